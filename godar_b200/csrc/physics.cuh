@@ -53,6 +53,38 @@ GD_DEV T S_shelter(T hfi, T hfj, T deltan, T cosa, T sina, T uf, T vf)
     return (T)1 - D * G;
 }
 
+// Both directions of one pair and medium: s_ij = S_shelter(hfi, hfj, dn,
+// cosa, sina, ..) and s_ji = S_shelter(hfj, hfi, dn, -cosa, -sina, ..).  The
+// second direction's cosine is the first one's negative, exactly, and a
+// factor with a negative cosine is 1 - D * (0 * costheta) = 1 exactly wherever
+// D is finite, as is one with a zero cosine: so one exponential and one set of
+// quotients give both.  (D is finite for finite positive freeboards and a
+// quotient dn / costheta that is a number.)
+template <typename T>
+GD_DEV void shelter_pair(T hfi, T hfj, T deltan, T cosa, T sina, T uf, T vf, T &s_ij, T &s_ji)
+{
+    const T wnorm = M<T>::sqrt_(uf * uf + vf * vf) + (T)1e-20;
+    const T costheta = (uf * cosa + vf * sina) / wnorm;
+    const bool plain = hfi > (T)0 && hfj > (T)0 && isfinite(hfi) && isfinite(hfj) && deltan == deltan;
+    if (plain && costheta == (T)0 && deltan != (T)0) {
+        s_ij = s_ji = (T)1;
+    } else if (plain && isfinite(costheta) && costheta != (T)0) {
+        const bool fwd = costheta > (T)0;
+        const T ct = fabs(costheta), hi = fwd ? hfi : hfj, hj = fwd ? hfj : hfi;
+        const T c018 = (T)(double)0.18f;
+        const T ex = M<T>::exp_(-((c018 * fabs(deltan / ct)) / hj));
+        const T D = ((T)1 - ((T)1 - heaviside(deltan)) * ((T)1 - ex))
+                    - (heaviside(deltan) * heaviside(hi - hj)) * ((T)1 - hj / hi);
+        const T G = heaviside(ct) * ct;
+        const T S = (T)1 - D * G;
+        s_ij = fwd ? S : (T)1;
+        s_ji = fwd ? (T)1 : S;
+    } else {
+        s_ij = S_shelter<T>(hfi, hfj, deltan, cosa, sina, uf, vf);
+        s_ji = S_shelter<T>(hfj, hfi, deltan, -cosa, -sina, uf, vf);
+    }
+}
+
 // ridging.f90:88-99 / 74-86: thickness increase of one floe (FP64 always)
 GD_DEV void apply_dh(const InstParams &P, Shape &s, double Vol)
 {
@@ -255,10 +287,8 @@ GD_DEV PairRes<T> pair_compute(const InstParams &P, double dx, double dy, double
         // sheltering (forcing.f90:162-186), wind of the lower-id floe
         const T hfai = (T)si.hfa, hfaj = (T)sj.hfa, hfwi = (T)si.hfw, hfwj = (T)sj.hfw;
         const T ua = (T)uai, va = (T)vai, uw = (T)uwi, vw = (T)vwi;
-        R.a_ij = S_shelter<T>(hfai, hfaj, dn, cosa, sina, ua, va);
-        R.w_ij = S_shelter<T>(hfwi, hfwj, dn, cosa, sina, uw, vw);
-        R.a_ji = S_shelter<T>(hfaj, hfai, dn, -cosa, -sina, ua, va);
-        R.w_ji = S_shelter<T>(hfwj, hfwi, dn, -cosa, -sina, uw, vw);
+        shelter_pair<T>(hfai, hfaj, dn, cosa, sina, ua, va, R.a_ij, R.a_ji);
+        shelter_pair<T>(hfwi, hfwj, dn, cosa, sina, uw, vw, R.w_ij, R.w_ji);
     }
     // stress magnitude of stepper.f90:238-271 (last contact forces of the pair)
     R.S = M<T>::sqrt_(H.fcn * H.fcn + H.fct * H.fct) + M<T>::sqrt_(sfbn * sfbn + sfbt * sfbt);

@@ -59,7 +59,7 @@ GD_DEV void bond_store(const Views &V, int bi, int side, const BondLocal &B)
 // groups: each group is written and read only when its flag says so (a
 // bond on a plain step: the first and the third).
 struct __align__(32) PairRec64 {
-    double cosa, sina, ri_l, rj_l;     // any term (PR_CONTACT, PR_BOND, PR_SHEL, PR_DIAG)
+    double cosa, sina, ri_l, rj_l;     // any sum (PR_CONTACT, PR_BOND, PR_DIAG)
     double fcn, fcr, fct, mcc;         // PR_CONTACT
     double fbn, fbt, mji, mij;         // PR_BOND
     double ac, vol, sbt, S;            // diagnostic step: ac (contact), sbt (bond), S (PR_DIAG); vol: a ridging event
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(128) k_pairs_fp64(Views V, int cur, FP64Lists 
                       && stress_term(R.S, R.cosa, R.ri_l, R.sina) == 0.0))
             f |= PR_DIAG;
         PairRec64 &Q = rec[p];
-        if (f & (PR_CONTACT | PR_BOND | PR_SHEL | PR_DIAG)) {
+        if (f & (PR_CONTACT | PR_BOND | PR_DIAG)) {
             Q.cosa = R.cosa; Q.sina = R.sina; Q.ri_l = R.ri_l; Q.rj_l = R.rj_l;
         }
         if (f & PR_CONTACT) {
@@ -320,7 +320,7 @@ GD_DEV PairRes<double> rec_load(const PairRec64 *rec, int p, unsigned f, bool di
     R.vol = 0.0;
     R.who = (f & PR_WHO1) ? 1 : (f & PR_WHO2) ? 2 : 0;
     const PairRec64 &Q = rec[p];
-    if (f & (PR_CONTACT | PR_BOND | PR_SHEL | PR_DIAG)) {
+    if (f & (PR_CONTACT | PR_BOND | PR_DIAG)) {
         R.cosa = Q.cosa; R.sina = Q.sina; R.ri_l = Q.ri_l; R.rj_l = Q.rj_l;
     }
     if (f & PR_CONTACT) {

@@ -473,10 +473,9 @@ __global__ void __launch_bounds__(256, 3) k_pairs_mixed(Views V, int cur, int di
                     const float dn = (float)((Si.r + Sj.r) - dist);
                     const float hfai = Pm.f_hfa * C.hi_l, hfaj = Pm.f_hfa * C.hj_l;
                     const float hfwi = Pm.f_hfw * C.hi_l, hfwj = Pm.f_hfw * C.hj_l;
-                    const float a_ij = S_shelter<float>(hfai, hfaj, dn, cosa, sina, ua, va);
-                    const float w_ij = S_shelter<float>(hfwi, hfwj, dn, cosa, sina, uw, vw);
-                    const float a_ji = S_shelter<float>(hfaj, hfai, dn, -cosa, -sina, ua, va);
-                    const float w_ji = S_shelter<float>(hfwj, hfwi, dn, -cosa, -sina, uw, vw);
+                    float a_ij, a_ji, w_ij, w_ji;
+                    shelter_pair<float>(hfai, hfaj, dn, cosa, sina, ua, va, a_ij, a_ji);
+                    shelter_pair<float>(hfwi, hfwj, dn, cosa, sina, uw, vw, w_ij, w_ji);
                     B.rec[2 * (size_t)e + 1] = make_float4(a_ji, w_ji, a_ij, w_ij);
                 }
                 f1 |= PF_REC;

@@ -199,11 +199,12 @@ GD_DEV int global_step(const Views &V, int sic) { return *V.step_base + sic; }
 // still run (expired_at is then this step, not below it).  The kernels
 // before the floe update in a step stop on any ST_ABORT state: an expiry
 // they see was raised by an earlier step.
-GD_DEV bool floe_update_stopped(const Views &V, int sic)
+// base: the chunk's first global step number, -1: in device memory.
+GD_DEV bool floe_update_stopped(const Views &V, int base, int sic)
 {
     const int s = *(volatile const int *)V.status;
     if (s & (ST_ABORT & ~ST_EXPIRED)) return true;
-    return (s & ST_EXPIRED) && *(volatile const int *)V.expired_at < global_step(V, sic);
+    return (s & ST_EXPIRED) && *(volatile const int *)V.expired_at < (base >= 0 ? base + sic : global_step(V, sic));
 }
 
 // Programmatic dependent launch of the step kernels.  A step kernel launched
@@ -217,6 +218,51 @@ GD_DEV void step_kernel_entry()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// The kernels that run whole steps of a small batch in one launch
+// (k_steps_fp64, k_steps_mixed): one cluster of up to SMALL_CLUSTER blocks.
+constexpr int SMALL_THREADS = 256;
+constexpr int SMALL_CLUSTER = 16;
+// lanes that sum one floe, and floes a block sums at a time
+constexpr int GRP = 8;
+constexpr int GRP_FLOES = SMALL_THREADS / GRP;
+
+// Barrier over every thread of the grid, which is one block or one cluster:
+// writes before it are visible after it (release at the arrival, acquire at
+// the wait, cluster scope).
+GD_DEV void cluster_sync()
+{
+    if (gridDim.x == 1) {
+        __syncthreads();
+    } else {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    }
+}
+
+// One thread: the status word and the first expired step into pinned host
+// memory.
+GD_DEV void publish_status(const Views &V, int *out)
+{
+    ((volatile int *)out)[0] = *(volatile const int *)V.status;
+    ((volatile int *)out)[1] = *(volatile const int *)V.expired_at;
+    __threadfence_system();
+}
+
+// The same by the last block of a grid to get here (every block calls it
+// once, all threads; done: a counter that is zero between kernels).
+GD_DEV void publish_status_last(const Views &V, int *done, int *out)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(done, 1) == (int)gridDim.x - 1) {
+            *done = 0;
+            __threadfence();
+            publish_status(V, out);
+        }
+    }
 }
 
 GD_DEV double wrap_d(double d, double L, bool per)

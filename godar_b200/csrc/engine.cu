@@ -260,7 +260,19 @@ struct Engine {
     // off by default: the overlap gains about 2% of a step on the benchmark
     // ensemble, and kernels sharing the GPU make per-kernel times meaningless
     bool overlap_bonds = false;
+    bool shelter_any = false;      // some field of the batch has sheltering
     bool walls_any = false;        // some field of the batch has a solid wall
+    // Batches of at most SMALL_FLOES_* floes run their steps as one or two
+    // launches (launch_small): below these sizes the five kernels of a step
+    // are mostly gaps and one thread's latency; above them the registers of
+    // the merged kernels cost more than the launches.  Measured, us a step
+    // (merged / five kernels): FP64 bonded fields 43.8 / 46.8 at 65,536 floes,
+    // 95 / 84 at 140,000; mixed 37.9 / 43.4 at 140,000, 600 / 340 at 2.2 M.
+    // GODAR_FUSED=0 turns it off, as does any switch that asks for a
+    // particular launch of the five step kernels.
+    bool fused_on = true;
+    static constexpr int SMALL_FLOES_FP64 = 64 * 1024;
+    static constexpr int SMALL_FLOES_MIXED = 148 * 1024;
 
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::atomic<size_t> bytes{0};
@@ -279,6 +291,8 @@ struct Engine {
     double accum_ms = 0.0;
     bool timing_open = false;
     unsigned long long counters[4] = {0, 0, 0, 0};
+    bool counting = false;             // the last call launched a diagnostic step
+    unsigned long long *h_counters = nullptr;   // pinned
     // Verlet skin = max(1 m, skin_frac (r_max + rtree)); a rebuild costs
     // about 25 ms on 2.2M floes, and 1% keeps rebuilds hundreds to thousands
     // of steps apart on the benchmark fields while shortening the rows
@@ -389,6 +403,7 @@ struct Engine {
     // the global number of the next step to launch, counted from the last
     // rebuild; kernels read the running chunk's first one from step_base_b
     int gbase = 0;
+    // (its second int counts the blocks of a chunk's last kernel, launch_small)
     Buf step_base_b;
     // asynchronous steps (godar_batch_step_async): chunks launched whose
     // status has not been read yet, oldest first.  Each has a pinned slot
@@ -396,6 +411,7 @@ struct Engine {
     struct Pending {
         int base, K, c0, slot;
         bool diag;                 // its last step produced the diagnostics
+        bool small;                // it was one launch (launch_small)
         std::vector<double> uvw;   // the uniform forcing it ran with (empty: as admitted)
     };
     static constexpr int RING = 16;
@@ -423,8 +439,7 @@ struct Engine {
         for (auto e : kev) cudaEventDestroy(e);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
-        if (h_status) cudaFreeHost(h_status);
-        if (h_ring) cudaFreeHost(h_ring);
+        if (h_counters) cudaFreeHost(h_counters);
         for (auto e : ring_ev)
             if (e) cudaEventDestroy(e);
         for (int q = 0; q < FRING; q++) {
@@ -482,12 +497,14 @@ struct Engine {
         CK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
         CK(cudaEventCreate(&ev0));
         CK(cudaEventCreate(&ev1));
-        CK(cudaMallocHost(&h_status, 4 * sizeof(int)));
-        CK(cudaMallocHost(&h_ring, RING * 4 * sizeof(int)));
+        // one pinned block: the counters, the status mirror, the ring
+        CK(cudaMallocHost(&h_counters, sizeof(counters) + (4 + RING * 4) * sizeof(int)));
+        h_status = (int *)(h_counters + 4);
+        h_ring = h_status + 4;
         for (auto &e : ring_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         for (auto &e : fring_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        TRY(step_base_b.ensure(sizeof(int), &bytes, &mp));
-        CK(cudaMemsetAsync(step_base_b.p, 0, sizeof(int), st));
+        TRY(step_base_b.ensure(2 * sizeof(int), &bytes, &mp));
+        CK(cudaMemsetAsync(step_base_b.p, 0, 2 * sizeof(int), st));
         TRY(status.ensure(2 * sizeof(int), &bytes, &mp));
         TRY(counters_b.ensure(4 * sizeof(unsigned long long), &bytes, &mp));
         TRY(tmp_cnt.ensure(sizeof(int), &bytes, &mp));
@@ -544,6 +561,8 @@ struct Engine {
         if (bl) tune_on = false;
         const char *ob = getenv("GODAR_OVERLAP_BONDS");
         if (ob) overlap_bonds = atoi(ob) != 0;
+        const char *fu = getenv("GODAR_FUSED");
+        fused_on = (!fu || atoi(fu) != 0) && !bl && !bv && !ob && test_wait_spins == 0;
         const char *gr = getenv("GODAR_GRAPHS");
         if (gr) graphs_on = atoi(gr) != 0;
 
@@ -910,10 +929,16 @@ struct Engine {
         }
         if (c_tot >= (1LL << 31)) { set_err("too many cells"); return GODAR_ERR_CAPACITY; }
         ridging_any = false;
+        shelter_any = false;
         walls_any = false;
         for (const Inst &I : insts) {
             ridging_any = ridging_any || I.prm.ridging != 0;
+            shelter_any = shelter_any || I.prm.shelter != 0;
             walls_any = walls_any || has_walls(I.prm.boundary);
+            // a restored field may carry wall histories that its next step clears
+            if (I.pending && I.rx)
+                for (const auto *w : {&I.rx->dtb1, &I.rx->dtb2, &I.rx->thb1, &I.rx->thb2})
+                    for (double d : *w) walls_any = walls_any || d != 0.0 || std::signbit(d);
         }
         const bool migrate = have_rows && oldN > 0;
         std::unique_ptr<FloeSet> oldF = std::move(F);
@@ -1452,7 +1477,8 @@ struct Engine {
             launch_row_sums_fp64(V, side, diag, pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
                                  fupn_b.as<int>(), fsum_b.as<double>(), cfg_block(bs[3]), st);
             if (ev) TRY(record(ev[4], capturing));
-            launch_floes_fp64(V, side, diag, sic, fsum_b.as<double>(), nwork_b.as<int>(), cfg_block(bs[4]), st);
+            launch_floes_fp64(V, side, diag, sic, walls_any ? 1 : 0, fsum_b.as<double>(), nwork_b.as<int>(),
+                              cfg_block(bs[4]), st);
             if (ev)
                 for (int q = 5; q < NEV; q++) TRY(record(ev[q], capturing));
         } else {
@@ -1484,6 +1510,36 @@ struct Engine {
             if (ev) TRY(record(ev[5], capturing));
         }
         return GODAR_OK;
+    }
+
+    // Whether this batch's chunks run as one launch.  A call whose steps are
+    // timed kernel by kernel runs the kernels.
+    bool small_batch(int every) const {
+        return fused_on && every == 0 && N > 0 && N <= (prec == GODAR_PREC_FP64 ? SMALL_FLOES_FP64 : SMALL_FLOES_MIXED);
+    }
+
+    // K steps from side c0 in one launch; out receives the status word and
+    // the first expired step.  False (and off from then on) where a cluster
+    // launch is not available.
+    bool launch_small(int K, int c0, int diag_last, int *out) {
+        Views V = views();
+        V.pdl = step_pdl();
+        bool ok;
+        if (prec == GODAR_PREC_FP64)
+            ok = launch_steps_fp64(V, c0, K, diag_last, gbase, (int)Lc, (int)E, shelter_any ? 1 : 0, fplist_b.as<int>(),
+                                   erow_up.as<unsigned>(), pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
+                                   fupn_b.as<int>(), fsum_b.as<double>(), out, step_base_b.as<int>() + 1, st);
+        else
+            ok = launch_steps_mixed(V, c0, K, diag_last, gbase, (int)Ec, (int)E, NB, shelter_any ? 1 : 0, ridging_any ? 1 : 0,
+                                    clist_b.as<int2>(), clist_b.as<int2>() + Ecap, erow_up.as<unsigned>(),
+                                    bflag_b.as<unsigned char>(), mixed_bufs(), out, step_base_b.as<int>() + 1, st);
+        if (!ok) {
+            cudaGetLastError();
+            fused_on = false;
+            return false;
+        }
+        graph_launches++;
+        return true;
     }
 
     int max_cfg() const {
@@ -1551,7 +1607,7 @@ struct Engine {
 
     int prepare(int nsteps) {
         TRY(commit());
-        if (N == 0 || nsteps <= 0 || !graphs_on || tune_left > 0) return GODAR_OK;
+        if (N == 0 || nsteps <= 0 || !graphs_on || tune_left > 0 || small_batch(phase_every)) return GODAR_OK;
         int c = cur, remaining = nsteps, ch = chunk;
         while (remaining > 0 && graphs_on) {
             int K = std::min(remaining, ch);
@@ -1598,6 +1654,22 @@ struct Engine {
         return GODAR_OK;
     }
 
+    // The counters of a call's diagnostic step start at zero; a call without
+    // one leaves them zero, and neither clears nor reads the device's.
+    int open_counters() {
+        counting = diagnostics;
+        if (counting) CK(cudaMemsetAsync(counters_b.p, 0, sizeof(counters), st));
+        return GODAR_OK;
+    }
+
+    // ... and are read once the stream is idle (which this waits for).
+    int close_counters() {
+        if (counting) CK(cudaMemcpyAsync(h_counters, counters_b.p, sizeof(counters), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        for (int k = 0; k < 4; k++) counters[k] = counting ? h_counters[k] : 0;
+        return GODAR_OK;
+    }
+
     // Advances every instance by nsteps; diagnostics on the last step.
     int run(int nsteps) {
         TRY(commit());
@@ -1606,10 +1678,11 @@ struct Engine {
         // that side (one step from the gathered side only reads it)
         for (int q = 0; q < 2; q++)
             if (gath_rec[q] && !(nsteps == 1 && gath_side[q] == cur)) CK(cudaStreamWaitEvent(st, ev_gath[q], 0));
-        CK(cudaMemsetAsync(counters_b.p, 0, sizeof(counters), st));
+        TRY(open_counters());
         if (!timing_open) { CK(cudaEventRecord(ev0, st)); timing_open = true; }
-        // tune once, and again only if the batch grew more than 4x since
-        if (tune_on && (tuned_n == 0 || N > 4 * tuned_n) && tune_left == 0) {
+        // tune once, and again only if the batch grew more than 4x since (a
+        // batch whose chunks are one launch has nothing to tune)
+        if (tune_on && !small_batch(phase_every) && (tuned_n == 0 || N > 4 * tuned_n) && tune_left == 0) {
             tune_left = TUNE_ROUNDS * max_cfg();
             tuned_n = N;
             for (int q = 0; q < NPH; q++)
@@ -1617,16 +1690,20 @@ struct Engine {
         }
         int remaining = nsteps;
         while (remaining > 0) {
-            const bool tuning = tune_left > 0;
-            // a tuning chunk runs one step per candidate; otherwise chunks are
-            // powers of two so that their graphs are reused
+            bool small = small_batch(phase_every);
+            const bool tuning = tune_left > 0 && !small;
+            // a tuning chunk runs one step per candidate; otherwise chunks of
+            // the five kernels are powers of two so that their graphs are reused
             int K = tuning ? std::min(remaining, max_cfg()) : std::min(remaining, chunk);
-            if (!tuning) while (K & (K - 1)) K &= K - 1;
+            if (!tuning && !small) while (K & (K - 1)) K &= K - 1;
             const int diag_last = (diagnostics && remaining == K) ? 1 : 0;
             int bs[NPH];
             for (int q = 0; q < NPH; q++) bs[q] = blk[q];
-            launch_set_int(step_base_b.as<int>(), gbase, st);
-            if (tuning) {
+            small = small && launch_small(K, cur, diag_last, h_status);
+            if (!small) launch_set_int(step_base_b.as<int>(), gbase, st);
+            if (small) {
+                // launched
+            } else if (tuning) {
                 // each tuning step uses the next candidate for every kernel
                 for (int k = 0; k < K; k++) {
                     int bk[NPH];
@@ -1646,7 +1723,8 @@ struct Engine {
             // working bond records
             if (prec != GODAR_PREC_FP64 && NB > 0) wdirty = true;
             CK(cudaGetLastError());
-            CK(cudaMemcpyAsync(h_status, status.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+            // (a small batch's kernel has written the status word itself)
+            if (!small) CK(cudaMemcpyAsync(h_status, status.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
             const int stt = h_status[0];
             if (stt & ST_NAN) { set_err("non-finite floe state"); return GODAR_ERR_NAN; }
@@ -1657,7 +1735,7 @@ struct Engine {
             gbase += K;
             const bool conc = concurrent_bonds();
             for (int k = 0; k < done; k++) {
-                if (!tuning && !(phase_every > 0 && k % phase_every == 0)) continue;
+                if (small || (!tuning && !(phase_every > 0 && k % phase_every == 0))) continue;
                 phase_steps++;
                 const cudaEvent_t *E7 = &kev[NEV * k];
                 float tstep = 0.f;
@@ -1709,11 +1787,9 @@ struct Engine {
                     drop_graphs();
                 }
             }
-            launches += done;
-            kernel_launches += (long long)done * kernels_per_step();
+            account(done, small);
             cur ^= (done & 1);
             remaining -= done;
-            for (auto &I : insts) I.steps += done;
             if (stt & ST_EXPIRED) {
                 // a rebuild rewrites the other side: the copy must be done
                 for (int q = 0; q < 2; q++)
@@ -1724,9 +1800,8 @@ struct Engine {
                 chunk = std::min(chunk * 2, 256);
             }
         }
-        CK(cudaMemcpyAsync(counters, counters_b.p, sizeof(counters), cudaMemcpyDeviceToHost, st));
         CK(cudaEventRecord(ev1, st));
-        CK(cudaStreamSynchronize(st));
+        TRY(close_counters());
         float ms = 0.f;
         CK(cudaEventElapsedTime(&ms, ev0, ev1));
         timing_open = false;
@@ -1745,34 +1820,40 @@ struct Engine {
     // membership change waits or without CUDA graphs.
     int run_async(int nsteps) {
         if (nsteps <= 0) return GODAR_OK;
-        const bool tune_due = tune_on && (tuned_n == 0 || N > 4 * tuned_n);
-        if (dirty || !have_rows || N == 0 || !graphs_on || tune_left > 0 || tune_due) {
+        const bool tune_due = tune_left > 0 || (tune_on && (tuned_n == 0 || N > 4 * tuned_n));
+        // (queued steps are never timed kernel by kernel)
+        if (dirty || !have_rows || N == 0 || (!small_batch(0) && (!graphs_on || tune_due))) {
             TRY(resolve());
             return run(nsteps);
         }
         const size_t before = pend.size();
         for (int q = 0; q < 2; q++)
             if (gath_rec[q] && !(nsteps == 1 && gath_side[q] == cur)) CK(cudaStreamWaitEvent(st, ev_gath[q], 0));
-        CK(cudaMemsetAsync(counters_b.p, 0, sizeof(counters), st));
+        TRY(open_counters());
         if (!timing_open) { CK(cudaEventRecord(ev0, st)); timing_open = true; }
         int remaining = nsteps;
         while (remaining > 0) {
             if ((int)pend.size() >= RING) TRY(resolve_front(pend.size()));
             int K = std::min(remaining, chunk);
-            while (K & (K - 1)) K &= K - 1;
+            bool small = small_batch(0);
+            if (!small) while (K & (K - 1)) K &= K - 1;
             const int diag_last = (diagnostics && remaining == K) ? 1 : 0;
             Pending P;
             P.base = gbase; P.K = K; P.c0 = cur; P.slot = ring_next;
             P.diag = diag_last != 0;
             P.uvw = cur_uvw;
             ring_next = (ring_next + 1) % RING;
-            launch_set_int(step_base_b.as<int>(), gbase, st);
-            // queued steps record no timing events: nothing reads them
-            TRY(launch_chunk(K, cur, diag_last, blk, false, 0));
+            int *hs = h_ring + 4 * P.slot;
+            small = small && launch_small(K, cur, diag_last, hs);
+            P.small = small;
+            if (!small) {
+                launch_set_int(step_base_b.as<int>(), gbase, st);
+                // queued steps record no timing events: nothing reads them
+                TRY(launch_chunk(K, cur, diag_last, blk, false, 0));
+                CK(cudaMemcpyAsync(hs, status.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+            }
             if (prec != GODAR_PREC_FP64 && NB > 0) wdirty = true;
             CK(cudaGetLastError());
-            int *hs = h_ring + 4 * P.slot;
-            CK(cudaMemcpyAsync(hs, status.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
             CK(cudaEventRecord(ring_ev[P.slot], st));
             pend.push_back(std::move(P));
             cur ^= (K & 1);
@@ -1783,9 +1864,9 @@ struct Engine {
     }
 
     // Time steps counted as done.
-    void account(int done) {
+    void account(int done, bool small) {
         launches += done;
-        kernel_launches += (long long)done * kernels_per_step();
+        kernel_launches += small ? 1 : (long long)done * kernels_per_step();
         for (auto &I : insts) I.steps += done;
     }
 
@@ -1805,7 +1886,7 @@ struct Engine {
                 return GODAR_ERR_TIMEOUT;
             }
             if (stt & ST_EXPIRED) return redo_after_expiry();
-            account(P.K);
+            account(P.K, P.small);
             chunk = std::min(chunk * 2, 256);
             pend.pop_front();
             n--;
@@ -1825,7 +1906,7 @@ struct Engine {
         std::vector<Redo> redo;
         if (P.K > done) redo.push_back({P.K - done, P.diag, P.uvw});
         for (size_t i = 1; i < pend.size(); i++) redo.push_back({pend[i].K, pend[i].diag, pend[i].uvw});
-        account(done);
+        account(done, P.small);
         cur = P.c0 ^ (done & 1);
         pend.clear();
         for (int q = 0; q < 2; q++)
@@ -1851,9 +1932,8 @@ struct Engine {
     int resolve() {
         if (pend.empty()) return GODAR_OK;
         TRY(resolve_front(pend.size()));
-        CK(cudaMemcpyAsync(counters, counters_b.p, sizeof(counters), cudaMemcpyDeviceToHost, st));
         CK(cudaEventRecord(ev1, st));
-        CK(cudaStreamSynchronize(st));
+        TRY(close_counters());
         if (timing_open) {
             float ms = 0.f;
             CK(cudaEventElapsedTime(&ms, ev0, ev1));

@@ -29,6 +29,33 @@ inline void launch_step(bool pdl, void (*kern)(Params...), int grid, int block, 
     cudaLaunchKernelEx(&c, kern, args...);
 }
 
+// Launches a kernel of whole steps (k_steps_fp64, k_steps_mixed) as one
+// cluster of enough blocks to give every one of `items` a thread, at most
+// SMALL_CLUSTER.  False if the launch was refused.
+template <typename... Params, typename... Args>
+inline bool launch_cluster(bool pdl, void (*kern)(Params...), long long items, cudaStream_t st, Args... args)
+{
+    static const bool wide =
+        cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    const int most = wide ? SMALL_CLUSTER : 8;
+    int blocks = 1;
+    while (blocks < most && (long long)blocks * SMALL_THREADS < items) blocks *= 2;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)blocks);
+    c.blockDim = dim3(SMALL_THREADS);
+    c.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)blocks;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = pdl ? 2 : 1;
+    return cudaLaunchKernelEx(&c, kern, args...) == cudaSuccess;
+}
+
 void scan_excl(const int *in, int *out, int n, int *scratch, cudaStream_t st);
 void radix_sort(uint32_t *keys, int *vals, uint32_t *keys_alt, int *vals_alt, int n, int bits,
                 int *counts, int *scratch, cudaStream_t st);
@@ -67,8 +94,29 @@ void launch_row_sums_fp64(const Views &V, int cur, int diag, const unsigned char
 // screen (plist, pos[N] of them; pos: N + 1 ints; tmp: 2 E entries).
 void launch_fp64_rows(const Views &V, int side, int E, const unsigned *erow, unsigned char *listed, int *up_n,
                       int *lo_n, int2 *tmp, int *pos, int *scan_scratch, int *plist, cudaStream_t st);
-void launch_floes_fp64(const Views &V, int cur, int diag, int sic, const double *fs, int *nwork, int block,
+void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, const double *fs, int *nwork, int block,
                        cudaStream_t st);
+// K whole steps of a small batch (n marked positions, E owner entries;
+// shelter: some field of the batch has sheltering; drag: 8 N doubles; out:
+// pinned host memory for the status word and the first expired step; done: an
+// int that is zero): as one launch of one cluster up to ONE_CLUSTER_* items
+// (positions, bonds and floes), else as two launches a step.  False if the
+// launch was refused.
+constexpr int ONE_CLUSTER_FP64 = 1024, ONE_CLUSTER_MIXED = 4096;
+bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int shelter,
+                       const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
+                       const int *up_n, double *drag, int *out, int *done, cudaStream_t st);
+
+// Rounds of GRP_FLOES floes that a block of the two-launch step sums by
+// groups of lanes; 0: one thread per floe.
+inline int group_rounds(int N, int shelter)
+{
+    const int wave = 148 * 2 * GRP_FLOES;     // floes of one round of every block that fits the GPU at once
+    int r = 1;
+    while (r < GRP && N > r * wave) r *= 2;
+    return shelter || r == 1 ? r : 0;
+}
+
 // Mixed precision: (b) one lane per pair with warp-segmented sums, (b') the
 // partners' shares gathered the same way, (c)-(e) one thread per floe.
 struct MixedBufs {
@@ -119,6 +167,12 @@ void launch_bonds_mixed(const Views &V, int cur, int diag, int NB, MixedBufs B, 
                         unsigned test_spins, cudaStream_t st);
 void launch_floes_mixed(const Views &V, int cur, int diag, int sic, int walls, MixedBufs B, int block,
                         cudaStream_t st);
+
+// The same on the mixed path (n contact-list items eb/stl, bfl: the live-bond
+// flags of both sides).
+bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
+                        int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
+                        int *done, cudaStream_t st);
 
 // Checkpoints: pair histories out and back in.
 void launch_hist_list(const Views &V, int cur, int off, int n, int fp64, int hs, int *count, int *pi, int *pj,

@@ -55,11 +55,43 @@ void launch_row_sums_fp64(const Views &V, int cur, int diag, const unsigned char
     else launch_step(V.pdl != 0, k_row_sums_fp64<false>, fp64_grid(V.N, block), block, st, V, cur, pfl, r, lo_n, up_n, fs);
 }
 
-void launch_floes_fp64(const Views &V, int cur, int diag, int sic, const double *fs, int *nwork, int block,
+void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, const double *fs, int *nwork, int block,
                        cudaStream_t st)
 {
-    if (diag) launch_step(V.pdl != 0, k_floes_fp64<true>, fp64_grid(V.N, block), block, st, V, cur, sic, fs, nwork);
-    else launch_step(V.pdl != 0, k_floes_fp64<false>, fp64_grid(V.N, block), block, st, V, cur, sic, fs, nwork);
+    const int grid = fp64_grid(V.N, block);
+    if (walls) {
+        if (diag) launch_step(V.pdl != 0, k_floes_fp64<true, true>, grid, block, st, V, cur, sic, fs, nwork);
+        else launch_step(V.pdl != 0, k_floes_fp64<false, true>, grid, block, st, V, cur, sic, fs, nwork);
+    } else {
+        if (diag) launch_step(V.pdl != 0, k_floes_fp64<true, false>, grid, block, st, V, cur, sic, fs, nwork);
+        else launch_step(V.pdl != 0, k_floes_fp64<false, false>, grid, block, st, V, cur, sic, fs, nwork);
+    }
+}
+
+bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int shelter,
+                       const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
+                       const int *up_n, double *drag, int *out, int *done, cudaStream_t st)
+{
+    SmallArgs64 A;
+    A.cur = cur; A.K = K; A.diag_last = diag_last; A.base = base;
+    A.n = n; A.E = E; A.plist = plist; A.erow = erow; A.pfl = pfl; A.rec = (PairRec64 *)rec;
+    A.lo_n = lo_n; A.up_n = up_n; A.drag = drag; A.out = out; A.done = done;
+    const long long items = (long long)n + V.N;
+    if (!shelter && items <= ONE_CLUSTER_FP64) return launch_cluster(V.pdl != 0, k_steps_fp64, items, st, V, A);
+    const int rounds = group_rounds(V.N, shelter);
+    for (int k = 0; k < K; k++) {
+        const int c = cur ^ (k & 1);
+        const bool diag = diag_last && k == K - 1;
+        const int gp = fp64_grid((long long)(diag ? E : n) + 32 + V.N, 128);
+        if (diag) launch_step(V.pdl != 0, k_step_pairs_fp64<true>, gp, 128, st, V, A, c);
+        else launch_step(V.pdl != 0, k_step_pairs_fp64<false>, gp, 128, st, V, A, c);
+        if (diag) launch_step(V.pdl != 0, k_step_floes_fp64<true>, fp64_grid(V.N, 64), 64, st, V, A, c, k);
+        else if (rounds == 0) launch_step(V.pdl != 0, k_step_floes_fp64<false>, fp64_grid(V.N, 64), 64, st, V, A, c, k);
+        else
+            launch_step(V.pdl != 0, k_step_floes_grp_fp64, (V.N + rounds * GRP_FLOES - 1) / (rounds * GRP_FLOES),
+                        SMALL_THREADS, st, V, A, c, k, rounds);
+    }
+    return true;
 }
 
 // Owner entries [0, E) at a rebuild (floes on side `side`, at the rebuild

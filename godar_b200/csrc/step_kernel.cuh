@@ -79,6 +79,33 @@ enum : unsigned char {
 
 GD_DEV double stress_term(double S, double c1, double rl, double c2) { return ((S * c1) * rl) * c2; }
 
+// A candidate without contact, bond or sheltering: its tangential and rolling
+// histories are reset (most are zero already; h01: the stored ones) and, on
+// a diagnostic step, its stress record and overlap written: pair_compute's
+// normal, stress magnitude (no bond forces) and overlap, by the same
+// expressions.  Returns the pair's flags.
+template <bool DIAG>
+GD_DEV unsigned quiet_candidate(const Views &V, Hist4<double> *Hs, int p, double dx, double dy, double dist,
+                                double deltan, double ri, double rj, double2 h01, PairRec64 *rec)
+{
+    if (__double_as_longlong(h01.x) | __double_as_longlong(h01.y)) *(double2 *)&Hs[p] = make_double2(0.0, 0.0);
+    unsigned f = PR_CAND;
+    if (DIAG) {
+        const double2 fc = *(const double2 *)&Hs[p].fcn;
+        const double S = sqrt(fc.x * fc.x + fc.y * fc.y) + sqrt(0.0 * 0.0 + 0.0 * 0.0);
+        const double cosa = -dx / dist, sina = -dy / dist;
+        if (!(stress_term(S, cosa, ri, cosa) == 0.0 && stress_term(S, sina, ri, sina) == 0.0
+              && stress_term(S, sina, ri, cosa) == 0.0 && stress_term(S, cosa, ri, sina) == 0.0)) {
+            f |= PR_DIAG;
+            PairRec64 &Q = rec[p];
+            Q.cosa = cosa; Q.sina = sina; Q.ri_l = ri; Q.rj_l = rj;
+            Q.S = S;
+        }
+        V.pdn[p] = (float)deltan;
+    }
+    return f;
+}
+
 // Owner entries, first pass (few registers): the FP64 distance (kept for
 // the row sort) and the candidate test, and the entries that need no pair
 // physics finished here.  A non-candidate keeps its history and bond state.
@@ -160,27 +187,9 @@ __global__ void __launch_bounds__(256) k_pairs_fp64_screen(Views V, int cur, int
                     heavy = general || bi[k] >= 0;
                     bond_only = !general && bi[k] >= 0;
                     if (!heavy) {
-                        // reset_contact: deltat and thetarelc to +0 (most already are)
-                        if (__double_as_longlong(h01[k].x) | __double_as_longlong(h01[k].y))
-                            *(double2 *)&Hs[p[k]] = make_double2(0.0, 0.0);
-                        unsigned f = PR_CAND;
-                        if (DIAG) {
-                            // pair_compute's normal, stress magnitude (no bond
-                            // forces) and overlap, by the same expressions
-                            const double2 fc = *(const double2 *)&Hs[p[k]].fcn;
-                            const double S = sqrt(fc.x * fc.x + fc.y * fc.y) + sqrt(0.0 * 0.0 + 0.0 * 0.0);
-                            const double cosa = -dx / dist, sina = -dy / dist;
-                            const double ri = rg[k];
-                            if (!(stress_term(S, cosa, ri, cosa) == 0.0 && stress_term(S, sina, ri, sina) == 0.0
-                                  && stress_term(S, sina, ri, cosa) == 0.0 && stress_term(S, cosa, ri, sina) == 0.0)) {
-                                f |= PR_DIAG;
-                                PairRec64 &Q = rec[p[k]];
-                                Q.cosa = cosa; Q.sina = sina; Q.ri_l = ri; Q.rj_l = rt[k];
-                                Q.S = S;
-                            }
-                            V.pdn[p[k]] = (float)deltan;
-                            n_cand++;
-                        }
+                        const unsigned f = quiet_candidate<DIAG>(V, Hs, p[k], dx, dy, dist, deltan, rg[k], rt[k], h01[k],
+                                                                 rec);
+                        if (DIAG) n_cand++;
                         pfl[p[k]] = f;
                     }
                 }
@@ -210,6 +219,83 @@ __global__ void __launch_bounds__(256) k_pairs_fp64_screen(Views V, int cur, int
     }
 }
 
+// Counts of a diagnostic step, per thread.
+struct Counts64 { unsigned long long cand, cont, bond, plast; };
+
+// The counts added to the counters (every lane of the warp calls it).
+GD_DEV void add_counts(const Counts64 &C, unsigned long long *counters)
+{
+    unsigned long long c[4] = {C.cand, C.cont, C.bond, C.plast};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) c[q] += __shfl_down_sync(0xffffffffu, c[q], o);
+        if ((threadIdx.x & 31) == 0 && c[q]) atomicAdd(&counters[q], c[q]);
+    }
+}
+
+// The pair physics of one candidate (pair p, owner slot g, partner slot t,
+// bond bi or -1, offset dx, dy): history and bond in place, the record
+// groups its flags name.
+template <bool BONDS, bool DIAG>
+GD_DEV void pair_work64(const Views &V, int cur, Hist4<double> *Hs, int p, int g, int t, int bi, double dx, double dy,
+                        unsigned char *pfl, PairRec64 *rec, Counts64 &C)
+{
+    const InstParams &P = V.P[V.inst[g]];
+    const bool shel = !BONDS && P.shelter != 0;
+    const double r = V.r[cur][g];
+    // the screen's distance, by the same expression
+    const double dist = sqrt(dx * dx + dy * dy);
+    Hist4<double> H = Hs[p];
+    BondLocal BL;
+    if (bi >= 0) bond_load(V, bi, 0, BL);
+    const Shape si = make_shape(P, r, V.h[cur][g]);
+    const Shape sj = make_shape(P, V.r[cur][t], V.h[cur][t]);
+    double ua = 0.0, va = 0.0, uw = 0.0, vw = 0.0;
+    if (shel) wind_at(P, V.field, V.x[cur][g], V.y[cur][g], ua, va, uw, vw);
+    const PairRes<double> R = pair_compute<double, !BONDS>(P, dx, dy, dist, V.u[cur][g], V.v[cur][g], V.om[cur][g],
+                                                   V.u[cur][t], V.v[cur][t], V.om[cur][t], si, sj,
+                                                   ua, va, uw, vw, H, bi >= 0 ? &BL : nullptr, shel);
+    Hs[p] = H;
+    if (bi >= 0) bond_store(V, bi, 0, BL);
+
+    unsigned f = PR_CAND;
+    if (R.contact) f |= PR_CONTACT;
+    if (R.bond_on) f |= PR_BOND;
+    if (R.who == 1) f |= PR_WHO1;
+    else if (R.who == 2) f |= PR_WHO2;
+    if (shel && !(R.a_ij == 1.0 && R.a_ji == 1.0 && R.w_ij == 1.0 && R.w_ji == 1.0)) f |= PR_SHEL;
+    // a stress term of +-0 leaves a sum unchanged (the sums start at +0
+    // and never become -0), so only nonzero ones (NaN included) count
+    if (DIAG && !(stress_term(R.S, R.cosa, R.ri_l, R.cosa) == 0.0 && stress_term(R.S, R.sina, R.ri_l, R.sina) == 0.0
+                  && stress_term(R.S, R.sina, R.ri_l, R.cosa) == 0.0
+                  && stress_term(R.S, R.cosa, R.ri_l, R.sina) == 0.0))
+        f |= PR_DIAG;
+    PairRec64 &Q = rec[p];
+    if (f & (PR_CONTACT | PR_BOND | PR_DIAG)) {
+        Q.cosa = R.cosa; Q.sina = R.sina; Q.ri_l = R.ri_l; Q.rj_l = R.rj_l;
+    }
+    if (f & PR_CONTACT) {
+        Q.fcn = R.fcn; Q.fcr = R.fcr; Q.fct = R.fct; Q.mcc = R.mcc;
+        if (DIAG) Q.ac = R.ac;
+    }
+    if (f & (PR_WHO1 | PR_WHO2)) Q.vol = R.vol;
+    if (f & PR_BOND) {
+        Q.fbn = R.fbn; Q.fbt = R.fbt; Q.mji = R.mji; Q.mij = R.mij;
+        if (DIAG) Q.sbt = R.sbt;
+    }
+    if (f & PR_DIAG) Q.S = R.S;
+    if (f & PR_SHEL) { Q.a_ij = R.a_ij; Q.a_ji = R.a_ji; Q.w_ij = R.w_ij; Q.w_ji = R.w_ji; }
+    pfl[p] = (unsigned char)f;
+    if (DIAG) {
+        V.pdn[p] = (float)R.deltan;
+        C.cand++;
+        C.cont += R.contact;
+        C.bond += R.bond_on;
+        C.plast += R.who != 0;
+    }
+}
+
 // A work list: the pair physics of every remaining candidate, once.
 // BONDS: list 1 (bonded, no contact, no sheltering), with the contact
 // branch compiled out.  DIAG: a diagnostic step (stress records, overlaps,
@@ -219,10 +305,9 @@ __global__ void __launch_bounds__(128) k_pairs_fp64(Views V, int cur, FP64Lists 
                                                     PairRec64 *rec)
 {
     step_kernel_entry();
-    constexpr bool diag = DIAG;
     if (*(volatile int *)V.status & ST_ABORT) return;
     Hist4<double> *Hs = (Hist4<double> *)V.hist[0];   // in place: one thread per pair
-    unsigned long long n_cand = 0, n_cont = 0, n_bond = 0, n_plast = 0;
+    Counts64 C = {0, 0, 0, 0};
     const int stride = gridDim.x * blockDim.x;
     const int n = *(volatile const int *)&L.n[BONDS];
     const FP64Item *work = L.work[BONDS];
@@ -231,82 +316,21 @@ __global__ void __launch_bounds__(128) k_pairs_fp64(Views V, int cur, FP64Lists 
         // pair's offset along
         const FP64Item w = work[k];
         const int p = w.p, g = w.g, t = w.t, bi = w.bi;
-        const InstParams &P = V.P[V.inst[g]];
-        const bool shel = !BONDS && P.shelter != 0;
-        const double r = V.r[cur][g];
-        const double dx = w.dx, dy = w.dy;
-        // the screen's distance, by the same expression
-        const double dist = sqrt(dx * dx + dy * dy);
-        Hist4<double> H = Hs[p];
-        BondLocal BL;
-        if (bi >= 0) bond_load(V, bi, 0, BL);
-        const Shape si = make_shape(P, r, V.h[cur][g]);
-        const Shape sj = make_shape(P, V.r[cur][t], V.h[cur][t]);
-        double ua = 0.0, va = 0.0, uw = 0.0, vw = 0.0;
-        if (shel) wind_at(P, V.field, V.x[cur][g], V.y[cur][g], ua, va, uw, vw);
-        const PairRes<double> R = pair_compute<double, !BONDS>(P, dx, dy, dist, V.u[cur][g], V.v[cur][g], V.om[cur][g],
-                                                       V.u[cur][t], V.v[cur][t], V.om[cur][t], si, sj,
-                                                       ua, va, uw, vw, H, bi >= 0 ? &BL : nullptr, shel);
-        Hs[p] = H;
-        if (bi >= 0) bond_store(V, bi, 0, BL);
-
-        unsigned f = PR_CAND;
-        if (R.contact) f |= PR_CONTACT;
-        if (R.bond_on) f |= PR_BOND;
-        if (R.who == 1) f |= PR_WHO1;
-        else if (R.who == 2) f |= PR_WHO2;
-        if (shel && !(R.a_ij == 1.0 && R.a_ji == 1.0 && R.w_ij == 1.0 && R.w_ji == 1.0)) f |= PR_SHEL;
-        // a stress term of +-0 leaves a sum unchanged (the sums start at +0
-        // and never become -0), so only nonzero ones (NaN included) count
-        if (diag && !(stress_term(R.S, R.cosa, R.ri_l, R.cosa) == 0.0 && stress_term(R.S, R.sina, R.ri_l, R.sina) == 0.0
-                      && stress_term(R.S, R.sina, R.ri_l, R.cosa) == 0.0
-                      && stress_term(R.S, R.cosa, R.ri_l, R.sina) == 0.0))
-            f |= PR_DIAG;
-        PairRec64 &Q = rec[p];
-        if (f & (PR_CONTACT | PR_BOND | PR_DIAG)) {
-            Q.cosa = R.cosa; Q.sina = R.sina; Q.ri_l = R.ri_l; Q.rj_l = R.rj_l;
-        }
-        if (f & PR_CONTACT) {
-            Q.fcn = R.fcn; Q.fcr = R.fcr; Q.fct = R.fct; Q.mcc = R.mcc;
-            if (diag) Q.ac = R.ac;
-        }
-        if (f & (PR_WHO1 | PR_WHO2)) Q.vol = R.vol;
-        if (f & PR_BOND) {
-            Q.fbn = R.fbn; Q.fbt = R.fbt; Q.mji = R.mji; Q.mij = R.mij;
-            if (diag) Q.sbt = R.sbt;
-        }
-        if (f & PR_DIAG) Q.S = R.S;
-        if (f & PR_SHEL) { Q.a_ij = R.a_ij; Q.a_ji = R.a_ji; Q.w_ij = R.w_ij; Q.w_ji = R.w_ji; }
-        pfl[p] = (unsigned char)f;
-        if (diag) {
-            V.pdn[p] = (float)R.deltan;
-            n_cand++;
-            n_cont += R.contact;
-            n_bond += R.bond_on;
-            n_plast += R.who != 0;
-        }
+        pair_work64<BONDS, DIAG>(V, cur, Hs, p, g, t, bi, w.dx, w.dy, pfl, rec, C);
     }
 
-    if (diag) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            n_cand += __shfl_down_sync(0xffffffffu, n_cand, o);
-            n_cont += __shfl_down_sync(0xffffffffu, n_cont, o);
-            n_bond += __shfl_down_sync(0xffffffffu, n_bond, o);
-            n_plast += __shfl_down_sync(0xffffffffu, n_plast, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            atomicAdd(&V.counters[0], n_cand);
-            atomicAdd(&V.counters[1], n_cont);
-            atomicAdd(&V.counters[2], n_bond);
-            atomicAdd(&V.counters[3], n_plast);
-        }
-    }
+    if (DIAG) add_counts(C, V.counters);
 }
 
 // The pair result one floe's sums need, from the pair's record.  A group the
 // flags leave out holds values that make its terms no-ops: no contact, no
 // bond, shelter factors of exactly 1 (what the pair computed), stress of 0.
+GD_DEV double4 load_group(const double *q)
+{
+    const double2 u = ((const double2 *)q)[0], v = ((const double2 *)q)[1];
+    return make_double4(u.x, u.y, v.x, v.y);
+}
+
 GD_DEV PairRes<double> rec_load(const PairRec64 *rec, int p, unsigned f, bool diag)
 {
     PairRes<double> R;
@@ -321,19 +345,25 @@ GD_DEV PairRes<double> rec_load(const PairRec64 *rec, int p, unsigned f, bool di
     R.who = (f & PR_WHO1) ? 1 : (f & PR_WHO2) ? 2 : 0;
     const PairRec64 &Q = rec[p];
     if (f & (PR_CONTACT | PR_BOND | PR_DIAG)) {
-        R.cosa = Q.cosa; R.sina = Q.sina; R.ri_l = Q.ri_l; R.rj_l = Q.rj_l;
+        const double4 q = load_group(&Q.cosa);
+        R.cosa = q.x; R.sina = q.y; R.ri_l = q.z; R.rj_l = q.w;
     }
     if (f & PR_CONTACT) {
-        R.fcn = Q.fcn; R.fcr = Q.fcr; R.fct = Q.fct; R.mcc = Q.mcc;
+        const double4 q = load_group(&Q.fcn);
+        R.fcn = q.x; R.fcr = q.y; R.fct = q.z; R.mcc = q.w;
         if (diag) R.ac = Q.ac;
     }
     if (R.who) R.vol = Q.vol;
     if (f & PR_BOND) {
-        R.fbn = Q.fbn; R.fbt = Q.fbt; R.mji = Q.mji; R.mij = Q.mij;
+        const double4 q = load_group(&Q.fbn);
+        R.fbn = q.x; R.fbt = q.y; R.mji = q.z; R.mij = q.w;
         if (diag) R.sbt = Q.sbt;
     }
     if (f & PR_DIAG) R.S = Q.S;
-    if (f & PR_SHEL) { R.a_ij = Q.a_ij; R.a_ji = Q.a_ji; R.w_ij = Q.w_ij; R.w_ji = Q.w_ji; }
+    if (f & PR_SHEL) {
+        const double4 q = load_group(&Q.a_ij);
+        R.a_ij = q.x; R.a_ji = q.y; R.w_ij = q.z; R.w_ji = q.w;
+    }
     return R;
 }
 
@@ -405,13 +435,67 @@ GD_DEV void sort_own(const Views &V, int cur, int a0, int a1)
     }
 }
 
-// Floes [0, N), first part: the ordered sums of the floe's pairs' records
-// and its pairs' ridging events, in the reference's order (partners of
-// lower id in ascending id, then its own row in the kd-tree's order).  Every
-// row holds first the pairs that can act on a step without diagnostics
-// before the next rebuild (lo_n / up_n of them), then the others, each part
-// in the row's order: a plain step walks the first part only; a diagnostic
-// step, on which every candidate adds its stress, walks both parts merged.
+// The ordered sums of floe g's pairs' records (A) and its shape after its
+// pairs' ridging events, in the reference's order (partners of lower id in
+// ascending id, then its own row in the kd-tree's order).  Every row holds
+// first the pairs that can act on a step without diagnostics before the next
+// rebuild (lo_n / up_n of them), then the others, each part in the row's
+// order: a plain step walks the first part only; a diagnostic step, on which
+// every candidate adds its stress, walks both parts merged.
+template <bool DIAG>
+GD_DEV Shape row_sums64(const Views &V, int cur, int g, const InstParams &P, const unsigned char *pfl,
+                        const PairRec64 *rec, const int *lo_n, const int *up_n, Acc<double> &A)
+{
+    const bool shel = P.shelter != 0;
+    A.fcx = A.fcy = A.mc = A.fbx = A.fby = A.mb = 0.0;
+    A.tac = A.pc = A.tab = A.pb = 0.0;
+    A.sxx = A.syy = A.sxy = A.syx = 0.0;
+    A.hsfa = A.hsfw = shel ? 1.0 : 0.0;
+    Shape run = make_shape(P, V.r[cur][g], V.h[cur][g]);
+    const int l0 = V.lo_off[g], l1 = V.lo_off[g + 1], lm = l0 + lo_n[g];
+    const int el = V.up_off[g], e1 = V.up_off[g + 1], em = el + up_n[g];
+
+    if (!DIAG) {
+        row_sum<false, true>(V.ent_lo, l0, lm, pfl, rec, P, A, run, shel);
+        sort_own(V, cur, el, em);
+        row_sum<false, false>(V.ent_up, el, em, pfl, rec, P, A, run, shel);
+    } else {
+        // ---- partners of lower id (the floe is the reference's "j"):
+        // the two parts merged by ascending id
+        int a = l0, b = lm;
+        int ida = a < lm ? V.id[cur][V.ent_lo[a].x] : 0, idb = b < l1 ? V.id[cur][V.ent_lo[b].x] : 0;
+        while (a < lm || b < l1) {
+            int take;
+            if (b >= l1 || (a < lm && ida < idb)) {
+                take = a++;
+                if (a < lm) ida = V.id[cur][V.ent_lo[a].x];
+            } else {
+                take = b++;
+                if (b < l1) idb = V.id[cur][V.ent_lo[b].x];
+            }
+            const int p = V.ent_lo[take].y;
+            add_pair<true, true>(rec, p, pfl[p], P, A, run, shel);
+        }
+        // ---- own row (the floe is "i"): each part sorted, merged by
+        // (distance, id)
+        sort_own(V, cur, el, em);
+        sort_own(V, cur, em, e1);
+        a = el;
+        b = em;
+        while (a < em || b < e1) {
+            bool first = b >= e1;
+            if (!first && a < em) {
+                const double da = V.edist[a], db = V.edist[b];
+                first = da < db || (da == db && V.id[cur][V.ent_up[a].x] < V.id[cur][V.ent_up[b].x]);
+            }
+            const int p = V.ent_up[first ? a++ : b++].y;
+            add_pair<true, false>(rec, p, pfl[p], P, A, run, shel);
+        }
+    }
+    return run;
+}
+
+// Floes [0, N), first part: the ordered sums.
 template <bool DIAG>
 __global__ void __launch_bounds__(128) k_row_sums_fp64(Views V, int cur, const unsigned char *pfl,
                                                        const PairRec64 *rec, const int *lo_n, const int *up_n,
@@ -422,54 +506,8 @@ __global__ void __launch_bounds__(128) k_row_sums_fp64(Views V, int cur, const u
     const size_t N = (size_t)V.N;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < V.N; g += gridDim.x * blockDim.x) {
         const InstParams &P = V.P[V.inst[g]];
-        const bool shel = P.shelter != 0;
         Acc<double> A;
-        A.fcx = A.fcy = A.mc = A.fbx = A.fby = A.mb = 0.0;
-        A.tac = A.pc = A.tab = A.pb = 0.0;
-        A.sxx = A.syy = A.sxy = A.syx = 0.0;
-        A.hsfa = A.hsfw = shel ? 1.0 : 0.0;
-        Shape run = make_shape(P, V.r[cur][g], V.h[cur][g]);
-        const int l0 = V.lo_off[g], l1 = V.lo_off[g + 1], lm = l0 + lo_n[g];
-        const int el = V.up_off[g], e1 = V.up_off[g + 1], em = el + up_n[g];
-
-        if (!DIAG) {
-            row_sum<false, true>(V.ent_lo, l0, lm, pfl, rec, P, A, run, shel);
-            sort_own(V, cur, el, em);
-            row_sum<false, false>(V.ent_up, el, em, pfl, rec, P, A, run, shel);
-        } else {
-            // ---- partners of lower id (the floe is the reference's "j"):
-            // the two parts merged by ascending id
-            int a = l0, b = lm;
-            int ida = a < lm ? V.id[cur][V.ent_lo[a].x] : 0, idb = b < l1 ? V.id[cur][V.ent_lo[b].x] : 0;
-            while (a < lm || b < l1) {
-                int take;
-                if (b >= l1 || (a < lm && ida < idb)) {
-                    take = a++;
-                    if (a < lm) ida = V.id[cur][V.ent_lo[a].x];
-                } else {
-                    take = b++;
-                    if (b < l1) idb = V.id[cur][V.ent_lo[b].x];
-                }
-                const int p = V.ent_lo[take].y;
-                add_pair<true, true>(rec, p, pfl[p], P, A, run, shel);
-            }
-            // ---- own row (the floe is "i"): each part sorted, merged by
-            // (distance, id)
-            sort_own(V, cur, el, em);
-            sort_own(V, cur, em, e1);
-            a = el;
-            b = em;
-            while (a < em || b < e1) {
-                bool first = b >= e1;
-                if (!first && a < em) {
-                    const double da = V.edist[a], db = V.edist[b];
-                    first = da < db || (da == db && V.id[cur][V.ent_up[a].x] < V.id[cur][V.ent_up[b].x]);
-                }
-                const int p = V.ent_up[first ? a++ : b++].y;
-                add_pair<true, false>(rec, p, pfl[p], P, A, run, shel);
-            }
-        }
-
+        const Shape run = row_sums64<DIAG>(V, cur, g, P, pfl, rec, lo_n, up_n, A);
         fs[FS64_FCX * N + g] = A.fcx; fs[FS64_FCY * N + g] = A.fcy; fs[FS64_MC * N + g] = A.mc;
         fs[FS64_FBX * N + g] = A.fbx; fs[FS64_FBY * N + g] = A.fby; fs[FS64_MB * N + g] = A.mb;
         fs[FS64_HSFA * N + g] = A.hsfa; fs[FS64_HSFW * N + g] = A.hsfw;
@@ -483,90 +521,265 @@ __global__ void __launch_bounds__(128) k_row_sums_fp64(Views V, int cur, const u
     }
 }
 
-// Floes [0, N), second part: walls with the shape after the floe's pair
-// events, drag and Coriolis with the final shape, totals and the FP64
-// update.  The shape after the events is make_shape of the radius and
-// thickness the sums wrote (apply_dh ends with make_shape too).
-template <bool DIAG>
+// The sums of one floe on a plain step by a group of GRP lanes.  One thread
+// per floe spends its time on a chain of loads a row entry long (row, flag,
+// record), and a step waits for its longest row: a large floe among small
+// ones, or any row of a sheltering field, whose every candidate has a record
+// (measured on 512 floes of such a field: 36 us of a 48 us step).  Here the
+// lanes load entries, flags and records side by side.
+//
+// The order of every sum is row_sums64's.  Only pairs in contact or bonded
+// add to the force sums: they are listed in shared memory, the partner row's
+// in row order, the own row's ranked by (distance, id), and their records are
+// then added one after the other, each handed round from the lane that loaded
+// it; every lane of the group holds the same sums.  A shelter factor only
+// lowers a minimum, whose result does not depend on the order as long as no
+// factor is NaN; each lane keeps its own and they are merged at the end.  A
+// floe with a NaN factor, or with more than CAP pairs to list, goes the
+// sequential way on the group's first lane.
+constexpr int GRP_CAP = 24;
+
+struct GroupList {
+    double d[GRP_CAP];
+    int p[GRP_CAP], id[GRP_CAP];
+    int q[GRP_CAP];               // pair index by rank
+    unsigned char f[GRP_CAP], fq[GRP_CAP];
+};
+
+GD_DEV double shfl_grp(double v, int src) { return __shfl_sync(0xffffffffu, v, src, GRP); }
+
+// on: whether this group has a floe (g); every lane of the warp calls.  The
+// result is valid in the group's first lane.
+GD_DEV void group_sums64(const Views &V, int cur, bool on, int g, const unsigned char *pfl, const PairRec64 *rec,
+                         const int *lo_n, const int *up_n, GroupList &L, Acc<double> &A, Shape &run)
+{
+    const int lane = threadIdx.x & 31, sub = lane & (GRP - 1);
+    const unsigned gmask = ((1u << GRP) - 1u) << (lane & ~(GRP - 1)), below = (1u << lane) - 1u;
+    const InstParams &P = V.P[on ? V.inst[g] : 0];
+    const bool shel = P.shelter != 0;
+    A.fcx = A.fcy = A.mc = A.fbx = A.fby = A.mb = 0.0;
+    A.hsfa = A.hsfw = shel ? 1.0 : 0.0;
+    int e0[2] = {0, 0}, e1[2] = {0, 0};
+    if (on) {
+        run = make_shape(P, V.r[cur][g], V.h[cur][g]);
+        e0[0] = V.lo_off[g]; e1[0] = e0[0] + lo_n[g];
+        e0[1] = V.up_off[g]; e1[1] = e0[1] + up_n[g];
+    }
+    int m = 0, mlo = 0;             // pairs listed, of the partner row
+    bool seq = false;
+#pragma unroll
+    for (int side = 0; side < 2; side++) {
+        const int2 *ent = side ? V.ent_up : V.ent_lo;
+        for (int b = e0[side]; __any_sync(0xffffffffu, b < e1[side]); b += GRP) {
+            const int e = b + sub;
+            int p = 0, id = 0;
+            unsigned f = 0;
+            double d = 0.0;
+            if (e < e1[side]) {
+                const int2 en = ent[e];
+                p = en.y;
+                f = pfl[p];
+                if (side) {
+                    d = V.edist[e];
+                    id = V.id[cur][en.x];
+                }
+            }
+            if (f & PR_SHEL) {
+                const double4 q = load_group(&rec[p].a_ij);
+                const double fa = side ? q.y : q.x, fw = side ? q.w : q.z;
+                seq |= fa != fa || fw != fw;
+                A.hsfa = tmin(A.hsfa, fa);
+                A.hsfw = tmin(A.hsfw, fw);
+            }
+            const bool add = (f & (PR_CONTACT | PR_BOND)) != 0;
+            const unsigned bal = __ballot_sync(0xffffffffu, add) & gmask;
+            const int k = m + __popc(bal & below);
+            if (add && k < GRP_CAP) {
+                L.p[k] = p; L.f[k] = (unsigned char)f;
+                L.d[k] = d; L.id[k] = id;
+            }
+            m += __popc(bal);
+        }
+        if (side == 0) mlo = m;
+    }
+    seq = (__ballot_sync(0xffffffffu, seq) & gmask) != 0 || m > GRP_CAP;
+    if (seq) m = mlo = 0;
+    __syncwarp();
+    // the own row's pairs by (distance, id)
+    for (int k = sub; k < m; k += GRP) {
+        int at = k;
+        if (k >= mlo) {
+            at = mlo;
+            for (int j = mlo; j < m; j++) at += L.d[j] < L.d[k] || (L.d[j] == L.d[k] && L.id[j] < L.id[k]);
+        }
+        L.q[at] = L.p[k];
+        L.fq[at] = L.f[k];
+    }
+    __syncwarp();
+    for (int b = 0; __any_sync(0xffffffffu, b < m); b += GRP) {
+        double4 qa, qb;
+        qa = qb = make_double4(0.0, 0.0, 0.0, 0.0);
+        if (b + sub < m) {
+            const PairRec64 &Q = rec[L.q[b + sub]];
+            qa = load_group(&Q.cosa);
+            qb = load_group(L.fq[b + sub] & PR_CONTACT ? &Q.fcn : &Q.fbn);
+        }
+        for (int j = 0; j < GRP && __any_sync(0xffffffffu, b + j < m); j++) {
+            PairRes<double> R;
+            R.cosa = shfl_grp(qa.x, j); R.sina = shfl_grp(qa.y, j);
+            R.ri_l = shfl_grp(qa.z, j); R.rj_l = shfl_grp(qa.w, j);
+            const double bx = shfl_grp(qb.x, j), by = shfl_grp(qb.y, j);
+            const double bz = shfl_grp(qb.z, j), bw = shfl_grp(qb.w, j);
+            if (b + j >= m) continue;
+            const unsigned f = L.fq[b + j];
+            const int p = L.q[b + j];
+            R.contact = (f & PR_CONTACT) != 0;
+            R.bond_on = (f & PR_BOND) != 0;
+            if (R.contact) { R.fcn = bx; R.fcr = by; R.fct = bz; R.mcc = bw; }
+            if (R.bond_on) {
+                R.fbn = bx; R.fbt = by; R.mji = bz; R.mij = bw;
+                if (R.contact) {
+                    const double4 q = load_group(&rec[p].fbn);
+                    R.fbn = q.x; R.fbt = q.y; R.mji = q.z; R.mij = q.w;
+                }
+            }
+            if (b + j < mlo) {
+                acc_side_j(A, R, P.lambda_lb, false, false);
+                if (f & PR_WHO2) apply_dh(P, run, rec[p].vol);
+            } else {
+                acc_side_i(A, R, P.lambda_lb, false, false);
+                if (f & PR_WHO1) apply_dh(P, run, rec[p].vol);
+            }
+        }
+    }
+#pragma unroll
+    for (int o = GRP / 2; o > 0; o >>= 1) {
+        A.hsfa = tmin(A.hsfa, __shfl_xor_sync(0xffffffffu, A.hsfa, o));
+        A.hsfw = tmin(A.hsfw, __shfl_xor_sync(0xffffffffu, A.hsfw, o));
+    }
+    if (seq && on && sub == 0) run = row_sums64<false>(V, cur, g, P, pfl, rec, lo_n, up_n, A);
+    __syncwarp();
+}
+
+// Floe g, second part: walls with the shape after the floe's pair events
+// (run), drag and Coriolis with the final shape, totals and the FP64 update
+// of step sic of a chunk (base: the chunk's first global step number, -1: in
+// device memory).  The shape after the events is make_shape of its radius and
+// thickness (apply_dh ends with make_shape too).  drag: the floe's drag and
+// Coriolis terms computed ahead with its start-of-step shape (eight planes;
+// null: none), taken if no event changed the shape.  Returns the wall events.
+template <bool DIAG, bool WALLS>
+GD_DEV int floe_update64(const Views &V, int cur, int base, int sic, int g, const InstParams &P, const Acc<double> &A,
+                         Shape run, const double *drag)
+{
+    const int nxt = cur ^ 1;
+    const bool px = P.boundary & BC_PERIODIC_X, py = P.boundary & BC_PERIODIC_Y;
+    const double x = V.x[cur][g], y = V.y[cur][g], th = V.th[cur][g];
+    const double u = V.u[cur][g], v = V.v[cur][g], om = V.om[cur][g];
+    const double r0 = V.r[cur][g], h0 = V.h[cur][g];
+
+    // ---- walls with the shape after this floe's pair events (a batch
+    // without walls neither reads nor writes the wall histories, which are
+    // zero on both sides)
+    WallOut W;
+    int wev = 0;
+    if (WALLS) {
+        double dtb1 = V.dtb1[cur][g], dtb2 = V.dtb2[cur][g];
+        double thb1 = V.thb1[cur][g], thb2 = V.thb2[cur][g];
+        verify_bc(P, x, y, u, v, om, run, dtb1, dtb2, thb1, thb2, W, wev);
+        V.dtb1[nxt][g] = dtb1; V.dtb2[nxt][g] = dtb2;
+        V.thb1[nxt][g] = thb1; V.thb2[nxt][g] = thb2;
+    } else {
+        W.fx_bc = W.fy_bc = W.m_bc = 0.0;
+        W.sxx = W.syy = W.sxy = W.syx = 0.0;
+        W.ta_bc = W.p_bc = 0.0;
+    }
+
+    // ---- drag and Coriolis with the final shape
+    Drag<double> D;
+    if (drag && run.r == r0 && run.h == h0) {
+        const size_t N = (size_t)V.N;
+        D.fax = drag[0 * N + g]; D.fay = drag[1 * N + g]; D.fwx = drag[2 * N + g]; D.fwy = drag[3 * N + g];
+        D.ma = drag[4 * N + g]; D.mw = drag[5 * N + g]; D.fcorx = drag[6 * N + g]; D.fcory = drag[7 * N + g];
+    } else {
+        double ua, va, uw, vw;
+        wind_at(P, V.field, x, y, ua, va, uw, vw);
+        D = forcing<double>(P, run, u, v, om, ua, va, uw, vw, A.hsfa, A.hsfw);
+    }
+
+    // ---- totals and integration (FP64)
+    const double fcx = A.fcx, fcy = A.fcy, fbx = A.fbx, fby = A.fby, mc = A.mc, mb = A.mb;
+    const double fax = D.fax, fay = D.fay, fwx = D.fwx, fwy = D.fwy;
+    const double tfx = ((((fcx + fbx) + fax) + fwx) + D.fcorx) + W.fx_bc;
+    const double tfy = ((((fcy + fby) + fay) + fwy) + D.fcory) + W.fy_bc;
+    const double mt = (((mc + mb) + D.ma) + D.mw) + W.m_bc;
+    const double dt = P.dt;
+    const double u1 = u + (tfx / run.mass) * dt;
+    const double v1 = v + (tfy / run.mass) * dt;
+    const double om1 = om + (mt / run.inertia) * dt;
+    double x1 = x + u1 * dt;
+    double y1 = y + v1 * dt;
+    const double th1 = th + om1 * dt;
+    if (px) { if (x1 < 0.0) x1 = x1 + P.nx; else if (x1 >= P.nx) x1 = x1 - P.nx; }
+    if (py) { if (y1 < 0.0) y1 = y1 + P.ny; else if (y1 >= P.ny) y1 = y1 - P.ny; }
+    V.x[nxt][g] = x1; V.y[nxt][g] = y1; V.th[nxt][g] = th1;
+    V.u[nxt][g] = u1; V.v[nxt][g] = v1; V.om[nxt][g] = om1;
+    V.r[nxt][g] = run.r; V.h[nxt][g] = run.h;
+
+    // ---- neighbour-list validity and finiteness
+    const double ddx = wrap_d(x1 - V.x0[cur][g], P.nx, px), ddy = wrap_d(y1 - V.y0[cur][g], P.ny, py);
+    const double half = 0.5 * P.skin;
+    if (ddx * ddx + ddy * ddy > half * half) {
+        atomicOr(V.status, ST_EXPIRED);
+        atomicMin(V.expired_at, base >= 0 ? base + sic : global_step(V, sic));
+    }
+    if (!(isfinite(x1) && isfinite(y1) && isfinite(u1) && isfinite(v1) && isfinite(om1) && isfinite(th1)))
+        atomicOr(V.status, ST_NAN);
+
+    if (DIAG) {
+        const size_t N = (size_t)V.N;
+        const double rr = run.r;
+        const double sxx = (A.sxx + W.sxx) + (fax + fwx) * rr;
+        const double syy = (A.syy + W.syy) + (fay + fwy) * rr;
+        const double sxy = (A.sxy + W.sxy) + 0.0;
+        const double syx = (A.syx + W.syx) + 0.0;
+        const double tac = A.tac, tab = A.tab;
+        const double pa = tac != 0.0 ? A.pc / tac : 0.0;
+        const double pbv = tab != 0.0 ? A.pb / tab : 0.0;
+        const double pw = W.ta_bc != 0.0 ? W.p_bc / W.ta_bc : 0.0;
+        double *D0 = V.diag;
+        D0[0 * N + g] = tfx; D0[1 * N + g] = tfy; D0[2 * N + g] = fcx; D0[3 * N + g] = fcy;
+        D0[4 * N + g] = fbx; D0[5 * N + g] = fby; D0[6 * N + g] = mt; D0[7 * N + g] = mc;
+        D0[8 * N + g] = mb; D0[9 * N + g] = sxx; D0[10 * N + g] = syy; D0[11 * N + g] = sxy;
+        D0[12 * N + g] = syx; D0[13 * N + g] = (pa + pbv) + pw;
+    }
+    return DIAG ? wev : 0;
+}
+
+// Floes [0, N), second part, from the sums of the first.
+template <bool DIAG, bool WALLS>
 __global__ void __launch_bounds__(128) k_floes_fp64(Views V, int cur, int sic, const double *fs, int *nwork)
 {
     step_kernel_entry();
     // the work lists were used by the pair kernels before this one
     if (blockIdx.x == 0 && threadIdx.x < 2) nwork[threadIdx.x] = 0;
-    if (floe_update_stopped(V, sic)) return;
-    const int nxt = cur ^ 1;
+    if (floe_update_stopped(V, -1, sic)) return;
     const size_t N = (size_t)V.N;
     unsigned long long n_plast = 0;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < V.N; g += gridDim.x * blockDim.x) {
         const InstParams &P = V.P[V.inst[g]];
-        const bool px = P.boundary & BC_PERIODIC_X, py = P.boundary & BC_PERIODIC_Y;
-        const double x = V.x[cur][g], y = V.y[cur][g], th = V.th[cur][g];
-        const double u = V.u[cur][g], v = V.v[cur][g], om = V.om[cur][g];
-        double dtb1 = V.dtb1[cur][g], dtb2 = V.dtb2[cur][g];
-        double thb1 = V.thb1[cur][g], thb2 = V.thb2[cur][g];
-        double ua, va, uw, vw;
-        wind_at(P, V.field, x, y, ua, va, uw, vw);
-        Shape run = make_shape(P, fs[FS64_R * N + g], fs[FS64_H * N + g]);
-
-        // ---- walls with the shape after this floe's pair events
-        WallOut W;
-        int wev = 0;
-        verify_bc(P, x, y, u, v, om, run, dtb1, dtb2, thb1, thb2, W, wev);
-        n_plast += DIAG ? wev : 0;
-
-        // ---- drag and Coriolis with the final shape
-        const Drag<double> D = forcing<double>(P, run, u, v, om, ua, va, uw, vw, fs[FS64_HSFA * N + g],
-                                               fs[FS64_HSFW * N + g]);
-
-        // ---- totals and integration (FP64)
-        const double fcx = fs[FS64_FCX * N + g], fcy = fs[FS64_FCY * N + g];
-        const double fbx = fs[FS64_FBX * N + g], fby = fs[FS64_FBY * N + g];
-        const double mc = fs[FS64_MC * N + g], mb = fs[FS64_MB * N + g];
-        const double fax = D.fax, fay = D.fay, fwx = D.fwx, fwy = D.fwy;
-        const double tfx = ((((fcx + fbx) + fax) + fwx) + D.fcorx) + W.fx_bc;
-        const double tfy = ((((fcy + fby) + fay) + fwy) + D.fcory) + W.fy_bc;
-        const double mt = (((mc + mb) + D.ma) + D.mw) + W.m_bc;
-        const double dt = P.dt;
-        const double u1 = u + (tfx / run.mass) * dt;
-        const double v1 = v + (tfy / run.mass) * dt;
-        const double om1 = om + (mt / run.inertia) * dt;
-        double x1 = x + u1 * dt;
-        double y1 = y + v1 * dt;
-        const double th1 = th + om1 * dt;
-        if (px) { if (x1 < 0.0) x1 = x1 + P.nx; else if (x1 >= P.nx) x1 = x1 - P.nx; }
-        if (py) { if (y1 < 0.0) y1 = y1 + P.ny; else if (y1 >= P.ny) y1 = y1 - P.ny; }
-        V.x[nxt][g] = x1; V.y[nxt][g] = y1; V.th[nxt][g] = th1;
-        V.u[nxt][g] = u1; V.v[nxt][g] = v1; V.om[nxt][g] = om1;
-        V.r[nxt][g] = run.r; V.h[nxt][g] = run.h;
-        V.dtb1[nxt][g] = dtb1; V.dtb2[nxt][g] = dtb2;
-        V.thb1[nxt][g] = thb1; V.thb2[nxt][g] = thb2;
-
-        // ---- neighbour-list validity and finiteness
-        const double ddx = wrap_d(x1 - V.x0[cur][g], P.nx, px), ddy = wrap_d(y1 - V.y0[cur][g], P.ny, py);
-        const double half = 0.5 * P.skin;
-        if (ddx * ddx + ddy * ddy > half * half) {
-            atomicOr(V.status, ST_EXPIRED);
-            atomicMin(V.expired_at, global_step(V, sic));
-        }
-        if (!(isfinite(x1) && isfinite(y1) && isfinite(u1) && isfinite(v1) && isfinite(om1) && isfinite(th1)))
-            atomicOr(V.status, ST_NAN);
-
+        Acc<double> A;
+        A.fcx = fs[FS64_FCX * N + g]; A.fcy = fs[FS64_FCY * N + g]; A.mc = fs[FS64_MC * N + g];
+        A.fbx = fs[FS64_FBX * N + g]; A.fby = fs[FS64_FBY * N + g]; A.mb = fs[FS64_MB * N + g];
+        A.hsfa = fs[FS64_HSFA * N + g]; A.hsfw = fs[FS64_HSFW * N + g];
         if (DIAG) {
-            const double rr = run.r;
-            const double sxx = (fs[FS64_SXX * N + g] + W.sxx) + (fax + fwx) * rr;
-            const double syy = (fs[FS64_SYY * N + g] + W.syy) + (fay + fwy) * rr;
-            const double sxy = (fs[FS64_SXY * N + g] + W.sxy) + 0.0;
-            const double syx = (fs[FS64_SYX * N + g] + W.syx) + 0.0;
-            const double tac = fs[FS64_TAC * N + g], tab = fs[FS64_TAB * N + g];
-            const double pa = tac != 0.0 ? fs[FS64_PC * N + g] / tac : 0.0;
-            const double pbv = tab != 0.0 ? fs[FS64_PB * N + g] / tab : 0.0;
-            const double pw = W.ta_bc != 0.0 ? W.p_bc / W.ta_bc : 0.0;
-            double *D0 = V.diag;
-            D0[0 * N + g] = tfx; D0[1 * N + g] = tfy; D0[2 * N + g] = fcx; D0[3 * N + g] = fcy;
-            D0[4 * N + g] = fbx; D0[5 * N + g] = fby; D0[6 * N + g] = mt; D0[7 * N + g] = mc;
-            D0[8 * N + g] = mb; D0[9 * N + g] = sxx; D0[10 * N + g] = syy; D0[11 * N + g] = sxy;
-            D0[12 * N + g] = syx; D0[13 * N + g] = (pa + pbv) + pw;
+            A.tac = fs[FS64_TAC * N + g]; A.pc = fs[FS64_PC * N + g];
+            A.tab = fs[FS64_TAB * N + g]; A.pb = fs[FS64_PB * N + g];
+            A.sxx = fs[FS64_SXX * N + g]; A.syy = fs[FS64_SYY * N + g];
+            A.sxy = fs[FS64_SXY * N + g]; A.syx = fs[FS64_SYX * N + g];
         }
+        const Shape run = make_shape(P, fs[FS64_R * N + g], fs[FS64_H * N + g]);
+        n_plast += floe_update64<DIAG, WALLS>(V, cur, -1, sic, g, P, A, run, nullptr);
     }
 
     if (DIAG) {
@@ -574,6 +787,190 @@ __global__ void __launch_bounds__(128) k_floes_fp64(Views V, int cur, int sic, c
         for (int o = 16; o > 0; o >>= 1) n_plast += __shfl_down_sync(0xffffffffu, n_plast, o);
         if ((threadIdx.x & 31) == 0 && n_plast) atomicAdd(&V.counters[3], n_plast);
     }
+}
+
+// ---------------------------------------------------------------- small batches
+// A batch of few floes is bound by the latency of one thread's dependent
+// loads and FP64 operations and by the gaps between kernels, not by any
+// rate.  k_steps_fp64 runs a chunk of K whole steps in one launch of one
+// cluster (or one block): the screen and the pair physics of every entry in
+// one pass, each thread carrying its pair from the distance to the record,
+// beside the drag and Coriolis terms of every floe (they need the pairs only
+// where an event changes the shape or in a sheltering field, where the update
+// computes them again); a cluster barrier; the ordered sums and the update of
+// every floe; a cluster barrier.  Two barriers a step stand in for five
+// kernels.  Every value is computed by the functions the five kernels use.
+struct SmallArgs64 {
+    int cur, K, diag_last, base;   // first side, steps, diagnostics on the last one, global number of the first
+    int n, E;                      // marked positions (plist), owner entries
+    const int *plist;
+    const unsigned *erow;
+    unsigned char *pfl;
+    PairRec64 *rec;
+    const int *lo_n, *up_n;
+    double *drag;                  // [8][N]
+    int *out;                      // pinned host memory: the status word and the first expired step
+    int *done;                     // blocks of k_step_floes_fp64 that have finished
+};
+
+// One owner entry: k_pairs_fp64_screen and k_pairs_fp64 in one.
+template <bool DIAG>
+GD_DEV void pair_entry64(const Views &V, int cur, int e, const unsigned *erow, unsigned char *pfl, PairRec64 *rec,
+                         Counts64 &C)
+{
+    Hist4<double> *Hs = (Hist4<double> *)V.hist[0];
+    const int g = (int)erow[e];
+    const int2 en = V.ent_up[e];
+    const int t = en.x, p = en.y;
+    const InstParams &P = V.P[V.inst[g]];
+    const bool px = P.boundary & BC_PERIODIC_X, py = P.boundary & BC_PERIODIC_Y;
+    const double rg = V.r[cur][g], rt = V.r[cur][t];
+    const int bi = V.bidx[p];
+    const double2 h01 = *(const double2 *)&Hs[p];
+    const double dx = wrap_d(V.x[cur][g] - V.x[cur][t], P.nx, px);
+    const double dy = wrap_d(V.y[cur][g] - V.y[cur][t], P.ny, py);
+    const double dist = sqrt(dx * dx + dy * dy);
+    V.edist[e] = dist;
+    if (!(dist <= rg + P.rtree)) {
+        // history and bond state stay as they are
+        pfl[p] = 0;
+        if (DIAG) V.pdn[p] = __int_as_float(0x7fc00000);
+        return;
+    }
+    const double deltan = (rg + rt) - dist;
+    if (deltan > 0.0 || P.shelter != 0 || bi >= 0) {
+        pair_work64<false, DIAG>(V, cur, Hs, p, g, t, bi, dx, dy, pfl, rec, C);
+    } else {
+        pfl[p] = (unsigned char)quiet_candidate<DIAG>(V, Hs, p, dx, dy, dist, deltan, rg, rt, h01, rec);
+        if (DIAG) C.cand++;
+    }
+}
+
+template <bool DIAG>
+GD_DEV void small_pairs64(const Views &V, const SmallArgs64 &A, int cur)
+{
+    const int nthr = gridDim.x * blockDim.x;
+    const int n = DIAG ? A.E : A.n;
+    const int n0 = (n + 31) & ~31;      // the floes start on a warp of their own
+    const size_t N = (size_t)V.N;
+    Counts64 C = {0, 0, 0, 0};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n0 + V.N; i += nthr) {
+        if (i < n) {
+            pair_entry64<DIAG>(V, cur, DIAG ? i : A.plist[i], A.erow, A.pfl, A.rec, C);
+        } else if (i >= n0) {
+            const int g = i - n0;
+            const InstParams &P = V.P[V.inst[g]];
+            if (P.shelter != 0) continue;
+            double ua, va, uw, vw;
+            wind_at(P, V.field, V.x[cur][g], V.y[cur][g], ua, va, uw, vw);
+            const Drag<double> D = forcing<double>(P, make_shape(P, V.r[cur][g], V.h[cur][g]), V.u[cur][g],
+                                                   V.v[cur][g], V.om[cur][g], ua, va, uw, vw, 0.0, 0.0);
+            A.drag[0 * N + g] = D.fax; A.drag[1 * N + g] = D.fay; A.drag[2 * N + g] = D.fwx;
+            A.drag[3 * N + g] = D.fwy; A.drag[4 * N + g] = D.ma; A.drag[5 * N + g] = D.mw;
+            A.drag[6 * N + g] = D.fcorx; A.drag[7 * N + g] = D.fcory;
+        }
+    }
+    __syncwarp();
+    if (DIAG) add_counts(C, V.counters);
+}
+
+// The floes' sums and update, one thread per floe.
+template <bool DIAG>
+GD_DEV void small_floes64(const Views &V, const SmallArgs64 &A, int cur, int sic)
+{
+    const int nthr = gridDim.x * blockDim.x;
+    Counts64 C = {0, 0, 0, 0};
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < V.N; g += nthr) {
+        const InstParams &P = V.P[V.inst[g]];
+        Acc<double> S;
+        const Shape run = row_sums64<DIAG>(V, cur, g, P, A.pfl, A.rec, A.lo_n, A.up_n, S);
+        C.plast += floe_update64<DIAG, true>(V, cur, A.base, sic, g, P, S, run, P.shelter != 0 ? nullptr : A.drag);
+    }
+    __syncwarp();
+    if (DIAG) add_counts(C, V.counters);
+}
+
+__global__ void __launch_bounds__(SMALL_THREADS, 1) k_steps_fp64(Views V, SmallArgs64 A)
+{
+    step_kernel_entry();
+    for (int k = 0; k < A.K; k++) {
+        // the same answer in every thread: the status is written between the
+        // two barriers of a step only
+        if (*(volatile int *)V.status & ST_ABORT) break;
+        const int cur = A.cur ^ (k & 1);
+        const bool diag = A.diag_last && k == A.K - 1;
+        if (diag) small_pairs64<true>(V, A, cur);
+        else small_pairs64<false>(V, A, cur);
+        cluster_sync();
+        if (diag) small_floes64<true>(V, A, cur, k);
+        else small_floes64<false>(V, A, cur, k);
+        cluster_sync();
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) publish_status(V, A.out);
+}
+
+// The two halves of a step as ordinary grids, for batches with more work
+// than one cluster does quickly: two launches a step instead of five.  The
+// second one of a chunk's last step publishes the status word.
+template <bool DIAG>
+__global__ void __launch_bounds__(128) k_step_pairs_fp64(Views V, SmallArgs64 A, int cur)
+{
+    step_kernel_entry();
+    if (*(volatile int *)V.status & ST_ABORT) return;
+    small_pairs64<DIAG>(V, A, cur);
+}
+
+template <bool DIAG>
+__global__ void __launch_bounds__(128) k_step_floes_fp64(Views V, SmallArgs64 A, int cur, int sic)
+{
+    step_kernel_entry();
+    if (!floe_update_stopped(V, A.base, sic)) small_floes64<DIAG>(V, A, cur, sic);
+    if (sic == A.K - 1) publish_status_last(V, A.done, A.out);
+}
+
+// The second half of a plain step with the floes' sums by groups of lanes: a
+// block sums GRP_FLOES floes at a time, `rounds` times (at most GRP), then
+// gives every floe's update a thread.
+__global__ void __launch_bounds__(SMALL_THREADS, 2) k_step_floes_grp_fp64(Views V, SmallArgs64 A, int cur, int sic,
+                                                                          int rounds)
+{
+    __shared__ GroupList list[GRP_FLOES];
+    __shared__ double sum[10][SMALL_THREADS];
+    __shared__ int stopped;
+    step_kernel_entry();
+    // one answer per block: another block may raise an expiry meanwhile
+    if (threadIdx.x == 0) stopped = floe_update_stopped(V, A.base, sic);
+    __syncthreads();
+    const int grp = threadIdx.x / GRP, per = rounds * GRP_FLOES;
+    for (int g0 = blockIdx.x * per; !stopped && g0 < V.N; g0 += gridDim.x * per) {
+        for (int r = 0; r < rounds; r++) {
+            const int at = r * GRP_FLOES + grp;
+            const bool on = g0 + at < V.N;
+            Acc<double> S;
+            Shape run;
+            run.r = run.h = 0.0;
+            group_sums64(V, cur, on, g0 + at, A.pfl, A.rec, A.lo_n, A.up_n, list[grp], S, run);
+            if (on && threadIdx.x % GRP == 0) {
+                sum[0][at] = S.fcx; sum[1][at] = S.fcy; sum[2][at] = S.mc;
+                sum[3][at] = S.fbx; sum[4][at] = S.fby; sum[5][at] = S.mb;
+                sum[6][at] = S.hsfa; sum[7][at] = S.hsfw;
+                sum[8][at] = run.r; sum[9][at] = run.h;
+            }
+        }
+        __syncthreads();
+        const int q = threadIdx.x, g = g0 + q;
+        if (q < per && g < V.N) {
+            const InstParams &P = V.P[V.inst[g]];
+            Acc<double> S;
+            S.fcx = sum[0][q]; S.fcy = sum[1][q]; S.mc = sum[2][q];
+            S.fbx = sum[3][q]; S.fby = sum[4][q]; S.mb = sum[5][q];
+            S.hsfa = sum[6][q]; S.hsfw = sum[7][q];
+            const Shape run = make_shape(P, sum[8][q], sum[9][q]);
+            floe_update64<false, true>(V, cur, A.base, sic, g, P, S, run, P.shelter != 0 ? nullptr : A.drag);
+        }
+        __syncthreads();
+    }
+    if (sic == A.K - 1) publish_status_last(V, A.done, A.out);
 }
 
 }  // namespace godar

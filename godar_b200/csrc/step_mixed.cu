@@ -297,6 +297,21 @@ GD_DEV bool screen_test(const Views &V, const Snap *S, int2 *eb, int k, const in
     return false;
 }
 
+// D of the step from side cur: the previous step's D and largest step (side
+// cur ^ 1); one thread publishes it and clears the slot this step's update
+// fills.
+GD_DEV float advance_bound(int cur, const MixedBufs &B)
+{
+    const int o = cur ^ 1;
+    const float Dk = __fadd_ru(__uint_as_float(__ldcg(B.dsp + 2 + o)),
+                               __fmul_ru(__fsqrt_ru(__uint_as_float(__ldcg(B.dsp + o))), 1.00001f));
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        B.dsp[2 + cur] = __float_as_uint(Dk);
+        B.dsp[cur] = 0u;
+    }
+    return Dk;
+}
+
 // Appends entry e of every lane with `heavy` to the work list, with its
 // slots st where known (st.x >= 0), one atomic per warp; every lane of the
 // warp must call it.
@@ -329,15 +344,7 @@ __global__ void __launch_bounds__(256) k_pairs_screen(Views V, int cur, int diag
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int stride = gridDim.x * blockDim.x;
     const int nit = (P + stride - 1) / stride;
-    // D of this step: the previous step's D and largest step (side cur ^ 1);
-    // one thread publishes it and clears the slot this step's update fills
-    const int o = cur ^ 1;
-    const float Dk = __fadd_ru(__uint_as_float(__ldcg(B.dsp + 2 + o)),
-                               __fmul_ru(__fsqrt_ru(__uint_as_float(__ldcg(B.dsp + o))), 1.00001f));
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        B.dsp[2 + cur] = __float_as_uint(Dk);
-        B.dsp[cur] = 0u;
-    }
+    const float Dk = advance_bound(cur, B);
     // a diagnostic step computes every owner entry: the pair kernel walks
     // them itself, without a work list
     if (diag || !eb) return;
@@ -390,6 +397,108 @@ __global__ void __launch_bounds__(256) k_pairs_screen(Views V, int cur, int diag
     }
 }
 
+// The pair physics of owner entry e (slots s, t): contact forces, ridging
+// event, sheltering, history update, record and flags.
+GD_DEV void pair_mixed(const Views &V, const Snap *S, Hist4<float> *Hh, int diag, int e, int s, int t,
+                       const MixedBufs &B, unsigned long long &n_cand, unsigned long long &n_cont,
+                       unsigned long long &n_plast)
+{
+    const unsigned f0 = B.pfl[e];
+    // the entry's own records, loaded beside the snapshots rather than
+    // after the distance test
+    const Hist4<float> Hraw = Hh[e];
+    const int bix = V.bidx[e];
+    const int wix = bix >= 0 ? B.winv[bix] : -1;
+    const Snap Si = S[s], Sj = S[t];      // s has the lower id: the reference's "i"
+    const InstParams &Pm = V.P[Si.inst];
+    const bool px = Pm.boundary & BC_PERIODIC_X, py = Pm.boundary & BC_PERIODIC_Y;
+    const bool shel = Pm.shelter != 0;
+    const double dx = wrap_d(Si.x - Sj.x, Pm.nx, px), dy = wrap_d(Si.y - Sj.y, Pm.ny, py);
+    const double d2 = dx * dx + dy * dy;
+    unsigned f1 = f0 & PF_HIST;
+    const double dist = sqrt(d2);
+    if (dist <= Si.r + Pm.rtree) {
+        Hist4<float> H;
+        if ((f0 & PF_HIST) || diag) H = Hraw;
+        else { H.deltat = 0.f; H.thetarelc = 0.f; H.fcn = 0.f; H.fct = 0.f; }
+        const float fd = (float)dist;
+        const float cosa = (float)(-dx) / fd;
+        const float sina = (float)(-dy) / fd;
+        ContactOut C;
+        int bi = -1;
+        bool bond_active = false;
+        if ((Si.r + Sj.r) - dist > 0.0) {
+            // the bond's working index; its state at the start of the
+            // step (the bond kernel may be updating it at the same time)
+            bi = wix;
+            if (bi >= 0) {
+                bond_active = B.bfl_rd[bi] == 1;
+            }
+        }
+        contact_mixed(Pm, dist, cosa, sina, Si, Sj, H, bond_active, C);
+        if (C.contact || (f0 & PF_HIST)) {
+            Hh[e] = H;
+            f1 = (H.deltat != 0.f || H.thetarelc != 0.f) ? PF_HIST : 0u;
+        }
+        if (C.who != 0 && bi >= 0) {
+            // tell the bond kernel the pair's post-event radius
+            const float rl = C.who == 1 ? C.ri_l : -C.rj_l;
+            B.wdyn[bi].pad = __float_as_int(rl);
+        }
+        // force records only where a force or shelter factor can be
+        // nonzero, so that entries off the contact list never carry one
+        if (C.contact || shel) {
+            B.rec[2 * (size_t)e] = make_float4(C.fx, C.fy, C.mi, C.mj);
+            if (shel) {
+                double a0, a1, a2, a3;
+                wind_at(Pm, V.field, Si.x, Si.y, a0, a1, a2, a3);
+                const float ua = (float)a0, va = (float)a1, uw = (float)a2, vw = (float)a3;
+                const float dn = (float)((Si.r + Sj.r) - dist);
+                const float hfai = Pm.f_hfa * C.hi_l, hfaj = Pm.f_hfa * C.hj_l;
+                const float hfwi = Pm.f_hfw * C.hi_l, hfwj = Pm.f_hfw * C.hj_l;
+                float a_ij, a_ji, w_ij, w_ji;
+                shelter_pair<float>(hfai, hfaj, dn, cosa, sina, ua, va, a_ij, a_ji);
+                shelter_pair<float>(hfwi, hfwj, dn, cosa, sina, uw, vw, w_ij, w_ji);
+                B.rec[2 * (size_t)e + 1] = make_float4(a_ji, w_ji, a_ij, w_ij);
+            }
+            f1 |= PF_REC;
+            if (C.who != 0) {
+                const double rex = C.who == 1 ? C.vol / ((Pm.pi * (Si.r * Si.r)) * (double)Si.h)
+                                              : C.vol / ((Pm.pi * (Sj.r * Sj.r)) * (double)Sj.h);
+                B.rx[e] = C.who == 1 ? make_float2((float)rex, 0.f) : make_float2(0.f, (float)rex);
+                f1 |= PF_REX;
+            }
+        }
+        if (diag) {
+            // contact part of the stress sums (stepper.f90:238-271); the
+            // reference's S adds the bond force, done per bond.  A pair
+            // out of contact whose last normal and tangential forces are
+            // zero (it has not touched since it entered the rows) adds
+            // only zeros: it leaves no record (a sum that starts at +0
+            // never becomes -0, so adding a zero changes no bit)
+            const float Sc = sqrtf(H.fcn * H.fcn + H.fct * H.fct);
+            if (C.contact || Sc != 0.f) {
+                f1 |= PF_DG;
+                const float rl = C.ri_l;
+                B.pdg[2 * (size_t)e] = make_float4(C.ac, -(C.fcn * C.ac), -(((Sc * cosa) * rl) * cosa),
+                                                   -(((Sc * sina) * rl) * sina));
+                B.pdg[2 * (size_t)e + 1] = make_float4(-(((Sc * sina) * rl) * cosa),
+                                                       -(((Sc * cosa) * rl) * sina), 0.f, 0.f);
+            }
+            V.pdn[e] = (float)((Si.r + Sj.r) - dist);
+            n_cand++;
+            n_cont += C.contact;
+            n_plast += C.who != 0;
+        }
+    } else if (diag) {
+        V.pdn[e] = __int_as_float(0x7fc00000);
+    }
+    if (f1 != f0) {
+        B.pfl[e] = (unsigned char)f1;
+        B.lfl[B.lo_of[e]] = (unsigned char)(f1 & ~PF_HIST);
+    }
+}
+
 // Pairs of the work list: contact forces, ridging events, sheltering,
 // history updates and records.
 __global__ void __launch_bounds__(256, 3) k_pairs_mixed(Views V, int cur, int diag, int P, const unsigned *erow,
@@ -420,100 +529,7 @@ __global__ void __launch_bounds__(256, 3) k_pairs_mixed(Views V, int cur, int di
             s = st.x;
             t = st.y;
         }
-        const unsigned f0 = B.pfl[e];
-        // the entry's own records, loaded beside the snapshots rather than
-        // after the distance test
-        const Hist4<float> Hraw = Hh[e];
-        const int bix = V.bidx[e];
-        const int wix = bix >= 0 ? B.winv[bix] : -1;
-        const Snap Si = S[s], Sj = S[t];      // s has the lower id: the reference's "i"
-        const InstParams &Pm = V.P[Si.inst];
-        const bool px = Pm.boundary & BC_PERIODIC_X, py = Pm.boundary & BC_PERIODIC_Y;
-        const bool shel = Pm.shelter != 0;
-        const double dx = wrap_d(Si.x - Sj.x, Pm.nx, px), dy = wrap_d(Si.y - Sj.y, Pm.ny, py);
-        const double d2 = dx * dx + dy * dy;
-        unsigned f1 = f0 & PF_HIST;
-        const double dist = sqrt(d2);
-        if (dist <= Si.r + Pm.rtree) {
-            Hist4<float> H;
-            if ((f0 & PF_HIST) || diag) H = Hraw;
-            else { H.deltat = 0.f; H.thetarelc = 0.f; H.fcn = 0.f; H.fct = 0.f; }
-            const float fd = (float)dist;
-            const float cosa = (float)(-dx) / fd;
-            const float sina = (float)(-dy) / fd;
-            ContactOut C;
-            int bi = -1;
-            bool bond_active = false;
-            if ((Si.r + Sj.r) - dist > 0.0) {
-                // the bond's working index; its state at the start of the
-                // step (the bond kernel may be updating it at the same time)
-                bi = wix;
-                if (bi >= 0) {
-                    bond_active = B.bfl_rd[bi] == 1;
-                }
-            }
-            contact_mixed(Pm, dist, cosa, sina, Si, Sj, H, bond_active, C);
-            if (C.contact || (f0 & PF_HIST)) {
-                Hh[e] = H;
-                f1 = (H.deltat != 0.f || H.thetarelc != 0.f) ? PF_HIST : 0u;
-            }
-            if (C.who != 0 && bi >= 0) {
-                // tell the bond kernel the pair's post-event radius
-                const float rl = C.who == 1 ? C.ri_l : -C.rj_l;
-                B.wdyn[bi].pad = __float_as_int(rl);
-            }
-            // force records only where a force or shelter factor can be
-            // nonzero, so that entries off the contact list never carry one
-            if (C.contact || shel) {
-                B.rec[2 * (size_t)e] = make_float4(C.fx, C.fy, C.mi, C.mj);
-                if (shel) {
-                    double a0, a1, a2, a3;
-                    wind_at(Pm, V.field, Si.x, Si.y, a0, a1, a2, a3);
-                    const float ua = (float)a0, va = (float)a1, uw = (float)a2, vw = (float)a3;
-                    const float dn = (float)((Si.r + Sj.r) - dist);
-                    const float hfai = Pm.f_hfa * C.hi_l, hfaj = Pm.f_hfa * C.hj_l;
-                    const float hfwi = Pm.f_hfw * C.hi_l, hfwj = Pm.f_hfw * C.hj_l;
-                    float a_ij, a_ji, w_ij, w_ji;
-                    shelter_pair<float>(hfai, hfaj, dn, cosa, sina, ua, va, a_ij, a_ji);
-                    shelter_pair<float>(hfwi, hfwj, dn, cosa, sina, uw, vw, w_ij, w_ji);
-                    B.rec[2 * (size_t)e + 1] = make_float4(a_ji, w_ji, a_ij, w_ij);
-                }
-                f1 |= PF_REC;
-                if (C.who != 0) {
-                    const double rex = C.who == 1 ? C.vol / ((Pm.pi * (Si.r * Si.r)) * (double)Si.h)
-                                                  : C.vol / ((Pm.pi * (Sj.r * Sj.r)) * (double)Sj.h);
-                    B.rx[e] = C.who == 1 ? make_float2((float)rex, 0.f) : make_float2(0.f, (float)rex);
-                    f1 |= PF_REX;
-                }
-            }
-            if (diag) {
-                // contact part of the stress sums (stepper.f90:238-271); the
-                // reference's S adds the bond force, done per bond.  A pair
-                // out of contact whose last normal and tangential forces are
-                // zero (it has not touched since it entered the rows) adds
-                // only zeros: it leaves no record (a sum that starts at +0
-                // never becomes -0, so adding a zero changes no bit)
-                const float Sc = sqrtf(H.fcn * H.fcn + H.fct * H.fct);
-                if (C.contact || Sc != 0.f) {
-                    f1 |= PF_DG;
-                    const float rl = C.ri_l;
-                    B.pdg[2 * (size_t)e] = make_float4(C.ac, -(C.fcn * C.ac), -(((Sc * cosa) * rl) * cosa),
-                                                       -(((Sc * sina) * rl) * sina));
-                    B.pdg[2 * (size_t)e + 1] = make_float4(-(((Sc * sina) * rl) * cosa),
-                                                           -(((Sc * cosa) * rl) * sina), 0.f, 0.f);
-                }
-                V.pdn[e] = (float)((Si.r + Sj.r) - dist);
-                n_cand++;
-                n_cont += C.contact;
-                n_plast += C.who != 0;
-            }
-        } else if (diag) {
-            V.pdn[e] = __int_as_float(0x7fc00000);
-        }
-        if (f1 != f0) {
-            B.pfl[e] = (unsigned char)f1;
-            B.lfl[B.lo_of[e]] = (unsigned char)(f1 & ~PF_HIST);
-        }
+        pair_mixed(V, S, Hh, diag, e, s, t, B, n_cand, n_cont, n_plast);
     }
     if (diag) {
         warp_count(n_cand, V.counters, 0);
@@ -794,6 +810,81 @@ GD_DEV unsigned long long flag_word(const unsigned char *fl, int w, int e0, int 
     return word & (mhi & ~mlo) & bits;
 }
 
+// What the update of one floe needs of its pairs and bonds (FP32 sums).
+struct FloeSum32 {
+    float fcx, fcy, mc, fbx, fby, mb, sca, scw, rex;
+    float tac, pc, tab, pb, sxx, syy, sxy, syx;      // diagnostic steps
+};
+
+template <bool DIAG>
+GD_DEV void floe_sum(const Views &V, const MixedBufs &B, int g, FloeSum32 &F)
+{
+    constexpr bool diag = DIAG;
+    const bool shel = V.P[V.inst[g]].shelter != 0;
+    // contact and bond sums (FP32) in the order: own row, partner row,
+    // own bonds, partner bonds
+    float fcx = 0.f, fcy = 0.f, mc = 0.f, fbx = 0.f, fby = 0.f, mb = 0.f;
+    float sca = 1.f, scw = 1.f, rex = 0.f;
+    float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = make_float4(0.f, 0.f, 0.f, 0.f);   // tac pc sxx syy | sxy syx
+    float tab = 0.f, pbs = 0.f;
+    // flag bytes are read eight at a time; most pairs leave no record
+    const unsigned long long want = diag ? 0x0e0e0e0e0e0e0e0eULL : 0x0a0a0a0a0a0a0a0aULL;
+    const int e0 = V.up_off[g], e1 = V.up_off[g + 1];
+    const int l0 = V.lo_off[g], l1 = V.lo_off[g + 1];
+    for (int w = e0 >> 3; e1 > e0 && w <= (e1 - 1) >> 3; w++) {
+        unsigned long long bits = flag_word(B.pfl, w, e0, e1, want);
+        while (bits) {
+            const int byte = (__ffsll((long long)bits) - 1) >> 3;
+            const unsigned f = (unsigned)(bits >> (8 * byte)) & 0xffu;
+            bits &= ~(0xffULL << (8 * byte));
+            const int e = (w << 3) + byte;
+            if (f & PF_REC) {
+                const float4 r0 = B.rec[2 * (size_t)e];
+                fcx += r0.x; fcy += r0.y; mc += r0.z;
+                if (shel) {
+                    const float4 r1 = B.rec[2 * (size_t)e + 1];
+                    sca = fminf(sca, r1.x); scw = fminf(scw, r1.y);
+                }
+                if (f & PF_REX) { const float o = B.rx[e].x; rex = (rex + o) + rex * o; }
+            }
+            if (f & PF_DG) { add4(q0, B.pdg[2 * (size_t)e]); add4(q1, B.pdg[2 * (size_t)e + 1]); }
+        }
+    }
+    for (int w = l0 >> 3; l1 > l0 && w <= (l1 - 1) >> 3; w++) {
+        unsigned long long bits = flag_word(B.lfl, w, l0, l1, want);
+        while (bits) {
+            const int byte = (__ffsll((long long)bits) - 1) >> 3;
+            const unsigned f = (unsigned)(bits >> (8 * byte)) & 0xffu;
+            bits &= ~(0xffULL << (8 * byte));
+            const int p = V.ent_lo[(w << 3) + byte].y;
+            if (f & PF_REC) {
+                const float4 r0 = B.rec[2 * (size_t)p];
+                fcx -= r0.x; fcy -= r0.y; mc += r0.w;
+                if (shel) {
+                    const float4 r1 = B.rec[2 * (size_t)p + 1];
+                    sca = fminf(sca, r1.z); scw = fminf(scw, r1.w);
+                }
+                if (f & PF_REX) { const float o = B.rx[p].y; rex = (rex + o) + rex * o; }
+            }
+            if (f & PF_DG) { add4(q0, B.pdg[2 * (size_t)p]); add4(q1, B.pdg[2 * (size_t)p + 1]); }
+        }
+    }
+    for (int k = B.bfo[g]; k < B.bfo[g + 1]; k++) {
+        const float4 rb = B.brec[k];
+        fbx += rb.x; fby += rb.y; mb += rb.z;
+        if (diag) {
+            const float4 d0 = B.bdg[2 * (size_t)k], d1 = B.bdg[2 * (size_t)k + 1];
+            tab += d0.x; pbs += d0.y; q0.z += d0.z; q0.w += d0.w; q1.x += d1.x; q1.y += d1.y;
+        }
+    }
+    F.fcx = fcx; F.fcy = fcy; F.mc = mc; F.fbx = fbx; F.fby = fby; F.mb = mb;
+    F.sca = sca; F.scw = scw; F.rex = rex;
+    if (DIAG) {
+        F.tac = q0.x; F.pc = q0.y; F.tab = tab; F.pb = pbs;
+        F.sxx = q0.z; F.syy = q0.w; F.sxy = q1.x; F.syx = q1.y;
+    }
+}
+
 // Per floe: the sums of its flagged pair records (own row, partner row) and
 // of its bond records, in that order, FP32.  Few registers, so that many
 // floes' dependent loads are in flight at once.
@@ -801,78 +892,135 @@ template <bool DIAG>
 __global__ void __launch_bounds__(256, 8) k_floe_sums(Views V, MixedBufs B)
 {
     step_kernel_entry();
-    constexpr bool diag = DIAG;
     // the work list of the next step starts empty (the pair kernels of this
     // step have completed)
     if (blockIdx.x == 0 && threadIdx.x == 0) *B.nwork = 0;
     if (*(volatile int *)V.status & ST_ABORT) return;
     const int stride = gridDim.x * blockDim.x;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < V.N; g += stride) {
-        const bool shel = V.P[V.inst[g]].shelter != 0;
-        // contact and bond sums (FP32) in the order: own row, partner row,
-        // own bonds, partner bonds
-        float fcx = 0.f, fcy = 0.f, mc = 0.f, fbx = 0.f, fby = 0.f, mb = 0.f;
-        float sca = 1.f, scw = 1.f, rex = 0.f;
-        float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = make_float4(0.f, 0.f, 0.f, 0.f);   // tac pc sxx syy | sxy syx
-        float tab = 0.f, pbs = 0.f;
-        // flag bytes are read eight at a time; most pairs leave no record
-        const unsigned long long want = diag ? 0x0e0e0e0e0e0e0e0eULL : 0x0a0a0a0a0a0a0a0aULL;
-        const int e0 = V.up_off[g], e1 = V.up_off[g + 1];
-        const int l0 = V.lo_off[g], l1 = V.lo_off[g + 1];
-        for (int w = e0 >> 3; e1 > e0 && w <= (e1 - 1) >> 3; w++) {
-            unsigned long long bits = flag_word(B.pfl, w, e0, e1, want);
-            while (bits) {
-                const int byte = (__ffsll((long long)bits) - 1) >> 3;
-                const unsigned f = (unsigned)(bits >> (8 * byte)) & 0xffu;
-                bits &= ~(0xffULL << (8 * byte));
-                const int e = (w << 3) + byte;
-                if (f & PF_REC) {
-                    const float4 r0 = B.rec[2 * (size_t)e];
-                    fcx += r0.x; fcy += r0.y; mc += r0.z;
-                    if (shel) {
-                        const float4 r1 = B.rec[2 * (size_t)e + 1];
-                        sca = fminf(sca, r1.x); scw = fminf(scw, r1.y);
-                    }
-                    if (f & PF_REX) { const float o = B.rx[e].x; rex = (rex + o) + rex * o; }
-                }
-                if (f & PF_DG) { add4(q0, B.pdg[2 * (size_t)e]); add4(q1, B.pdg[2 * (size_t)e + 1]); }
-            }
-        }
-        for (int w = l0 >> 3; l1 > l0 && w <= (l1 - 1) >> 3; w++) {
-            unsigned long long bits = flag_word(B.lfl, w, l0, l1, want);
-            while (bits) {
-                const int byte = (__ffsll((long long)bits) - 1) >> 3;
-                const unsigned f = (unsigned)(bits >> (8 * byte)) & 0xffu;
-                bits &= ~(0xffULL << (8 * byte));
-                const int p = V.ent_lo[(w << 3) + byte].y;
-                if (f & PF_REC) {
-                    const float4 r0 = B.rec[2 * (size_t)p];
-                    fcx -= r0.x; fcy -= r0.y; mc += r0.w;
-                    if (shel) {
-                        const float4 r1 = B.rec[2 * (size_t)p + 1];
-                        sca = fminf(sca, r1.z); scw = fminf(scw, r1.w);
-                    }
-                    if (f & PF_REX) { const float o = B.rx[p].y; rex = (rex + o) + rex * o; }
-                }
-                if (f & PF_DG) { add4(q0, B.pdg[2 * (size_t)p]); add4(q1, B.pdg[2 * (size_t)p + 1]); }
-            }
-        }
-        for (int k = B.bfo[g]; k < B.bfo[g + 1]; k++) {
-            const float4 rb = B.brec[k];
-            fbx += rb.x; fby += rb.y; mb += rb.z;
-            if (diag) {
-                const float4 d0 = B.bdg[2 * (size_t)k], d1 = B.bdg[2 * (size_t)k + 1];
-                tab += d0.x; pbs += d0.y; q0.z += d0.z; q0.w += d0.w; q1.x += d1.x; q1.y += d1.y;
-            }
-        }
-        B.fsum[2 * (size_t)g] = make_float4(fcx, fcy, mc, fbx);
-        B.fsum[2 * (size_t)g + 1] = make_float4(fby, mb, sca, scw);
-        B.frex[g] = rex;
-        if (diag) {
-            B.fdg[2 * (size_t)g] = make_float4(q0.x, q0.y, tab, pbs);
-            B.fdg[2 * (size_t)g + 1] = make_float4(q0.z, q0.w, q1.x, q1.y);
+        FloeSum32 F;
+        floe_sum<DIAG>(V, B, g, F);
+        B.fsum[2 * (size_t)g] = make_float4(F.fcx, F.fcy, F.mc, F.fbx);
+        B.fsum[2 * (size_t)g + 1] = make_float4(F.fby, F.mb, F.sca, F.scw);
+        B.frex[g] = F.rex;
+        if (DIAG) {
+            B.fdg[2 * (size_t)g] = make_float4(F.tac, F.pc, F.tab, F.pb);
+            B.fdg[2 * (size_t)g + 1] = make_float4(F.sxx, F.syy, F.sxy, F.syx);
         }
     }
+}
+
+// The largest squared step of a warp's floes, which the next step's
+// screening adds to its bound: one atomic per warp, and only where it raises
+// the maximum.
+GD_DEV void raise_step(unsigned dmx, unsigned *top)
+{
+    const unsigned am = __activemask();
+    const unsigned wm = __reduce_max_sync(am, dmx);
+    if ((int)(threadIdx.x & 31) == __ffs(am) - 1 && wm > __ldcg(top)) atomicMax(top, wm);
+}
+
+// Floe g of step sic of a chunk (base: the chunk's first global step number,
+// -1: in device memory): walls, ridging, drag, Coriolis and the FP64 update
+// from its sums.  drag: its drag and Coriolis terms computed ahead with its
+// start-of-step shape (null: none), taken if no event changed the shape.
+// Returns its squared step (FP32 bits, rounded up).
+template <bool DIAG, bool WALLS>
+GD_DEV unsigned floe_update(const Views &V, int cur, int base, int sic, int g, const FloeSum32 &F, const float4 *drag)
+{
+    const int nxt = cur ^ 1;
+    const int ig = V.inst[g];
+    const InstParams &P = V.P[ig];
+    const bool px = P.boundary & BC_PERIODIC_X, py = P.boundary & BC_PERIODIC_Y;
+    const bool shel = P.shelter != 0;
+    const bool walls = WALLS && has_walls(P.boundary);
+    const float rex = F.rex;
+    const float fcx = F.fcx, fcy = F.fcy, mc = F.mc, fbx = F.fbx, fby = F.fby, mb = F.mb;
+    const float sca = F.sca, scw = F.scw;
+    const double x = V.x[cur][g], y = V.y[cur][g], th = V.th[cur][g];
+    const double u = V.u[cur][g], v = V.v[cur][g], om = V.om[cur][g];
+    const double r = V.r[cur][g], h = V.h[cur][g];
+    double dtb1 = 0.0, dtb2 = 0.0, thb1 = 0.0, thb2 = 0.0;
+    if (walls) {
+        dtb1 = V.dtb1[cur][g]; dtb2 = V.dtb2[cur][g];
+        thb1 = V.thb1[cur][g]; thb2 = V.thb2[cur][g];
+    }
+    // ridging of this floe's pairs (volume pi r^2 h kept)
+    Shape run = shape_mixed(P, r, h);
+    if (rex != 0.f) {
+        const double h1 = h + h * (double)rex;
+        run = shape_mixed(P, r * sqrt(h / h1), h1);
+    }
+    WallOut W;
+    int wev = 0;
+    if (walls) {
+        verify_bc(P, x, y, u, v, om, run, dtb1, dtb2, thb1, thb2, W, wev);
+    } else {
+        W.fx_bc = W.fy_bc = W.m_bc = 0.0;
+        W.sxx = W.syy = W.sxy = W.syx = 0.0;
+        W.ta_bc = W.p_bc = 0.0;
+    }
+    Drag<float> D;
+    if (drag && rex == 0.f && wev == 0) {
+        const float4 d0 = drag[2 * (size_t)g], d1 = drag[2 * (size_t)g + 1];
+        D.fax = d0.x; D.fay = d0.y; D.fwx = d0.z; D.fwy = d0.w;
+        D.ma = d1.x; D.mw = d1.y; D.fcorx = d1.z; D.fcory = d1.w;
+    } else {
+        double ua, va, uw, vw;
+        wind_at(P, V.field, x, y, ua, va, uw, vw);
+        D = forcing<float>(P, run, u, v, om, ua, va, uw, vw, shel ? sca : 0.f, shel ? scw : 0.f);
+    }
+    const double fax = D.fax, fay = D.fay, fwx = D.fwx, fwy = D.fwy;
+    const double tfx = (((((double)fcx + (double)fbx) + fax) + fwx) + (double)D.fcorx) + W.fx_bc;
+    const double tfy = (((((double)fcy + (double)fby) + fay) + fwy) + (double)D.fcory) + W.fy_bc;
+    const double mt = ((((double)mc + (double)mb) + (double)D.ma) + (double)D.mw) + W.m_bc;
+    const double dt = P.dt;
+    // FP64 update, the divisions by mass and inertia as two reciprocals
+    const double inv_m = 1.0 / run.mass, inv_i = 1.0 / run.inertia;
+    const double u1 = u + (tfx * inv_m) * dt;
+    const double v1 = v + (tfy * inv_m) * dt;
+    const double om1 = om + (mt * inv_i) * dt;
+    double x1 = x + u1 * dt;
+    double y1 = y + v1 * dt;
+    const double th1 = th + om1 * dt;
+    if (px) { if (x1 < 0.0) x1 = x1 + P.nx; else if (x1 >= P.nx) x1 = x1 - P.nx; }
+    if (py) { if (y1 < 0.0) y1 = y1 + P.ny; else if (y1 >= P.ny) y1 = y1 - P.ny; }
+    V.x[nxt][g] = x1; V.y[nxt][g] = y1; V.th[nxt][g] = th1;
+    V.u[nxt][g] = u1; V.v[nxt][g] = v1; V.om[nxt][g] = om1;
+    V.r[nxt][g] = run.r; V.h[nxt][g] = run.h;
+    if (walls) {
+        V.dtb1[nxt][g] = dtb1; V.dtb2[nxt][g] = dtb2;
+        V.thb1[nxt][g] = thb1; V.thb2[nxt][g] = thb2;
+    }
+    V.snap[nxt][g] = pack_snap(x1, y1, run, u1, v1, om1, ig);
+    const double ddx = wrap_d(x1 - V.x0[cur][g], P.nx, px), ddy = wrap_d(y1 - V.y0[cur][g], P.ny, py);
+    const double half = 0.5 * P.skin;
+    if (ddx * ddx + ddy * ddy > half * half) {
+        atomicOr(V.status, ST_EXPIRED);
+        atomicMin(V.expired_at, base >= 0 ? base + sic : global_step(V, sic));
+    }
+    const double sdx = wrap_d(x1 - x, P.nx, px), sdy = wrap_d(y1 - y, P.ny, py);
+    const unsigned moved = __float_as_uint(__double2float_ru(sdx * sdx + sdy * sdy));
+    if (!(isfinite(x1) && isfinite(y1) && isfinite(u1) && isfinite(v1) && isfinite(om1) && isfinite(th1)))
+        atomicOr(V.status, ST_NAN);
+    if (DIAG) {
+        const size_t N = (size_t)V.N;
+        const double rr = run.r;
+        const double tac = F.tac;
+        const double pa = tac != 0.0 ? (double)F.pc / tac : 0.0;
+        const double pbv = F.tab != 0.f ? (double)F.pb / (double)F.tab : 0.0;
+        const double pw = W.ta_bc != 0.0 ? W.p_bc / W.ta_bc : 0.0;
+        double *D0 = V.diag;
+        D0[0 * N + g] = tfx; D0[1 * N + g] = tfy; D0[2 * N + g] = fcx; D0[3 * N + g] = fcy;
+        D0[4 * N + g] = fbx; D0[5 * N + g] = fby; D0[6 * N + g] = mt; D0[7 * N + g] = mc;
+        D0[8 * N + g] = mb;
+        D0[9 * N + g] = ((double)F.sxx + W.sxx) + (fax + fwx) * rr;
+        D0[10 * N + g] = ((double)F.syy + W.syy) + (fay + fwy) * rr;
+        D0[11 * N + g] = ((double)F.sxy + W.sxy) + 0.0;
+        D0[12 * N + g] = ((double)F.syx + W.syx) + 0.0;
+        D0[13 * N + g] = (pa + pbv) + pw;
+    }
+    return moved;
 }
 
 // Per floe: walls, ridging, drag, Coriolis and the FP64 update from the
@@ -884,103 +1032,316 @@ template <bool DIAG, bool WALLS>
 __global__ void __launch_bounds__(256, WALLS ? 2 : 4) k_floes_mixed(Views V, int cur, int sic, MixedBufs B)
 {
     step_kernel_entry();
-    if (floe_update_stopped(V, sic)) return;
-    const int nxt = cur ^ 1;
+    if (floe_update_stopped(V, -1, sic)) return;
     const int stride = gridDim.x * blockDim.x;
     unsigned dmx = 0;      // largest squared step of this thread's floes (FP32 bits)
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < V.N; g += stride) {
-        const int ig = V.inst[g];
-        const InstParams &P = V.P[ig];
-        const bool px = P.boundary & BC_PERIODIC_X, py = P.boundary & BC_PERIODIC_Y;
-        const bool shel = P.shelter != 0;
-        const bool walls = WALLS && has_walls(P.boundary);
+        FloeSum32 F;
         const float4 s0 = B.fsum[2 * (size_t)g], s1 = B.fsum[2 * (size_t)g + 1];
-        const float rex = B.frex[g];
-        const float fcx = s0.x, fcy = s0.y, mc = s0.z, fbx = s0.w, fby = s1.x, mb = s1.y;
-        const float sca = s1.z, scw = s1.w;
-        const double x = V.x[cur][g], y = V.y[cur][g], th = V.th[cur][g];
-        const double u = V.u[cur][g], v = V.v[cur][g], om = V.om[cur][g];
-        const double r = V.r[cur][g], h = V.h[cur][g];
-        double dtb1 = 0.0, dtb2 = 0.0, thb1 = 0.0, thb2 = 0.0;
-        if (walls) {
-            dtb1 = V.dtb1[cur][g]; dtb2 = V.dtb2[cur][g];
-            thb1 = V.thb1[cur][g]; thb2 = V.thb2[cur][g];
-        }
-        // ridging of this floe's pairs (volume pi r^2 h kept)
-        Shape run = shape_mixed(P, r, h);
-        if (rex != 0.f) {
-            const double h1 = h + h * (double)rex;
-            run = shape_mixed(P, r * sqrt(h / h1), h1);
-        }
-        WallOut W;
-        int wev = 0;
-        if (walls) {
-            verify_bc(P, x, y, u, v, om, run, dtb1, dtb2, thb1, thb2, W, wev);
-        } else {
-            W.fx_bc = W.fy_bc = W.m_bc = 0.0;
-            W.sxx = W.syy = W.sxy = W.syx = 0.0;
-            W.ta_bc = W.p_bc = 0.0;
-        }
-        double ua, va, uw, vw;
-        wind_at(P, V.field, x, y, ua, va, uw, vw);
-        const Drag<float> D = forcing<float>(P, run, u, v, om, ua, va, uw, vw, shel ? sca : 0.f, shel ? scw : 0.f);
-        const double fax = D.fax, fay = D.fay, fwx = D.fwx, fwy = D.fwy;
-        const double tfx = (((((double)fcx + (double)fbx) + fax) + fwx) + (double)D.fcorx) + W.fx_bc;
-        const double tfy = (((((double)fcy + (double)fby) + fay) + fwy) + (double)D.fcory) + W.fy_bc;
-        const double mt = ((((double)mc + (double)mb) + (double)D.ma) + (double)D.mw) + W.m_bc;
-        const double dt = P.dt;
-        // FP64 update, the divisions by mass and inertia as two reciprocals
-        const double inv_m = 1.0 / run.mass, inv_i = 1.0 / run.inertia;
-        const double u1 = u + (tfx * inv_m) * dt;
-        const double v1 = v + (tfy * inv_m) * dt;
-        const double om1 = om + (mt * inv_i) * dt;
-        double x1 = x + u1 * dt;
-        double y1 = y + v1 * dt;
-        const double th1 = th + om1 * dt;
-        if (px) { if (x1 < 0.0) x1 = x1 + P.nx; else if (x1 >= P.nx) x1 = x1 - P.nx; }
-        if (py) { if (y1 < 0.0) y1 = y1 + P.ny; else if (y1 >= P.ny) y1 = y1 - P.ny; }
-        V.x[nxt][g] = x1; V.y[nxt][g] = y1; V.th[nxt][g] = th1;
-        V.u[nxt][g] = u1; V.v[nxt][g] = v1; V.om[nxt][g] = om1;
-        V.r[nxt][g] = run.r; V.h[nxt][g] = run.h;
-        if (walls) {
-            V.dtb1[nxt][g] = dtb1; V.dtb2[nxt][g] = dtb2;
-            V.thb1[nxt][g] = thb1; V.thb2[nxt][g] = thb2;
-        }
-        V.snap[nxt][g] = pack_snap(x1, y1, run, u1, v1, om1, ig);
-        const double ddx = wrap_d(x1 - V.x0[cur][g], P.nx, px), ddy = wrap_d(y1 - V.y0[cur][g], P.ny, py);
-        const double half = 0.5 * P.skin;
-        if (ddx * ddx + ddy * ddy > half * half) {
-            atomicOr(V.status, ST_EXPIRED);
-            atomicMin(V.expired_at, global_step(V, sic));
-        }
-        const double sdx = wrap_d(x1 - x, P.nx, px), sdy = wrap_d(y1 - y, P.ny, py);
-        dmx = max(dmx, __float_as_uint(__double2float_ru(sdx * sdx + sdy * sdy)));
-        if (!(isfinite(x1) && isfinite(y1) && isfinite(u1) && isfinite(v1) && isfinite(om1) && isfinite(th1)))
-            atomicOr(V.status, ST_NAN);
+        F.fcx = s0.x; F.fcy = s0.y; F.mc = s0.z; F.fbx = s0.w; F.fby = s1.x; F.mb = s1.y;
+        F.sca = s1.z; F.scw = s1.w;
+        F.rex = B.frex[g];
         if (DIAG) {
-            const float4 d0 = B.fdg[2 * (size_t)g], d1 = B.fdg[2 * (size_t)g + 1];   // tac pc tab pb | sxx syy sxy syx
-            const size_t N = (size_t)V.N;
-            const double rr = run.r;
-            const double tac = d0.x;
-            const double pa = tac != 0.0 ? (double)d0.y / tac : 0.0;
-            const double pbv = d0.z != 0.f ? (double)d0.w / (double)d0.z : 0.0;
-            const double pw = W.ta_bc != 0.0 ? W.p_bc / W.ta_bc : 0.0;
-            double *D0 = V.diag;
-            D0[0 * N + g] = tfx; D0[1 * N + g] = tfy; D0[2 * N + g] = fcx; D0[3 * N + g] = fcy;
-            D0[4 * N + g] = fbx; D0[5 * N + g] = fby; D0[6 * N + g] = mt; D0[7 * N + g] = mc;
-            D0[8 * N + g] = mb;
-            D0[9 * N + g] = ((double)d1.x + W.sxx) + (fax + fwx) * rr;
-            D0[10 * N + g] = ((double)d1.y + W.syy) + (fay + fwy) * rr;
-            D0[11 * N + g] = ((double)d1.z + W.sxy) + 0.0;
-            D0[12 * N + g] = ((double)d1.w + W.syx) + 0.0;
-            D0[13 * N + g] = (pa + pbv) + pw;
+            const float4 d0 = B.fdg[2 * (size_t)g], d1 = B.fdg[2 * (size_t)g + 1];
+            F.tac = d0.x; F.pc = d0.y; F.tab = d0.z; F.pb = d0.w;
+            F.sxx = d1.x; F.syy = d1.y; F.sxy = d1.z; F.syx = d1.w;
+        }
+        dmx = max(dmx, floe_update<DIAG, WALLS>(V, cur, -1, sic, g, F, nullptr));
+    }
+    raise_step(dmx, B.dsp + cur);
+}
+
+// Enough blocks for two full waves at any block size (148 SMs x 2048
+// threads), so that small blocks do not cap the resident warps; the kernels
+// stride over the rest.
+static int grid_of(long long n, int block)
+{
+    return (int)std::max(1LL, std::min<long long>((n + block - 1) / block, 148LL * (4096 / block)));
+}
+
+// ---------------------------------------------------------------- small batches
+// k_steps_mixed: a chunk of K whole steps of a small batch in one launch of
+// one cluster (or one block), as k_steps_fp64 does for the FP64 path: the
+// screen's test and the pair physics in one pass, beside the bonds and the
+// drag and Coriolis terms of every floe; a cluster barrier; the sums and the
+// update of every floe; a cluster barrier.  Where a field of the batch has
+// ridging the bonds follow the pairs (an event tells the bond the pair's new
+// radius), behind a third barrier.
+struct SmallArgs32 {
+    int cur, K, diag_last, base;   // first side, steps, diagnostics on the last one, global number of the first
+    int n, E, NB, ridging;         // contact-list items, owner entries, bonds
+    int2 *eb;
+    const int2 *stl;
+    const unsigned *erow;
+    unsigned char *bfl;            // live-bond flags of both sides
+    float4 *drag;                  // [2N]
+    int *out;                      // pinned host memory: the status word and the first expired step
+    int *done;                     // blocks of k_step_floes_mixed that have finished
+};
+
+GD_DEV void small_pairs32(const Views &V, const SmallArgs32 &A, const MixedBufs &B, int cur, int diag,
+                          int first, int nthr)
+{
+    const Snap *S = V.snap[cur];
+    Hist4<float> *Hh = (Hist4<float> *)V.hist[0];
+    const float Dk = advance_bound(cur, B);
+    const float thr = __fadd_ru(2.f * Dk, 1e-6f);
+    const int n = diag ? A.E : A.n;
+    // the bonds, unless they follow the pairs, and the floes start on warps
+    // of their own
+    const int n0 = (n + 31) & ~31;
+    const int n1 = n0 + (A.ridging ? 0 : (A.NB + 31) & ~31);
+    unsigned long long n_cand = 0, n_cont = 0, n_plast = 0, n_bond = 0;
+    for (int i = first; i < n1 + V.N; i += nthr) {
+        if (i < n) {
+            int e = i, s, t;
+            if (diag) {
+                s = (int)A.erow[e];
+                t = V.ent_up[e].x;
+            } else {
+                const int2 c = A.eb[i];
+                if (__int_as_float(c.y) > thr) continue;
+                e = c.x;
+                const int2 st = A.stl[i];
+                s = st.x;
+                t = st.y;
+                if (!screen_test(V, S, A.eb, i, c, st, (unsigned)B.pfl[e], Dk, B)) continue;
+            }
+            pair_mixed(V, S, Hh, diag, e, s, t, B, n_cand, n_cont, n_plast);
+        } else if (i >= n0 && i - n0 < A.NB && i < n1) {
+            const int b = i - n0;
+            n_bond += bond_step(V, S, diag, b, B.bsp[b], B.wdyn[b], B.bst[b], B.brec, B.bdg, B.bfl_wr, B.wdyn);
+        } else if (i >= n1) {
+            const int g = i - n1;
+            const InstParams &P = V.P[V.inst[g]];
+            if (P.shelter != 0) continue;
+            double ua, va, uw, vw;
+            wind_at(P, V.field, V.x[cur][g], V.y[cur][g], ua, va, uw, vw);
+            const Drag<float> D = forcing<float>(P, shape_mixed(P, V.r[cur][g], V.h[cur][g]), V.u[cur][g],
+                                                 V.v[cur][g], V.om[cur][g], ua, va, uw, vw, 0.f, 0.f);
+            A.drag[2 * (size_t)g] = make_float4(D.fax, D.fay, D.fwx, D.fwy);
+            A.drag[2 * (size_t)g + 1] = make_float4(D.ma, D.mw, D.fcorx, D.fcory);
         }
     }
-    // the largest step, which the next step's screening adds to its bound:
-    // one atomic per warp, and only where it raises the maximum
-    const unsigned am = __activemask();
-    const unsigned wm = __reduce_max_sync(am, dmx);
-    if ((int)(threadIdx.x & 31) == __ffs(am) - 1 && wm > __ldcg(B.dsp + cur)) atomicMax(B.dsp + cur, wm);
+    __syncwarp();
+    if (diag) {
+        warp_count(n_cand, V.counters, 0);
+        warp_count(n_cont, V.counters, 1);
+        warp_count(n_bond, V.counters, 2);
+        warp_count(n_plast, V.counters, 3);
+    }
+}
+
+// The sums of one floe on a plain step by a group of GRP lanes (see
+// group_sums64): entries, flags, records and bond records are loaded side by
+// side, and what adds to a sum is handed round in floe_sum's order, so every
+// lane of the group holds the same sums.  A record of zeros (a sheltered pair
+// out of contact) leaves every sum as it is; a shelter factor lowers a
+// minimum, in any order.  on: whether this group has a floe; every lane of
+// the warp calls.
+GD_DEV float shfl_grp(float v, int src) { return __shfl_sync(0xffffffffu, v, src, GRP); }
+
+GD_DEV void group_sum32(const Views &V, const MixedBufs &B, bool on, int g, FloeSum32 &F)
+{
+    const int lane = threadIdx.x & 31, sub = lane & (GRP - 1);
+    const bool shel = on && V.P[V.inst[g]].shelter != 0;
+    F.fcx = F.fcy = F.mc = F.fbx = F.fby = F.mb = 0.f;
+    F.sca = F.scw = 1.f;
+    F.rex = 0.f;
+    const int k0 = on ? B.bfo[g] : 0, k1 = on ? B.bfo[g + 1] : 0;
+#pragma unroll
+    for (int side = 0; side < 2; side++) {
+        const int *off = side ? V.lo_off : V.up_off;
+        const unsigned char *fl = side ? B.lfl : B.pfl;
+        const int e0 = on ? off[g] : 0, e1 = on ? off[g + 1] : 0;
+        for (int b = e0; __any_sync(0xffffffffu, b < e1); b += GRP) {
+            const int e = b + sub;
+            unsigned f = e < e1 ? fl[e] : 0u;
+            int p = e;
+            float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (f & PF_REC) {
+                if (side) p = V.ent_lo[e].y;
+                r0 = B.rec[2 * (size_t)p];
+                if (shel) {
+                    const float4 r1 = B.rec[2 * (size_t)p + 1];
+                    F.sca = fminf(F.sca, side ? r1.z : r1.x);
+                    F.scw = fminf(F.scw, side ? r1.w : r1.y);
+                }
+            }
+            const bool add = (f & PF_REX) || r0.x != 0.f || r0.y != 0.f || r0.z != 0.f || r0.w != 0.f;
+            unsigned left = __ballot_sync(0xffffffffu, add) >> (lane & ~(GRP - 1)) & ((1u << GRP) - 1u);
+            while (__any_sync(0xffffffffu, left != 0)) {
+                const int j = left ? __ffs(left) - 1 : 0;
+                const float x = shfl_grp(r0.x, j), y = shfl_grp(r0.y, j);
+                const float m = shfl_grp(side ? r0.w : r0.z, j);
+                const unsigned fj = __shfl_sync(0xffffffffu, f, j, GRP);
+                const int pj = __shfl_sync(0xffffffffu, p, j, GRP);
+                if (left) {
+                    if (side) { F.fcx -= x; F.fcy -= y; } else { F.fcx += x; F.fcy += y; }
+                    F.mc += m;
+                    if (fj & PF_REX) {
+                        const float2 rx = B.rx[pj];
+                        const float o = side ? rx.y : rx.x;
+                        F.rex = (F.rex + o) + F.rex * o;
+                    }
+                    left &= left - 1;
+                }
+            }
+        }
+    }
+    for (int b = k0; __any_sync(0xffffffffu, b < k1); b += GRP) {
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (b + sub < k1) q = B.brec[b + sub];
+        for (int j = 0; j < GRP && __any_sync(0xffffffffu, b + j < k1); j++) {
+            const float x = shfl_grp(q.x, j), y = shfl_grp(q.y, j), m = shfl_grp(q.z, j);
+            if (b + j < k1) { F.fbx += x; F.fby += y; F.mb += m; }
+        }
+    }
+#pragma unroll
+    for (int o = GRP / 2; o > 0; o >>= 1) {
+        F.sca = fminf(F.sca, __shfl_xor_sync(0xffffffffu, F.sca, o));
+        F.scw = fminf(F.scw, __shfl_xor_sync(0xffffffffu, F.scw, o));
+    }
+}
+
+// The floes' sums and update, one thread per floe.
+template <bool DIAG>
+GD_DEV void small_floes32(const Views &V, const SmallArgs32 &A, const MixedBufs &B, int cur, int sic)
+{
+    const int nthr = gridDim.x * blockDim.x;
+    unsigned dmx = 0;
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < V.N; g += nthr) {
+        FloeSum32 F;
+        floe_sum<DIAG>(V, B, g, F);
+        const bool shel = V.P[V.inst[g]].shelter != 0;
+        dmx = max(dmx, floe_update<DIAG, true>(V, cur, A.base, sic, g, F, shel ? nullptr : A.drag));
+    }
+    __syncwarp();
+    raise_step(dmx, B.dsp + cur);
+}
+
+__global__ void __launch_bounds__(SMALL_THREADS, 1) k_steps_mixed(Views V, SmallArgs32 A, MixedBufs B)
+{
+    step_kernel_entry();
+    const int first = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
+    for (int k = 0; k < A.K; k++) {
+        // the same answer in every thread: the status is written between the
+        // last two barriers of a step only
+        if (*(volatile int *)V.status & ST_ABORT) break;
+        const int cur = A.cur ^ (k & 1);
+        const int diag = A.diag_last && k == A.K - 1;
+        B.bfl_rd = A.bfl + (size_t)cur * A.NB;
+        B.bfl_wr = A.bfl + (size_t)(cur ^ 1) * A.NB;
+        small_pairs32(V, A, B, cur, diag, first, nthr);
+        cluster_sync();
+        if (A.ridging && A.NB > 0) {
+            unsigned long long n_bond = 0;
+            for (int b = first; b < A.NB; b += nthr)
+                n_bond += bond_step(V, V.snap[cur], diag, b, B.bsp[b], B.wdyn[b], B.bst[b], B.brec, B.bdg, B.bfl_wr,
+                                    B.wdyn);
+            __syncwarp();
+            if (diag) warp_count(n_bond, V.counters, 2);
+            cluster_sync();
+        }
+        if (diag) small_floes32<true>(V, A, B, cur, k);
+        else small_floes32<false>(V, A, B, cur, k);
+        cluster_sync();
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) publish_status(V, A.out);
+}
+
+// The two halves of a step as ordinary grids, for batches with more work
+// than one cluster does quickly: two launches a step instead of five (three
+// where the bonds follow the pairs).  The last one of a chunk's last step
+// publishes the status word.
+__global__ void __launch_bounds__(128) k_step_pairs_mixed(Views V, SmallArgs32 A, MixedBufs B, int cur, int diag)
+{
+    step_kernel_entry();
+    if (*(volatile int *)V.status & ST_ABORT) return;
+    small_pairs32(V, A, B, cur, diag, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
+template <bool DIAG>
+__global__ void __launch_bounds__(128) k_step_floes_mixed(Views V, SmallArgs32 A, MixedBufs B, int cur, int sic)
+{
+    step_kernel_entry();
+    if (!floe_update_stopped(V, A.base, sic)) small_floes32<DIAG>(V, A, B, cur, sic);
+    if (sic == A.K - 1) publish_status_last(V, A.done, A.out);
+}
+
+// The second half of a plain step with the floes' sums by groups of lanes
+// (k_step_floes_grp_fp64).
+__global__ void __launch_bounds__(SMALL_THREADS, 2) k_step_floes_grp_mixed(Views V, SmallArgs32 A, MixedBufs B,
+                                                                           int cur, int sic, int rounds)
+{
+    __shared__ float sum[9][SMALL_THREADS];
+    __shared__ int stopped;
+    step_kernel_entry();
+    // one answer per block: another block may raise an expiry meanwhile
+    if (threadIdx.x == 0) stopped = floe_update_stopped(V, A.base, sic);
+    __syncthreads();
+    const int grp = threadIdx.x / GRP, per = rounds * GRP_FLOES;
+    unsigned dmx = 0;
+    for (int g0 = blockIdx.x * per; !stopped && g0 < V.N; g0 += gridDim.x * per) {
+        for (int r = 0; r < rounds; r++) {
+            const int at = r * GRP_FLOES + grp;
+            const bool on = g0 + at < V.N;
+            FloeSum32 F;
+            group_sum32(V, B, on, g0 + at, F);
+            if (on && threadIdx.x % GRP == 0) {
+                sum[0][at] = F.fcx; sum[1][at] = F.fcy; sum[2][at] = F.mc;
+                sum[3][at] = F.fbx; sum[4][at] = F.fby; sum[5][at] = F.mb;
+                sum[6][at] = F.sca; sum[7][at] = F.scw; sum[8][at] = F.rex;
+            }
+        }
+        __syncthreads();
+        const int q = threadIdx.x, g = g0 + q;
+        if (q < per && g < V.N) {
+            FloeSum32 F;
+            F.fcx = sum[0][q]; F.fcy = sum[1][q]; F.mc = sum[2][q];
+            F.fbx = sum[3][q]; F.fby = sum[4][q]; F.mb = sum[5][q];
+            F.sca = sum[6][q]; F.scw = sum[7][q]; F.rex = sum[8][q];
+            const bool shel = V.P[V.inst[g]].shelter != 0;
+            dmx = max(dmx, floe_update<false, true>(V, cur, A.base, sic, g, F, shel ? nullptr : A.drag));
+        }
+        __syncthreads();
+    }
+    if (!stopped) raise_step(dmx, B.dsp + cur);
+    if (sic == A.K - 1) publish_status_last(V, A.done, A.out);
+}
+
+bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
+                        int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
+                        int *done, cudaStream_t st)
+{
+    SmallArgs32 A;
+    A.cur = cur; A.K = K; A.diag_last = diag_last; A.base = base;
+    A.n = n; A.E = E; A.NB = NB; A.ridging = ridging;
+    A.eb = eb; A.stl = stl; A.erow = erow; A.bfl = bfl;
+    A.drag = B.fsum;      // two float4 a floe: the sums stay in registers here
+    A.out = out;
+    A.done = done;
+    const long long all = (long long)n + NB + V.N;
+    if (!shelter && all <= ONE_CLUSTER_MIXED) return launch_cluster(V.pdl != 0, k_steps_mixed, all, st, V, A, B);
+    const int rounds = group_rounds(V.N, shelter);
+    for (int k = 0; k < K; k++) {
+        const int c = cur ^ (k & 1);
+        const int diag = diag_last && k == K - 1;
+        B.bfl_rd = A.bfl + (size_t)c * NB;
+        B.bfl_wr = A.bfl + (size_t)(c ^ 1) * NB;
+        const long long items = (long long)(diag ? E : n) + (ridging ? 0 : NB) + 64 + V.N;
+        launch_step(V.pdl != 0, k_step_pairs_mixed, grid_of(items, 128), 128, st, V, A, B, c, diag);
+        if (ridging && NB > 0)
+            launch_step(V.pdl != 0, k_bonds_mixed, grid_of(NB, 128), 128, st, V, c, diag, NB, B.bsp, B.bst, B.brec,
+                        B.bdg, B.bfl_wr, B.wdyn);
+        if (diag) launch_step(V.pdl != 0, k_step_floes_mixed<true>, grid_of(V.N, 64), 64, st, V, A, B, c, k);
+        else if (rounds == 0)
+            launch_step(V.pdl != 0, k_step_floes_mixed<false>, grid_of(V.N, 64), 64, st, V, A, B, c, k);
+        else
+            launch_step(V.pdl != 0, k_step_floes_grp_mixed, (V.N + rounds * GRP_FLOES - 1) / (rounds * GRP_FLOES),
+                        SMALL_THREADS, st, V, A, B, c, k, rounds);
+    }
+    return true;
 }
 
 // Row (slot) of every entry of a CSR.
@@ -1167,14 +1528,6 @@ __global__ void k_contact_fill(Views V, int side, int P, const unsigned *erow, c
         eb[pos[e]] = make_int2(e, __float_as_int(gap));
         stl[pos[e]] = make_int2(s, t);
     }
-}
-
-// Enough blocks for two full waves at any block size (148 SMs x 2048
-// threads), so that small blocks do not cap the resident warps; the kernels
-// stride over the rest.
-static int grid_of(long long n, int block)
-{
-    return (int)std::max(1LL, std::min<long long>((n + block - 1) / block, 148LL * (4096 / block)));
 }
 
 void launch_mixed_rows_init(int P, const int2 *ent_lo, const void *hist, int *lo_of, unsigned char *pfl,

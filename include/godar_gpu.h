@@ -363,8 +363,10 @@ int godar_batch_set_phase_timing(godar_batch *b, int every);
  * lane: 0 = 8, 1 = 4, 2 = 16; the bonds: 1 = records streamed through shared
  * memory by bulk copies), chosen by the online autotuner over the first steps
  * of a batch (or the block size of GODAR_BLOCK, variant 0); whether chunks of
- * steps run as captured CUDA graphs, and how many graph launches there
- * were.  Environment: GODAR_TUNE=0 disables the tuner, GODAR_TUNE_LOG=1
+ * steps run as captured CUDA graphs, and how many chunks ran as a whole (a
+ * graph launch, or on small batches the merged step kernels, which have no
+ * configuration to choose: GODAR_FUSED=0 runs the five kernels instead).
+ * Environment: GODAR_TUNE=0 disables the tuner, GODAR_TUNE_LOG=1
  * prints its measurements, GODAR_BOND_VARIANT=v fixes the bond kernel's
  * variant, GODAR_GRAPHS=0 disables the graphs; GODAR_OVERLAP_BONDS=1 runs
  * the mixed bond kernel on a second stream beside the pair kernels (batches

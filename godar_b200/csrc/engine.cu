@@ -293,6 +293,10 @@ struct Engine {
     unsigned long long counters[4] = {0, 0, 0, 0};
     bool counting = false;             // the last call launched a diagnostic step
     unsigned long long *h_counters = nullptr;   // pinned
+    // two pinned slots for read-backs (copy_out)
+    static constexpr size_t STAGE_SLOT = 128 << 10;
+    char *h_stage = nullptr;
+    cudaEvent_t stage_ev[2] = {};
     // Verlet skin = max(1 m, skin_frac (r_max + rtree)); a rebuild costs
     // about 25 ms on 2.2M floes, and 1% keeps rebuilds hundreds to thousands
     // of steps apart on the benchmark fields while shortening the rows
@@ -397,7 +401,7 @@ struct Engine {
     // outputs and status
     // status: two ints, the status word and the global number of the first
     // step that expired (INT_MAX: none), read back together after each chunk
-    Buf diag, status, counters_b, tmp_out, tmp_i, tmp_j, tmp_v, tmp_cnt;
+    Buf diag, status, counters_b, tmp_out, tmp_v, tmp_cnt;
     // pinned status mirror
     int *h_status = nullptr;
     // the global number of the next step to launch, counted from the last
@@ -440,6 +444,8 @@ struct Engine {
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (h_counters) cudaFreeHost(h_counters);
+        for (auto e : stage_ev)
+            if (e) cudaEventDestroy(e);
         for (auto e : ring_ev)
             if (e) cudaEventDestroy(e);
         for (int q = 0; q < FRING; q++) {
@@ -498,9 +504,12 @@ struct Engine {
         CK(cudaEventCreate(&ev0));
         CK(cudaEventCreate(&ev1));
         // one pinned block: the counters, the status mirror, the ring
-        CK(cudaMallocHost(&h_counters, sizeof(counters) + (4 + RING * 4) * sizeof(int)));
+        constexpr size_t small_pinned = sizeof(counters) + (4 + RING * 4) * sizeof(int);
+        CK(cudaMallocHost(&h_counters, small_pinned + 2 * STAGE_SLOT));
         h_status = (int *)(h_counters + 4);
         h_ring = h_status + 4;
+        h_stage = (char *)h_counters + small_pinned;
+        for (auto &e : stage_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         for (auto &e : ring_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         for (auto &e : fring_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         TRY(step_base_b.ensure(2 * sizeof(int), &bytes, &mp));
@@ -1951,16 +1960,76 @@ struct Engine {
         return GODAR_OK;
     }
 
-    int get_field(int handle, int field, double *out) {
-        if (!out || field < 0 || field >= GODAR_F_COUNT) { set_err("bad field"); return GODAR_ERR_BAD_INPUT; }
+    int get_field(int handle, int field, double *out) { return get_fields(handle, 1, &field, &out); }
+
+    // Fields of one instance: gathered side by side by one kernel, then copied
+    // out through the pinned slots (a kernel, a pageable copy and a wait for
+    // each of 22 fields took 20 us a field).
+    int get_fields(int handle, int nf, const int *fields, double *const *outs) {
+        for (int q = 0; q < nf; q++)
+            if (!outs[q] || fields[q] < 0 || fields[q] >= GODAR_F_COUNT) { set_err("bad field"); return GODAR_ERR_BAD_INPUT; }
         Inst *I = find(handle);
         if (!I) { set_err("unknown instance"); return GODAR_ERR_NOT_FOUND; }
         // other fields' admissions and removals wait for the next step: this
         // field's slots stay valid until then
         if (I->pending) TRY(commit());
-        launch_gather_field(views(), cur, 0, I->off, I->n, field, tmp_out.as<double>(), st);
-        CK(cudaMemcpyAsync(out, tmp_out.p, (size_t)I->n * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
+        const size_t one = (size_t)I->n * 8;
+        // as many fields at a time as 32 MB hold; the rebuild's row scratch is
+        // free between steps and mostly large enough
+        const int per = (int)std::max<size_t>(1, std::min<size_t>(24, (32u << 20) / one));
+        const size_t need = std::min(nf, per) * one;
+        double *dev = ent2.as<double>();
+        if (ent2.bytes < need) {
+            TRY(tmp_out.ensure(need, &bytes, &mp));
+            dev = tmp_out.as<double>();
+        }
+        for (int q0 = 0; q0 < nf; q0 += per) {
+            FieldList F;
+            F.n = std::min(nf - q0, per);
+            char *dst[24];
+            size_t len[24];
+            for (int q = 0; q < F.n; q++) {
+                F.code[q] = fields[q0 + q];
+                dst[q] = (char *)outs[q0 + q];
+                len[q] = one;
+            }
+            launch_gather_fields(views(), cur, I->off, I->n, F, dev, st);
+            TRY(copy_out((const char *)dev, F.n, dst, len));
+        }
+        return GODAR_OK;
+    }
+
+    // Device memory from dev on to `parts` host ranges one after the other
+    // (null: skipped), complete on return.  The copies go through two pinned
+    // slots, so that the host moves one slot to the caller while the next one
+    // fills; a copy to pageable memory would be staged by the driver, one wait
+    // a range.
+    int copy_out(const char *dev, int parts, char *const *dst, const size_t *len) {
+        size_t total = 0;
+        for (int q = 0; q < parts; q++) total += len[q];
+        const size_t chunks = (total + STAGE_SLOT - 1) / STAGE_SLOT;
+        int part = 0;
+        size_t at = 0;                       // start of `part` in the range
+        auto drain = [&](size_t c) -> int {
+            CK(cudaEventSynchronize(stage_ev[c & 1]));
+            const char *src = h_stage + (c & 1) * STAGE_SLOT;
+            size_t o = c * STAGE_SLOT;
+            const size_t end = std::min(total, o + STAGE_SLOT);
+            while (o < end) {
+                while (o >= at + len[part]) at += len[part++];
+                const size_t n = std::min(end, at + len[part]) - o;
+                if (dst[part]) std::memcpy(dst[part] + (o - at), src + (o - c * STAGE_SLOT), n);
+                o += n;
+            }
+            return GODAR_OK;
+        };
+        for (size_t c = 0; c < chunks; c++) {
+            if (c >= 2) TRY(drain(c - 2));
+            CK(cudaMemcpyAsync(h_stage + (c & 1) * STAGE_SLOT, dev + c * STAGE_SLOT,
+                               std::min(STAGE_SLOT, total - c * STAGE_SLOT), cudaMemcpyDeviceToHost, st));
+            CK(cudaEventRecord(stage_ev[c & 1], st));
+        }
+        for (size_t c = chunks > 2 ? chunks - 2 : 0; c < chunks; c++) TRY(drain(c));
         return GODAR_OK;
     }
 
@@ -2116,34 +2185,42 @@ struct Engine {
         // field's slots stay valid until then
         if (I->pending) TRY(commit());
         if (which == 2) TRY(sync_bonds());
-        // count first, then fill
-        CK(cudaMemsetAsync(tmp_cnt.p, 0, sizeof(int), st));
-        launch_list_pairs(views(), cur, 0, I->off, I->n, which, nullptr, nullptr, nullptr, 0, tmp_cnt.as<int>(), st);
-        int total = 0;
-        CK(cudaMemcpyAsync(&total, tmp_cnt.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        if (count) *count = total;
-        if (total == 0 || cap <= 0) return GODAR_OK;
-        TRY(tmp_i.ensure((size_t)total * 4, &bytes, &mp)); TRY(tmp_j.ensure((size_t)total * 4, &bytes, &mp));
-        TRY(tmp_v.ensure((size_t)total * 8, &bytes, &mp));
-        CK(cudaMemsetAsync(tmp_cnt.p, 0, sizeof(int), st));
-        launch_list_pairs(views(), cur, 0, I->off, I->n, which, tmp_i.as<int>(), tmp_j.as<int>(), tmp_v.as<double>(),
-                          total, tmp_cnt.as<int>(), st);
-        std::vector<int> hi(total), hj(total);
-        std::vector<double> hv(total);
-        CK(cudaMemcpyAsync(hi.data(), tmp_i.p, (size_t)total * 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(hj.data(), tmp_j.p, (size_t)total * 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(hv.data(), tmp_v.p, (size_t)total * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        std::vector<int> ord(total);
-        std::iota(ord.begin(), ord.end(), 0);
-        std::sort(ord.begin(), ord.end(), [&](int a, int b) { return hi[a] != hi[b] ? hi[a] < hi[b] : hj[a] < hj[b]; });
-        const int m = std::min(cap, total);
-        for (int k = 0; k < m; k++) {
-            if (pi) pi[k] = hi[ord[k]];
-            if (pj) pj[k] = hj[ord[k]];
-            if (val) val[k] = hv[ord[k]];
+        // the list's first `want` pairs in one pass; how many there are comes
+        // back beside them, or before them where they do not fit a staging slot
+        const long long bound = which == 2 ? I->nb : E;
+        int want = (int)std::max(0LL, std::min<long long>(cap, bound));
+        auto launch = [&](int m) {
+            double *v = tmp_v.as<double>();
+            int *i = (int *)(v + m);
+            launch_list_pairs(views(), cur, I->off, I->n, which, m, i, i + m, v, tmp_cnt.as<int>(), cnt.as<int>(),
+                              row_off2.as<int>(), scan_scratch.as<int>(), st);
+        };
+        int *h_total = h_status + 2;
+        if ((size_t)want * 16 > STAGE_SLOT) {
+            launch(0);
+            CK(cudaMemcpyAsync(h_total, tmp_cnt.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+            want = std::min(want, *h_total);
         }
+        TRY(tmp_v.ensure(std::max<size_t>((size_t)want * 16, 16), &bytes, &mp));
+        launch(want);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(h_total, tmp_cnt.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+        if ((size_t)want * 16 <= STAGE_SLOT) {
+            if (want > 0) CK(cudaMemcpyAsync(h_stage, tmp_v.p, (size_t)want * 16, cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+            const int m = std::min(want, *h_total);
+            const double *v = (const double *)h_stage;
+            const int *i = (const int *)(v + want);
+            if (val && m > 0) std::memcpy(val, v, (size_t)m * 8);
+            if (pi && m > 0) std::memcpy(pi, i, (size_t)m * 4);
+            if (pj && m > 0) std::memcpy(pj, i + want, (size_t)m * 4);
+        } else {
+            char *dst[3] = {(char *)val, (char *)pi, (char *)pj};
+            const size_t len[3] = {(size_t)want * 8, (size_t)want * 4, (size_t)want * 4};
+            TRY(copy_out((const char *)tmp_v.p, 3, dst, len));
+        }
+        if (count) *count = *h_total;
         return GODAR_OK;
     }
 };
@@ -2355,9 +2432,17 @@ int godar_gpu_download(godar_ctx *c, double *const *floe_out, int which, int32_t
 {
     if (!c) return GODAR_ERR_BAD_INPUT;
     if (count) *count = 0;
-    if (floe_out)
+    if (floe_out && c->handle >= 0) {
+        GODAR_CTX_RESOLVED(c);
+        int fields[GODAR_F_COUNT], nf = 0;
+        double *outs[GODAR_F_COUNT];
+        for (int f = 0; f < GODAR_F_COUNT; f++)
+            if (floe_out[f]) { fields[nf] = f; outs[nf++] = floe_out[f]; }
+        TRY(c->eng.get_fields(c->handle, nf, fields, outs));
+    } else if (floe_out) {
         for (int f = 0; f < GODAR_F_COUNT; f++)
             if (floe_out[f]) TRY(godar_gpu_get_floe_field(c, f, floe_out[f]));
+    }
     if (which >= 0) TRY(godar_gpu_get_pairs(c, which, pair_i, pair_j, pair_val, cap, count));
     return GODAR_OK;
 }

@@ -184,10 +184,17 @@ void launch_hist_inject(const Views &V, int cur, int off, int nh, const int *pi,
 // histories deltat_bc1, deltat_bc2, theta_bc1, theta_bc2.
 constexpr int GATHER_DTB1 = 100;
 void launch_gather_field(const Views &V, int cur, int inst, int off, int n, int field, double *out, cudaStream_t st);
+// Several fields of the instance at slots [off, off + n) in id order, field q
+// at out + q n.
+struct FieldList { int n; int code[24]; };
+void launch_gather_fields(const Views &V, int cur, int off, int n, const FieldList &F, double *out, cudaStream_t st);
 // Per instance: momentum x, y, kinetic energy, largest speed (4 doubles).
 void launch_instance_summary(const Views &V, int cur, double *out, cudaStream_t st);
-void launch_list_pairs(const Views &V, int cur, int inst, int off, int n, int which, int *pi, int *pj,
-                       double *val, int cap, int *count, cudaStream_t st);
+// A pair list (0 candidates, 1 contacts, 2 live bonds) of the instance at
+// slots [off, off + n), ascending in (i, j): its first cap pairs and, in
+// total, its length.  cnt, base: n + 1 ints each.
+void launch_list_pairs(const Views &V, int cur, int off, int n, int which, int cap, int *pi, int *pj, double *val,
+                       int *total, int *cnt, int *base, int *scan_scratch, cudaStream_t st);
 
 // Batch relayout (membership changes).
 void launch_gather_floes(const Views &Vo, int so, const Views &Vn, int sn, const int *repack, int n, cudaStream_t st);

@@ -6,60 +6,169 @@
 
 namespace godar {
 
+// One value of the state (field codes GODAR_F_*, GATHER_DTB1 ..) or of the
+// last diagnostic step.
+GD_DEV double field_value(const Views &V, int cur, int s, int field)
+{
+    switch (field) {
+    case 0: return V.x[cur][s];
+    case 1: return V.y[cur][s];
+    case 2: return V.u[cur][s];
+    case 3: return V.v[cur][s];
+    case 4: return V.r[cur][s];
+    case 5: return V.h[cur][s];
+    case 6: return V.th[cur][s];
+    case 7: return V.om[cur][s];
+    // wall histories, for checkpoints
+    case GATHER_DTB1: return V.dtb1[cur][s];
+    case GATHER_DTB1 + 1: return V.dtb2[cur][s];
+    case GATHER_DTB1 + 2: return V.thb1[cur][s];
+    case GATHER_DTB1 + 3: return V.thb2[cur][s];
+    default: return V.diag[(size_t)(field - 8) * V.N + s];
+    }
+}
+
 // all = 0: one instance at slots [off, off+n), out in its id order; all = 1:
 // every instance, out concatenated by instance (offset P.off) in id order.
 __global__ void k_gather_field(Views V, int cur, int off, int n, int field, double *out, int all)
 {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const int s = off + k;
-        double val;
-        switch (field) {
-        case 0: val = V.x[cur][s]; break;
-        case 1: val = V.y[cur][s]; break;
-        case 2: val = V.u[cur][s]; break;
-        case 3: val = V.v[cur][s]; break;
-        case 4: val = V.r[cur][s]; break;
-        case 5: val = V.h[cur][s]; break;
-        case 6: val = V.th[cur][s]; break;
-        case 7: val = V.om[cur][s]; break;
-        // wall histories, for checkpoints (GATHER_DTB1 ..)
-        case GATHER_DTB1: val = V.dtb1[cur][s]; break;
-        case GATHER_DTB1 + 1: val = V.dtb2[cur][s]; break;
-        case GATHER_DTB1 + 2: val = V.thb1[cur][s]; break;
-        case GATHER_DTB1 + 3: val = V.thb2[cur][s]; break;
-        default: val = V.diag[(size_t)(field - 8) * V.N + s]; break;
-        }
-        out[(all ? V.P[V.inst[s]].off : 0) + V.id[cur][s]] = val;
+        out[(all ? V.P[V.inst[s]].off : 0) + V.id[cur][s]] = field_value(V, cur, s, field);
     }
 }
 
-// which: 0 candidates, 1 contacts (pdn of the last diagnostic step), 2 bonds
-__global__ void k_list_pairs(Views V, int cur, int off, int n, int which, int *pi, int *pj, double *val,
-                             int cap, int *count)
+// Several fields of one instance at slots [off, off+n), each in id order:
+// field q at out + q n.
+__global__ void k_gather_fields(Views V, int cur, int off, int n, FieldList F, double *out)
+{
+    const int q = blockIdx.y;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
+        out[(size_t)q * n + V.id[cur][off + k]] = field_value(V, cur, off + k, F.code[q]);
+}
+
+// The pair lists.  which: 0 candidates, 1 contacts (pdn of the last
+// diagnostic step), 2 live bonds.  A list is in ascending (i, j): the pairs
+// are counted by their lower id, the counts scanned, and every floe writes its
+// own pairs at its place, ascending in j, so the host has nothing to sort
+// (sorting there took most of a read-back: 0.4 ms for 5,300 bonds).
+
+// The pairs of row item k (0 .. n-1) of the instance at [off, off + n): for
+// lists 0 and 1 those of slot off + k, for bonds those of reference id k.
+// Calls f(j, value); returns the lower id.
+template <class F>
+GD_DEV int row_pairs(const Views &V, int cur, int off, int which, int k, F f)
+{
+    if (which == 2) {
+        for (int b = V.bond_off[off + k]; b < V.bond_off[off + k + 1]; b++) {
+            const BondDyn d = V.bdyn[cur][b];
+            if (d.flag == 1) f(V.bond_hi[b], d.dmg);
+        }
+        return k;
+    }
+    const int s = off + k;
+    for (int e = V.up_off[s]; e < V.up_off[s + 1]; e++) {
+        const int2 en = V.ent_up[e];
+        const float dn = V.pdn[en.y];
+        if (dn != dn || (which == 1 && !(dn > 0.0f))) continue;
+        f(V.id[cur][en.x], (double)dn);
+    }
+    return V.id[cur][s];
+}
+
+GD_DEV int count_row(const Views &V, int cur, int off, int which, int k, int &id)
+{
+    int c = 0;
+    id = row_pairs(V, cur, off, which, k, [&](int, double) { c++; });
+    return c;
+}
+
+// Row item k's pairs at their place: base[id], each inserted in ascending j
+// among those already there.
+GD_DEV void write_row(const Views &V, int cur, int off, int which, int k, const int *base, int cap, int *pi, int *pj,
+                      double *val)
+{
+    const int i = which == 2 ? k : V.id[cur][off + k];
+    const int a = base[i];
+    int m = a;
+    row_pairs(V, cur, off, which, k, [&](int j, double v) {
+        if (m < cap) {
+            int q = m;
+            while (q > a && pj[q - 1] > j) {
+                pj[q] = pj[q - 1];
+                val[q] = val[q - 1];
+                q--;
+            }
+            pi[m] = i;
+            pj[q] = j;
+            val[q] = v;
+        } else {
+            // past the caller's capacity: the largest j of this row leaves
+            int q = cap;
+            while (q > a && pj[q - 1] > j) {
+                if (q < cap) { pj[q] = pj[q - 1]; val[q] = val[q - 1]; }
+                q--;
+            }
+            if (q < cap) { pj[q] = j; val[q] = v; }
+        }
+        m++;
+    });
+}
+
+__global__ void k_list_counts(Views V, int cur, int off, int n, int which, int *cnt)
 {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const int s = off + k;
-        const int ids = V.id[cur][s];
-        if (which == 2) {
-            const int gl = off + ids;
-            for (int b = V.bond_off[gl]; b < V.bond_off[gl + 1]; b++) {
-                const BondDyn d = V.bdyn[cur][b];
-                if (d.flag != 1) continue;
-                const int q = atomicAdd(count, 1);
-                if (q < cap) { pi[q] = ids; pj[q] = V.bond_hi[b]; val[q] = d.dmg; }
-            }
-            continue;
-        }
-        const int e0 = V.up_off[s], e1 = V.up_off[s + 1];
-        for (int e = e0; e < e1; e++) {
-            const int2 en = V.ent_up[e];
-            const float dn = V.pdn[en.y];
-            if (dn != dn) continue;
-            if (which == 1 && !(dn > 0.0f)) continue;
-            const int q = atomicAdd(count, 1);
-            if (q < cap) { pi[q] = ids; pj[q] = V.id[cur][en.x]; val[q] = (double)dn; }
-        }
+        int id;
+        const int c = count_row(V, cur, off, which, k, id);
+        cnt[id] = c;
     }
+}
+
+__global__ void k_list_fill(Views V, int cur, int off, int n, int which, const int *base, int cap, int *pi, int *pj,
+                            double *val)
+{
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
+        write_row(V, cur, off, which, k, base, cap, pi, pj, val);
+}
+
+// The whole list of a field of up to LIST_ONE_BLOCK floes by one block, the
+// counts in shared memory: one launch instead of six (count, three of the
+// scan, fill), which is what a list of a few thousand pairs costs.
+constexpr int LIST_ONE_BLOCK = 8192;
+__global__ void __launch_bounds__(1024) k_list_pairs(Views V, int cur, int off, int n, int which, int cap, int *pi,
+                                                     int *pj, double *val, int *total)
+{
+    __shared__ int cnt[LIST_ONE_BLOCK];
+    __shared__ int sums[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int k = tid; k < n; k += 1024) {
+        int id;
+        const int c = count_row(V, cur, off, which, k, id);
+        cnt[id] = c;
+    }
+    __syncthreads();
+    const int per = (n + 1023) / 1024, k0 = min(tid * per, n), k1 = min(k0 + per, n);
+    int own = 0;
+    for (int k = k0; k < k1; k++) own += cnt[k];
+    int pre = own;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, pre, o);
+        if (lane >= o) pre += v;
+    }
+    if (lane == 31) sums[warp] = pre;
+    __syncthreads();
+    int before = 0;
+    for (int w = 0; w < warp; w++) before += sums[w];
+    int at = before + pre - own;
+    if (tid == 1023) *total = before + pre;
+    for (int k = k0; k < k1; k++) {
+        const int c = cnt[k];
+        cnt[k] = at;
+        at += c;
+    }
+    __syncthreads();
+    if (cap > 0)
+        for (int k = tid; k < n; k += 1024) write_row(V, cur, off, which, k, cnt, cap, pi, pj, val);
 }
 
 // Per instance (one block each): total momentum (x, y), kinetic energy of
@@ -111,12 +220,24 @@ void launch_gather_field(const Views &V, int cur, int inst, int off, int n, int 
     k_gather_field<<<grid < 2048 ? grid : 2048, 256, 0, st>>>(V, cur, off, n, field, out, inst < 0 ? 1 : 0);
 }
 
-void launch_list_pairs(const Views &V, int cur, int inst, int off, int n, int which, int *pi, int *pj,
-                       double *val, int cap, int *count, cudaStream_t st)
+void launch_gather_fields(const Views &V, int cur, int off, int n, const FieldList &F, double *out, cudaStream_t st)
 {
-    (void)inst;
-    const int grid = n > 0 ? (n + 127) / 128 : 1;
-    k_list_pairs<<<grid < 2048 ? grid : 2048, 128, 0, st>>>(V, cur, off, n, which, pi, pj, val, cap, count);
+    const int grid = n > 0 ? (n + 255) / 256 : 1;
+    k_gather_fields<<<dim3(grid < 1024 ? grid : 1024, F.n), 256, 0, st>>>(V, cur, off, n, F, out);
+}
+
+void launch_list_pairs(const Views &V, int cur, int off, int n, int which, int cap, int *pi, int *pj, double *val,
+                       int *total, int *cnt, int *base, int *scan_scratch, cudaStream_t st)
+{
+    if (n <= LIST_ONE_BLOCK) {
+        k_list_pairs<<<1, 1024, 0, st>>>(V, cur, off, n, which, cap, pi, pj, val, total);
+        return;
+    }
+    const int grid = (n + 127) / 128 < 2048 ? (n + 127) / 128 : 2048;
+    k_list_counts<<<grid, 128, 0, st>>>(V, cur, off, n, which, cnt);
+    scan_excl(cnt, base, n, scan_scratch, st);
+    cudaMemcpyAsync(total, base + n, sizeof(int), cudaMemcpyDeviceToDevice, st);
+    if (cap > 0) k_list_fill<<<grid, 128, 0, st>>>(V, cur, off, n, which, base, cap, pi, pj, val);
 }
 
 }  // namespace godar

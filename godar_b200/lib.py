@@ -201,7 +201,7 @@ class Stepper:
         return out
 
     def floes(self, names=None) -> dict:
-        return {k: self.field(k) for k in (names or FLOE_FIELDS)}
+        return self.download(names)[0]
 
     def set_diagnostics(self, on: bool):
         _check(load().godar_gpu_set_diagnostics(self._h, 1 if on else 0))
@@ -227,7 +227,10 @@ class Stepper:
         """Per-floe outputs (all, or `names`) and optionally one pair list in
         one call (godar_gpu_download)."""
         names = list(names or FLOE_FIELDS)
-        outs = {k: np.empty(self.n, dtype=np.float64) for k in names}
+        # one block for all fields: its pages are touched here for the first
+        # time, and numpy asks for huge ones from 4 MB on
+        block = np.empty((len(names), self.n), dtype=np.float64)
+        outs = {k: block[q] for q, k in enumerate(names)}
         ptrs = (ctypes.c_void_p * len(FLOE_FIELDS))()
         for k, a in outs.items():
             ptrs[FIELD_ID[k]] = a.ctypes.data

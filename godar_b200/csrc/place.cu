@@ -16,8 +16,18 @@
 //      the overlaps, 12 iterations), keeping the first position that is free;
 //   2. a free position is kept if no free position of a disk of the class
 //      with a lower index overlaps it (the others retry next round).
-// Every list is ordered (cells by key, disks by index within a cell), so a
-// placement depends only on its inputs and seed.
+// Every list is ordered (disks by index within a cell), so a placement
+// depends only on its inputs and seed.
+//
+// What bounds a round is not any rate but the chain of one disk's attempts
+// (8 positions of 12 iterations, each over up to four cells) and the host
+// between the kernels.  A warp takes a disk, four lanes an attempt, so its
+// eight positions relax side by side and four placed disks are tested at once;
+// the cell lists are built by counting (their places by a scan, the order in
+// a cell restored by a sort of its few entries), which needs no length on the
+// host; all memory is drawn once; and the host reads one number a round.
+// 32,768 disks at 66 %: 39-50 ms with one thread per disk, radix sorts and
+// allocations per round, 9-11 ms so; 65,536 polydisperse ones 61 and 16 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -75,38 +85,68 @@ GD_DEV void cell_span(double lo, double hi, double cw, int nc, int per, int &a, 
 
 GD_DEV int wrapc(int c, int nc, int per) { return per ? ((c % nc) + nc) % nc : c; }
 
-// Coverage of the placed disks: one (cell, disk) item per cell that a placed
-// disk's bounding box meets.
-__global__ void k_cover_count(int n, const double *x, const double *y, const double *r,
-                              const unsigned char *placed, PGrid G, int *cnt)
+// A placed disk as a cell's list holds it.
+struct __align__(32) Cover {
+    double x, y, r;
+    int j, pad;
+};
+
+// Coverage of the placed disks: one entry per cell that a placed disk's
+// bounding box meets, counted (FILL = false) and written (true; cnt: how many
+// of each cell's entries are still to come).  The first `big` disks, which may
+// meet more than COVER_ALONE cells each, are spread over the whole grid.
+constexpr double COVER_ALONE = 4096.0;
+template <bool FILL>
+__global__ void k_cover(int n, int big, const double *x, const double *y, const double *r,
+                        const unsigned char *placed, PGrid G, int *cnt, const int *off, int *list)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int c = 0;
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
+    for (int i = 0; i < n; i++) {
+        int first = tid, stride = nthr;
+        if (i >= big) {
+            // from here on a thread per disk
+            i = max(i, big + tid);
+            if (i >= n) break;
+            first = 0;
+            stride = 1;
+        }
         if (placed[i]) {
             int ax, bx, ay, by;
             cell_span(x[i] - r[i], x[i] + r[i], G.cwx, G.ncx, G.px, ax, bx);
             cell_span(y[i] - r[i], y[i] + r[i], G.cwy, G.ncy, G.py, ay, by);
-            c = max(0, bx - ax + 1) * max(0, by - ay + 1);
+            const int w = max(0, bx - ax + 1), cells = w * max(0, by - ay + 1);
+            for (int k = first; k < cells; k += stride) {
+                const int c = wrapc(ay + k / w, G.ncy, G.py) * G.ncx + wrapc(ax + k % w, G.ncx, G.px);
+                if (FILL) list[off[c] + atomicSub(&cnt[c], 1) - 1] = i;
+                else atomicAdd(&cnt[c], 1);
+            }
         }
-        cnt[i] = c;
+        if (i >= big) i += nthr - 1;
     }
 }
 
-__global__ void k_cover_fill(int n, const double *x, const double *y, const double *r,
-                             const unsigned char *placed, PGrid G, const int *off, uint32_t *key, int *val)
+// Every cell's entries in ascending index, with their disks.
+__global__ void k_cover_order(int ncell, const int *off, int *list, const double *x, const double *y, const double *r,
+                              Cover *cov)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (!placed[i]) continue;
-        int ax, bx, ay, by;
-        cell_span(x[i] - r[i], x[i] + r[i], G.cwx, G.ncx, G.px, ax, bx);
-        cell_span(y[i] - r[i], y[i] + r[i], G.cwy, G.ncy, G.py, ay, by);
-        int q = off[i];
-        for (int cy = ay; cy <= by; cy++)
-            for (int cx = ax; cx <= bx; cx++) {
-                key[q] = (uint32_t)(wrapc(cy, G.ncy, G.py) * G.ncx + wrapc(cx, G.ncx, G.px));
-                val[q] = i;
-                q++;
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x) {
+        const int a = off[c], b = off[c + 1];
+        for (int k = a + 1; k < b; k++) {
+            const int v = list[k];
+            int q = k;
+            while (q > a && list[q - 1] > v) {
+                list[q] = list[q - 1];
+                q--;
             }
+            list[q] = v;
+        }
+        for (int k = a; k < b; k++) {
+            const int j = list[k];
+            Cover e;
+            e.x = x[j]; e.y = y[j]; e.r = r[j];
+            e.j = j; e.pad = 0;
+            cov[k] = e;
+        }
     }
 }
 
@@ -118,65 +158,102 @@ GD_DEV bool in_span(int w, int a, int b, int nc, int per)
     return ((w - a) % nc + nc) % nc <= b - a;
 }
 
-// Step 1: free positions of the unplaced disks [c0, c1).  A candidate spans
-// at most 2 x 2 cells (cells are at least twice the class's largest
-// radius); a placed disk met in several of them is counted in the first.
-__global__ void k_trial(int c0, int c1, const double *r, const unsigned char *placed, const double *x,
-                        const double *y, PGrid G, const int *cstart, const int *cend, const int *cov,
-                        uint64_t seed, int round, int attempts, unsigned char *cand, double *tx, double *ty)
+// Step 1: free positions of the unplaced disks [c0, c1), a warp per disk, four
+// lanes per attempt.  A candidate spans at most 2 x 2 cells (cells are at
+// least twice the class's largest radius); a placed disk met in several of
+// them is counted in the first.  The lanes of an attempt test a cell's
+// entries four at a time; the pushes are added in the entries' order.  The
+// disk takes the free position of its first successful attempt, so an attempt
+// after a successful one stops.
+constexpr int ATTEMPTS = 8;
+__global__ void __launch_bounds__(256) k_trial(int c0, int c1, const double *r, const unsigned char *placed, PGrid G,
+                                               const int *off, const Cover *cov, uint64_t seed, int round,
+                                               unsigned char *cand, double *tx, double *ty)
 {
-    for (int i = c0 + blockIdx.x * blockDim.x + threadIdx.x; i < c1; i += gridDim.x * blockDim.x) {
-        cand[i] = 0;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, sub = lane & 3, att = lane >> 2, quad = lane & ~3;
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    for (int i = c0 + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < c1; i += warps) {
+        if (lane == 0) cand[i] = 0;
         if (placed[i]) continue;
         const double rad = r[i];
         const double xlo = G.px ? 0.0 : rad, xhi = G.px ? G.Lx : G.Lx - rad;
         const double ylo = G.py ? 0.0 : rad, yhi = G.py ? G.Ly : G.Ly - rad;
         if (!(xhi > xlo && yhi > ylo)) continue;
         uint64_t s = mix64(seed ^ (0x632be59bd9b4e019ULL * (uint64_t)(i + 1))) ^ mix64((uint64_t)round + 1);
-        bool found = false;
-        for (int a = 0; a < attempts && !found; a++) {
-            double cx = xlo + (xhi - xlo) * uni(s);
-            double cy = ylo + (yhi - ylo) * uni(s);
-            for (int it = 0; it < 12; it++) {
-                int ax, bx, ay, by;
+        // attempt a takes the generator's values 2 a and 2 a + 1
+        s += 2 * (uint64_t)att * 0x9e3779b97f4a7c15ULL;
+        double cx = xlo + (xhi - xlo) * uni(s);
+        double cy = ylo + (yhi - ylo) * uni(s);
+        bool live = true, found = false;
+        for (int it = 0; it < 12; it++) {
+            int ax = 0, bx = -1, ay = 0, by = -1;
+            if (live) {
                 cell_span(cx - rad, cx + rad, G.cwx, G.ncx, G.px, ax, bx);
                 cell_span(cy - rad, cy + rad, G.cwy, G.ncy, G.py, ay, by);
-                int wxs[2], wys[2];
-                const int nxs = min(bx - ax + 1, 2), nys = min(by - ay + 1, 2);
-                for (int k = 0; k < nxs; k++) wxs[k] = wrapc(ax + k, G.ncx, G.px);
-                for (int k = 0; k < nys; k++) wys[k] = wrapc(ay + k, G.ncy, G.py);
-                double mx = 0.0, my = 0.0;
-                int hits = 0;
-                for (int ci = 0; ci < nxs * nys; ci++) {
-                    const int wx = wxs[ci % nxs], wy = wys[ci / nxs];
-                    const int cell = wy * G.ncx + wx;
-                    for (int q = cstart[cell]; q < cend[cell]; q++) {
-                        const int j = cov[q];
-                        const double dx = pwrap(cx - x[j], G.Lx, G.px), dy = pwrap(cy - y[j], G.Ly, G.py);
+            }
+            const int nxs = min(bx - ax + 1, 2), nys = min(by - ay + 1, 2);
+            const int wx0 = wrapc(ax, G.ncx, G.px), wx1 = wrapc(ax + 1, G.ncx, G.px);
+            const int wy0 = wrapc(ay, G.ncy, G.py), wy1 = wrapc(ay + 1, G.ncy, G.py);
+            const int cells = live ? nxs * nys : 0;
+            double mx = 0.0, my = 0.0;
+            int hits = 0;
+            for (int ci = 0; ci < 4; ci++) {
+                if (!__any_sync(full, ci < cells)) break;
+                int q = 0, q1 = 0;
+                if (ci < cells) {
+                    const int cell = (ci / nxs ? wy1 : wy0) * G.ncx + (ci % nxs ? wx1 : wx0);
+                    q = off[cell];
+                    q1 = off[cell + 1];
+                }
+                for (; __any_sync(full, q < q1); q += 4) {
+                    bool hit = false;
+                    double px = 0.0, py = 0.0, push = 0.0;
+                    bool apart = false;
+                    if (q + sub < q1) {
+                        const Cover e = cov[q + sub];
+                        const double dx = pwrap(cx - e.x, G.Lx, G.px), dy = pwrap(cy - e.y, G.Ly, G.py);
                         const double d = sqrt(dx * dx + dy * dy);
-                        const double sep = rad + r[j];
-                        if (!(d < sep)) continue;
-                        int jax, jbx, jay, jby;
-                        cell_span(x[j] - r[j], x[j] + r[j], G.cwx, G.ncx, G.px, jax, jbx);
-                        cell_span(y[j] - r[j], y[j] + r[j], G.cwy, G.ncy, G.py, jay, jby);
-                        bool seen = false;
-                        for (int cj = 0; cj < ci && !seen; cj++)
-                            seen = in_span(wxs[cj % nxs], jax, jbx, G.ncx, G.px) &&
-                                   in_span(wys[cj / nxs], jay, jby, G.ncy, G.py);
-                        if (seen) continue;
-                        const double push = (sep - d) * 1.0001 + 1e-9 * sep;
-                        if (d > 0) { mx += dx / d * push; my += dy / d * push; }
-                        else mx += push;
+                        const double sep = rad + e.r;
+                        if (d < sep) {
+                            int jax, jbx, jay, jby;
+                            cell_span(e.x - e.r, e.x + e.r, G.cwx, G.ncx, G.px, jax, jbx);
+                            cell_span(e.y - e.r, e.y + e.r, G.cwy, G.ncy, G.py, jay, jby);
+                            bool seen = false;
+                            for (int cj = 0; cj < ci && !seen; cj++)
+                                seen = in_span(cj % nxs ? wx1 : wx0, jax, jbx, G.ncx, G.px) &&
+                                       in_span(cj / nxs ? wy1 : wy0, jay, jby, G.ncy, G.py);
+                            if (!seen) {
+                                hit = true;
+                                push = (sep - d) * 1.0001 + 1e-9 * sep;
+                                apart = d > 0;
+                                if (apart) { px = dx / d; py = dy / d; }
+                            }
+                        }
+                    }
+                    // the attempt's hits in order
+                    const unsigned mine = __ballot_sync(full, hit) >> quad & 15u;
+                    for (int k = 0; k < 4; k++) {
+                        if (!__any_sync(full, mine >> k & 1u)) continue;
+                        const double hx = __shfl_sync(full, px, k, 4), hy = __shfl_sync(full, py, k, 4);
+                        const double hp = __shfl_sync(full, push, k, 4);
+                        const bool ha = __shfl_sync(full, (int)apart, k, 4) != 0;
+                        if (!(mine >> k & 1u)) continue;
+                        if (ha) { mx += hx * hp; my += hy * hp; }
+                        else mx += hp;
                         hits++;
                     }
                 }
-                if (!hits) {
-                    cand[i] = 1;
-                    tx[i] = cx;
-                    ty[i] = cy;
-                    found = true;
-                    break;
-                }
+            }
+            if (live && !hits) {
+                found = true;
+                live = false;
+            }
+            // attempts after a successful one stop
+            const unsigned ok = __ballot_sync(full, found);
+            if (ok && att > (__ffs(ok) - 1) >> 2) live = false;
+            if (!__any_sync(full, live)) break;
+            if (live) {
                 cx += mx;
                 cy += my;
                 if (G.px) cx -= G.Lx * floor(cx / G.Lx);
@@ -185,36 +262,45 @@ __global__ void k_trial(int c0, int c1, const double *r, const unsigned char *pl
                 else cy = fmin(fmax(cy, ylo), yhi);
             }
         }
+        const unsigned ok = __ballot_sync(full, found);
+        if (ok && lane == __ffs(ok) - 1) {
+            cand[i] = 1;
+            tx[i] = cx;
+            ty[i] = cy;
+        }
     }
 }
 
-__global__ void k_cand_keys(int c0, int c1, const unsigned char *cand, const double *tx, const double *ty, PGrid G,
-                            uint32_t *key, int *val)
+GD_DEV int cand_cell(const PGrid &G, double x, double y)
+{
+    const int cx = min(max((int)floor(x / G.cwx), 0), G.ncx - 1);
+    const int cy = min(max((int)floor(y / G.cwy), 0), G.ncy - 1);
+    return cy * G.ncx + cx;
+}
+
+// The free positions by cell (k_cover's two passes).
+template <bool FILL>
+__global__ void k_cands(int c0, int c1, const unsigned char *cand, const double *tx, const double *ty, PGrid G,
+                        int *cnt, const int *off, int *list)
 {
     for (int i = c0 + blockIdx.x * blockDim.x + threadIdx.x; i < c1; i += gridDim.x * blockDim.x) {
-        const int k = i - c0;
-        if (cand[i]) {
-            const int cx = min(max((int)floor(tx[i] / G.cwx), 0), G.ncx - 1);
-            const int cy = min(max((int)floor(ty[i] / G.cwy), 0), G.ncy - 1);
-            key[k] = (uint32_t)(cy * G.ncx + cx);
-        } else {
-            key[k] = 0xffffffffu;      // sorts last, never looked up
-        }
-        val[k] = i;
+        if (!cand[i]) continue;
+        const int c = cand_cell(G, tx[i], ty[i]);
+        if (FILL) list[off[c] + atomicSub(&cnt[c], 1) - 1] = i;
+        else atomicAdd(&cnt[c], 1);
     }
 }
 
 // Step 2: a free position is kept unless a free position of a lower-index
 // disk of the class overlaps it (class radii are at most half a cell, so
 // such a disk's centre lies in one of the 3 x 3 cells around).
-__global__ void k_accept(int c0, int c1, const double *r, unsigned char *cand, const double *tx, const double *ty,
-                         PGrid G, const int *cstart, const int *cend, const int *vals, unsigned char *placed,
-                         double *x, double *y, int *nplaced)
+__global__ void k_accept(int c0, int c1, const double *r, const unsigned char *cand, const double *tx,
+                         const double *ty, PGrid G, const int *off, const int *list, unsigned char *placed, double *x,
+                         double *y, int *nplaced)
 {
     for (int i = c0 + blockIdx.x * blockDim.x + threadIdx.x; i < c1; i += gridDim.x * blockDim.x) {
         if (!cand[i]) continue;
-        const int cx = min(max((int)floor(tx[i] / G.cwx), 0), G.ncx - 1);
-        const int cy = min(max((int)floor(ty[i] / G.cwy), 0), G.ncy - 1);
+        const int own = cand_cell(G, tx[i], ty[i]), cx = own % G.ncx, cy = own / G.ncx;
         bool ok = true;
         for (int dyc = -1; dyc <= 1 && ok; dyc++)
             for (int dxc = -1; dxc <= 1 && ok; dxc++) {
@@ -224,8 +310,8 @@ __global__ void k_accept(int c0, int c1, const double *r, unsigned char *cand, c
                 // small grids: a wrapped neighbour may repeat the own cell or
                 // another; repeats only repeat the same tests
                 const int cell = yy * G.ncx + xx;
-                for (int q = cstart[cell]; q < cend[cell]; q++) {
-                    const int j = vals[q];
+                for (int q = off[cell]; q < off[cell + 1]; q++) {
+                    const int j = list[q];
                     if (j >= i) continue;
                     const double dx = pwrap(tx[i] - tx[j], G.Lx, G.px), dy = pwrap(ty[i] - ty[j], G.Ly, G.py);
                     if (sqrt(dx * dx + dy * dy) < r[i] + r[j]) { ok = false; break; }
@@ -240,14 +326,15 @@ __global__ void k_accept(int c0, int c1, const double *r, unsigned char *cand, c
     }
 }
 
-struct DevMem {
-    std::vector<void *> ptrs;
-    ~DevMem() { for (void *p : ptrs) cudaFree(p); }
-    template <class T> T *get(size_t count) {
-        void *p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) return nullptr;
-        ptrs.push_back(p);
-        return (T *)p;
+// One device allocation, cut into pieces of 256-byte alignment.
+struct Arena {
+    char *base = nullptr;
+    size_t used = 0;
+    ~Arena() { if (base) cudaFree(base); }
+    template <class T> T *take(size_t count) {
+        T *p = (T *)(base + used);
+        used += (std::max<size_t>(count, 1) * sizeof(T) + 255) & ~(size_t)255;
+        return p;
     }
 };
 
@@ -270,107 +357,97 @@ int place_disks(int n, const double *r_in, double Lx, double Ly, int px, int py,
     const double rmin = std::max(rs[n - 1], 1e-9);
     auto cls = [&](double v) { return (int)std::floor(std::log2(std::max(v / rmin, 1.0))); };
 
-    DevMem M;
-    double *r = M.get<double>(n), *x = M.get<double>(n), *y = M.get<double>(n);
-    double *tx = M.get<double>(n), *ty = M.get<double>(n);
-    unsigned char *placed = M.get<unsigned char>(n), *cand = M.get<unsigned char>(n);
-    int *cnt = M.get<int>(n + 1), *off = M.get<int>(n + 1), *counter = M.get<int>(4);
-    if (!r || !x || !y || !tx || !ty || !placed || !cand || !cnt || !off || !counter) {
-        set_last_error("device allocation failed");
-        return GODAR_ERR_NOMEM;
-    }
-    cudaMemcpy(r, rs.data(), (size_t)n * 8, cudaMemcpyHostToDevice);
-    cudaMemset(placed, 0, (size_t)n);
-    cudaMemset(counter, 0, 16);
-    int total_placed = 0;
-    int k0 = 0;
-    while (k0 < n) {
+    // the classes and their grids; the most cells of one and the most cells
+    // the bounding boxes of all disks placed by its end can meet
+    struct Class { int k0, k1, big; PGrid G; };
+    std::vector<Class> classes;
+    long long cells = 1, covers = 1;
+    int widest = 1;
+    for (int k0 = 0; k0 < n;) {
         // the class of disk k0: every disk down to half its class's radius
+        Class C;
+        C.k0 = k0;
         const int c = cls(rs[k0]);
         int k1 = k0;
         while (k1 < n && cls(rs[k1]) == c) k1++;
-        const double R = rs[k0];
-        PGrid G;
+        C.k1 = k1;
+        PGrid &G = C.G;
         G.Lx = Lx; G.Ly = Ly; G.px = px; G.py = py;
-        const double cell = std::max(2.0 * R, 1e-9);
+        const double cell = std::max(2.0 * rs[k0], 1e-9);
         G.ncx = std::max(1, std::min(8192, (int)std::floor(Lx / cell)));
         G.ncy = std::max(1, std::min(8192, (int)std::floor(Ly / cell)));
         G.cwx = Lx / G.ncx;
         G.cwy = Ly / G.ncy;
-        const long long ncell = (long long)G.ncx * G.ncy;
-        int *cstart = M.get<int>(ncell), *cend = M.get<int>(ncell);
-        int *c2s = M.get<int>(ncell), *c2e = M.get<int>(ncell);
-        const int m = k1 - k0;
-        uint32_t *ck = M.get<uint32_t>(m), *cka = M.get<uint32_t>(m);
-        int *cv = M.get<int>(m), *cva = M.get<int>(m);
-        const int nt2 = (m + 2047) / 2048;
-        int *rsc2 = M.get<int>(256 * (size_t)nt2 + 1), *scr2 = M.get<int>(256 * (size_t)nt2 / 2048 + 64 + m / 2048 + 64);
-        if (!cstart || !cend || !c2s || !c2e || !ck || !cka || !cv || !cva || !rsc2 || !scr2) {
-            set_last_error("device allocation failed");
-            return GODAR_ERR_NOMEM;
+        double met = 0.0;
+        C.big = 0;
+        for (int k = 0; k < k1; k++) {
+            const double own = std::min((double)G.ncx, std::floor(2.0 * rs[k] / G.cwx) + 2.0) *
+                               std::min((double)G.ncy, std::floor(2.0 * rs[k] / G.cwy) + 2.0);
+            met += own;
+            if (own > COVER_ALONE) C.big = k + 1;
         }
-        const int bits = std::max(1, (int)std::ceil(std::log2((double)std::max<long long>(ncell + 1, 2))));
+        if (met >= 2147483647.0) { set_last_error("too many cells covered"); return GODAR_ERR_NOMEM; }
+        covers = std::max(covers, (long long)met);
+        cells = std::max(cells, (long long)G.ncx * G.ncy);
+        widest = std::max(widest, k1 - k0);
+        classes.push_back(C);
+        k0 = k1;
+    }
+    const size_t nc = (size_t)cells;
+    const auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    Arena M;
+    const size_t want = 5 * up((size_t)n * 8) + 2 * up((size_t)n) + 2 * up((nc + 1) * 4) + 2 * up(nc * 4) +
+                        up((nc / 2048 + 64) * 4) + up((size_t)covers * 4) + up((size_t)covers * sizeof(Cover)) +
+                        up((size_t)widest * 4) + up(16);
+    if (cudaMalloc(&M.base, want) != cudaSuccess) {
+        cudaGetLastError();
+        M.base = nullptr;
+        set_last_error("device allocation failed");
+        return GODAR_ERR_NOMEM;
+    }
+    double *r = M.take<double>(n), *x = M.take<double>(n), *y = M.take<double>(n);
+    double *tx = M.take<double>(n), *ty = M.take<double>(n);
+    unsigned char *placed = M.take<unsigned char>(n), *cand = M.take<unsigned char>(n);
+    // per cell: places in the lists of placed disks and of free positions, and
+    // the counts they come from (zero between uses: the second pass of each
+    // list counts them down)
+    int *off = M.take<int>(nc + 1), *off2 = M.take<int>(nc + 1), *cnt = M.take<int>(nc), *cnt2 = M.take<int>(nc);
+    int *scr = M.take<int>(nc / 2048 + 64);
+    int *list = M.take<int>((size_t)covers);
+    Cover *cov = M.take<Cover>((size_t)covers);
+    int *list2 = M.take<int>(widest), *counter = M.take<int>(4);
+    cudaMemcpy(r, rs.data(), (size_t)n * 8, cudaMemcpyHostToDevice);
+    cudaMemset(placed, 0, (size_t)n);
+    cudaMemset(cnt, 0, nc * 4);
+    cudaMemset(cnt2, 0, nc * 4);
+    cudaMemset(counter, 0, 16);
+    int total_placed = 0;
+    for (const Class &C : classes) {
+        const PGrid G = C.G;
+        const int k0 = C.k0, k1 = C.k1, m = k1 - k0, ncell = G.ncx * G.ncy;
         int left = m;
         for (int round = 0; round < max_rounds && left > 0; round++) {
-            // coverage of every disk placed so far
-            k_cover_count<<<grid_n(n, 256), 256>>>(n, x, y, r, placed, G, cnt);
-            int *scr1 = nullptr;
-            {
-                const int nt = (n + 2047) / 2048;
-                scr1 = M.get<int>(256 * (size_t)nt / 2048 + 64 + (size_t)n / 2048 + 64);
-            }
-            scan_excl(cnt, off, n, scr1, 0);
-            int P = 0;
-            cudaMemcpy(&P, off + n, sizeof(int), cudaMemcpyDeviceToHost);
-            uint32_t *key = M.get<uint32_t>(P), *keya = M.get<uint32_t>(P);
-            int *val = M.get<int>(P), *vala = M.get<int>(P);
-            const int nt = (P + 2047) / 2048;
-            int *rsc = M.get<int>(256 * (size_t)nt + 1), *scr = M.get<int>(256 * (size_t)nt / 2048 + 64 + P / 2048 + 64);
-            if (!scr1 || !key || !keya || !val || !vala || !rsc || !scr) {
-                set_last_error("device allocation failed");
-                return GODAR_ERR_NOMEM;
-            }
-            cudaMemset(cstart, 0, (size_t)ncell * 4);
-            cudaMemset(cend, 0, (size_t)ncell * 4);
-            if (P > 0) {
-                k_cover_fill<<<grid_n(n, 256), 256>>>(n, x, y, r, placed, G, off, key, val);
-                radix_sort(key, val, keya, vala, P, bits, rsc, scr, 0);
-                launch_cell_ranges(key, P, cstart, cend, 0);
-            }
+            // coverage of every disk placed so far (they come before k1)
+            k_cover<false><<<grid_n(C.big ? 1 << 20 : k1, 256), 256>>>(k1, C.big, x, y, r, placed, G, cnt, nullptr, nullptr);
+            scan_excl(cnt, off, ncell, scr, 0);
+            k_cover<true><<<grid_n(C.big ? 1 << 20 : k1, 256), 256>>>(k1, C.big, x, y, r, placed, G, cnt, off, list);
+            k_cover_order<<<grid_n(ncell, 128), 128>>>(ncell, off, list, x, y, r, cov);
             // step 1
-            k_trial<<<grid_n(m, 128), 128>>>(k0, k1, r, placed, x, y, G, cstart, cend, val, seed, round, 8, cand,
-                                              tx, ty);
-            // step 2: free positions by cell
-            k_cand_keys<<<grid_n(m, 256), 256>>>(k0, k1, cand, tx, ty, G, ck, cv);
-            radix_sort(ck, cv, cka, cva, m, 32, rsc2, scr2, 0);
-            cudaMemset(c2s, 0, (size_t)ncell * 4);
-            cudaMemset(c2e, 0, (size_t)ncell * 4);
-            // keys of disks without a free position (0xffffffff) sort last:
-            // ranges only for the real cells
-            int mc = 0;
-            {
-                std::vector<uint32_t> hk(m);
-                cudaMemcpy(hk.data(), ck, (size_t)m * 4, cudaMemcpyDeviceToHost);
-                mc = (int)(std::lower_bound(hk.begin(), hk.end(), 0xffffffffu) - hk.begin());
-            }
-            if (mc > 0) launch_cell_ranges(ck, mc, c2s, c2e, 0);
-            cudaMemset(counter, 0, sizeof(int));
-            k_accept<<<grid_n(m, 128), 128>>>(k0, k1, r, cand, tx, ty, G, c2s, c2e, cv, placed, x, y, counter);
+            k_trial<<<grid_n((long long)m * 32, 256), 256>>>(k0, k1, r, placed, G, off, cov, seed, round, cand, tx, ty);
+            // step 2
+            k_cands<false><<<grid_n(m, 256), 256>>>(k0, k1, cand, tx, ty, G, cnt2, nullptr, nullptr);
+            scan_excl(cnt2, off2, ncell, scr, 0);
+            k_cands<true><<<grid_n(m, 256), 256>>>(k0, k1, cand, tx, ty, G, cnt2, off2, list2);
+            k_accept<<<grid_n(m, 128), 128>>>(k0, k1, r, cand, tx, ty, G, off2, list2, placed, x, y, counter);
             int got = 0;
             if (cudaMemcpy(&got, counter, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) {
                 set_last_error("placement kernels failed");
                 return GODAR_ERR_CUDA;
             }
-            left -= got;
-            total_placed += got;
-            // this round's temporaries
-            for (int q = 0; q < 7; q++) {
-                cudaFree(M.ptrs.back());
-                M.ptrs.pop_back();
-            }
+            left -= got - total_placed;
+            total_placed = got;
         }
         if (left > 0) break;     // the caller enlarges the domain
-        k0 = k1;
     }
     std::vector<double> hx(n), hy(n);
     std::vector<unsigned char> hp(n);

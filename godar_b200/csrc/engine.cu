@@ -71,6 +71,11 @@ struct Pool {
     cudaStream_t st = nullptr;      // allocations are ordered on this stream
 };
 
+// Set while an engine whose streams are idle frees its buffers: nothing is in
+// flight that a free would have to wait for, and the pool is drained once at
+// the end (EngineRes).
+thread_local bool g_idle_free = false;
+
 struct Buf {
     void *p = nullptr;
     size_t bytes = 0;
@@ -81,7 +86,9 @@ struct Buf {
     ~Buf() { free_mem(); }
     void free_mem() {
         if (!p) return;
-        if (pooled) {
+        if (pooled && g_idle_free) {
+            cudaFreeAsync(p, nullptr);
+        } else if (pooled) {
             // whatever any stream still does with the buffer ends first, and
             // the memory is back in the pool before the call returns
             cudaDeviceSynchronize();
@@ -217,15 +224,155 @@ void restart_bonds(const Inst &I, HostBonds &B)
 }  // namespace
 
 // ====================================================================== Engine
-struct PoolOwner {
+// What an engine needs of the driver besides its buffers: streams, events,
+// pinned memory and the memory pool.  Creating and destroying them takes
+// 1.5-8 ms, more than the whole first step of a field of a few thousand
+// floes, so a destroyed engine's set is kept for the next one on the same
+// device and context: at most RES_KEPT sets, each holding at most
+// RES_KEPT_BYTES of device memory; what is over is given back to the driver.
+// A set belongs to one engine at a time and comes back with its streams idle.
+constexpr size_t RES_KEPT = 4;
+constexpr size_t RES_KEPT_BYTES = 64u << 20;
+constexpr int RES_RING = 16, RES_FRING = 4;
+constexpr size_t STAGE_SLOT = 128 << 10;      // one of two pinned read-back slots
+
+struct EngineRes {
+    int dev = -1;
+    unsigned long long ctx = 0;       // the context's id (0: unknown, never kept)
+    cudaStream_t st = nullptr, st2 = nullptr, stc = nullptr, stg = nullptr;
+    cudaEvent_t ev_state = nullptr, ev_fork = nullptr, ev_join = nullptr, ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev_gath[2] = {}, ev_copy[2] = {}, stage_ev[2] = {}, ring_ev[RES_RING] = {}, fring_ev[RES_FRING] = {};
+    // one pinned block: four counters, the status mirror (four ints), four ints
+    // per ring slot, the two read-back slots
+    static constexpr size_t SMALL_PINNED = 4 * 8 + (4 + RES_RING * 4) * 4;
+    char *pinned = nullptr;
+    cudaMemPool_t pool = nullptr;
+
+    EngineRes() = default;
+    EngineRes(const EngineRes &) = delete;
+    EngineRes &operator=(const EngineRes &) = delete;
+    ~EngineRes() {
+        for (cudaEvent_t e : {ev_state, ev_fork, ev_join, ev0, ev1, ev_gath[0], ev_gath[1], ev_copy[0], ev_copy[1],
+                              stage_ev[0], stage_ev[1]})
+            if (e) cudaEventDestroy(e);
+        for (auto e : ring_ev) if (e) cudaEventDestroy(e);
+        for (auto e : fring_ev) if (e) cudaEventDestroy(e);
+        for (cudaStream_t t : {st2, stc, stg, st})
+            if (t) cudaStreamDestroy(t);
+        if (pinned) cudaFreeHost(pinned);
+        if (pool) cudaMemPoolDestroy(pool);
+    }
+
+    int create() {
+        for (cudaStream_t *t : {&st, &st2, &stc, &stg}) CK(cudaStreamCreateWithFlags(t, cudaStreamNonBlocking));
+        for (cudaEvent_t *e : {&ev_state, &ev_fork, &ev_join, &ev_gath[0], &ev_gath[1], &ev_copy[0], &ev_copy[1],
+                               &stage_ev[0], &stage_ev[1]})
+            CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        for (auto &e : ring_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        for (auto &e : fring_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        CK(cudaEventCreate(&ev0));
+        CK(cudaEventCreate(&ev1));
+        CK(cudaMallocHost(&pinned, SMALL_PINNED + 2 * STAGE_SLOT));
+        int pools = 0;
+        cudaDeviceGetAttribute(&pools, cudaDevAttrMemoryPoolsSupported, dev);
+        if (pools) {
+            cudaMemPoolProps pp = {};
+            pp.allocType = cudaMemAllocationTypePinned;
+            pp.location.type = cudaMemLocationTypeDevice;
+            pp.location.id = dev;
+            CK(cudaMemPoolCreate(&pool, &pp));
+            unsigned long long keep = ~0ULL;
+            CK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        }
+        cudaGetLastError();
+        return GODAR_OK;
+    }
+
+    // The id of the calling thread's current context: unlike its handle, never
+    // used again after the context is destroyed.  0 if it cannot be had.
+    static unsigned long long context_id() {
+        typedef int (*GetFn)(void **);
+        typedef int (*IdFn)(void *, unsigned long long *);
+        static const auto fns = [] {
+            void *get = nullptr, *id = nullptr;
+            cudaDriverEntryPointQueryResult q;
+            if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &get, cudaEnableDefault, &q) != cudaSuccess ||
+                q != cudaDriverEntryPointSuccess)
+                get = nullptr;
+            if (cudaGetDriverEntryPoint("cuCtxGetId", &id, cudaEnableDefault, &q) != cudaSuccess ||
+                q != cudaDriverEntryPointSuccess)
+                id = nullptr;
+            cudaGetLastError();
+            return std::make_pair((GetFn)get, (IdFn)id);
+        }();
+        void *ctx = nullptr;
+        unsigned long long v = 0;
+        if (!fns.first || !fns.second || fns.first(&ctx) != 0 || !ctx || fns.second(ctx, &v) != 0) return 0;
+        return v;
+    }
+
+    // (never destroyed: the process may end after the driver has shut down)
+    static std::mutex &lock() { static std::mutex *m = new std::mutex; return *m; }
+    static std::vector<EngineRes *> &kept() { static auto *v = new std::vector<EngineRes *>; return *v; }
+
+    static int acquire(EngineRes **out) {
+        int dev = 0;
+        CK(cudaGetDevice(&dev));
+        CK(cudaFree(nullptr));            // the device's context exists and is current
+        const unsigned long long ctx = context_id();
+        {
+            std::lock_guard<std::mutex> lk(lock());
+            auto &v = kept();
+            for (size_t k = v.size(); k-- > 0;)
+                if (v[k]->dev == dev && ctx != 0 && v[k]->ctx == ctx) {
+                    *out = v[k];
+                    v.erase(v.begin() + k);
+                    return GODAR_OK;
+                }
+        }
+        auto r = std::make_unique<EngineRes>();
+        r->dev = dev;
+        r->ctx = ctx;
+        TRY(r->create());
+        *out = r.release();
+        return GODAR_OK;
+    }
+
+    // Back from an engine whose streams are idle and whose buffers are freed.
+    static void release(EngineRes *r) {
+        if (!r) return;
+        bool ok = cudaStreamSynchronize(nullptr) == cudaSuccess;
+        if (r->pool) ok = ok && cudaMemPoolTrimTo(r->pool, RES_KEPT_BYTES) == cudaSuccess;
+        cudaGetLastError();
+        if (ok && r->ctx != 0 && r->ctx == context_id()) {
+            std::lock_guard<std::mutex> lk(lock());
+            auto &v = kept();
+            // sets of a context that is gone went with it
+            for (size_t k = v.size(); k-- > 0;)
+                if (v[k]->dev == r->dev && v[k]->ctx != r->ctx) v.erase(v.begin() + k);
+            if (v.size() < RES_KEPT) {
+                v.push_back(r);
+                return;
+            }
+        }
+        delete r;
+    }
+};
+
+struct ResOwner {
+    EngineRes *r = nullptr;
     Pool mp;
-    ~PoolOwner() { if (mp.pool) cudaMemPoolDestroy(mp.pool); }
+    ~ResOwner() {
+        g_idle_free = false;
+        EngineRes::release(r);
+    }
 };
 
 struct Engine {
-    // first member, so that it is destroyed after every buffer drawn from it
-    PoolOwner po;
-    Pool &mp = po.mp;
+    // first member, so that it is destroyed after every buffer drawn from its
+    // pool; the streams, events and pinned memory below are this set's
+    ResOwner res;
+    Pool &mp = res.mp;
     int prec = GODAR_PREC_FP64;
     size_t budget = 0;
     cudaStream_t st = nullptr;
@@ -294,7 +441,6 @@ struct Engine {
     bool counting = false;             // the last call launched a diagnostic step
     unsigned long long *h_counters = nullptr;   // pinned
     // two pinned slots for read-backs (copy_out)
-    static constexpr size_t STAGE_SLOT = 128 << 10;
     char *h_stage = nullptr;
     cudaEvent_t stage_ev[2] = {};
     // Verlet skin = max(1 m, skin_frac (r_max + rtree)); a rebuild costs
@@ -418,7 +564,7 @@ struct Engine {
         bool small;                // it was one launch (launch_small)
         std::vector<double> uvw;   // the uniform forcing it ran with (empty: as admitted)
     };
-    static constexpr int RING = 16;
+    static constexpr int RING = RES_RING;
     std::deque<Pending> pend;
     int *h_ring = nullptr;
     cudaEvent_t ring_ev[RING] = {};
@@ -426,7 +572,7 @@ struct Engine {
     std::vector<double> cur_uvw;   // the last uniform forcing set since the last relayout
     // pinned copies of the uniform forcing for its queued uploads (a copy
     // from pageable memory may wait for the stream)
-    static constexpr int FRING = 4;
+    static constexpr int FRING = RES_FRING;
     double *fring[FRING] = {};
     size_t fring_cap = 0;          // doubles per buffer
     cudaEvent_t fring_ev[FRING] = {};
@@ -441,28 +587,10 @@ struct Engine {
         if (st) cudaStreamSynchronize(st);
         drop_graphs();
         for (auto e : kev) cudaEventDestroy(e);
-        if (ev0) cudaEventDestroy(ev0);
-        if (ev1) cudaEventDestroy(ev1);
-        if (h_counters) cudaFreeHost(h_counters);
-        for (auto e : stage_ev)
-            if (e) cudaEventDestroy(e);
-        for (auto e : ring_ev)
-            if (e) cudaEventDestroy(e);
-        for (int q = 0; q < FRING; q++) {
+        for (int q = 0; q < FRING; q++)
             if (fring[q]) cudaFreeHost(fring[q]);
-            if (fring_ev[q]) cudaEventDestroy(fring_ev[q]);
-        }
-        if (ev_fork) cudaEventDestroy(ev_fork);
-        if (ev_join) cudaEventDestroy(ev_join);
-        if (st2) cudaStreamDestroy(st2);
-        if (stc) cudaStreamDestroy(stc);
-        if (stg) cudaStreamDestroy(stg);
-        for (int q = 0; q < 2; q++) {
-            if (ev_gath[q]) cudaEventDestroy(ev_gath[q]);
-            if (ev_copy[q]) cudaEventDestroy(ev_copy[q]);
-        }
-        if (ev_state) cudaEventDestroy(ev_state);
-        if (st) cudaStreamDestroy(st);
+        if (st2) cudaStreamSynchronize(st2);
+        g_idle_free = true;      // until ResOwner has the buffers back
     }
 
     int init(int precision, size_t bud) {
@@ -474,44 +602,23 @@ struct Engine {
             set_err("no CUDA device visible");
             return GODAR_ERR_NO_DEVICE;
         }
-        CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-        CK(cudaStreamCreateWithFlags(&st2, cudaStreamNonBlocking));
-        CK(cudaStreamCreateWithFlags(&stc, cudaStreamNonBlocking));
-        CK(cudaStreamCreateWithFlags(&stg, cudaStreamNonBlocking));
+        TRY(EngineRes::acquire(&res.r));
+        const EngineRes &R = *res.r;
+        st = R.st; st2 = R.st2; stc = R.stc; stg = R.stg;
+        ev_state = R.ev_state; ev_fork = R.ev_fork; ev_join = R.ev_join; ev0 = R.ev0; ev1 = R.ev1;
         for (int q = 0; q < 2; q++) {
-            CK(cudaEventCreateWithFlags(&ev_gath[q], cudaEventDisableTiming));
-            CK(cudaEventCreateWithFlags(&ev_copy[q], cudaEventDisableTiming));
+            ev_gath[q] = R.ev_gath[q];
+            ev_copy[q] = R.ev_copy[q];
+            stage_ev[q] = R.stage_ev[q];
         }
-        {
-            int dev = 0, pools = 0;
-            CK(cudaGetDevice(&dev));
-            cudaDeviceGetAttribute(&pools, cudaDevAttrMemoryPoolsSupported, dev);
-            if (pools) {
-                cudaMemPoolProps pp = {};
-                pp.allocType = cudaMemAllocationTypePinned;
-                pp.location.type = cudaMemLocationTypeDevice;
-                pp.location.id = dev;
-                CK(cudaMemPoolCreate(&mp.pool, &pp));
-                unsigned long long keep = ~0ULL;
-                CK(cudaMemPoolSetAttribute(mp.pool, cudaMemPoolAttrReleaseThreshold, &keep));
-                mp.st = st;
-            }
-            cudaGetLastError();
-        }
-        CK(cudaEventCreateWithFlags(&ev_state, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
-        CK(cudaEventCreate(&ev0));
-        CK(cudaEventCreate(&ev1));
-        // one pinned block: the counters, the status mirror, the ring
-        constexpr size_t small_pinned = sizeof(counters) + (4 + RING * 4) * sizeof(int);
-        CK(cudaMallocHost(&h_counters, small_pinned + 2 * STAGE_SLOT));
+        for (int q = 0; q < RING; q++) ring_ev[q] = R.ring_ev[q];
+        for (int q = 0; q < FRING; q++) fring_ev[q] = R.fring_ev[q];
+        h_counters = (unsigned long long *)R.pinned;
         h_status = (int *)(h_counters + 4);
         h_ring = h_status + 4;
-        h_stage = (char *)h_counters + small_pinned;
-        for (auto &e : stage_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        for (auto &e : ring_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        for (auto &e : fring_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        h_stage = R.pinned + EngineRes::SMALL_PINNED;
+        mp.pool = R.pool;
+        mp.st = st;
         TRY(step_base_b.ensure(2 * sizeof(int), &bytes, &mp));
         CK(cudaMemsetAsync(step_base_b.p, 0, 2 * sizeof(int), st));
         TRY(status.ensure(2 * sizeof(int), &bytes, &mp));

@@ -2,55 +2,37 @@
 // (KdTree build, kdtree_utils.f90:21-24; radius query kNearest,
 // stepper.f90:77-78).
 //
-// Pipeline of one rebuild (all instances of a batch at once):
-//   1. cell key of every floe (its instance's first key + row-major cell)
-//   2. stable LSD radix sort of (key, slot), 8-bit digits, as many passes as
-//      the key range needs
-//   3. gather the floe state into cell order (the other ping-pong side)
-//   4. first/last slot of every non-empty cell
-//   5. count, scan and fill the symmetric neighbour superset: every t with
-//      dist(s,t) <= r_lo + rtree + skin, lo = the floe of lower id; rows are
-//      sorted (lower-id partners by id, then higher-id partners by distance;
-//      by id in the mixed path)
-//   6. link every lower entry to the record of its pair (owned by the
-//      lower-id floe's upper entry), migrate contact histories from the
-//      previous rows by reference ids, and link bonds.
+// One rebuild (all instances of a batch at once):
+//   1. k_cell_count, scan, k_cell_scatter: the cell list, by counting (the
+//      cell of a floe: its instance's first cell + row-major cell)
+//   2. k_cell_place: the floes' state gathered into cell order on the other
+//      ping-pong side, floes of one cell in their previous order
+//   3. k_nbr_count, scan, k_nbr_fill: the symmetric neighbour superset, every
+//      t with dist(s,t) <= r_lo + rtree + skin, lo = the floe of lower id, as
+//      owner rows (partners of higher id, by distance; by id in the mixed path)
+//      and partner rows (partners of lower id, by id)
+//   4. k_row_finish: the pair index of every partner entry (the entry of the
+//      lower-id floe's owner row that points back), contact histories from
+//      the previous rows by reference ids, bond indices, and what else a
+//      fresh row holds
 // The step kernel filters the superset with the exact candidate predicate
 // every step, so the candidate set is the kd-tree's radius query exactly as
 // long as no floe moved more than skin/2 since the rebuild (checked every
 // step).  This file is compiled with --fmad=false: distances must round
 // exactly as in the step kernel and the CPU oracle.
-#include "common.cuh"
+//
+// What bounds it: on small fields the chains of dependent loads of one thread
+// per floe (cells, floes, rows) and the number of launches; on large ones the
+// same chains at partial occupancy.  So a group of eight lanes takes a floe,
+// reads each stencil row as one range, and ranks a row's entries by counting
+// instead of inserting them one by one; and the list is built by counting
+// (6 launches where the radix sort took 11-16).
+#include <algorithm>
+
+#include "cells.cuh"
 #include "kernels.h"
 
 namespace godar {
-
-// ------------------------------------------------------------ cell keys
-GD_DEV void cell_of(const InstParams &P, double x, double y, int &cx, int &cy)
-{
-    // clamp before the integer conversion so that non-finite or far-away
-    // positions land in an edge cell
-    double fx = x / P.cw, fy = y / P.ch;
-    if (!(fx >= 0.0)) fx = 0.0;
-    if (!(fy >= 0.0)) fy = 0.0;
-    if (fx > (double)P.ncx) fx = (double)P.ncx;
-    if (fy > (double)P.ncy) fy = (double)P.ncy;
-    cx = (int)floor(fx);
-    cy = (int)floor(fy);
-    cx = cx < 0 ? 0 : (cx >= P.ncx ? P.ncx - 1 : cx);
-    cy = cy < 0 ? 0 : (cy >= P.ncy ? P.ncy - 1 : cy);
-}
-
-__global__ void k_cell_keys(Views V, int cur, uint32_t *keys, int *vals)
-{
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < V.N; g += gridDim.x * blockDim.x) {
-        const InstParams &P = V.P[V.inst[g]];
-        int cx, cy;
-        cell_of(P, V.x[cur][g], V.y[cur][g], cx, cy);
-        keys[g] = (uint32_t)(P.coff + (long long)cy * P.ncx + cx);
-        vals[g] = g;
-    }
-}
 
 // ------------------------------------------------------------ radix sort
 // Tile of RS_THREADS x RS_ITEMS keys per block; item k of the tile is key
@@ -236,17 +218,44 @@ void radix_sort(uint32_t *keys, int *vals, uint32_t *keys_alt, int *vals_alt, in
     }
 }
 
-// ------------------------------------------------------------ permutation
-// new slot s takes the floe at pre-sort slot vals[s]; old_slot[s] is that
-// floe's slot in the previous layout (repack[] maps pre-sort slots to the
-// previous layout; -1 for floes new to the batch).
-__global__ void k_permute(Views V, int cur, const int *vals, const int *repack, int *old_slot)
+// ------------------------------------------------------------ cell list
+// Floes [s0, s0 + n): their cells and how many each cell has (cnt, zero
+// before); after the scan, the cells' floes in any order (cnt back to zero).
+__global__ void k_cell_count(Views V, int cur, int s0, int n, uint32_t *keys, int *cnt)
+{
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const int s = s0 + k;
+        const uint32_t c = cell_key(V.P[V.inst[s]], V.x[cur][s], V.y[cur][s]);
+        keys[k] = c;
+        atomicAdd(&cnt[c], 1);
+    }
+}
+
+__global__ void k_cell_scatter(int s0, int n, const uint32_t *keys, const int *coff, int *cnt, int *list)
+{
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const uint32_t c = keys[k];
+        list[coff[c] + atomicSub(&cnt[c], 1) - 1] = s0 + k;
+    }
+}
+
+// The floes in cell order, those of a cell in ascending previous slot (a
+// floe's place: how many of its cell's floes come before it); old_slot: the
+// floe's slot in the previous layout (repack maps pre-sort slots to it; -1 for
+// floes new to the batch).
+__global__ void k_cell_place(Views V, int cur, const uint32_t *keys, const int *coff, const int *list,
+                             const int *repack, int *old_slot)
 {
     const int nxt = cur ^ 1;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x) {
-        const int o = vals[s];
-        V.x[nxt][s] = V.x[cur][o];
-        V.y[nxt][s] = V.y[cur][o];
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < V.N; q += gridDim.x * blockDim.x) {
+        const int o = list[q];
+        const uint32_t c = keys[o];
+        const int a = coff[c], b = coff[c + 1];
+        int s = a;
+        for (int k = a; k < b; k++) s += list[k] < o;
+        const double x = V.x[cur][o], y = V.y[cur][o];
+        V.x[nxt][s] = x;
+        V.y[nxt][s] = y;
         V.th[nxt][s] = V.th[cur][o];
         V.u[nxt][s] = V.u[cur][o];
         V.v[nxt][s] = V.v[cur][o];
@@ -258,186 +267,194 @@ __global__ void k_permute(Views V, int cur, const int *vals, const int *repack, 
         V.thb1[nxt][s] = V.thb1[cur][o];
         V.thb2[nxt][s] = V.thb2[cur][o];
         V.id[nxt][s] = V.id[cur][o];
-        V.x0[nxt][s] = V.x[cur][o];
-        V.y0[nxt][s] = V.y[cur][o];
+        V.x0[nxt][s] = x;
+        V.y0[nxt][s] = y;
         old_slot[s] = repack ? repack[o] : o;
     }
 }
 
-__global__ void k_cell_ranges(const uint32_t *keys, int n, int *cstart, int *cend)
-{
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        const uint32_t k = keys[s];
-        if (s == 0 || keys[s - 1] != k) cstart[k] = s;
-        if (s == n - 1 || keys[s + 1] != k) cend[k] = s + 1;
-    }
-}
-
 // ------------------------------------------------------------ neighbour rows
-// Visits every floe t != s of s's instance within the stencil and calls
-// f(t, dist, id of t) when dist <= r_lo + rtree + skin.
+// Floe s against every floe of the stencil around it that falls to this lane:
+// f(t, dist, id of t) when t != s and dist <= r_lo + rtree + skin.
 template <class F>
-GD_DEV void for_superset(const Views &V, int side, const int *cstart, const int *cend, int s, F f)
+GD_DEV void for_superset(const Views &V, int side, const int *coff, int s, int sub, F f)
 {
     const InstParams &P = V.P[V.inst[s]];
     const double xs = V.x[side][s], ys = V.y[side][s], rs = V.r[side][s];
     const int ids = V.id[side][s];
     const bool px = P.boundary & BC_PERIODIC_X, py = P.boundary & BC_PERIODIC_Y;
-    int cx, cy;
-    cell_of(P, xs, ys, cx, cy);
-    int x0 = cx - P.kx, x1 = cx + P.kx, y0 = cy - P.ky, y1 = cy + P.ky;
-    if (px && x1 - x0 + 1 >= P.ncx) { x0 = 0; x1 = P.ncx - 1; }
-    if (py && y1 - y0 + 1 >= P.ncy) { y0 = 0; y1 = P.ncy - 1; }
-    for (int yy = y0; yy <= y1; yy++) {
-        int wy = yy;
-        if (py) wy = (yy % P.ncy + P.ncy) % P.ncy;
-        else if (yy < 0 || yy >= P.ncy) continue;
-        for (int xx = x0; xx <= x1; xx++) {
-            int wx = xx;
-            if (px) wx = (xx % P.ncx + P.ncx) % P.ncx;
-            else if (xx < 0 || xx >= P.ncx) continue;
-            const long long c = P.coff + (long long)wy * P.ncx + wx;
-            const int t0 = cstart[c], t1 = cend[c];
-            for (int t = t0; t < t1; t++) {
-                if (t == s) continue;
-                const double dx = wrap_d(xs - V.x[side][t], P.nx, px);
-                const double dy = wrap_d(ys - V.y[side][t], P.ny, py);
-                const double d = sqrt(dx * dx + dy * dy);
-                const int idt = V.id[side][t];
-                const double rlo = ids < idt ? rs : V.r[side][t];
-                if (d <= (rlo + P.rtree) + P.skin) f(t, d, idt);
-            }
+    walk_cells(P, xs, ys, coff, sub, [&](int t) {
+        if (t == s) return;
+        const double dx = wrap_d(xs - V.x[side][t], P.nx, px);
+        const double dy = wrap_d(ys - V.y[side][t], P.ny, py);
+        const double d = sqrt(dx * dx + dy * dy);
+        const int idt = V.id[side][t];
+        const double rlo = ids < idt ? rs : V.r[side][t];
+        if (d <= (rlo + P.rtree) + P.skin) f(t, d, idt);
+    });
+}
+
+// cnt[s], cnt[N + s]: the partners of lower and of higher id of every floe.
+__global__ void __launch_bounds__(256) k_nbr_count(Views V, int side, const int *coff, int *cnt)
+{
+    const int sub = threadIdx.x & (GRP - 1);
+    const int groups = gridDim.x * (blockDim.x / GRP);
+    // every lane of a warp runs the same rounds (the sums are warp-wide)
+    for (int s0 = blockIdx.x * (blockDim.x / GRP) + (threadIdx.x & ~31) / GRP; s0 < V.N; s0 += groups) {
+        const int s = s0 + (threadIdx.x & 31) / GRP;
+        int lo = 0, up = 0;
+        if (s < V.N) {
+            const int ids = V.id[side][s];
+            for_superset(V, side, coff, s, sub, [&](int, double, int idt) { if (idt < ids) lo++; else up++; });
+        }
+#pragma unroll
+        for (int o = GRP / 2; o > 0; o >>= 1) {
+            lo += __shfl_xor_sync(0xffffffffu, lo, o);
+            up += __shfl_xor_sync(0xffffffffu, up, o);
+        }
+        if (s < V.N && sub == 0) {
+            cnt[s] = lo;
+            cnt[V.N + s] = up;
         }
     }
 }
 
-__global__ void k_nbr_count(Views V, int side, const int *cstart, const int *cend, int *cnt)
+// Whether entry (da, ida) comes before (db, idb) in a row: partner rows and,
+// with up_by_id, owner rows by id; owner rows else by (distance, id).
+// up_by_id: the mixed path, whose per-floe sums follow the row order: the
+// order then depends only on the reference ids, not on when the rows were
+// built (the FP64 path re-sorts its owner rows by distance every step, the
+// kd-tree's order).
+GD_DEV bool row_before(double da, int ida, double db, int idb, bool by_dist)
 {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x) {
-        int c = 0;
-        for_superset(V, side, cstart, cend, s, [&](int, double, int) { c++; });
-        cnt[s] = c;
+    return by_dist ? da < db || (da == db && ida < idb) : ida < idb;
+}
+
+// The rows of every floe: off2 is the scan of k_nbr_count's counts (partner
+// rows from off2[s], owner rows from off2[N + s] - off2[N]).  A group collects
+// its floe's entries in shared memory and places each by its rank; a floe with
+// more than ROW_CAP partners is written unordered and its rows sorted in
+// place by one lane (dist: their distances, owner rows).
+constexpr int ROW_CAP = 112;
+__global__ void __launch_bounds__(128) k_nbr_fill(Views V, int side, const int *coff, const int *off2, int up_by_id,
+                                                  int *lo_off, int *up_off, int2 *ent_lo, int2 *ent_up, double *dist)
+{
+    __shared__ GroupBag<ROW_CAP> bags[128 / GRP];
+    const int sub = threadIdx.x & (GRP - 1);
+    GroupBag<ROW_CAP> &B = bags[threadIdx.x / GRP];
+    const int groups = gridDim.x * (blockDim.x / GRP), N = V.N, P = off2[N];
+    for (int s0 = blockIdx.x * (blockDim.x / GRP) + (threadIdx.x & ~31) / GRP; s0 < N; s0 += groups) {
+        const int s = s0 + (threadIdx.x & 31) / GRP;
+        if (sub == 0) B.n[0] = B.n[1] = 0;
+        __syncwarp();
+        const bool on = s < N;
+        const int ids = on ? V.id[side][s] : 0;
+        const int lo = on ? off2[s] : 0, up = on ? off2[N + s] - P : 0;
+        const int m = on ? off2[s + 1] - lo + (off2[N + s + 1] - P) - up : 0;
+        if (on && sub == 0) {
+            lo_off[s] = lo;
+            up_off[s] = up;
+            if (s == N - 1) {
+                lo_off[N] = P;
+                up_off[N] = P;
+            }
+        }
+        if (on && m <= ROW_CAP) {
+            for_superset(V, side, coff, s, sub, [&](int t, double d, int idt) {
+                const int k = atomicAdd(&B.n[0], 1);
+                B.t[k] = t;
+                B.id[k] = idt;
+                B.d[k] = d;
+            });
+        } else if (on) {
+            for_superset(V, side, coff, s, sub, [&](int t, double d, int idt) {
+                const int u = idt > ids, k = atomicAdd(&B.n[u], 1);
+                // .y holds the partner's id while the row is sorted
+                (u ? ent_up : ent_lo)[(u ? up : lo) + k] = make_int2(t, idt);
+                if (u) dist[up + k] = d;
+            });
+        }
+        __syncwarp();
+        if (on && m <= ROW_CAP) {
+            for (int k = sub; k < m; k += GRP) {
+                const int idk = B.id[k];
+                const double dk = B.d[k];
+                const bool u = idk > ids;
+                int at = 0;
+                for (int j = 0; j < m; j++)
+                    at += (B.id[j] > ids) == u && row_before(B.d[j], B.id[j], dk, idk, u && !up_by_id);
+                if (u) ent_up[up + at] = make_int2(B.t[k], up + at);      // the pair's index: its own place
+                else ent_lo[lo + at] = make_int2(B.t[k], -1);
+            }
+        } else if (on && sub == 0) {
+            for (int u = 0; u < 2; u++) {
+                int2 *e = u ? ent_up + up : ent_lo + lo;
+                double *d = dist + up;
+                const int n = B.n[u];
+                for (int a = 1; a < n; a++) {
+                    const int2 ea = e[a];
+                    const double da = u ? d[a] : 0.0;
+                    int b = a - 1;
+                    while (b >= 0 && row_before(da, ea.y, u ? d[b] : 0.0, e[b].y, u && !up_by_id)) {
+                        e[b + 1] = e[b];
+                        if (u) d[b + 1] = d[b];
+                        b--;
+                    }
+                    e[b + 1] = ea;
+                    if (u) d[b + 1] = da;
+                }
+                for (int a = 0; a < n; a++) e[a].y = u ? up + a : -1;
+            }
+        }
+        __syncwarp();
     }
 }
 
-// fills the rows of the new generation (ent2/edist2 at row_off2) and sorts
-// each row: partners of lower id ascending by id, then partners of higher id
-// ascending by (distance, id).
-// up_by_id: the partners of higher id by id as well (the mixed path, whose
-// per-floe sums follow the row order: the order then depends only on the
-// reference ids, not on when the rows were built); otherwise by distance
-// (the FP64 path re-sorts them by distance every step, the kd-tree's order).
-__global__ void k_nbr_fill(Views V, int side, const int *cstart, const int *cend, const int *row_off2,
-                           int2 *ent2, double *dist2, int *nlo2, int up_by_id)
+// What the fresh rows hold besides the partners; a group per floe.
+// Partner entries: the pair's index (ST_ROW_OVERFLOW if the partner's owner
+// row does not point back) and, mixed, its inverse and no record flag.  Owner
+// entries: row, bond index (bonds are sorted by the partner's id), no overlap,
+// and the contact history by reference ids from the previous rows (old_up_off
+// null: zero); mixed, the history flag.
+template <typename H4, bool MIXED>
+__global__ void __launch_bounds__(256) k_row_finish(Views V, int side, const int *old_slot, const int *old_up_off,
+                                                    const int2 *old_ent_up, const int *old_id, const H4 *old_hist,
+                                                    const int *up_off, const int *lo_off, const int2 *ent_up,
+                                                    int2 *ent_lo, H4 *hist, int *bidx, unsigned *erow, float *pdn,
+                                                    unsigned char *pfl, unsigned char *lfl, int *lo_of)
 {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x) {
-        const int e0 = row_off2[s], e1 = row_off2[s + 1];
-        int k = e0;
-        // .y holds the partner's id while the row is sorted (no gathers in
-        // the comparisons); it becomes the pair index afterwards
-        for_superset(V, side, cstart, cend, s, [&](int t, double d, int idt) {
-            if (k < e1) { ent2[k] = make_int2(t, idt); dist2[k] = d; }
-            k++;
-        });
+    const int sub = threadIdx.x & (GRP - 1);
+    const int groups = gridDim.x * (blockDim.x / GRP);
+    for (int s = blockIdx.x * (blockDim.x / GRP) + threadIdx.x / GRP; s < V.N; s += groups) {
         const int ids = V.id[side][s];
-        // insertion sort by (upper?, upper && !up_by_id ? dist : 0, id)
-        int nlo = 0;
-        for (int a = e0; a < e1; a++) {
-            const int2 ea = ent2[a];
-            const double da = dist2[a];
-            const int ida = ea.y;
-            const bool ua = ida > ids;
-            if (!ua) nlo++;
-            int b = a - 1;
-            while (b >= e0) {
-                const int idb = ent2[b].y;
-                const bool ub = idb > ids;
-                const double db = dist2[b];
-                bool gt;   // entry b sorts after entry a
-                if (ub != ua) gt = ub;
-                else if (!ua || up_by_id) gt = idb > ida;
-                else gt = (db > da) || (db == da && idb > ida);
-                if (!gt) break;
-                ent2[b + 1] = ent2[b];
-                dist2[b + 1] = db;
-                b--;
-            }
-            ent2[b + 1] = ea;
-            dist2[b + 1] = da;
-        }
-        nlo2[s] = nlo;
-        for (int a = e0 + nlo; a < e1; a++) ent2[a].y = a;   // pair record = upper entry
-    }
-}
-
-// pair index of every lower entry: the upper entry of the partner's row that
-// points back at s
-__global__ void k_nbr_link(Views V, const int *row_off2, const int *nlo2, int2 *ent2)
-{
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x) {
-        const int e0 = row_off2[s], el = e0 + nlo2[s];
-        for (int e = e0; e < el; e++) {
-            const int t = ent2[e].x;
-            const int q0 = row_off2[t] + nlo2[t], q1 = row_off2[t + 1];
+        for (int e = lo_off[s] + sub; e < lo_off[s + 1]; e += GRP) {
+            const int t = ent_lo[e].x;
             int found = -1;
-            for (int q = q0; q < q1; q++)
-                if (ent2[q].x == s) { found = q; break; }
-            ent2[e].y = found;
+            for (int q = up_off[t]; q < up_off[t + 1]; q++)
+                if (ent_up[q].x == s) { found = q; break; }
+            ent_lo[e].y = found;
             if (found < 0) atomicOr(V.status, ST_ROW_OVERFLOW);
+            if (MIXED) {
+                if (found >= 0) lo_of[found] = e;
+                lfl[e] = 0;
+            }
         }
-    }
-}
-
-// Splits the combined rows into the partner CSR (ent_lo: partners of lower
-// id, ascending id; .y = the pair's index) and the owner CSR (ent_up:
-// partners of higher id, ascending distance - ascending id in the mixed path;
-// .y = own index = pair index).
-__global__ void k_split_rows(int N, const int *row_off2, const int *nlo2, const int2 *ent2, const int *lo_off,
-                             const int *up_off, int2 *ent_lo, int2 *ent_up)
-{
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < N; s += gridDim.x * blockDim.x) {
-        const int e0 = row_off2[s], nl = nlo2[s], e1 = row_off2[s + 1];
-        const int lo0 = lo_off[s], up0 = up_off[s];
-        for (int k = 0; k < nl; k++) {
-            const int2 en = ent2[e0 + k];
-            const int t = en.x, q = en.y;     // q: combined index of the owner entry in t's row
-            const int pidx = q < 0 ? -1 : up_off[t] + (q - row_off2[t] - nlo2[t]);
-            ent_lo[lo0 + k] = make_int2(t, pidx);
-        }
-        for (int k = 0; k < e1 - e0 - nl; k++) {
-            const int e = e0 + nl + k;
-            ent_up[up0 + k] = make_int2(ent2[e].x, up0 + k);
-        }
-    }
-}
-
-// Contact histories of the new pairs, taken from the previous pairs by
-// reference ids; bond index of every pair.
-template <typename H4>
-__global__ void k_migrate(Views V, int side_new, const int *old_slot, const int *old_up_off, const int2 *old_ent_up,
-                          const int *old_id, const H4 *old_hist, const int *up_off2, const int2 *ent_up2, H4 *hist2,
-                          int *bidx2)
-{
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x) {
+        const int e0 = up_off[s], e1 = up_off[s + 1];
+        if (e0 == e1) continue;
         const InstParams &P = V.P[V.inst[s]];
-        const int ids = V.id[side_new][s];
         const int os = old_slot[s];
-        const int e0 = up_off2[s], e1 = up_off2[s + 1];
+        const int q0 = os >= 0 && old_up_off ? old_up_off[os] : 0, q1 = os >= 0 && old_up_off ? old_up_off[os + 1] : 0;
         const int gl = P.off + ids;
         const int b0 = V.bond_off[gl], b1 = V.bond_off[gl + 1];
-        for (int e = e0; e < e1; e++) {
-            const int idt = V.id[side_new][ent_up2[e].x];
+        for (int e = e0 + sub; e < e1; e += GRP) {
+            const int idt = V.id[side][ent_up[e].x];
             H4 h;
             h.deltat = 0; h.thetarelc = 0; h.fcn = 0; h.fct = 0;
-            if (os >= 0 && old_up_off) {
-                const int q0 = old_up_off[os], q1 = old_up_off[os + 1];
-                for (int q = q0; q < q1; q++) {
-                    const int2 oe = old_ent_up[q];
-                    if (old_id[oe.x] == idt) { h = old_hist[oe.y]; break; }
-                }
+            for (int q = q0; q < q1; q++) {
+                const int2 oe = old_ent_up[q];
+                if (old_id[oe.x] == idt) { h = old_hist[oe.y]; break; }
             }
-            hist2[e] = h;
-            // bonds of this floe are sorted by the partner's id
+            hist[e] = h;
             int lo = b0, hi = b1 - 1, bi = -1;
             while (lo <= hi) {
                 const int mid = (lo + hi) >> 1;
@@ -445,11 +462,16 @@ __global__ void k_migrate(Views V, int side_new, const int *old_slot, const int 
                 if (v == idt) { bi = mid; break; }
                 if (v < idt) lo = mid + 1; else hi = mid - 1;
             }
-            bidx2[e] = bi;
+            bidx[e] = bi;
+            erow[e] = (unsigned)s;
+            pdn[e] = __int_as_float(-1);       // a NaN: not a candidate
+            if (MIXED) pfl[e] = h.deltat != 0 || h.thetarelc != 0 ? 1 : 0;     // PF_HIST
         }
     }
 }
 
+// Ids and rebuild positions on both sides (after the histories moved: they
+// are found by the previous layout's ids).
 __global__ void k_copy_ids(Views V, int from)
 {
     const int to = from ^ 1;
@@ -461,73 +483,55 @@ __global__ void k_copy_ids(Views V, int from)
 }
 
 // ------------------------------------------------------------ host side
-static int grid_for(int n, int block) { return n <= 0 ? 1 : (int)std::min<long long>((n + block - 1) / block, 148LL * 16); }
-
-void launch_cell_keys(const Views &V, int cur, uint32_t *keys, int *vals, cudaStream_t st)
+static int grid_for(long long n, int block)
 {
-    k_cell_keys<<<grid_for(V.N, 256), 256, 0, st>>>(V, cur, keys, vals);
+    return n <= 0 ? 1 : (int)std::min<long long>((n + block - 1) / block, 148LL * 16);
 }
 
-void launch_permute(const Views &V, int cur, const int *vals, const int *repack, int *old_slot, cudaStream_t st)
+void launch_cell_list(const Views &V, int cur, int s0, int n, long long C, uint32_t *keys, int *cnt, int *coff,
+                      int *list, int *scan_scratch, cudaStream_t st)
 {
-    k_permute<<<grid_for(V.N, 256), 256, 0, st>>>(V, cur, vals, repack, old_slot);
+    cudaMemsetAsync(cnt, 0, (size_t)C * 4, st);
+    k_cell_count<<<grid_for(n, 256), 256, 0, st>>>(V, cur, s0, n, keys, cnt);
+    scan_excl(cnt, coff, (int)C, scan_scratch, st);
+    k_cell_scatter<<<grid_for(n, 256), 256, 0, st>>>(s0, n, keys, coff, cnt, list);
 }
 
-void launch_cell_ranges(const uint32_t *keys, int n, int *cstart, int *cend, cudaStream_t st)
+void launch_cell_place(const Views &V, int cur, const uint32_t *keys, const int *coff, const int *list,
+                       const int *repack, int *old_slot, cudaStream_t st)
 {
-    k_cell_ranges<<<grid_for(n, 256), 256, 0, st>>>(keys, n, cstart, cend);
+    k_cell_place<<<grid_for(V.N, 256), 256, 0, st>>>(V, cur, keys, coff, list, repack, old_slot);
 }
 
-void launch_nbr_count(const Views &V, int side, const int *cstart, const int *cend, int *cnt, cudaStream_t st)
+void launch_nbr_count(const Views &V, int side, const int *coff, int *cnt, int *off2, int *scan_scratch,
+                      cudaStream_t st)
 {
-    k_nbr_count<<<grid_for(V.N, 128), 128, 0, st>>>(V, side, cstart, cend, cnt);
+    k_nbr_count<<<grid_for((long long)V.N * GRP, 256), 256, 0, st>>>(V, side, coff, cnt);
+    scan_excl(cnt, off2, 2 * V.N, scan_scratch, st);
 }
 
-void launch_nbr_fill(const Views &V, int side, const int *cstart, const int *cend, const int *row_off2,
-                     int2 *ent2, double *dist2, int *nlo2, int up_by_id, cudaStream_t st)
+void launch_nbr_fill(const Views &V, int side, const int *coff, const int *off2, int up_by_id, int *lo_off,
+                     int *up_off, int2 *ent_lo, int2 *ent_up, double *dist, cudaStream_t st)
 {
-    k_nbr_fill<<<grid_for(V.N, 128), 128, 0, st>>>(V, side, cstart, cend, row_off2, ent2, dist2, nlo2, up_by_id);
+    k_nbr_fill<<<grid_for((long long)V.N * GRP, 128), 128, 0, st>>>(V, side, coff, off2, up_by_id, lo_off, up_off,
+                                                                    ent_lo, ent_up, dist);
 }
 
-void launch_nbr_link(const Views &V, const int *row_off2, const int *nlo2, int2 *ent2, cudaStream_t st)
+void launch_row_finish(const Views &V, int mixed, int side, const int *old_slot, const int *old_up_off,
+                       const int2 *old_ent_up, const int *old_id, const void *old_hist, const int *up_off,
+                       const int *lo_off, const int2 *ent_up, int2 *ent_lo, void *hist, int *bidx, unsigned *erow,
+                       float *pdn, unsigned char *pfl, unsigned char *lfl, int *lo_of, cudaStream_t st)
 {
-    k_nbr_link<<<grid_for(V.N, 128), 128, 0, st>>>(V, row_off2, nlo2, ent2);
-}
-
-void launch_split_rows(int N, const int *row_off2, const int *nlo2, const int2 *ent2, const int *lo_off,
-                       const int *up_off, int2 *ent_lo, int2 *ent_up, cudaStream_t st)
-{
-    k_split_rows<<<grid_for(N, 128), 128, 0, st>>>(N, row_off2, nlo2, ent2, lo_off, up_off, ent_lo, ent_up);
-}
-
-void launch_migrate(const Views &V, int fp64, int side_new, const int *old_slot, const int *old_up_off,
-                    const int2 *old_ent_up, const int *old_id, const void *old_hist, const int *up_off2,
-                    const int2 *ent_up2, void *hist2, int *bidx2, cudaStream_t st)
-{
-    if (fp64)
-        k_migrate<Hist4<double>><<<grid_for(V.N, 128), 128, 0, st>>>(
-            V, side_new, old_slot, old_up_off, old_ent_up, old_id, (const Hist4<double> *)old_hist, up_off2,
-            ent_up2, (Hist4<double> *)hist2, bidx2);
+    const int grid = grid_for((long long)V.N * GRP, 256);
+    if (mixed)
+        k_row_finish<Hist4<float>, true><<<grid, 256, 0, st>>>(
+            V, side, old_slot, old_up_off, old_ent_up, old_id, (const Hist4<float> *)old_hist, up_off, lo_off, ent_up,
+            ent_lo, (Hist4<float> *)hist, bidx, erow, pdn, pfl, lfl, lo_of);
     else
-        k_migrate<Hist4<float>><<<grid_for(V.N, 128), 128, 0, st>>>(
-            V, side_new, old_slot, old_up_off, old_ent_up, old_id, (const Hist4<float> *)old_hist, up_off2,
-            ent_up2, (Hist4<float> *)hist2, bidx2);
-}
-
-__global__ void k_row_lengths(int N, const int *row_off2, const int *nlo2, int *nup)
-{
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < N; s += gridDim.x * blockDim.x)
-        nup[s] = row_off2[s + 1] - row_off2[s] - nlo2[s];
-}
-
-void launch_row_lengths(int N, const int *row_off2, const int *nlo2, int *nup, cudaStream_t st)
-{
-    k_row_lengths<<<grid_for(N, 256), 256, 0, st>>>(N, row_off2, nlo2, nup);
-}
-
-void launch_copy_ids(const Views &V, int from, cudaStream_t st)
-{
-    k_copy_ids<<<grid_for(V.N, 256), 256, 0, st>>>(V, from);
+        k_row_finish<Hist4<double>, false><<<grid, 256, 0, st>>>(
+            V, side, old_slot, old_up_off, old_ent_up, old_id, (const Hist4<double> *)old_hist, up_off, lo_off, ent_up,
+            ent_lo, (Hist4<double> *)hist, bidx, erow, pdn, pfl, lfl, lo_of);
+    k_copy_ids<<<grid_for(V.N, 256), 256, 0, st>>>(V, side);
 }
 
 }  // namespace godar

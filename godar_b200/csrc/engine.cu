@@ -115,9 +115,8 @@ struct Buf {
     }
     void release(std::atomic<size_t> *acct) { if (p) { free_mem(); if (acct) *acct -= bytes; } p = nullptr; bytes = 0; }
     template <class T> T *as() const { return (T *)p; }
+    void swap(Buf &o) { std::swap(p, o.p); std::swap(bytes, o.bytes); std::swap(pooled, o.pooled); }
 };
-
-inline int ilog2ceil(uint64_t v) { int b = 0; while ((1ULL << b) < v) b++; return b; }
 
 // ------------------------------------------------------------ instances
 struct HostBonds {           // one instance's bond table, id order
@@ -538,10 +537,11 @@ struct Engine {
     Buf flisted_b, fupn_b, flon_b, fpart_b, fpos_b, fplist_b;
     long long Lc = 0;
     long long Ec = 0;             // mixed path: owner entries on the contact list
-    Buf brec, bdg, bsp, bst32, bflag_b, wdyn_b, wsp_b, winv_b, perm_b, wfo_b, bfo, slot_of, blo_start, blo_end, bkeys, bvals, bkeys_alt, bvals_alt, brs_counts, bscan;
-    Buf row_off2, nlo2, ent2, dist2, cnt, old_slot;
-    Buf up_off2, lo_off2, nup, ent_up2, ent_lo2, bidx2, hist2;
-    Buf keys, vals, keys_alt, vals_alt, rs_counts, scan_scratch, cstart, cend;
+    Buf brec, bdg, bsp, bst32, bflag_b, wdyn_b, wsp_b, winv_b, perm_b, bfo, slot_of, blo_b, blist_b;
+    // (rows under construction; they change places with the primary ones)
+    Buf row_off2, dist2, cnt, old_slot;
+    Buf up_off2, lo_off2, ent_up2, ent_lo2, bidx2, hist2;
+    Buf keys, vals, scan_scratch, coff_b, ccnt_b;
     // mixed path: the screening's displacement bound (see k_pairs_screen)
     Buf dsp_b;
     // outputs and status
@@ -894,15 +894,13 @@ struct Engine {
     int alloc_scratch(int n) {
         auto ens = [&](Buf &b, size_t s) { return b.ensure(s, &bytes, &mp); };
         TRY(ens(inst_b, (size_t)n * 4));
-        TRY(ens(row_off2, (size_t)(n + 1) * 4)); TRY(ens(nlo2, (size_t)(n + 1) * 4));
+        TRY(ens(row_off2, (size_t)(2 * n + 1) * 4));
         TRY(ens(up_off2, (size_t)(n + 1) * 4)); TRY(ens(lo_off2, (size_t)(n + 1) * 4));
-        TRY(ens(nup, (size_t)(n + 1) * 4));
-        TRY(ens(cnt, (size_t)(n + 1) * 4)); TRY(ens(old_slot, (size_t)n * 4));
+        TRY(ens(cnt, (size_t)(2 * n + 1) * 4)); TRY(ens(old_slot, (size_t)n * 4));
         TRY(ens(keys, (size_t)n * 4)); TRY(ens(vals, (size_t)n * 4));
-        TRY(ens(keys_alt, (size_t)n * 4)); TRY(ens(vals_alt, (size_t)n * 4));
-        const size_t ntiles = (n + 2047) / 2048;
-        TRY(ens(rs_counts, (256 * ntiles + 1) * 4));
-        TRY(ens(scan_scratch, (256 * ntiles / 2048 + 64 + n / 2048 + 64) * 4));
+        // scans over 2 n counts and over the cells
+        TRY(ens(scan_scratch, ((2 * (size_t)n + (size_t)C) / 2048 + 64) * 4));
+        TRY(ens(coff_b, (size_t)(C + 1) * 4)); TRY(ens(ccnt_b, (size_t)std::max<long long>(C, 1) * 4));
         TRY(ens(diag, (size_t)14 * n * 8));
         TRY(ens(tmp_out, (size_t)n * 8));
         return GODAR_OK;
@@ -933,13 +931,10 @@ struct Engine {
         TRY(ens(rule_b, (size_t)ni * sizeof(BondRule)));
         std::vector<BondRule> r = bond_rules(fresh);
         CK(cudaMemcpyAsync(rule_b.p, r.data(), r.size() * sizeof(BondRule), cudaMemcpyHostToDevice, st));
-        CK(cudaMemsetAsync(cstart.p, 0, (size_t)C * 4, st));
-        CK(cudaMemsetAsync(cend.p, 0, (size_t)C * 4, st));
-        const int bits = std::max(1, ilog2ceil((uint64_t)std::max<long long>(C, 2)));
-        launch_bond_init_count(views(), 0, s0, n, rule_b.as<BondRule>(), keys.as<uint32_t>(), vals.as<int>(),
-                               keys_alt.as<uint32_t>(), vals_alt.as<int>(), bits, rs_counts.as<int>(),
-                               scan_scratch.as<int>(), cstart.as<int>(), cend.as<int>(), cnt.as<int>(),
-                               row_off2.as<int>(), st);
+        launch_cell_list(views(), 0, s0, n, C, keys.as<uint32_t>(), ccnt_b.as<int>(), coff_b.as<int>(), vals.as<int>(),
+                         scan_scratch.as<int>(), st);
+        launch_bond_init_count(views(), 0, s0, n, rule_b.as<BondRule>(), coff_b.as<int>(), vals.as<int>(),
+                               scan_scratch.as<int>(), cnt.as<int>(), row_off2.as<int>(), st);
         // per fresh field: its bonds = scan[last] - scan[first]
         std::vector<int> fi, la, which;
         for (int k = 0; k < ni; k++)
@@ -972,8 +967,8 @@ struct Engine {
     int fill_fresh_bonds(int s0, const std::vector<char> &fresh) {
         std::vector<BondRule> r = bond_rules(fresh);
         CK(cudaMemcpyAsync(rule_b.p, r.data(), r.size() * sizeof(BondRule), cudaMemcpyHostToDevice, st));
-        launch_bond_init_fill(views(), 0, s0, N - s0, rule_b.as<BondRule>(), cstart.as<int>(), cend.as<int>(),
-                              vals.as<int>(), row_off2.as<int>(), BS->bond_off.as<int>(), BS->bond_hi.as<int>(),
+        launch_bond_init_fill(views(), 0, s0, N - s0, rule_b.as<BondRule>(), coff_b.as<int>(), vals.as<int>(),
+                              row_off2.as<int>(), BS->bond_off.as<int>(), BS->bond_hi.as<int>(),
                               BS->bstat.as<BondStat>(), BS->bdyn[0].as<BondDyn>(), st);
         CK(cudaGetLastError());
         return GODAR_OK;
@@ -1061,10 +1056,10 @@ struct Engine {
         std::unique_ptr<BondSet> oldB = std::move(BS);
         F = spareF ? std::move(spareF) : std::make_unique<FloeSet>();
         BS = spareB ? std::move(spareB) : std::make_unique<BondSet>();
-        TRY(alloc_floe_set(*F, n_tot));
-        TRY(alloc_scratch(n_tot));
         const int old_cur = cur;
         N = n_tot; C = c_tot;
+        TRY(alloc_floe_set(*F, n_tot));
+        TRY(alloc_scratch(n_tot));
         const int sn = 0;
         auto up = [&](void *dst, const void *src, size_t nbytes) -> int {
             if (nbytes) CK(cudaMemcpyAsync(dst, src, nbytes, cudaMemcpyHostToDevice, st));
@@ -1076,8 +1071,6 @@ struct Engine {
         hparams = hp;
         TRY(field_b.ensure(std::max<size_t>(hfield.size(), 1) * 8, &bytes, &mp));
         TRY(up(field_b.p, hfield.data(), hfield.size() * 8));
-        TRY(cstart.ensure((size_t)std::max<long long>(C, 1) * 4, &bytes, &mp));
-        TRY(cend.ensure((size_t)std::max<long long>(C, 1) * 4, &bytes, &mp));
         // resident floes, device to device
         TRY(repack_b.ensure((size_t)std::max(N, 1) * 4, &bytes, &mp));
         TRY(up(repack_b.p, repack.data(), (size_t)N * 4));
@@ -1341,54 +1334,29 @@ struct Engine {
         Views V = views();
         const int nxt = cur ^ 1;
         const bool have_old = have_rows && (repack ? migrate_from_old : true);
-        launch_cell_keys(V, cur, keys.as<uint32_t>(), vals.as<int>(), st);
-        const int bits = std::max(1, ilog2ceil((uint64_t)std::max<long long>(C, 2)));
-        radix_sort(keys.as<uint32_t>(), vals.as<int>(), keys_alt.as<uint32_t>(), vals_alt.as<int>(), N, bits,
-                   rs_counts.as<int>(), scan_scratch.as<int>(), st);
-        launch_permute(V, cur, vals.as<int>(), repack, old_slot.as<int>(), st);
-        CK(cudaMemsetAsync(cstart.p, 0, (size_t)C * 4, st));
-        CK(cudaMemsetAsync(cend.p, 0, (size_t)C * 4, st));
-        launch_cell_ranges(keys.as<uint32_t>(), N, cstart.as<int>(), cend.as<int>(), st);
-        launch_nbr_count(V, nxt, cstart.as<int>(), cend.as<int>(), cnt.as<int>(), st);
-        scan_excl(cnt.as<int>(), row_off2.as<int>(), N, scan_scratch.as<int>(), st);
-        int Enew = 0;
-        CK(cudaMemcpyAsync(&Enew, row_off2.as<int>() + N, sizeof(int), cudaMemcpyDeviceToHost, st));
+        launch_cell_list(V, cur, 0, N, C, keys.as<uint32_t>(), ccnt_b.as<int>(), coff_b.as<int>(), vals.as<int>(),
+                         scan_scratch.as<int>(), st);
+        launch_cell_place(V, cur, keys.as<uint32_t>(), coff_b.as<int>(), vals.as<int>(), repack, old_slot.as<int>(), st);
+        launch_nbr_count(V, nxt, coff_b.as<int>(), cnt.as<int>(), row_off2.as<int>(), scan_scratch.as<int>(), st);
+        // pairs, and entries of both rows (in the status mirror's spare ints)
+        int *h_n = h_status + 2;
+        CK(cudaMemcpyAsync(h_n, row_off2.as<int>() + N, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(h_n + 1, row_off2.as<int>() + 2 * N, sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        if (Enew < 0) { set_err("neighbour rows overflow int32"); return GODAR_ERR_CAPACITY; }
-        if (Enew % 2) { set_err("asymmetric neighbour rows"); return GODAR_ERR_CAPACITY; }
-        const int Pn = Enew / 2;
+        const int Pn = h_n[0], Enew = h_n[1];
+        if (Enew < 0 || Pn < 0) { set_err("neighbour rows overflow int32"); return GODAR_ERR_CAPACITY; }
+        if (Enew != 2 * Pn) { set_err("asymmetric neighbour rows"); return GODAR_ERR_CAPACITY; }
         const size_t he = hist_elem();
         auto ens = [&](Buf &b, size_t s) { return b.ensure(std::max<size_t>(s, 16), &bytes, &mp); };
-        TRY(ens(ent2, (size_t)Enew * 8)); TRY(ens(dist2, (size_t)Enew * 8));
-        TRY(ens(ent_up2, (size_t)Pn * 8)); TRY(ens(ent_lo2, (size_t)Pn * 8));
-        TRY(ens(bidx2, (size_t)Pn * 4)); TRY(ens(hist2, (size_t)Pn * he));
-        launch_nbr_fill(V, nxt, cstart.as<int>(), cend.as<int>(), row_off2.as<int>(), ent2.as<int2>(),
-                        dist2.as<double>(), nlo2.as<int>(), prec == GODAR_PREC_FP64 ? 0 : 1, st);
-        launch_nbr_link(V, row_off2.as<int>(), nlo2.as<int>(), ent2.as<int2>(), st);
-        // split into owner and partner rows
-        launch_row_lengths(N, row_off2.as<int>(), nlo2.as<int>(), nup.as<int>(), st);
-        scan_excl(nlo2.as<int>(), lo_off2.as<int>(), N, scan_scratch.as<int>(), st);
-        scan_excl(nup.as<int>(), up_off2.as<int>(), N, scan_scratch.as<int>(), st);
-        launch_split_rows(N, row_off2.as<int>(), nlo2.as<int>(), ent2.as<int2>(), lo_off2.as<int>(), up_off2.as<int>(), ent_lo2.as<int2>(), ent_up2.as<int2>(), st);
         const bool fp64 = prec == GODAR_PREC_FP64;
-        {
-            // without a previous generation of rows every history starts at zero
-            const int *o_up_off = have_old ? up_off.as<int>() : nullptr;
-            const int *o_id = old_ids ? old_ids : F->id[cur].as<int>();
-            launch_migrate(V, fp64, nxt, old_slot.as<int>(), o_up_off, ent_up.as<int2>(), o_id,
-                           hist[0].p, up_off2.as<int>(), ent_up2.as<int2>(), hist2.p, bidx2.as<int>(), st);
-            CK(cudaStreamSynchronize(st));
-        }
-        // the new generation becomes the primary rows
         if ((long long)Pn > Ecap) {
-            CK(cudaStreamSynchronize(st));
+            // what the previous rows hold in these does not outlive them
             const long long cap = (long long)(Pn * 1.25) + 1024;
-            Buf *pb[] = {&ent_up, &ent_lo, &bidx, &hist[0], &edist, &pdn, &erow_up, &lo_of, &pfl, &lfl,
+            Buf *pb[] = {&edist, &pdn, &erow_up, &lo_of, &pfl, &lfl,
                          &prec_b, &prx_b, &pdg_b, &work_b, &work_st_b, &clist_b, &cscan_b, &frec_b, &fwork1_b,
                          &flisted_b, &fpart_b, &fplist_b};
             for (Buf *b : pb) b->release(&bytes);
-            TRY(ens(ent_up, cap * 8)); TRY(ens(ent_lo, cap * 8)); TRY(ens(bidx, cap * 4));
-            TRY(ens(hist[0], cap * he)); TRY(ens(pdn, cap * 4));
+            TRY(ens(pdn, cap * 4));
             if (fp64) {
                 TRY(ens(edist, cap * 8));
                 TRY(ens(erow_up, cap * 4)); TRY(ens(pfl, cap + 16));
@@ -1405,22 +1373,24 @@ struct Engine {
             }
             Ecap = cap;
         }
-        if (up_off.bytes < (size_t)(N + 1) * 4 || lo_off.bytes < (size_t)(N + 1) * 4) {
-            CK(cudaStreamSynchronize(st));
-            TRY(ens(up_off, (size_t)(N + 1) * 4));
-            TRY(ens(lo_off, (size_t)(N + 1) * 4));
-        }
-        CK(cudaMemcpyAsync(up_off.p, up_off2.p, (size_t)(N + 1) * 4, cudaMemcpyDeviceToDevice, st));
-        CK(cudaMemcpyAsync(lo_off.p, lo_off2.p, (size_t)(N + 1) * 4, cudaMemcpyDeviceToDevice, st));
-        if (Pn) {
-            CK(cudaMemcpyAsync(ent_up.p, ent_up2.p, (size_t)Pn * 8, cudaMemcpyDeviceToDevice, st));
-            CK(cudaMemcpyAsync(ent_lo.p, ent_lo2.p, (size_t)Pn * 8, cudaMemcpyDeviceToDevice, st));
-            CK(cudaMemcpyAsync(bidx.p, bidx2.p, (size_t)Pn * 4, cudaMemcpyDeviceToDevice, st));
-            CK(cudaMemcpyAsync(hist[0].p, hist2.p, (size_t)Pn * he, cudaMemcpyDeviceToDevice, st));
-            CK(cudaMemsetAsync(pdn.p, 0xff, (size_t)Pn * 4, st));
-        }
-        launch_copy_ids(V, nxt, st);
-        launch_fill_erow(up_off.as<int>(), N, erow_up.as<unsigned>(), st);
+        TRY(ens(up_off2, (size_t)(N + 1) * 4)); TRY(ens(lo_off2, (size_t)(N + 1) * 4));
+        // (two ints an entry also serve the contact list's marks and positions)
+        TRY(ens(dist2, (size_t)(Ecap + 2) * 8));
+        TRY(ens(ent_up2, (size_t)Ecap * 8)); TRY(ens(ent_lo2, (size_t)Ecap * 8));
+        TRY(ens(bidx2, (size_t)Ecap * 4)); TRY(ens(hist2, (size_t)Ecap * he));
+        launch_nbr_fill(V, nxt, coff_b.as<int>(), row_off2.as<int>(), fp64 ? 0 : 1, lo_off2.as<int>(),
+                        up_off2.as<int>(), ent_lo2.as<int2>(), ent_up2.as<int2>(), dist2.as<double>(), st);
+        // without a previous generation of rows every history starts at zero
+        launch_row_finish(V, fp64 ? 0 : 1, nxt, old_slot.as<int>(), have_old ? up_off.as<int>() : nullptr,
+                          ent_up.as<int2>(), old_ids ? old_ids : F->id[cur].as<int>(), hist[0].p, up_off2.as<int>(),
+                          lo_off2.as<int>(), ent_up2.as<int2>(), ent_lo2.as<int2>(), hist2.p, bidx2.as<int>(),
+                          erow_up.as<unsigned>(), pdn.as<float>(), pfl.as<unsigned char>(), lfl.as<unsigned char>(),
+                          lo_of.as<int>(), st);
+        // the new generation becomes the primary rows
+        up_off.swap(up_off2); lo_off.swap(lo_off2);
+        ent_up.swap(ent_up2); ent_lo.swap(ent_lo2);
+        bidx.swap(bidx2); hist[0].swap(hist2);
+        V = views();
         if (fp64) {
             E = Pn;
             TRY(fp64_rows(nxt));
@@ -1430,8 +1400,6 @@ struct Engine {
         // per-floe sums: the FP64 path's ordered record sums, the mixed path's window partials
         TRY(fsum_b.ensure((size_t)N * (fp64 ? 8 * FP64_FLOE_SUMS : 32), &bytes, &mp));
         if (!fp64) {
-            launch_mixed_rows_init(Pn, ent_lo.as<int2>(), hist[0].p, lo_of.as<int>(), pfl.as<unsigned char>(),
-                                   lfl.as<unsigned char>(), st);
             TRY(frex_b.ensure((size_t)N * 4, &bytes, &mp));
             TRY(fdg_b.ensure((size_t)N * 32, &bytes, &mp));
             launch_pack_snap(V, nxt, st);
@@ -1456,7 +1424,7 @@ struct Engine {
     int contact_list(int side, int P) {
         Ec = 0;
         if (P <= 0) return GODAR_OK;
-        int *mark = ent2.as<int>(), *pos = mark + P;
+        int *mark = dist2.as<int>(), *pos = mark + P;
         launch_contact_list(views(), side, P, erow_up.as<unsigned>(), pfl.as<unsigned char>(), mark, pos,
                             cscan_b.as<int>(), clist_b.as<int2>(), clist_b.as<int2>() + Ecap, st);
         int ec = 0;
@@ -1489,7 +1457,7 @@ struct Engine {
         B.pfl = pfl.as<unsigned char>(); B.lfl = lfl.as<unsigned char>(); B.lo_of = lo_of.as<int>();
         B.rec = prec_b.as<float4>(); B.rx = prx_b.as<float2>(); B.pdg = pdg_b.as<float4>();
         B.brec = brec.as<float4>(); B.bdg = bdg.as<float4>(); B.bsp = wsp_b.as<int4>(); B.wdyn = wdyn_b.as<BondDyn>(); B.winv = winv_b.as<int>();
-        B.blo_start = blo_start.as<int>(); B.blo_end = blo_end.as<int>(); B.blo_idx = bvals.as<int>();
+        
         B.work = work_b.as<int>(); B.nwork = nwork_b.as<int>(); B.work_st = work_st_b.as<int2>();
         B.bfo = bfo.as<int>(); B.bst = bst32.as<BondGeom32>();
         B.fsum = fsum_b.as<float4>(); B.frex = frex_b.as<float>(); B.fdg = fdg_b.as<float4>();
@@ -1511,36 +1479,24 @@ struct Engine {
 
     int mixed_bond_lists(int side) {
         auto ens = [&](Buf &b, size_t sz) { return b.ensure(std::max<size_t>(sz, 16), &bytes, &mp); };
-        TRY(ens(slot_of, (size_t)N * 4)); TRY(ens(blo_start, (size_t)N * 4)); TRY(ens(blo_end, (size_t)N * 4));
         TRY(ens(bfo, (size_t)(N + 1) * 4));
-        CK(cudaMemsetAsync(blo_start.p, 0, (size_t)N * 4, st));
-        CK(cudaMemsetAsync(blo_end.p, 0, (size_t)N * 4, st));
         if (NB == 0) {
             CK(cudaMemsetAsync(bfo.p, 0, (size_t)(N + 1) * 4, st));
             return GODAR_OK;
         }
-        const size_t nt = ((size_t)NB + 2047) / 2048;
+        TRY(ens(slot_of, (size_t)N * 4)); TRY(ens(blo_b, (size_t)(N + 1) * 4)); TRY(ens(blist_b, (size_t)NB * 4));
         TRY(ens(brec, (size_t)NB * 32)); TRY(ens(bdg, (size_t)NB * 64)); TRY(ens(bsp, (size_t)NB * 16));
         TRY(ens(bst32, (size_t)NB * sizeof(BondGeom32)));
         TRY(ens(bflag_b, (size_t)NB * 2));
         TRY(ens(wdyn_b, (size_t)NB * sizeof(BondDyn))); TRY(ens(wsp_b, (size_t)NB * 16));
-        TRY(ens(winv_b, (size_t)NB * 4)); TRY(ens(perm_b, (size_t)NB * 4)); TRY(ens(wfo_b, (size_t)(N + 1) * 4));
-        TRY(ens(bkeys, (size_t)NB * 4)); TRY(ens(bvals, (size_t)NB * 4));
-        TRY(ens(bkeys_alt, (size_t)NB * 4)); TRY(ens(bvals_alt, (size_t)NB * 4));
-        TRY(ens(brs_counts, (256 * nt + 1) * 4));
-        TRY(ens(bscan, (256 * nt / 2048 + 64 + (size_t)NB / 2048 + 64) * 4));
-        Views V = views();
-        launch_bond_slots(V, side, slot_of.as<int>(), bsp.as<int4>(), bkeys.as<uint32_t>(), bvals.as<int>(), st);
-        const int bits = std::max(1, ilog2ceil((uint64_t)std::max(N, 2)));
-        radix_sort(bkeys.as<uint32_t>(), bvals.as<int>(), bkeys_alt.as<uint32_t>(), bvals_alt.as<int>(), NB, bits,
-                   brs_counts.as<int>(), bscan.as<int>(), st);
-        launch_cell_ranges(bkeys.as<uint32_t>(), NB, blo_start.as<int>(), blo_end.as<int>(), st);
-        launch_bond_positions(V, side, blo_start.as<int>(), blo_end.as<int>(), bvals.as<int>(), cnt.as<int>(),
-                              bfo.as<int>(), scan_scratch.as<int>(), bsp.as<int4>(), st);
+        TRY(ens(winv_b, (size_t)NB * 4)); TRY(ens(perm_b, (size_t)NB * 4));
         CK(cudaMemsetAsync(brec.p, 0, (size_t)NB * 32, st));
-        launch_bond_work(V, side, NB, cnt.as<int>(), wfo_b.as<int>(), scan_scratch.as<int>(), perm_b.as<int>(),
-                         BS->bstat.as<BondStat>(), BS->bdyn[0].as<BondDyn>(), bsp.as<int4>(), bst32.as<BondGeom32>(),
-                         wdyn_b.as<BondDyn>(), wsp_b.as<int4>(), winv_b.as<int>(), bflag_b.as<unsigned char>(), st);
+        // (old_slot and the rows' counts and offsets are free by now)
+        launch_bond_lists(views(), side, NB, slot_of.as<int>(), bsp.as<int4>(), old_slot.as<int>(), blo_b.as<int>(),
+                          blist_b.as<int>(), cnt.as<int>(), row_off2.as<int>(), scan_scratch.as<int>(), bfo.as<int>(),
+                          perm_b.as<int>(), BS->bstat.as<BondStat>(), BS->bdyn[0].as<BondDyn>(),
+                          bst32.as<BondGeom32>(), wdyn_b.as<BondDyn>(), wsp_b.as<int4>(), winv_b.as<int>(),
+                          bflag_b.as<unsigned char>(), st);
         wnb = NB;
         wdirty = false;
         return GODAR_OK;
@@ -2085,8 +2041,8 @@ struct Engine {
         // free between steps and mostly large enough
         const int per = (int)std::max<size_t>(1, std::min<size_t>(24, (32u << 20) / one));
         const size_t need = std::min(nf, per) * one;
-        double *dev = ent2.as<double>();
-        if (ent2.bytes < need) {
+        double *dev = hist2.as<double>();
+        if (hist2.bytes < need) {
             TRY(tmp_out.ensure(need, &bytes, &mp));
             dev = tmp_out.as<double>();
         }

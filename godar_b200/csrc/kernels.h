@@ -59,20 +59,23 @@ inline bool launch_cluster(bool pdl, void (*kern)(Params...), long long items, c
 void scan_excl(const int *in, int *out, int n, int *scratch, cudaStream_t st);
 void radix_sort(uint32_t *keys, int *vals, uint32_t *keys_alt, int *vals_alt, int n, int bits,
                 int *counts, int *scratch, cudaStream_t st);
-void launch_cell_keys(const Views &V, int cur, uint32_t *keys, int *vals, cudaStream_t st);
-void launch_permute(const Views &V, int cur, const int *vals, const int *repack, int *old_slot, cudaStream_t st);
-void launch_cell_ranges(const uint32_t *keys, int n, int *cstart, int *cend, cudaStream_t st);
-void launch_nbr_count(const Views &V, int side, const int *cstart, const int *cend, int *cnt, cudaStream_t st);
-void launch_nbr_fill(const Views &V, int side, const int *cstart, const int *cend, const int *row_off2,
-                     int2 *ent2, double *dist2, int *nlo2, int up_by_id, cudaStream_t st);
-void launch_nbr_link(const Views &V, const int *row_off2, const int *nlo2, int2 *ent2, cudaStream_t st);
-void launch_split_rows(int N, const int *row_off2, const int *nlo2, const int2 *ent2, const int *lo_off,
-                       const int *up_off, int2 *ent_lo, int2 *ent_up, cudaStream_t st);
-void launch_row_lengths(int N, const int *row_off2, const int *nlo2, int *nup, cudaStream_t st);
-void launch_migrate(const Views &V, int fp64, int side_new, const int *old_slot, const int *old_up_off,
-                    const int2 *old_ent_up, const int *old_id, const void *old_hist, const int *up_off2,
-                    const int2 *ent_up2, void *hist2, int *bidx2, cudaStream_t st);
-void launch_copy_ids(const Views &V, int from, cudaStream_t st);
+// The cell list of floes [s0, s0 + n) over C cells: keys (n ints), the cells'
+// offsets coff (C + 1), their floes (list, n, any order within a cell); cnt: C.
+void launch_cell_list(const Views &V, int cur, int s0, int n, long long C, uint32_t *keys, int *cnt, int *coff,
+                      int *list, int *scan_scratch, cudaStream_t st);
+// The floes' state from side cur into cell order on the other side.
+void launch_cell_place(const Views &V, int cur, const uint32_t *keys, const int *coff, const int *list,
+                       const int *repack, int *old_slot, cudaStream_t st);
+// The counts of every floe's partners (cnt: 2 N) and their scan (off2: 2 N + 1;
+// off2[N] pairs), then the rows.
+void launch_nbr_count(const Views &V, int side, const int *coff, int *cnt, int *off2, int *scan_scratch,
+                      cudaStream_t st);
+void launch_nbr_fill(const Views &V, int side, const int *coff, const int *off2, int up_by_id, int *lo_off,
+                     int *up_off, int2 *ent_lo, int2 *ent_up, double *dist, cudaStream_t st);
+void launch_row_finish(const Views &V, int mixed, int side, const int *old_slot, const int *old_up_off,
+                       const int2 *old_ent_up, const int *old_id, const void *old_hist, const int *up_off,
+                       const int *lo_off, const int2 *ent_up, int2 *ent_lo, void *hist, int *bidx, unsigned *erow,
+                       float *pdn, unsigned char *pfl, unsigned char *lfl, int *lo_of, cudaStream_t st);
 
 // The FP64 time step: (b) a screen of every owner entry (distance,
 // candidate test, the entries that need no pair physics) and the pair
@@ -133,8 +136,6 @@ struct MixedBufs {
     const unsigned char *bfl_rd;   // [NB] live-bond flags at the start of the step
     unsigned char *bfl_wr;         // [NB] ... at its end (the other side)
     int4 *bsp;                  // [NB] slots of the bond's two floes, positions of their records (working order)
-    int *blo_start, *blo_end;   // [N] by global id: range of the floe's partner bonds in blo_idx
-    int *blo_idx;               // [NB] bond indices ordered by the higher id
     int *work, *nwork;          // [P] owner entries for the full pair computation, and their count
     int2 *work_st;              // [P] their row and partner slots (not on diagnostic steps)
     float4 *fsum;               // [2N] per floe: fcx fcy mc fbx | fby mb shelter(air) shelter(water)
@@ -144,18 +145,14 @@ struct MixedBufs {
                                 // the largest squared step of any floe (FP32 bits, rounded up),
                                 // then per side the cumulative bound D (FP32 bits); zero at a rebuild
 };
-void launch_fill_erow(const int *off, int N, unsigned *erow, cudaStream_t st);
 void launch_pack_snap(const Views &V, int side, cudaStream_t st);
-void launch_mixed_rows_init(int P, const int2 *ent_lo, const void *hist, int *lo_of, unsigned char *pfl,
-                            unsigned char *lfl, cudaStream_t st);
-void launch_bond_slots(const Views &V, int side, int *slot_of, int4 *bsp, uint32_t *pkey, int *pval,
+// The bonds' slots, record positions (bfo: N + 1) and working copies (perm:
+// nb) of fresh rows.  cnt: N, blo: N + 1, list: nb, n2: 2 N, o2: 2 N + 1.
+void launch_bond_lists(const Views &V, int side, int nb, int *slot_of, int4 *bsp, int *cnt, int *blo, int *list,
+                       int *n2, int *o2, int *scan_scratch, int *bfo, int *perm, const BondStat *in,
+                       const BondDyn *dyn, BondGeom32 *wst, BondDyn *wdyn, int4 *wsp, int *winv, unsigned char *wflag,
                        cudaStream_t st);
-void launch_bond_work(const Views &V, int side, int nb, int *cnt, int *wfo, int *scan_scratch, int *perm,
-                      const BondStat *in, const BondDyn *dyn, const int4 *bsp, BondGeom32 *wst, BondDyn *wdyn,
-                      int4 *wsp, int *winv, unsigned char *wflag, cudaStream_t st);
 void launch_bond_work_scatter(const int *perm, int nb, const BondDyn *wdyn, BondDyn *dyn, cudaStream_t st);
-void launch_bond_positions(const Views &V, int side, const int *blo_start, const int *blo_end, const int *blo_idx,
-                           int *cnt, int *bfo, int *scan_scratch, int4 *bsp, cudaStream_t st);
 void launch_pairs_screen(const Views &V, int cur, int diag, int P, int2 *eb, const int2 *stl,
                          MixedBufs B, int block, int variant, cudaStream_t st);
 void launch_contact_list(const Views &V, int side, int P, const unsigned *erow, const unsigned char *pfl, int *mark,
@@ -205,15 +202,14 @@ void launch_gather_bonds(const int *old_hi, const BondStat *old_st, const BondDy
                          BondStat *new_st, BondDyn *new_dy, const int *bmap, int nb, cudaStream_t st);
 void launch_set_int(int *p, int v, cudaStream_t st);
 
-// Bond creation at admission (bonds_init.cu): cell list over the admitted
-// floes [s0, s0 + n) on side `side`, per-floe bond counts and their scan;
-// per-field totals; the bond table's entries of the fresh fields.
-void launch_bond_init_count(const Views &V, int side, int s0, int n, const BondRule *rule, uint32_t *keys,
-                            int *vals, uint32_t *keys_alt, int *vals_alt, int key_bits, int *rs_counts,
-                            int *scan_scratch, int *cstart, int *cend, int *cnt, int *scan, cudaStream_t st);
+// Bond creation at admission (bonds_init.cu): per-floe bond counts of the
+// admitted floes [s0, s0 + n) on side `side` and their scan (coff, list: their
+// cell list); per-field totals; the bond table's entries of the fresh fields.
+void launch_bond_init_count(const Views &V, int side, int s0, int n, const BondRule *rule, const int *coff,
+                            const int *list, int *scan_scratch, int *cnt, int *scan, cudaStream_t st);
 void launch_bond_init_totals(const int *scan, const int *first, const int *last, int m, int *tot, cudaStream_t st);
-void launch_bond_init_fill(const Views &V, int side, int s0, int n, const BondRule *rule, const int *cstart,
-                           const int *cend, const int *vals, const int *scan, int *bond_off, int *bond_hi,
-                           BondStat *bstat, BondDyn *bdyn, cudaStream_t st);
+void launch_bond_init_fill(const Views &V, int side, int s0, int n, const BondRule *rule, const int *coff,
+                           const int *list, const int *scan, int *bond_off, int *bond_hi, BondStat *bstat,
+                           BondDyn *bdyn, cudaStream_t st);
 
 }  // namespace godar

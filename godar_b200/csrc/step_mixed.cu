@@ -1344,24 +1344,11 @@ bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base,
     return true;
 }
 
-// Row (slot) of every entry of a CSR.
-__global__ void k_fill_erow(const int *off, int N, unsigned *erow)
-{
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < N; s += gridDim.x * blockDim.x)
-        for (int e = off[s]; e < off[s + 1]; e++) erow[e] = (unsigned)s;
-}
-
 __global__ void k_pack_snap(Views V, int side)
 {
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < V.N; g += gridDim.x * blockDim.x)
         V.snap[side][g] = pack_snap(V.x[side][g], V.y[side][g], make_shape(V.P[V.inst[g]], V.r[side][g], V.h[side][g]),
                                     V.u[side][g], V.v[side][g], V.om[side][g], V.inst[g]);
-}
-
-void launch_fill_erow(const int *off, int N, unsigned *erow, cudaStream_t st)
-{
-    const int grid = N > 0 ? std::min((N + 255) / 256, 148 * 16) : 1;
-    k_fill_erow<<<grid, 256, 0, st>>>(off, N, erow);
 }
 
 void launch_pack_snap(const Views &V, int side, cudaStream_t st)
@@ -1371,29 +1358,17 @@ void launch_pack_snap(const Views &V, int side, cudaStream_t st)
 }
 
 
-// Per rebuild: the partner index of every owner entry, the pair flags from
-// the migrated histories, no records.
-__global__ void k_mixed_rows_init(int P, const int2 *ent_lo, const Hist4<float> *hist, int *lo_of,
-                                  unsigned char *pfl, unsigned char *lfl)
-{
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < P; k += gridDim.x * blockDim.x) {
-        const int p = ent_lo[k].y;
-        if (p >= 0 && p < P) lo_of[p] = k;
-        lfl[k] = 0;
-        const Hist4<float> H = hist[k];
-        pfl[k] = (H.deltat != 0.f || H.thetarelc != 0.f) ? PF_HIST : 0;
-    }
-}
-
-// Slot of every floe by global id (instance offset + reference id), then the
-// slots of both floes of every bond.
+// The bond lists of a rebuild.  Slot of every floe by global id (instance
+// offset + reference id).
 __global__ void k_slot_of(Views V, int side, int *slot_of)
 {
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x)
         slot_of[V.P[V.inst[s]].off + V.id[side][s]] = s;
 }
 
-__global__ void k_bond_slots(Views V, int side, const int *slot_of, int4 *bsp, uint32_t *pkey, int *pval)
+// Slots of both floes of every bond; cnt[gj]: the bonds in which global id gj
+// is the higher one.
+__global__ void k_bond_slots(Views V, int side, const int *slot_of, int4 *bsp, int *cnt)
 {
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x) {
         const int off = V.P[V.inst[s]].off;
@@ -1401,56 +1376,70 @@ __global__ void k_bond_slots(Views V, int side, const int *slot_of, int4 *bsp, u
         for (int b = V.bond_off[gl]; b < V.bond_off[gl + 1]; b++) {
             const int gj = off + V.bond_hi[b];
             reinterpret_cast<int2 *>(&bsp[b])[0] = make_int2(s, slot_of[gj]);
-            if (pkey) { pkey[b] = (uint32_t)gj; pval[b] = b; }
+            atomicAdd(&cnt[gj], 1);
         }
     }
 }
 
-// Per slot: the number of bond records (bonds where the floe is the lower
-// id, then those where it is the higher id); after the scan bfo, the record
-// positions of every bond.
-__global__ void k_bond_counts(Views V, int side, const int *blo_start, const int *blo_end, int *cnt)
+// The bonds of every higher id, in any order (blo: the scan of cnt, which
+// returns to zero).
+__global__ void k_bond_partners(Views V, int side, const int *blo, int *cnt, int *list)
 {
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x) {
-        const int gl = V.P[V.inst[s]].off + V.id[side][s];
-        cnt[s] = (V.bond_off[gl + 1] - V.bond_off[gl]) + (blo_end[gl] - blo_start[gl]);
+        const int off = V.P[V.inst[s]].off;
+        const int gl = off + V.id[side][s];
+        for (int b = V.bond_off[gl]; b < V.bond_off[gl + 1]; b++) {
+            const int gj = off + V.bond_hi[b];
+            list[blo[gj] + atomicSub(&cnt[gj], 1) - 1] = b;
+        }
     }
 }
 
-__global__ void k_bond_pos(Views V, int side, const int *blo_start, const int *blo_end, const int *blo_idx,
-                           const int *bfo, int4 *bsp)
+// Per slot: the number of bond records (bonds where the floe is the lower id,
+// then those where it is the higher id) at n2[s], and of its own bonds at
+// n2[N + s].
+__global__ void k_bond_counts(Views V, int side, const int *blo, int *n2)
 {
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x) {
+        const int gl = V.P[V.inst[s]].off + V.id[side][s];
+        const int own = V.bond_off[gl + 1] - V.bond_off[gl];
+        n2[s] = own + (blo[gl + 1] - blo[gl]);
+        n2[V.N + s] = own;
+    }
+}
+
+// From the scan o2 of k_bond_counts: the first bond record of every slot
+// (bfo), the record positions of every bond (own bonds in ascending partner
+// id, then those where the floe is the higher id in ascending lower id: the
+// table's order), and the bonds' working order, by the slot of the lower-id
+// floe.
+__global__ void k_bond_pos(Views V, int side, const int *blo, const int *list, const int *o2, int *bfo, int4 *bsp,
+                           int *perm)
+{
+    const int rec = o2[V.N];
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x) {
         const int gl = V.P[V.inst[s]].off + V.id[side][s];
         const int b0 = V.bond_off[gl], b1 = V.bond_off[gl + 1];
-        const int base = bfo[s];
-        for (int b = b0; b < b1; b++) bsp[b].z = base + (b - b0);
-        const int k0 = blo_start[gl], k1 = blo_end[gl];
-        for (int k = k0; k < k1; k++) bsp[blo_idx[k]].w = base + (b1 - b0) + (k - k0);
+        const int base = o2[s], w0 = o2[V.N + s] - rec;
+        bfo[s] = base;
+        if (s == V.N - 1) bfo[V.N] = rec;
+        for (int b = b0; b < b1; b++) {
+            bsp[b].z = base + (b - b0);
+            perm[w0 + (b - b0)] = b;
+        }
+        const int k0 = blo[gl], k1 = blo[gl + 1];
+        for (int k = k0; k < k1; k++) {
+            const int b = list[k];
+            int before = 0;
+            for (int j = k0; j < k1; j++) before += list[j] < b;
+            bsp[b].w = base + (b1 - b0) + before;
+        }
     }
 }
 
-// Per rebuild: the bonds' working order, by the slot of the lower-id floe
-// (wfo: first working index of every slot), and per working index the
-// dynamic record, the FP32 copy of the static record, slots and record
-// positions, both sides of the live-bond flag, and the inverse map.
-__global__ void k_bond_own_counts(Views V, int side, int *cnt)
-{
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x) {
-        const int gl = V.P[V.inst[s]].off + V.id[side][s];
-        cnt[s] = V.bond_off[gl + 1] - V.bond_off[gl];
-    }
-}
-
-__global__ void k_bond_perm(Views V, int side, const int *wfo, int *perm)
-{
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x) {
-        const int gl = V.P[V.inst[s]].off + V.id[side][s];
-        const int b0 = V.bond_off[gl], b1 = V.bond_off[gl + 1], base = wfo[s];
-        for (int b = b0; b < b1; b++) perm[base + (b - b0)] = b;
-    }
-}
-
+// Per working index the dynamic record, the FP32 copy of the static record,
+// slots and record positions, both sides of the live-bond flag, and the
+// inverse map.
 __global__ void k_bond_work_gather(Views V, const int *perm, int nb, const BondStat *in, const BondDyn *dyn,
                                    const int4 *bsp, BondGeom32 *wst, BondDyn *wdyn, int4 *wsp, int *winv,
                                    unsigned char *wflag)
@@ -1530,20 +1519,6 @@ __global__ void k_contact_fill(Views V, int side, int P, const unsigned *erow, c
     }
 }
 
-void launch_mixed_rows_init(int P, const int2 *ent_lo, const void *hist, int *lo_of, unsigned char *pfl,
-                            unsigned char *lfl, cudaStream_t st)
-{
-    if (P > 0)
-        k_mixed_rows_init<<<grid_of(P, 256), 256, 0, st>>>(P, ent_lo, (const Hist4<float> *)hist, lo_of, pfl, lfl);
-}
-
-void launch_bond_slots(const Views &V, int side, int *slot_of, int4 *bsp, uint32_t *pkey, int *pval,
-                       cudaStream_t st)
-{
-    k_slot_of<<<grid_of(V.N, 256), 256, 0, st>>>(V, side, slot_of);
-    k_bond_slots<<<grid_of(V.N, 128), 128, 0, st>>>(V, side, slot_of, bsp, pkey, pval);
-}
-
 void launch_contact_list(const Views &V, int side, int P, const unsigned *erow, const unsigned char *pfl, int *mark,
                          int *pos, int *scan_scratch, int2 *eb, int2 *stl, cudaStream_t st)
 {
@@ -1553,28 +1528,26 @@ void launch_contact_list(const Views &V, int side, int P, const unsigned *erow, 
     k_contact_fill<<<grid_of(P, 256), 256, 0, st>>>(V, side, P, erow, pfl, mark, pos, eb, stl);
 }
 
-void launch_bond_work(const Views &V, int side, int nb, int *cnt, int *wfo, int *scan_scratch, int *perm,
-                      const BondStat *in, const BondDyn *dyn, const int4 *bsp, BondGeom32 *wst, BondDyn *wdyn,
-                      int4 *wsp, int *winv, unsigned char *wflag, cudaStream_t st)
+void launch_bond_lists(const Views &V, int side, int nb, int *slot_of, int4 *bsp, int *cnt, int *blo, int *list,
+                       int *n2, int *o2, int *scan_scratch, int *bfo, int *perm, const BondStat *in,
+                       const BondDyn *dyn, BondGeom32 *wst, BondDyn *wdyn, int4 *wsp, int *winv, unsigned char *wflag,
+                       cudaStream_t st)
 {
-    if (nb <= 0) return;
-    k_bond_own_counts<<<grid_of(V.N, 256), 256, 0, st>>>(V, side, cnt);
-    scan_excl(cnt, wfo, V.N, scan_scratch, st);
-    k_bond_perm<<<grid_of(V.N, 128), 128, 0, st>>>(V, side, wfo, perm);
+    const int grid = grid_of(V.N, 128);
+    cudaMemsetAsync(cnt, 0, (size_t)V.N * 4, st);
+    k_slot_of<<<grid_of(V.N, 256), 256, 0, st>>>(V, side, slot_of);
+    k_bond_slots<<<grid, 128, 0, st>>>(V, side, slot_of, bsp, cnt);
+    scan_excl(cnt, blo, V.N, scan_scratch, st);
+    k_bond_partners<<<grid, 128, 0, st>>>(V, side, blo, cnt, list);
+    k_bond_counts<<<grid_of(V.N, 256), 256, 0, st>>>(V, side, blo, n2);
+    scan_excl(n2, o2, 2 * V.N, scan_scratch, st);
+    k_bond_pos<<<grid, 128, 0, st>>>(V, side, blo, list, o2, bfo, bsp, perm);
     k_bond_work_gather<<<grid_of(nb, 256), 256, 0, st>>>(V, perm, nb, in, dyn, bsp, wst, wdyn, wsp, winv, wflag);
 }
 
 void launch_bond_work_scatter(const int *perm, int nb, const BondDyn *wdyn, BondDyn *dyn, cudaStream_t st)
 {
     if (nb > 0) k_bond_work_scatter<<<grid_of(nb, 256), 256, 0, st>>>(perm, nb, wdyn, dyn);
-}
-
-void launch_bond_positions(const Views &V, int side, const int *blo_start, const int *blo_end, const int *blo_idx,
-                           int *cnt, int *bfo, int *scan_scratch, int4 *bsp, cudaStream_t st)
-{
-    k_bond_counts<<<grid_of(V.N, 256), 256, 0, st>>>(V, side, blo_start, blo_end, cnt);
-    scan_excl(cnt, bfo, V.N, scan_scratch, st);
-    k_bond_pos<<<grid_of(V.N, 128), 128, 0, st>>>(V, side, blo_start, blo_end, blo_idx, bfo, bsp);
 }
 
 void launch_pairs_screen(const Views &V, int cur, int diag, int P, int2 *eb, const int2 *stl,

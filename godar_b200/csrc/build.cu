@@ -413,7 +413,8 @@ __global__ void __launch_bounds__(128) k_nbr_fill(Views V, int side, const int *
 // What the fresh rows hold besides the partners; a group per floe.
 // Partner entries: the pair's index (ST_ROW_OVERFLOW if the partner's owner
 // row does not point back) and, mixed, its inverse and no record flag.  Owner
-// entries: row, bond index (bonds are sorted by the partner's id), no overlap,
+// entries: row, bond index (bonds are sorted by the partner's id; in the FP64
+// path counted in the working order, from wfo[s]), no overlap,
 // and the contact history by reference ids from the previous rows (old_up_off
 // null: zero); mixed, the history flag.
 template <typename H4, bool MIXED>
@@ -421,7 +422,7 @@ __global__ void __launch_bounds__(256) k_row_finish(Views V, int side, const int
                                                     const int2 *old_ent_up, const int *old_id, const H4 *old_hist,
                                                     const int *up_off, const int *lo_off, const int2 *ent_up,
                                                     int2 *ent_lo, H4 *hist, int *bidx, unsigned *erow, float *pdn,
-                                                    unsigned char *pfl, unsigned char *lfl, int *lo_of)
+                                                    unsigned char *pfl, unsigned char *lfl, int *lo_of, const int *wfo)
 {
     const int sub = threadIdx.x & (GRP - 1);
     const int groups = gridDim.x * (blockDim.x / GRP);
@@ -462,7 +463,7 @@ __global__ void __launch_bounds__(256) k_row_finish(Views V, int side, const int
                 if (v == idt) { bi = mid; break; }
                 if (v < idt) lo = mid + 1; else hi = mid - 1;
             }
-            bidx[e] = bi;
+            bidx[e] = !MIXED && bi >= 0 ? wfo[s] + (bi - b0) : bi;
             erow[e] = (unsigned)s;
             pdn[e] = __int_as_float(-1);       // a NaN: not a candidate
             if (MIXED) pfl[e] = h.deltat != 0 || h.thetarelc != 0 ? 1 : 0;     // PF_HIST
@@ -520,17 +521,18 @@ void launch_nbr_fill(const Views &V, int side, const int *coff, const int *off2,
 void launch_row_finish(const Views &V, int mixed, int side, const int *old_slot, const int *old_up_off,
                        const int2 *old_ent_up, const int *old_id, const void *old_hist, const int *up_off,
                        const int *lo_off, const int2 *ent_up, int2 *ent_lo, void *hist, int *bidx, unsigned *erow,
-                       float *pdn, unsigned char *pfl, unsigned char *lfl, int *lo_of, cudaStream_t st)
+                       float *pdn, unsigned char *pfl, unsigned char *lfl, int *lo_of, const int *wfo,
+                       cudaStream_t st)
 {
     const int grid = grid_for((long long)V.N * GRP, 256);
     if (mixed)
         k_row_finish<Hist4<float>, true><<<grid, 256, 0, st>>>(
             V, side, old_slot, old_up_off, old_ent_up, old_id, (const Hist4<float> *)old_hist, up_off, lo_off, ent_up,
-            ent_lo, (Hist4<float> *)hist, bidx, erow, pdn, pfl, lfl, lo_of);
+            ent_lo, (Hist4<float> *)hist, bidx, erow, pdn, pfl, lfl, lo_of, wfo);
     else
         k_row_finish<Hist4<double>, false><<<grid, 256, 0, st>>>(
             V, side, old_slot, old_up_off, old_ent_up, old_id, (const Hist4<double> *)old_hist, up_off, lo_off, ent_up,
-            ent_lo, (Hist4<double> *)hist, bidx, erow, pdn, pfl, lfl, lo_of);
+            ent_lo, (Hist4<double> *)hist, bidx, erow, pdn, pfl, lfl, lo_of, wfo);
     k_copy_ids<<<grid_for(V.N, 256), 256, 0, st>>>(V, side);
 }
 

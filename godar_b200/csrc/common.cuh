@@ -93,6 +93,11 @@ struct __align__(16) BondStat {
     float k_ax, k_sh1, k_sh2, k_r1, k_r2, ei_l, ea_l, inv_l;
 };
 
+// A bond's geometry in the FP64 path's working order.
+struct BondGeom64 {
+    double rb, hb, lb, sb, ib;
+};
+
 // The bond rule of one field for bond creation at admission (stepper.f90:93-101
 // with the relative limit and hashed fraction extensions): fresh = create
 // the field's bonds on the device; boff = its first index in the bond table.
@@ -151,7 +156,7 @@ struct Views {
     int *lo_off;           // [N+1]
     int2 *ent_up;          // [P]
     int2 *ent_lo;          // [P]
-    int *bidx;             // [P] bond index of the pair, -1 none
+    int *bidx;             // [P] bond index of the pair, -1 none (mixed path: in the table; FP64: in working order)
     void *hist[2];         // [P] Hist4<double> (FP64) or Hist4<float> (mixed), in place: both sides are one table
     float *pdn;            // [P] deltan of the last diagnostic step (NaN: not a candidate)
     double *edist;         // [P] FP64 path: the step's distance of every owner entry the screen visited (row order)
@@ -160,6 +165,8 @@ struct Views {
     int *bond_hi;          // [NB] higher id of the bond
     BondStat *bstat;       // [NB]
     BondDyn *bdyn[2];      // [NB] in place: both sides are one table
+    BondDyn *wdyn;         // [NB] FP64 path: the bonds' state and geometry in working order (bidx counts in it)
+    const BondGeom64 *wgeo;
     // mixed path: packed neighbour view of every floe, per side
     Snap *snap[2];
     // forcing grids
@@ -176,14 +183,13 @@ struct Views {
 
 #define GD_DEV __device__ __forceinline__
 
-// the FP64 pair work lists: [0] general, [1] bonded pairs out of contact
-// (no sheltering, no diagnostics); n[0], n[1] their lengths
+// the FP64 pair work list: contacts, and candidates of sheltering fields
 struct __align__(32) FP64Item {
     int p, g, t, bi;     // pair index, owner slot, partner slot, bond index
     double dx, dy;       // the pair's minimum-image offset x_g - x_t, y_g - y_t
 };
-struct FP64Lists {
-    FP64Item *work[2];
+struct FP64List {
+    FP64Item *work;
     int *n;
 };
 

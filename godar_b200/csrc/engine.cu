@@ -450,8 +450,8 @@ struct Engine {
     double kernel_ms = 0.0;        // device time inside step kernels
     long long launches = 0;        // time steps launched
     // the kernels of a time step: mixed [pair screen, pair work list, bonds,
-    // floe sums, floe update]; FP64 [entry screen, general work list, bond
-    // work list, row sums, floe update]
+    // floe sums, floe update]; FP64 [pairs, pair work list, none, row sums,
+    // floe update]
     static constexpr int NPH = 5;
     static constexpr int NEV = NPH + 2;   // timing events per step
     double phase_ms[NPH] = {0, 0, 0, 0, 0};
@@ -527,10 +527,10 @@ struct Engine {
     // mixed path: row of every owner entry, partner index, flags, pair records;
     // bond records, bond slots and the partner-bond lists
     Buf erow_up, lo_of, pfl, lfl, prec_b, prx_b, pdg_b, work_b, work_st_b, nwork_b, fsum_b, frex_b, fdg_b, clist_b, cscan_b;
-    // FP64 path: the pair records and the bond work list (the row of every
-    // owner entry, the pair flags and the general work list are the mixed
-    // path's erow_up, pfl and work_b)
-    Buf frec_b, fwork1_b;
+    // FP64 path: the pair records and the bonds' geometry in working order (the
+    // row of every owner entry, the pair flags, the work list and the bonds'
+    // working state are the mixed path's erow_up, pfl, work_b and wdyn_b)
+    Buf frec_b, wgeo_b;
     // FP64 path, per rebuild: the pairs that can act on a plain step before
     // the next rebuild (a byte per pair), their count at the head of every
     // row (owner, partner), and the list of their owner-row positions
@@ -634,15 +634,9 @@ struct Engine {
         const char *bl = getenv("GODAR_BLOCK");
         if (bl) block = std::max(32, atoi(bl));
         if (prec == GODAR_PREC_FP64) {
-            // five kernels: the screen (phase 0), the pair physics of the
-            // general and the bond work lists (phases 1, 2), the row sums
-            // (phase 3) and the floe update (phase 4); all but the screen at
-            // most 128 threads per block
-            // the screen: every block size with 2, 1 and 4 entries per lane
-            for (int v = 0; v < 3; v++)
-                for (int k = 0; k < 3; k++) cfg[0][3 * v + k] = (64 << k) | (v << 16);
-            ncfg[0] = 9;
-            for (int q = 1; q < NPH; q++) { ncfg[q] = 3; cfg[q][0] = 32; cfg[q][1] = 64; cfg[q][2] = 128; }
+            // the pairs (phase 0), the pair work list (1), the row sums (3)
+            // and the floe update (4); phase 2 is empty
+            for (int q = 0; q < NPH; q++) { ncfg[q] = 3; cfg[q][0] = 32; cfg[q][1] = 64; cfg[q][2] = 128; }
         } else {
             for (int q = 0; q < NPH; q++) {
                 ncfg[q] = 3;
@@ -658,7 +652,7 @@ struct Engine {
             ncfg[2] = 4;
         }
         if (bl)
-            for (int q = 0; q < NPH; q++) blk[q] = std::min(std::max(32, atoi(bl) & ~31), prec == GODAR_PREC_FP64 && q > 0 ? 128 : 256);
+            for (int q = 0; q < NPH; q++) blk[q] = std::min(std::max(32, atoi(bl) & ~31), prec == GODAR_PREC_FP64 ? 128 : 256);
         // GODAR_BOND_VARIANT: the mixed bond kernel's variant, fixed (the
         // tuner keeps choosing the other kernels' configurations)
         const char *bv = getenv("GODAR_BOND_VARIANT");
@@ -709,6 +703,7 @@ struct Engine {
         V.bidx = bidx.as<int>(); V.edist = edist.as<double>(); V.pdn = pdn.as<float>();
         V.bond_off = b.bond_off.as<int>(); V.bond_hi = b.bond_hi.as<int>();
         V.bstat = b.bstat.as<BondStat>();
+        V.wdyn = wdyn_b.as<BondDyn>(); V.wgeo = wgeo_b.as<BondGeom64>();
         V.field = field_b.as<double>();
         V.diag = diag.as<double>();
         V.status = status.as<int>(); V.expired_at = status.as<int>() + 1;
@@ -1353,14 +1348,14 @@ struct Engine {
             // what the previous rows hold in these does not outlive them
             const long long cap = (long long)(Pn * 1.25) + 1024;
             Buf *pb[] = {&edist, &pdn, &erow_up, &lo_of, &pfl, &lfl,
-                         &prec_b, &prx_b, &pdg_b, &work_b, &work_st_b, &clist_b, &cscan_b, &frec_b, &fwork1_b,
+                         &prec_b, &prx_b, &pdg_b, &work_b, &work_st_b, &clist_b, &cscan_b, &frec_b,
                          &flisted_b, &fpart_b, &fplist_b};
             for (Buf *b : pb) b->release(&bytes);
             TRY(ens(pdn, cap * 4));
             if (fp64) {
                 TRY(ens(edist, cap * 8));
                 TRY(ens(erow_up, cap * 4)); TRY(ens(pfl, cap + 16));
-                TRY(ens(work_b, cap * sizeof(FP64Item))); TRY(ens(fwork1_b, cap * sizeof(FP64Item)));
+                TRY(ens(work_b, cap * sizeof(FP64Item)));
                 TRY(ens(frec_b, cap * FP64_PAIR_REC_BYTES));
                 TRY(ens(flisted_b, cap + 16)); TRY(ens(fpart_b, cap * 16)); TRY(ens(fplist_b, cap * 4));
             } else {
@@ -1380,12 +1375,22 @@ struct Engine {
         TRY(ens(bidx2, (size_t)Ecap * 4)); TRY(ens(hist2, (size_t)Ecap * he));
         launch_nbr_fill(V, nxt, coff_b.as<int>(), row_off2.as<int>(), fp64 ? 0 : 1, lo_off2.as<int>(),
                         up_off2.as<int>(), ent_lo2.as<int2>(), ent_up2.as<int2>(), dist2.as<double>(), st);
+        if (fp64 && NB > 0) {
+            // the bonds' working order, which the pairs' bond indices count in
+            TRY(ens(wdyn_b, (size_t)NB * sizeof(BondDyn))); TRY(ens(wgeo_b, (size_t)NB * sizeof(BondGeom64)));
+            TRY(ens(perm_b, (size_t)NB * 4)); TRY(ens(blo_b, (size_t)(N + 1) * 4));
+            V = views();
+            launch_fp64_bonds(V, nxt, cnt.as<int>(), blo_b.as<int>(), scan_scratch.as<int>(), perm_b.as<int>(),
+                              wdyn_b.as<BondDyn>(), wgeo_b.as<BondGeom64>(), st);
+            wnb = NB;
+            wdirty = false;
+        }
         // without a previous generation of rows every history starts at zero
         launch_row_finish(V, fp64 ? 0 : 1, nxt, old_slot.as<int>(), have_old ? up_off.as<int>() : nullptr,
                           ent_up.as<int2>(), old_ids ? old_ids : F->id[cur].as<int>(), hist[0].p, up_off2.as<int>(),
                           lo_off2.as<int>(), ent_up2.as<int2>(), ent_lo2.as<int2>(), hist2.p, bidx2.as<int>(),
                           erow_up.as<unsigned>(), pdn.as<float>(), pfl.as<unsigned char>(), lfl.as<unsigned char>(),
-                          lo_of.as<int>(), st);
+                          lo_of.as<int>(), blo_b.as<int>(), st);
         // the new generation becomes the primary rows
         up_off.swap(up_off2); lo_off.swap(lo_off2);
         ent_up.swap(ent_up2); ent_lo.swap(ent_lo2);
@@ -1440,7 +1445,7 @@ struct Engine {
     int fp64_rows(int side) {
         auto ens = [&](Buf &b, size_t sz) { return b.ensure(std::max<size_t>(sz, 16), &bytes, &mp); };
         TRY(ens(fupn_b, (size_t)N * 4)); TRY(ens(flon_b, (size_t)N * 4)); TRY(ens(fpos_b, (size_t)(N + 1) * 4));
-        launch_fp64_rows(views(), side, (int)E, erow_up.as<unsigned>(), flisted_b.as<unsigned char>(),
+        launch_fp64_rows(views(), side, (int)E, erow_up.as<unsigned>(), pfl.as<unsigned char>(), flisted_b.as<unsigned char>(),
                          fupn_b.as<int>(), flon_b.as<int>(), fpart_b.as<int2>(), fpos_b.as<int>(),
                          scan_scratch.as<int>(), fplist_b.as<int>(), st);
         int lc = 0;
@@ -1470,7 +1475,7 @@ struct Engine {
     // the bonds by the partner's global id); bond records start at zero.
     // Writes the bond kernel's working records back to the bond table.
     int sync_bonds() {
-        if (prec != GODAR_PREC_FP64 && wdirty && wnb > 0 && BS)
+        if (wdirty && wnb > 0 && BS)
             launch_bond_work_scatter(perm_b.as<int>(), wnb, wdyn_b.as<BondDyn>(), BS->bdyn[0].as<BondDyn>(), st);
         wdirty = false;
         CK(cudaGetLastError());
@@ -1530,22 +1535,20 @@ struct Engine {
         // made the step slower (0.362 against 0.354 ms on 2.2 M floes).
         V.pdl = step_pdl() && N <= PDL_MAX_FLOES;
         if (ev) TRY(record(ev[0], capturing));
+        if (NB > 0) wdirty = true;
         if (prec == GODAR_PREC_FP64) {
-            FP64Lists L;
-            L.work[0] = work_b.as<FP64Item>();
-            L.work[1] = fwork1_b.as<FP64Item>();
+            FP64List L;
+            L.work = work_b.as<FP64Item>();
             L.n = nwork_b.as<int>();
             // a plain step visits the pairs that can act before the next
             // rebuild; a diagnostic step every owner entry
-            launch_pairs_fp64_screen(V, side, diag, diag ? (int)E : (int)Lc, diag ? nullptr : fplist_b.as<int>(),
-                                     erow_up.as<unsigned>(), pfl.as<unsigned char>(), L, frec_b.p, cfg_block(bs[0]),
-                                     cfg_variant(bs[0]), st);
+            launch_pairs_fp64(V, side, diag, diag ? (int)E : (int)Lc, diag ? nullptr : fplist_b.as<int>(),
+                              erow_up.as<unsigned>(), pfl.as<unsigned char>(), L, frec_b.p, cfg_block(bs[0]), st);
             if (ev) TRY(record(ev[1], capturing));
-            for (int l = 0; l < 2; l++) {
-                launch_pairs_fp64_work(V, side, diag, l, (int)E, pfl.as<unsigned char>(), L, frec_b.p,
-                                       cfg_block(bs[1 + l]), st);
-                if (ev) TRY(record(ev[2 + l], capturing));
-            }
+            launch_pairs_list_fp64(V, side, diag, (int)E, pfl.as<unsigned char>(), L, frec_b.p, cfg_block(bs[1]), st);
+            // (the third phase has no kernel of its own)
+            if (ev) TRY(record(ev[2], capturing));
+            if (ev) TRY(record(ev[3], capturing));
             launch_row_sums_fp64(V, side, diag, pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
                                  fupn_b.as<int>(), fsum_b.as<double>(), cfg_block(bs[3]), st);
             if (ev) TRY(record(ev[4], capturing));
@@ -1556,7 +1559,6 @@ struct Engine {
         } else {
             MixedBufs B = mixed_bufs();
             // live-bond flags ping-pong with the floe state's side
-            if (NB > 0) wdirty = true;
             B.bfl_rd = bflag_b.as<unsigned char>() + (size_t)side * NB;
             B.bfl_wr = bflag_b.as<unsigned char>() + (size_t)(side ^ 1) * NB;
             const bool conc = concurrent_bonds();
@@ -1621,7 +1623,7 @@ struct Engine {
     }
 
     int kernels_per_step() const {
-        return prec == GODAR_PREC_FP64 ? 5 : (E > 0 ? 2 : 0) + (NB > 0 ? 1 : 0) + 2;
+        return prec == GODAR_PREC_FP64 ? 4 : (E > 0 ? 2 : 0) + (NB > 0 ? 1 : 0) + 2;
     }
 
     // The graph of K steps from side c0, captured on first use.  Returns
@@ -1793,7 +1795,7 @@ struct Engine {
             }
             // the steps just launched (directly or as a graph) update the
             // working bond records
-            if (prec != GODAR_PREC_FP64 && NB > 0) wdirty = true;
+            if (NB > 0) wdirty = true;
             CK(cudaGetLastError());
             // (a small batch's kernel has written the status word itself)
             if (!small) CK(cudaMemcpyAsync(h_status, status.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1924,7 +1926,7 @@ struct Engine {
                 TRY(launch_chunk(K, cur, diag_last, blk, false, 0));
                 CK(cudaMemcpyAsync(hs, status.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
             }
-            if (prec != GODAR_PREC_FP64 && NB > 0) wdirty = true;
+            if (NB > 0) wdirty = true;
             CK(cudaGetLastError());
             CK(cudaEventRecord(ring_ev[P.slot], st));
             pend.push_back(std::move(P));

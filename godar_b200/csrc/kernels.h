@@ -75,30 +75,35 @@ void launch_nbr_fill(const Views &V, int side, const int *coff, const int *off2,
 void launch_row_finish(const Views &V, int mixed, int side, const int *old_slot, const int *old_up_off,
                        const int2 *old_ent_up, const int *old_id, const void *old_hist, const int *up_off,
                        const int *lo_off, const int2 *ent_up, int2 *ent_lo, void *hist, int *bidx, unsigned *erow,
-                       float *pdn, unsigned char *pfl, unsigned char *lfl, int *lo_of, cudaStream_t st);
+                       float *pdn, unsigned char *pfl, unsigned char *lfl, int *lo_of, const int *wfo,
+                       cudaStream_t st);
 
-// The FP64 time step: (b) a screen of every owner entry (distance,
-// candidate test, the entries that need no pair physics) and the pair
-// physics once per work-list entry, writing pair records and flags; the
-// ordered sums of every floe's records and its ridging events, into
-// FP64_FLOE_SUMS doubles per floe; (c)-(e) walls, forcing and the FP64
-// update (which also clears the work list).
+// The FP64 time step: (b) every owner entry's distance and candidate test,
+// with the pairs out of contact done there, and the pair physics of the work
+// list, writing pair records and flags; the ordered sums of every floe's
+// records and its ridging events, into FP64_FLOE_SUMS doubles per floe;
+// (c)-(e) walls, forcing and the FP64 update (which also clears the work list).
 constexpr int FP64_PAIR_REC_BYTES = 160;
 constexpr int FP64_FLOE_SUMS = 18;
-void launch_pairs_fp64_screen(const Views &V, int cur, int diag, int n, const int *plist, const unsigned *erow,
-                              unsigned char *pfl, FP64Lists L, void *rec, int block, int variant, cudaStream_t st);
-void launch_pairs_fp64_work(const Views &V, int cur, int diag, int list, int E, unsigned char *pfl, FP64Lists L,
-                            void *rec, int block, cudaStream_t st);
+void launch_pairs_fp64(const Views &V, int cur, int diag, int n, const int *plist, const unsigned *erow,
+                       unsigned char *pfl, FP64List L, void *rec, int block, cudaStream_t st);
+void launch_pairs_list_fp64(const Views &V, int cur, int diag, int E, unsigned char *pfl, FP64List L, void *rec,
+                            int block, cudaStream_t st);
 void launch_row_sums_fp64(const Views &V, int cur, int diag, const unsigned char *pfl, const void *rec,
                           const int *lo_n, const int *up_n, double *fs, int block, cudaStream_t st);
 // At a rebuild: the pairs that can act on a step without diagnostics before
 // the next one marked (listed[p]), every row reordered to hold them first
 // (up_n / lo_n per floe), and the list of their owner-row positions for the
 // screen (plist, pos[N] of them; pos: N + 1 ints; tmp: 2 E entries).
-void launch_fp64_rows(const Views &V, int side, int E, const unsigned *erow, unsigned char *listed, int *up_n,
-                      int *lo_n, int2 *tmp, int *pos, int *scan_scratch, int *plist, cudaStream_t st);
+// Also sets the pairs' flags before the first step.
+void launch_fp64_rows(const Views &V, int side, int E, const unsigned *erow, unsigned char *pfl,
+                      unsigned char *listed, int *up_n, int *lo_n, int2 *tmp, int *pos, int *scan_scratch, int *plist, cudaStream_t st);
 void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, const double *fs, int *nwork, int block,
                        cudaStream_t st);
+// At a rebuild: the bonds' working order (perm; wfo: N + 1, its first index of
+// every slot) and working copies.  cnt: N.
+void launch_fp64_bonds(const Views &V, int side, int *cnt, int *wfo, int *scan_scratch, int *perm, BondDyn *wdyn,
+                       BondGeom64 *wgeo, cudaStream_t st);
 // K whole steps of a small batch (n marked positions, E owner entries;
 // shelter: some field of the batch has sheltering; drag: 8 N doubles; out:
 // pinned host memory for the status word and the first expired step; done: an

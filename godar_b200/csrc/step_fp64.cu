@@ -15,36 +15,23 @@ static int fp64_grid(long long n, int block)
     return (int)std::max(1LL, std::min<long long>((n + block - 1) / block, 148LL * (4096 / block)));
 }
 
-template <int U>
-static void screen_u(const Views &V, int cur, int diag, int n, const int *plist, const unsigned *erow,
-                     unsigned char *pfl, FP64Lists L, PairRec64 *rec, int grid, int block, cudaStream_t st)
+void launch_pairs_fp64(const Views &V, int cur, int diag, int n, const int *plist, const unsigned *erow,
+                       unsigned char *pfl, FP64List L, void *rec, int block, cudaStream_t st)
 {
-    if (diag) launch_step(V.pdl != 0, k_pairs_fp64_screen<U, true>, grid, block, st, V, cur, n, plist, erow, pfl, L, rec);
-    else launch_step(V.pdl != 0, k_pairs_fp64_screen<U, false>, grid, block, st, V, cur, n, plist, erow, pfl, L, rec);
-}
-
-void launch_pairs_fp64_screen(const Views &V, int cur, int diag, int n, const int *plist, const unsigned *erow,
-                              unsigned char *pfl, FP64Lists L, void *rec, int block, int variant, cudaStream_t st)
-{
-    // variant: 0, 1, 2 = 2, 1, 4 entries per lane
-    const int u = variant == 1 ? 1 : variant == 2 ? 4 : 2;
-    const int grid = fp64_grid((n + u - 1) / u, block);
+    const int grid = fp64_grid(n, block);
     PairRec64 *r = (PairRec64 *)rec;
-    if (u == 1) screen_u<1>(V, cur, diag, n, plist, erow, pfl, L, r, grid, block, st);
-    else if (u == 2) screen_u<2>(V, cur, diag, n, plist, erow, pfl, L, r, grid, block, st);
-    else screen_u<4>(V, cur, diag, n, plist, erow, pfl, L, r, grid, block, st);
+    if (diag) launch_step(V.pdl != 0, k_pairs_fp64<true>, grid, block, st, V, cur, n, plist, erow, pfl, L, r);
+    else launch_step(V.pdl != 0, k_pairs_fp64<false>, grid, block, st, V, cur, n, plist, erow, pfl, L, r);
 }
 
-void launch_pairs_fp64_work(const Views &V, int cur, int diag, int list, int E, unsigned char *pfl, FP64Lists L,
-                            void *rec, int block, cudaStream_t st)
+void launch_pairs_list_fp64(const Views &V, int cur, int diag, int E, unsigned char *pfl, FP64List L, void *rec,
+                            int block, cudaStream_t st)
 {
     // the list's length is known on the device only: at most one wave, grid-stride
     const int grid = (int)std::max(1LL, std::min<long long>((E + block - 1) / block, 148LL * (1024 / block)));
     PairRec64 *r = (PairRec64 *)rec;
-    if (list && diag) launch_step(V.pdl != 0, k_pairs_fp64<true, true>, grid, block, st, V, cur, L, pfl, r);
-    else if (list) launch_step(V.pdl != 0, k_pairs_fp64<true, false>, grid, block, st, V, cur, L, pfl, r);
-    else if (diag) launch_step(V.pdl != 0, k_pairs_fp64<false, true>, grid, block, st, V, cur, L, pfl, r);
-    else launch_step(V.pdl != 0, k_pairs_fp64<false, false>, grid, block, st, V, cur, L, pfl, r);
+    if (diag) launch_step(V.pdl != 0, k_pairs_list_fp64<true>, grid, block, st, V, cur, L, pfl, r);
+    else launch_step(V.pdl != 0, k_pairs_list_fp64<false>, grid, block, st, V, cur, L, pfl, r);
 }
 
 void launch_row_sums_fp64(const Views &V, int cur, int diag, const unsigned char *pfl, const void *rec,
@@ -103,8 +90,8 @@ bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, 
 // without sheltering changes nothing on such a step (pair_compute resets a
 // history that is already zero).  Kept: pairs within reach (with a margin
 // far above rounding), bonded pairs, pairs with a history, every pair of a
-// sheltering field.
-__global__ void k_fp64_mark(Views V, int side, int E, const unsigned *erow, unsigned char *listed)
+// sheltering field.  Also the pairs' flags before the first step.
+__global__ void k_fp64_mark(Views V, int side, int E, const unsigned *erow, unsigned char *listed, unsigned char *pfl)
 {
     const Hist4<double> *H = (const Hist4<double> *)V.hist[0];
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < E; e += gridDim.x * blockDim.x) {
@@ -112,11 +99,10 @@ __global__ void k_fp64_mark(Views V, int side, int E, const unsigned *erow, unsi
         const InstParams &P = V.P[V.inst[g]];
         const int2 en = V.ent_up[e];
         const int t = en.x, p = en.y;
-        bool keep = P.shelter != 0 || V.bidx[p] >= 0;
-        if (!keep) {
-            const Hist4<double> h = H[p];
-            keep = (__double_as_longlong(h.deltat) | __double_as_longlong(h.thetarelc)) != 0;
-        }
+        const double2 h = *(const double2 *)&H[p];
+        const bool hist = (__double_as_longlong(h.x) | __double_as_longlong(h.y)) != 0;
+        pfl[p] = hist ? PR_HIST : 0;
+        bool keep = P.shelter != 0 || V.bidx[p] >= 0 || hist;
         if (!keep) {
             const bool px = P.boundary & BC_PERIODIC_X, py = P.boundary & BC_PERIODIC_Y;
             const double dx = wrap_d(V.x[side][g] - V.x[side][t], P.nx, px);
@@ -161,10 +147,46 @@ __global__ void k_fp64_list(const int *up_off, const int *up_n, const int *pos, 
     }
 }
 
-void launch_fp64_rows(const Views &V, int side, int E, const unsigned *erow, unsigned char *listed, int *up_n,
-                      int *lo_n, int2 *tmp, int *pos, int *scan_scratch, int *plist, cudaStream_t st)
+// The bonds' working order, by the slot of the lower-id floe: the own bonds of
+// every slot, counted; from their scan (wfo) the order itself and the working
+// copies.
+__global__ void k_fp64_bond_counts(Views V, int side, int *cnt)
 {
-    if (E > 0) k_fp64_mark<<<fp64_grid(E, 256), 256, 0, st>>>(V, side, E, erow, listed);
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x) {
+        const int gl = V.P[V.inst[s]].off + V.id[side][s];
+        cnt[s] = V.bond_off[gl + 1] - V.bond_off[gl];
+    }
+}
+
+__global__ void k_fp64_bond_work(Views V, int side, const int *wfo, int *perm, BondDyn *wdyn, BondGeom64 *wgeo)
+{
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < V.N; s += gridDim.x * blockDim.x) {
+        const int gl = V.P[V.inst[s]].off + V.id[side][s];
+        const int b0 = V.bond_off[gl], b1 = V.bond_off[gl + 1], w0 = wfo[s];
+        for (int b = b0; b < b1; b++) {
+            const int w = w0 + (b - b0);
+            const BondStat c = V.bstat[b];
+            BondGeom64 q;
+            q.rb = c.rb; q.hb = c.hb; q.lb = c.lb; q.sb = c.sb; q.ib = c.ib;
+            perm[w] = b;
+            wdyn[w] = V.bdyn[0][b];
+            wgeo[w] = q;
+        }
+    }
+}
+
+void launch_fp64_bonds(const Views &V, int side, int *cnt, int *wfo, int *scan_scratch, int *perm, BondDyn *wdyn,
+                       BondGeom64 *wgeo, cudaStream_t st)
+{
+    k_fp64_bond_counts<<<fp64_grid(V.N, 256), 256, 0, st>>>(V, side, cnt);
+    scan_excl(cnt, wfo, V.N, scan_scratch, st);
+    k_fp64_bond_work<<<fp64_grid(V.N, 128), 128, 0, st>>>(V, side, wfo, perm, wdyn, wgeo);
+}
+
+void launch_fp64_rows(const Views &V, int side, int E, const unsigned *erow, unsigned char *pfl,
+                      unsigned char *listed, int *up_n, int *lo_n, int2 *tmp, int *pos, int *scan_scratch, int *plist, cudaStream_t st)
+{
+    if (E > 0) k_fp64_mark<<<fp64_grid(E, 256), 256, 0, st>>>(V, side, E, erow, listed, pfl);
     k_fp64_partition<<<fp64_grid(V.N, 128), 128, 0, st>>>(V, listed, up_n, lo_n, tmp, E);
     scan_excl(up_n, pos, V.N, scan_scratch, st);
     k_fp64_list<<<fp64_grid(V.N, 128), 128, 0, st>>>(V.up_off, up_n, pos, V.N, plist);

@@ -1,14 +1,14 @@
 // One time step of every floe of a batch in FP64: the body of `stepper`
-// (stepper.f90:44-343) as three kernels, bit-identical to the reference's
+// (stepper.f90:44-343) as four kernels, bit-identical to the reference's
 // sequential order.
 //
-//   k_pairs_fp64_screen, one thread per owner entry (pair of candidates
-//   i < j by id, stored in the row of the lower-id floe i): the FP64
-//   distance of the pair and the candidate test (dist <= r_i + rtree,
-//   stepper.f90:89-92); entries that need no pair physics are finished
+//   k_pairs_fp64, one thread per owner entry (pair of candidates i < j by
+//   id, stored in the row of the lower-id floe i): the FP64 distance of the
+//   pair and the candidate test (dist <= r_i + rtree, stepper.f90:89-92);
+//   pairs that need no pair physics and bonded pairs out of contact are done
 //   there, the others go on a work list.
 //
-//   k_pairs_fp64, one thread per work-list entry: (b) contact
+//   k_pairs_list_fp64, one thread per work-list entry: contact
 //   (contact_forces.f90:1-87), ridging (ridging.f90:1-99), bond forces and
 //   damage (bonds.f90:74-212), sheltering (forcing.f90:162-186) and the
 //   stress magnitude (stepper.f90:238-271), computed ONCE per pair.  The
@@ -37,22 +37,24 @@
 
 namespace godar {
 
-GD_DEV void bond_load(const Views &V, int bi, int side, BondLocal &B)
+// Bond w of the working order (by the slot of the lower-id floe, as the pairs
+// are: a row's bonds are one stretch of memory).
+GD_DEV void bond_load(const Views &V, int w, BondLocal &B)
 {
-    const BondDyn d = V.bdyn[side][bi];
-    const BondStat c = V.bstat[bi];
+    const BondDyn d = V.wdyn[w];
+    const BondGeom64 c = V.wgeo[w];
     B.flag = d.flag;
     B.dmg = d.dmg; B.dnb = d.dnb; B.dtb = d.dtb; B.thji = d.thji; B.thij = d.thij;
     B.rb = c.rb; B.hb = c.hb; B.lb = c.lb; B.sb = c.sb; B.ib = c.ib;
 }
 
-GD_DEV void bond_store(const Views &V, int bi, int side, const BondLocal &B)
+GD_DEV void bond_store(const Views &V, int w, const BondLocal &B)
 {
     BondDyn d;
     d.dnb = B.dnb; d.dtb = B.dtb; d.thji = B.thji; d.thij = B.thij; d.dmg = B.dmg;
     d.flag = B.flag;
     d.pad = 0;
-    V.bdyn[side][bi] = d;
+    V.wdyn[w] = d;
 }
 
 // What one candidate pair adds to the sums of its two floes, in 32-byte
@@ -75,20 +77,29 @@ enum : unsigned char {
     PR_DIAG = 16,      // a stress term other than +-0 (diagnostic steps)
     PR_WHO1 = 32,      // ridging of the lower-id floe
     PR_WHO2 = 64,      // ridging of the higher-id floe
+    PR_HIST = 128,     // the pair's tangential or rolling history may be nonzero (kept while not a candidate)
 };
 
 GD_DEV double stress_term(double S, double c1, double rl, double c2) { return ((S * c1) * rl) * c2; }
 
-// A candidate without contact, bond or sheltering: its tangential and rolling
-// histories are reset (most are zero already; h01: the stored ones) and, on
-// a diagnostic step, its stress record and overlap written: pair_compute's
-// normal, stress magnitude (no bond forces) and overlap, by the same
-// expressions.  Returns the pair's flags.
+// reset_contact (reset.f90:1-15) of a candidate out of contact whose flags of
+// the last step say that its tangential or rolling history may be nonzero.
+// The flag spares every other pair the history's sector, read and written.
+GD_DEV void reset_history(Hist4<double> *Hs, int p, unsigned old)
+{
+    if (old & PR_HIST) *(double2 *)&Hs[p] = make_double2(0.0, 0.0);
+}
+
+// A candidate without contact, bond or sheltering (old: its flags of the last
+// step): its tangential and rolling histories are reset and, on a diagnostic
+// step, its stress record and overlap written: pair_compute's normal, stress
+// magnitude (no bond forces) and overlap, by the same expressions.  Returns
+// the pair's flags.
 template <bool DIAG>
 GD_DEV unsigned quiet_candidate(const Views &V, Hist4<double> *Hs, int p, double dx, double dy, double dist,
-                                double deltan, double ri, double rj, double2 h01, PairRec64 *rec)
+                                double deltan, double ri, double rj, unsigned old, PairRec64 *rec)
 {
-    if (__double_as_longlong(h01.x) | __double_as_longlong(h01.y)) *(double2 *)&Hs[p] = make_double2(0.0, 0.0);
+    reset_history(Hs, p, old);
     unsigned f = PR_CAND;
     if (DIAG) {
         const double2 fc = *(const double2 *)&Hs[p].fcn;
@@ -104,119 +115,6 @@ GD_DEV unsigned quiet_candidate(const Views &V, Hist4<double> *Hs, int p, double
         V.pdn[p] = (float)deltan;
     }
     return f;
-}
-
-// Owner entries, first pass (few registers): the FP64 distance (kept for
-// the row sort) and the candidate test, and the entries that need no pair
-// physics finished here.  A non-candidate keeps its history and bond state.
-// A candidate that is not in contact, has no bond and is in a field without
-// sheltering only has its tangential and rolling histories reset
-// (reset_contact, reset.f90:1-15) and, on a diagnostic step, its normal,
-// the stress magnitude of its history's last contact forces
-// (stepper.f90:238-271) and its overlap recorded: all pair_compute gives it.
-// The other candidates go on one of two work lists with their slots, bond
-// index and offset: bonded pairs out of contact in fields without
-// sheltering (work[1], most of them), and all others (work[0]).
-// A plain step visits the positions of plist only (n of them: the pairs
-// that can act before the next rebuild, see k_fp64_mark); a diagnostic step
-// every owner entry (plist null, n = E).
-// U entries per lane (a warp takes 32 U consecutive items): every load of
-// the U entries is issued before the first store, so that they overlap.
-template <int U, bool DIAG>
-__global__ void __launch_bounds__(256) k_pairs_fp64_screen(Views V, int cur, int n, const int *plist,
-                                                           const unsigned *erow, unsigned char *pfl, FP64Lists L,
-                                                           PairRec64 *rec)
-{
-    step_kernel_entry();
-    if (*(volatile int *)V.status & ST_ABORT) return;
-    Hist4<double> *Hs = (Hist4<double> *)V.hist[0];   // in place: one thread per pair
-    unsigned long long n_cand = 0;
-    const int lane = threadIdx.x & 31;
-    const int nwarps = gridDim.x * (blockDim.x >> 5);
-    // every lane of a warp runs the same iterations (the list append is warp-wide)
-    for (int b0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32 * U; b0 < n; b0 += nwarps * 32 * U) {
-        int g[U], t[U], p[U], bi[U];
-        double xg[U], yg[U], rg[U], xt[U], yt[U], rt[U];
-        double2 h01[U];
-        const InstParams *Pk[U];
-        int ek[U];
-#pragma unroll
-        for (int k = 0; k < U; k++) {
-            // lanes past the end read item 0 and store nothing
-            const int i = b0 + 32 * k + lane < n ? b0 + 32 * k + lane : 0;
-            ek[k] = plist ? plist[i] : i;
-        }
-#pragma unroll
-        for (int k = 0; k < U; k++) {
-            const int e = ek[k];
-            g[k] = (int)erow[e];
-            const int2 en = V.ent_up[e];
-            t[k] = en.x;
-            p[k] = en.y;
-        }
-#pragma unroll
-        for (int k = 0; k < U; k++) {
-            Pk[k] = &V.P[V.inst[g[k]]];
-            xg[k] = V.x[cur][g[k]]; yg[k] = V.y[cur][g[k]]; rg[k] = V.r[cur][g[k]];
-            xt[k] = V.x[cur][t[k]]; yt[k] = V.y[cur][t[k]]; rt[k] = V.r[cur][t[k]];
-            bi[k] = V.bidx[p[k]];
-            h01[k] = *(const double2 *)&Hs[p[k]];
-        }
-        double dxk[U], dyk[U];
-#pragma unroll
-        for (int k = 0; k < U; k++) {
-            const int e = ek[k];
-            bool heavy = false, bond_only = false;
-            dxk[k] = dyk[k] = 0.0;
-            if (b0 + 32 * k + lane < n) {
-                const InstParams &P = *Pk[k];
-                const bool px = P.boundary & BC_PERIODIC_X, py = P.boundary & BC_PERIODIC_Y;
-                const double dx = wrap_d(xg[k] - xt[k], P.nx, px);
-                const double dy = wrap_d(yg[k] - yt[k], P.ny, py);
-                dxk[k] = dx;
-                dyk[k] = dy;
-                const double dist = sqrt(dx * dx + dy * dy);
-                V.edist[e] = dist;
-                if (!(dist <= rg[k] + P.rtree)) {
-                    // history and bond state stay as they are
-                    pfl[p[k]] = 0;
-                    if (DIAG) V.pdn[p[k]] = __int_as_float(0x7fc00000);
-                } else {
-                    const double deltan = (rg[k] + rt[k]) - dist;
-                    const bool general = deltan > 0.0 || P.shelter != 0;
-                    heavy = general || bi[k] >= 0;
-                    bond_only = !general && bi[k] >= 0;
-                    if (!heavy) {
-                        const unsigned f = quiet_candidate<DIAG>(V, Hs, p[k], dx, dy, dist, deltan, rg[k], rt[k], h01[k],
-                                                                 rec);
-                        if (DIAG) n_cand++;
-                        pfl[p[k]] = f;
-                    }
-                }
-            }
-#pragma unroll
-            for (int l = 0; l < 2; l++) {
-                const bool mine = l ? bond_only : heavy && !bond_only;
-                const unsigned m = __ballot_sync(0xffffffffu, mine);
-                if (m) {
-                    int base = 0;
-                    if (lane == 0) base = atomicAdd(&L.n[l], __popc(m));
-                    base = __shfl_sync(0xffffffffu, base, 0);
-                    if (mine) {
-                        FP64Item it;
-                        it.p = p[k]; it.g = g[k]; it.t = t[k]; it.bi = bi[k];
-                        it.dx = dxk[k]; it.dy = dyk[k];
-                        L.work[l][base + __popc(m & ((1u << lane) - 1))] = it;
-                    }
-                }
-            }
-        }
-    }
-    if (DIAG) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) n_cand += __shfl_down_sync(0xffffffffu, n_cand, o);
-        if (lane == 0 && n_cand) atomicAdd(&V.counters[0], n_cand);
-    }
 }
 
 // Counts of a diagnostic step, per thread.
@@ -235,20 +133,26 @@ GD_DEV void add_counts(const Counts64 &C, unsigned long long *counters)
 }
 
 // The pair physics of one candidate (pair p, owner slot g, partner slot t,
-// bond bi or -1, offset dx, dy): history and bond in place, the record
-// groups its flags name.
+// working bond bi or -1, offset dx, dy, flags `old` of the last step): history
+// and bond in place, the record groups its flags name.  BONDS: for a bonded
+// pair out of contact in a field without sheltering, the contact branch
+// compiled out.  DIAG: a diagnostic step (stress records, overlaps, counts).
 template <bool BONDS, bool DIAG>
 GD_DEV void pair_work64(const Views &V, int cur, Hist4<double> *Hs, int p, int g, int t, int bi, double dx, double dy,
-                        unsigned char *pfl, PairRec64 *rec, Counts64 &C)
+                        unsigned old, unsigned char *pfl, PairRec64 *rec, Counts64 &C)
 {
     const InstParams &P = V.P[V.inst[g]];
     const bool shel = !BONDS && P.shelter != 0;
     const double r = V.r[cur][g];
     // the screen's distance, by the same expression
     const double dist = sqrt(dx * dx + dy * dy);
-    Hist4<double> H = Hs[p];
     BondLocal BL;
-    if (bi >= 0) bond_load(V, bi, 0, BL);
+    if (bi >= 0) bond_load(V, bi, BL);
+    // the history: a contact's, and on a diagnostic step the last contact
+    // forces of every pair
+    Hist4<double> H;
+    H.deltat = H.thetarelc = H.fcn = H.fct = 0.0;
+    if (DIAG || (!BONDS && (r + V.r[cur][t]) - dist > 0.0)) H = Hs[p];
     const Shape si = make_shape(P, r, V.h[cur][g]);
     const Shape sj = make_shape(P, V.r[cur][t], V.h[cur][t]);
     double ua = 0.0, va = 0.0, uw = 0.0, vw = 0.0;
@@ -256,11 +160,16 @@ GD_DEV void pair_work64(const Views &V, int cur, Hist4<double> *Hs, int p, int g
     const PairRes<double> R = pair_compute<double, !BONDS>(P, dx, dy, dist, V.u[cur][g], V.v[cur][g], V.om[cur][g],
                                                    V.u[cur][t], V.v[cur][t], V.om[cur][t], si, sj,
                                                    ua, va, uw, vw, H, bi >= 0 ? &BL : nullptr, shel);
-    Hs[p] = H;
-    if (bi >= 0) bond_store(V, bi, 0, BL);
-
     unsigned f = PR_CAND;
-    if (R.contact) f |= PR_CONTACT;
+    if (R.contact) {
+        Hs[p] = H;
+        f |= PR_CONTACT;
+        if (__double_as_longlong(H.deltat) | __double_as_longlong(H.thetarelc)) f |= PR_HIST;
+    } else {
+        reset_history(Hs, p, old);
+    }
+    if (bi >= 0) bond_store(V, bi, BL);
+
     if (R.bond_on) f |= PR_BOND;
     if (R.who == 1) f |= PR_WHO1;
     else if (R.who == 2) f |= PR_WHO2;
@@ -296,29 +205,97 @@ GD_DEV void pair_work64(const Views &V, int cur, Hist4<double> *Hs, int p, int g
     }
 }
 
-// A work list: the pair physics of every remaining candidate, once.
-// BONDS: list 1 (bonded, no contact, no sheltering), with the contact
-// branch compiled out.  DIAG: a diagnostic step (stress records, overlaps,
-// counts).
-template <bool BONDS, bool DIAG>
-__global__ void __launch_bounds__(128) k_pairs_fp64(Views V, int cur, FP64Lists L, unsigned char *pfl,
-                                                    PairRec64 *rec)
+// Owner entries: the FP64 distance (kept for the row sort), the candidate
+// test, and every pair that is not in contact in a field without sheltering.
+// A non-candidate keeps its history and bond state.  A candidate without a
+// bond is a quiet_candidate.  A bonded one goes through the pair physics with
+// the contact branch compiled out.  The others go on the work list with
+// their slots, bond index and offset.
+// A plain step visits the positions of plist only (n of them: the pairs that
+// can act before the next rebuild, see k_fp64_mark; nine in ten are bonded on
+// the benchmark's fields); a diagnostic step every owner entry (plist null,
+// n = E).
+// Latency bounds it (half its warps' registers are the bond's FP64 chain), so
+// what it waits for is kept short: the screen and the bonds were two kernels
+// with a 32-byte item a bond between them, each gathering both floes, the bond
+// state in reference order, and every pair's history read and written back.
+// 529,113 floes, 0.82 M bonds: 41 + 84 us then, 77 us now.
+template <bool DIAG>
+__global__ void __launch_bounds__(128) k_pairs_fp64(Views V, int cur, int n, const int *plist, const unsigned *erow,
+                                                    unsigned char *pfl, FP64List L, PairRec64 *rec)
+{
+    step_kernel_entry();
+    if (*(volatile int *)V.status & ST_ABORT) return;
+    Hist4<double> *Hs = (Hist4<double> *)V.hist[0];   // in place: one thread per pair
+    Counts64 C = {0, 0, 0, 0};
+    const int lane = threadIdx.x & 31;
+    const int stride = gridDim.x * blockDim.x;
+    // every lane of a warp runs the same iterations (the list append is warp-wide)
+    for (int i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += stride) {
+        const int i = i0 + lane;
+        const bool on = i < n;
+        // lanes past the end read item 0 and store nothing
+        const int e = plist ? plist[on ? i : 0] : on ? i : 0;
+        const int g = (int)erow[e];
+        const int2 en = V.ent_up[e];
+        const int t = en.x, p = en.y;
+        const InstParams &P = V.P[V.inst[g]];
+        const double rg = V.r[cur][g], rt = V.r[cur][t];
+        const int bi = V.bidx[p];
+        const unsigned old = pfl[p];
+        const bool px = P.boundary & BC_PERIODIC_X, py = P.boundary & BC_PERIODIC_Y;
+        const double dx = wrap_d(V.x[cur][g] - V.x[cur][t], P.nx, px);
+        const double dy = wrap_d(V.y[cur][g] - V.y[cur][t], P.ny, py);
+        const double dist = sqrt(dx * dx + dy * dy);
+        const double deltan = (rg + rt) - dist;
+        const bool cand = on && dist <= rg + P.rtree;
+        const bool heavy = cand && (deltan > 0.0 || P.shelter != 0);
+        if (on) V.edist[e] = dist;
+        const unsigned m = __ballot_sync(0xffffffffu, heavy);
+        if (m) {
+            int base = 0;
+            if (lane == 0) base = atomicAdd(L.n, __popc(m));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (heavy) {
+                FP64Item it;
+                it.p = p; it.g = g; it.t = t; it.bi = bi;
+                it.dx = dx; it.dy = dy;
+                L.work[base + __popc(m & ((1u << lane) - 1))] = it;
+            }
+        }
+        if (!on || heavy) continue;
+        if (!cand) {
+            // history and bond state stay as they are
+            pfl[p] = (unsigned char)(old & PR_HIST);
+            if (DIAG) V.pdn[p] = __int_as_float(0x7fc00000);
+        } else if (bi >= 0) {
+            pair_work64<true, DIAG>(V, cur, Hs, p, g, t, bi, dx, dy, old, pfl, rec, C);
+        } else {
+            pfl[p] = (unsigned char)quiet_candidate<DIAG>(V, Hs, p, dx, dy, dist, deltan, rg, rt, old, rec);
+            if (DIAG) C.cand++;
+        }
+    }
+    __syncwarp();
+    if (DIAG) add_counts(C, V.counters);
+}
+
+// The work list: contacts, and every candidate of a sheltering field.
+template <bool DIAG>
+__global__ void __launch_bounds__(128) k_pairs_list_fp64(Views V, int cur, FP64List L, unsigned char *pfl,
+                                                         PairRec64 *rec)
 {
     step_kernel_entry();
     if (*(volatile int *)V.status & ST_ABORT) return;
     Hist4<double> *Hs = (Hist4<double> *)V.hist[0];   // in place: one thread per pair
     Counts64 C = {0, 0, 0, 0};
     const int stride = gridDim.x * blockDim.x;
-    const int n = *(volatile const int *)&L.n[BONDS];
-    const FP64Item *work = L.work[BONDS];
+    const int n = *(volatile const int *)L.n;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
-        // the screen passes the pair, both slots, the bond index and the
-        // pair's offset along
-        const FP64Item w = work[k];
-        const int p = w.p, g = w.g, t = w.t, bi = w.bi;
-        pair_work64<BONDS, DIAG>(V, cur, Hs, p, g, t, bi, w.dx, w.dy, pfl, rec, C);
+        // the pair, both slots, the bond index and the pair's offset come along
+        const FP64Item w = L.work[k];
+        pair_work64<false, DIAG>(V, cur, Hs, w.p, w.g, w.t, w.bi, w.dx, w.dy, pfl[w.p], pfl, rec, C);
     }
-
+    __syncwarp();
     if (DIAG) add_counts(C, V.counters);
 }
 
@@ -404,7 +381,7 @@ GD_DEV void row_sum(const int2 *ent, int e0, int e1, const unsigned char *pfl, c
 #pragma unroll
         for (int k = 0; k < 4; k++) pk[k] = e + k < e1 ? ent[e + k].y : -1;
 #pragma unroll
-        for (int k = 0; k < 4; k++) fk[k] = pk[k] >= 0 ? pfl[pk[k]] : 0u;
+        for (int k = 0; k < 4; k++) fk[k] = pk[k] >= 0 ? pfl[pk[k]] & ~PR_HIST : 0u;
 #pragma unroll
         for (int k = 0; k < 4; k++)
             if (fk[k]) add_pair<DIAG, LO>(rec, pk[k], fk[k], P, A, run, shel);
@@ -474,7 +451,7 @@ GD_DEV Shape row_sums64(const Views &V, int cur, int g, const InstParams &P, con
                 if (b < l1) idb = V.id[cur][V.ent_lo[b].x];
             }
             const int p = V.ent_lo[take].y;
-            add_pair<true, true>(rec, p, pfl[p], P, A, run, shel);
+            add_pair<true, true>(rec, p, pfl[p] & ~PR_HIST, P, A, run, shel);
         }
         // ---- own row (the floe is "i"): each part sorted, merged by
         // (distance, id)
@@ -489,7 +466,7 @@ GD_DEV Shape row_sums64(const Views &V, int cur, int g, const InstParams &P, con
                 first = da < db || (da == db && V.id[cur][V.ent_up[a].x] < V.id[cur][V.ent_up[b].x]);
             }
             const int p = V.ent_up[first ? a++ : b++].y;
-            add_pair<true, false>(rec, p, pfl[p], P, A, run, shel);
+            add_pair<true, false>(rec, p, pfl[p] & ~PR_HIST, P, A, run, shel);
         }
     }
     return run;
@@ -761,8 +738,8 @@ template <bool DIAG, bool WALLS>
 __global__ void __launch_bounds__(128) k_floes_fp64(Views V, int cur, int sic, const double *fs, int *nwork)
 {
     step_kernel_entry();
-    // the work lists were used by the pair kernels before this one
-    if (blockIdx.x == 0 && threadIdx.x < 2) nwork[threadIdx.x] = 0;
+    // the work list was used by the pair kernels before this one
+    if (blockIdx.x == 0 && threadIdx.x == 0) *nwork = 0;
     if (floe_update_stopped(V, -1, sic)) return;
     const size_t N = (size_t)V.N;
     unsigned long long n_plast = 0;
@@ -813,7 +790,7 @@ struct SmallArgs64 {
     int *done;                     // blocks of k_step_floes_fp64 that have finished
 };
 
-// One owner entry: k_pairs_fp64_screen and k_pairs_fp64 in one.
+// One owner entry: k_pairs_fp64 and k_pairs_list_fp64 in one.
 template <bool DIAG>
 GD_DEV void pair_entry64(const Views &V, int cur, int e, const unsigned *erow, unsigned char *pfl, PairRec64 *rec,
                          Counts64 &C)
@@ -826,22 +803,22 @@ GD_DEV void pair_entry64(const Views &V, int cur, int e, const unsigned *erow, u
     const bool px = P.boundary & BC_PERIODIC_X, py = P.boundary & BC_PERIODIC_Y;
     const double rg = V.r[cur][g], rt = V.r[cur][t];
     const int bi = V.bidx[p];
-    const double2 h01 = *(const double2 *)&Hs[p];
+    const unsigned old = pfl[p];
     const double dx = wrap_d(V.x[cur][g] - V.x[cur][t], P.nx, px);
     const double dy = wrap_d(V.y[cur][g] - V.y[cur][t], P.ny, py);
     const double dist = sqrt(dx * dx + dy * dy);
     V.edist[e] = dist;
     if (!(dist <= rg + P.rtree)) {
         // history and bond state stay as they are
-        pfl[p] = 0;
+        pfl[p] = (unsigned char)(old & PR_HIST);
         if (DIAG) V.pdn[p] = __int_as_float(0x7fc00000);
         return;
     }
     const double deltan = (rg + rt) - dist;
     if (deltan > 0.0 || P.shelter != 0 || bi >= 0) {
-        pair_work64<false, DIAG>(V, cur, Hs, p, g, t, bi, dx, dy, pfl, rec, C);
+        pair_work64<false, DIAG>(V, cur, Hs, p, g, t, bi, dx, dy, old, pfl, rec, C);
     } else {
-        pfl[p] = (unsigned char)quiet_candidate<DIAG>(V, Hs, p, dx, dy, dist, deltan, rg, rt, h01, rec);
+        pfl[p] = (unsigned char)quiet_candidate<DIAG>(V, Hs, p, dx, dy, dist, deltan, rg, rt, old, rec);
         if (DIAG) C.cand++;
     }
 }

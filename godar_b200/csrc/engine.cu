@@ -118,6 +118,12 @@ struct Buf {
     void swap(Buf &o) { std::swap(p, o.p); std::swap(bytes, o.bytes); std::swap(pooled, o.pooled); }
 };
 
+// A piece of a Buf.
+struct Piece {
+    void *p = nullptr;
+    template <class T> T *as() const { return (T *)p; }
+};
+
 // ------------------------------------------------------------ instances
 struct HostBonds {           // one instance's bond table, id order
     std::vector<int> off;    // n+1
@@ -507,8 +513,9 @@ struct Engine {
     // floe state (two sides) and bond table, each in a set that a batch
     // relayout replaces as a whole
     struct FloeSet {
-        Buf x[2], y[2], th[2], u[2], v[2], om[2], r[2], h[2], dtb1[2], dtb2[2], thb1[2], thb2[2];
-        Buf id[2], x0[2], y0[2], snap[2];
+        Buf mem;                 // one allocation, cut into the arrays below
+        Piece x[2], y[2], th[2], u[2], v[2], om[2], r[2], h[2], dtb1[2], dtb2[2], thb1[2], thb2[2];
+        Piece id[2], x0[2], y0[2], snap[2];
     };
     struct BondSet {
         Buf bond_off, bond_hi, bstat, bdyn[1];   // bond state, updated in place
@@ -518,9 +525,9 @@ struct Engine {
     // the sets of the previous layout, the target of the next commit
     std::unique_ptr<FloeSet> spareF;
     std::unique_ptr<BondSet> spareB;
-    // commit scratch: old slot of every new slot, old index of every new
-    // bond, per-instance offset tables
-    Buf repack_b, small_b, bmap_b, rule_b;
+    // commit scratch: old slot of every new slot, the layout's table, bond
+    // creation's rules and totals
+    Buf repack_b, small_b, layout_b, rule_b;
     Buf inst_b, params_b, field_b;
     // rows (primary) and rebuild scratch (secondary)
     Buf up_off, lo_off, ent_up, ent_lo, bidx, hist[1], edist, pdn;
@@ -875,13 +882,20 @@ struct Engine {
     }
 
     int alloc_floe_set(FloeSet &f, int n) {
-        auto ens = [&](Buf &b, size_t s) { return b.ensure(s, &bytes, &mp); };
+        const auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+        const size_t one = up((size_t)n * 8), snap = prec == GODAR_PREC_FP64 ? 0 : up((size_t)n * sizeof(Snap));
+        TRY(f.mem.ensure(2 * (14 * one + up((size_t)n * 4) + snap), &bytes, &mp));
+        char *at = f.mem.as<char>();
+        const auto cut = [&](Piece &q, size_t b) {
+            q.p = at;
+            at += b;
+        };
         for (int s = 0; s < 2; s++) {
-            Buf *dd[] = {&f.x[s], &f.y[s], &f.th[s], &f.u[s], &f.v[s], &f.om[s], &f.r[s], &f.h[s], &f.dtb1[s],
-                         &f.dtb2[s], &f.thb1[s], &f.thb2[s], &f.x0[s], &f.y0[s]};
-            for (Buf *b : dd) TRY(ens(*b, (size_t)n * 8));
-            TRY(ens(f.id[s], (size_t)n * 4));
-            TRY(ens(f.snap[s], (size_t)n * sizeof(Snap)));
+            for (Piece *q : {&f.x[s], &f.y[s], &f.th[s], &f.u[s], &f.v[s], &f.om[s], &f.r[s], &f.h[s], &f.dtb1[s],
+                             &f.dtb2[s], &f.thb1[s], &f.thb2[s], &f.x0[s], &f.y0[s]})
+                cut(*q, one);
+            cut(f.id[s], up((size_t)n * 4));
+            cut(f.snap[s], snap);
         }
         return GODAR_OK;
     }
@@ -1017,15 +1031,10 @@ struct Engine {
             n_tot += I.n;
         }
         if ((long long)n_tot >= INT_MAX / 2) { set_err("too many floes"); return GODAR_ERR_CAPACITY; }
-        std::vector<int> repack(n_tot, -1), hinst(n_tot);
         std::vector<InstParams> hp(ni);
         std::vector<double> hfield;
         for (int k = 0; k < ni; k++) {
             Inst &I = insts[k];
-            for (int i = 0; i < I.n; i++) {
-                hinst[I.off + i] = k;
-                if (!I.pending) repack[I.off + i] = old_off[k] + i;
-            }
             hp[k] = make_params(I, c_tot, f_tot);
             c_tot += (long long)hp[k].ncx * hp[k].ncy;
             if (!I.field.empty()) {
@@ -1056,21 +1065,46 @@ struct Engine {
         TRY(alloc_floe_set(*F, n_tot));
         TRY(alloc_scratch(n_tot));
         const int sn = 0;
+        // uploads of up to a quarter of a megabyte go through the pinned
+        // read-back slots (idle here), the larger ones directly
+        size_t staged = 0;
         auto up = [&](void *dst, const void *src, size_t nbytes) -> int {
-            if (nbytes) CK(cudaMemcpyAsync(dst, src, nbytes, cudaMemcpyHostToDevice, st));
+            if (nbytes == 0) return GODAR_OK;
+            if (nbytes <= 2 * STAGE_SLOT) {
+                if (staged + nbytes > 2 * STAGE_SLOT) {
+                    CK(cudaStreamSynchronize(st));
+                    staged = 0;
+                }
+                std::memcpy(h_stage + staged, src, nbytes);
+                src = h_stage + staged;
+                staged += (nbytes + 15) & ~(size_t)15;
+            }
+            CK(cudaMemcpyAsync(dst, src, nbytes, cudaMemcpyHostToDevice, st));
             return GODAR_OK;
         };
-        TRY(up(inst_b.p, hinst.data(), (size_t)N * 4));
         TRY(params_b.ensure(std::max<size_t>(hp.size(), 1) * sizeof(InstParams), &bytes, &mp));
         TRY(up(params_b.p, hp.data(), hp.size() * sizeof(InstParams)));
         hparams = hp;
         TRY(field_b.ensure(std::max<size_t>(hfield.size(), 1) * 8, &bytes, &mp));
         TRY(up(field_b.p, hfield.data(), hfield.size() * 8));
-        // resident floes, device to device
+        // the layout's table, every slot's field and origin, and the resident
+        // floes, device to device
         TRY(repack_b.ensure((size_t)std::max(N, 1) * 4, &bytes, &mp));
-        TRY(up(repack_b.p, repack.data(), (size_t)N * 4));
+        std::vector<int> tab(4 * std::max(ni, 1), 0);
+        for (int k = 0; k < ni; k++) {
+            tab[k] = insts[k].off;
+            tab[ni + k] = old_off[k];
+            tab[3 * ni + k] = old_boff[k];
+        }
+        TRY(layout_b.ensure(tab.size() * 4, &bytes, &mp));
+        TRY(up(layout_b.p, tab.data(), tab.size() * 4));
+        RelayoutTable T;
+        T.ni = ni;
+        T.off = layout_b.as<int>(); T.old_off = T.off + ni; T.boff = T.off + 2 * ni; T.old_boff = T.off + 3 * ni;
         Views Vn = views();
-        if (oldF && oldN > 0) launch_gather_floes(make_views(*oldF, *oldB), old_cur, Vn, sn, repack_b.as<int>(), N, st);
+        if (N > 0)
+            launch_relayout_floes(oldF && oldN > 0 ? make_views(*oldF, *oldB) : Vn, old_cur, Vn, sn, T, inst_b.as<int>(),
+                                  repack_b.as<int>(), N, st);
         // admitted floes, host to device
         for (Inst &I : insts) {
             if (!I.pending) continue;
@@ -1084,15 +1118,7 @@ struct Engine {
                 TRY(up(F->dtb2[sn].as<double>() + o, I.rx->dtb2.data(), nb8));
                 TRY(up(F->thb1[sn].as<double>() + o, I.rx->thb1.data(), nb8));
                 TRY(up(F->thb2[sn].as<double>() + o, I.rx->thb2.data(), nb8));
-            } else {
-                CK(cudaMemsetAsync(F->dtb1[sn].as<double>() + o, 0, nb8, st));
-                CK(cudaMemsetAsync(F->dtb2[sn].as<double>() + o, 0, nb8, st));
-                CK(cudaMemsetAsync(F->thb1[sn].as<double>() + o, 0, nb8, st));
-                CK(cudaMemsetAsync(F->thb2[sn].as<double>() + o, 0, nb8, st));
             }
-            std::vector<int> ids(I.n);
-            std::iota(ids.begin(), ids.end(), 0);
-            TRY(up(F->id[sn].as<int>() + o, ids.data(), (size_t)I.n * 4));
         }
         // bonds: the fresh fields' counts from the device, then every
         // field's place in the table (instances in layout order)
@@ -1104,36 +1130,18 @@ struct Engine {
             nb_tot += I.nb;
         }
         NB = nb_tot;
-        std::vector<int> bmap(NB, -1);
-        for (int k = 0; k < ni; k++)
-            if (old_boff[k] >= 0)
-                for (int q = 0; q < insts[k].nb; q++) bmap[insts[k].boff + q] = old_boff[k] + q;
         auto ens = [&](Buf &b, size_t sz) { return b.ensure(std::max<size_t>(sz, 16), &bytes, &mp); };
         TRY(ens(BS->bond_off, (size_t)(N + 1) * 4));
         TRY(ens(BS->bond_hi, (size_t)NB * 4));
         TRY(ens(BS->bstat, (size_t)NB * sizeof(BondStat)));
         TRY(ens(BS->bdyn[0], (size_t)NB * sizeof(BondDyn)));
         if (oldB && oldN > 0) {
-            if (NB > 0 && oldNB > 0) {
-                TRY(bmap_b.ensure((size_t)NB * 4, &bytes, &mp));
-                TRY(up(bmap_b.p, bmap.data(), (size_t)NB * 4));
-                launch_gather_bonds(oldB->bond_hi.as<int>(), oldB->bstat.as<BondStat>(),
-                                    oldB->bdyn[0].as<BondDyn>(),
-                                    BS->bond_hi.as<int>(), BS->bstat.as<BondStat>(), BS->bdyn[sn].as<BondDyn>(),
-                                    bmap_b.as<int>(), NB, st);
-            }
-            std::vector<int> tab(4 * ni);
-            for (int k = 0; k < ni; k++) {
-                tab[k] = old_off[k];
-                tab[ni + k] = insts[k].off;
-                tab[2 * ni + k] = old_boff[k];
-                tab[3 * ni + k] = insts[k].boff;
-            }
-            TRY(small_b.ensure((size_t)std::max(4 * ni, 4) * 4, &bytes, &mp));
-            TRY(up(small_b.p, tab.data(), tab.size() * 4));
-            const int *t4 = small_b.as<int>();
-            launch_rebase_bond_off(oldB->bond_off.as<int>(), BS->bond_off.as<int>(), inst_b.as<int>(), t4, t4 + ni,
-                                   t4 + 2 * ni, t4 + 3 * ni, N, st);
+            for (int k = 0; k < ni; k++) tab[k] = insts[k].boff;
+            TRY(up(layout_b.as<int>() + 2 * ni, tab.data(), (size_t)ni * 4));
+            launch_relayout_bonds(oldB->bond_off.as<int>(), BS->bond_off.as<int>(), inst_b.as<int>(),
+                                  oldB->bond_hi.as<int>(), oldB->bstat.as<BondStat>(), oldB->bdyn[0].as<BondDyn>(),
+                                  BS->bond_hi.as<int>(), BS->bstat.as<BondStat>(), BS->bdyn[sn].as<BondDyn>(), T, N,
+                                  oldNB > 0 ? NB : 0, st);
         }
         if (std::any_of(gpu_bonds.begin(), gpu_bonds.end(), [](char c) { return c != 0; }))
             TRY(fill_fresh_bonds(first_pending, gpu_bonds));

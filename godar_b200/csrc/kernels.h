@@ -198,13 +198,17 @@ void launch_instance_summary(const Views &V, int cur, double *out, cudaStream_t 
 void launch_list_pairs(const Views &V, int cur, int off, int n, int which, int cap, int *pi, int *pj, double *val,
                        int *total, int *cnt, int *base, int *scan_scratch, cudaStream_t st);
 
-// Batch relayout (membership changes).
-void launch_gather_floes(const Views &Vo, int so, const Views &Vn, int sn, const int *repack, int n, cudaStream_t st);
-void launch_rebase_bond_off(const int *old_bond_off, int *new_bond_off, const int *inst, const int *old_slot_base,
-                            const int *new_slot_base, const int *old_bbase, const int *new_bbase, int n,
-                            cudaStream_t st);
-void launch_gather_bonds(const int *old_hi, const BondStat *old_st, const BondDyn *old_dy, int *new_hi,
-                         BondStat *new_st, BondDyn *new_dy, const int *bmap, int nb, cudaStream_t st);
+// Batch relayout (membership changes), per field: its first new slot and bond,
+// its first old ones (-1: admitted now).
+struct RelayoutTable {
+    int ni;
+    const int *off, *old_off, *boff, *old_boff;
+};
+void launch_relayout_floes(const Views &Vo, int so, const Views &Vn, int sn, const RelayoutTable &T, int *inst,
+                           int *repack, int n, cudaStream_t st);
+void launch_relayout_bonds(const int *old_bond_off, int *new_bond_off, const int *inst, const int *old_hi,
+                           const BondStat *old_st, const BondDyn *old_dy, int *new_hi, BondStat *new_st,
+                           BondDyn *new_dy, const RelayoutTable &T, int n, int nb, cudaStream_t st);
 void launch_set_int(int *p, int v, cudaStream_t st);
 
 // Bond creation at admission (bonds_init.cu): per-floe bond counts of the

@@ -243,17 +243,37 @@ void launch_list_pairs(const Views &V, int cur, int off, int n, int which, int c
 }  // namespace godar
 
 // ------------------------------------------------------------ relayout
-// Batch membership changes: resident floes move to their new slots
-// device-to-device (new slot g takes old slot repack[g]; -1 = a newly admitted
-// floe, uploaded from the host instead), and their bond records follow
-// (new bond q takes old bond bmap[q]).
+// Batch membership changes.  The host describes the new layout by a few
+// numbers a field (RelayoutTable); which field a slot or a bond belongs to, and
+// where it comes from, is found on the device.
 namespace godar {
 
-__global__ void k_gather_floes(Views Vo, int so, Views Vn, int sn, const int *repack, int n)
+// The last k in [0, n) with start[k] <= g (start[0] = 0, ascending).
+GD_DEV int field_at(const int *start, int n, int g)
+{
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (start[mid] <= g) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+// Every new slot: its field, where its floe was (repack, -1: admitted now),
+// and its state: a resident floe's from the previous layout; of an admitted
+// one its id and empty wall histories (the rest is uploaded).
+__global__ void k_relayout_floes(Views Vo, int so, Views Vn, int sn, RelayoutTable T, int *inst, int *repack, int n)
 {
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < n; g += gridDim.x * blockDim.x) {
-        const int o = repack[g];
-        if (o < 0) continue;
+        const int k = field_at(T.off, T.ni, g), i = g - T.off[k];
+        const int o = T.old_off[k] < 0 ? -1 : T.old_off[k] + i;
+        inst[g] = k;
+        repack[g] = o;
+        if (o < 0) {
+            Vn.dtb1[sn][g] = 0.0; Vn.dtb2[sn][g] = 0.0; Vn.thb1[sn][g] = 0.0; Vn.thb2[sn][g] = 0.0;
+            Vn.id[sn][g] = i;
+            continue;
+        }
         Vn.x[sn][g] = Vo.x[so][o]; Vn.y[sn][g] = Vo.y[so][o]; Vn.th[sn][g] = Vo.th[so][o];
         Vn.u[sn][g] = Vo.u[so][o]; Vn.v[sn][g] = Vo.v[so][o]; Vn.om[sn][g] = Vo.om[so][o];
         Vn.r[sn][g] = Vo.r[so][o]; Vn.h[sn][g] = Vo.h[so][o];
@@ -263,26 +283,25 @@ __global__ void k_gather_floes(Views Vo, int so, Views Vn, int sn, const int *re
     }
 }
 
-// bond_off of resident floes, rebased: the floe with reference id k of
-// instance b keeps its bonds at new index  old_off[old_base_b + k] -
-// old_bbase_b + new_bbase_b.  new_id_base[b] is the instance's first new slot.
-__global__ void k_rebase_bond_off(const int *old_bond_off, int *new_bond_off, const int *inst, const int *old_slot_base,
-                                  const int *new_slot_base, const int *old_bbase, const int *new_bbase, int n)
+// bond_off of resident floes, rebased (the floe with reference id k of field b
+// keeps its bonds), and the resident bonds moved.
+__global__ void k_relayout_bond_off(const int *old_bond_off, int *new_bond_off, const int *inst, RelayoutTable T,
+                                    int n)
 {
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < n; g += gridDim.x * blockDim.x) {
         const int b = inst[g];
-        if (old_slot_base[b] < 0) continue;
-        const int k = g - new_slot_base[b];
-        new_bond_off[g] = old_bond_off[old_slot_base[b] + k] - old_bbase[b] + new_bbase[b];
+        if (T.old_off[b] < 0) continue;
+        new_bond_off[g] = old_bond_off[T.old_off[b] + (g - T.off[b])] - T.old_boff[b] + T.boff[b];
     }
 }
 
-__global__ void k_gather_bonds(const int *old_hi, const BondStat *old_st, const BondDyn *old_dy, int *new_hi,
-                               BondStat *new_st, BondDyn *new_dy, const int *bmap, int nb)
+__global__ void k_relayout_bonds(const int *old_hi, const BondStat *old_st, const BondDyn *old_dy, int *new_hi,
+                                 BondStat *new_st, BondDyn *new_dy, RelayoutTable T, int nb)
 {
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nb; q += gridDim.x * blockDim.x) {
-        const int o = bmap[q];
-        if (o < 0) continue;
+        const int k = field_at(T.boff, T.ni, q);
+        if (T.old_boff[k] < 0) continue;
+        const int o = T.old_boff[k] + (q - T.boff[k]);
         new_hi[q] = old_hi[o];
         new_st[q] = old_st[o];
         new_dy[q] = old_dy[o];
@@ -291,23 +310,18 @@ __global__ void k_gather_bonds(const int *old_hi, const BondStat *old_st, const 
 
 static int rl_grid(int n) { return n > 0 ? ((n + 255) / 256 < 2368 ? (n + 255) / 256 : 2368) : 1; }
 
-void launch_gather_floes(const Views &Vo, int so, const Views &Vn, int sn, const int *repack, int n, cudaStream_t st)
+void launch_relayout_floes(const Views &Vo, int so, const Views &Vn, int sn, const RelayoutTable &T, int *inst,
+                           int *repack, int n, cudaStream_t st)
 {
-    k_gather_floes<<<rl_grid(n), 256, 0, st>>>(Vo, so, Vn, sn, repack, n);
+    k_relayout_floes<<<rl_grid(n), 256, 0, st>>>(Vo, so, Vn, sn, T, inst, repack, n);
 }
 
-void launch_rebase_bond_off(const int *old_bond_off, int *new_bond_off, const int *inst, const int *old_slot_base,
-                            const int *new_slot_base, const int *old_bbase, const int *new_bbase, int n,
-                            cudaStream_t st)
+void launch_relayout_bonds(const int *old_bond_off, int *new_bond_off, const int *inst, const int *old_hi,
+                           const BondStat *old_st, const BondDyn *old_dy, int *new_hi, BondStat *new_st,
+                           BondDyn *new_dy, const RelayoutTable &T, int n, int nb, cudaStream_t st)
 {
-    k_rebase_bond_off<<<rl_grid(n), 256, 0, st>>>(old_bond_off, new_bond_off, inst, old_slot_base, new_slot_base,
-                                                  old_bbase, new_bbase, n);
-}
-
-void launch_gather_bonds(const int *old_hi, const BondStat *old_st, const BondDyn *old_dy, int *new_hi,
-                         BondStat *new_st, BondDyn *new_dy, const int *bmap, int nb, cudaStream_t st)
-{
-    if (nb > 0) k_gather_bonds<<<rl_grid(nb), 256, 0, st>>>(old_hi, old_st, old_dy, new_hi, new_st, new_dy, bmap, nb);
+    k_relayout_bond_off<<<rl_grid(n), 256, 0, st>>>(old_bond_off, new_bond_off, inst, T, n);
+    if (nb > 0) k_relayout_bonds<<<rl_grid(nb), 256, 0, st>>>(old_hi, old_st, old_dy, new_hi, new_st, new_dy, T, nb);
 }
 
 __global__ void k_set_int(int *p, int v) { *p = v; }

@@ -188,13 +188,41 @@ __global__ void k_scan_add(int *out, int n, const int *tile_sums, const int *tot
     if (blockIdx.x == 0 && threadIdx.x == 0 && out_n) *out_n = *total;
 }
 
+// The whole scan by one block: a short one is three launches' latency
+// otherwise (a rebuild of a few hundred floes has five of them).
+constexpr int SC_SHORT = 8192;
+__global__ void __launch_bounds__(1024) k_scan_short(const int *in, int *out, int n)
+{
+    __shared__ int sh[32];
+    constexpr int PER = SC_SHORT / 1024;
+    const int base = threadIdx.x * PER;
+    int v[PER], s = 0;
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        v[k] = base + k < n ? in[base + k] : 0;
+        s += v[k];
+    }
+    int total;
+    int pre = block_excl_scan(s, sh, total);
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        if (base + k < n) out[base + k] = pre;
+        pre += v[k];
+    }
+    if (threadIdx.x == 0) out[n] = total;
+}
+
 void scan_excl(const int *in, int *out, int n, int *scratch, cudaStream_t st)
 {
     // scratch: ntiles + 1 ints; out must hold n + 1 ints
+    if (n <= SC_SHORT) {
+        k_scan_short<<<1, 1024, 0, st>>>(in, out, n);
+        return;
+    }
     const int ntiles = (n + SC_TILE - 1) / SC_TILE;
-    if (n > 0) k_scan_tiles<<<ntiles, SC_THREADS, 0, st>>>(in, out, n, scratch + 1);
+    k_scan_tiles<<<ntiles, SC_THREADS, 0, st>>>(in, out, n, scratch + 1);
     k_scan_sums<<<1, 1024, 0, st>>>(scratch + 1, ntiles, scratch);
-    k_scan_add<<<n > 0 ? (n + 255) / 256 : 1, 256, 0, st>>>(out, n, scratch + 1, scratch, out + n);
+    k_scan_add<<<(n + 255) / 256, 256, 0, st>>>(out, n, scratch + 1, scratch, out + n);
 }
 
 void radix_sort(uint32_t *keys, int *vals, uint32_t *keys_alt, int *vals_alt, int n, int bits,
@@ -483,6 +511,19 @@ __global__ void k_copy_ids(Views V, int from)
     }
 }
 
+// The state fresh rows start from: no error and no expiry, an empty work
+// list and, mixed, no displacement (the contact list holds the gaps at the
+// rebuild).
+__global__ void k_rows_ready(int *status, int *nwork, unsigned *dsp)
+{
+    if (threadIdx.x == 0) {
+        status[0] = 0;
+        status[1] = 0x7fffffff;
+    }
+    if (threadIdx.x < 2) nwork[threadIdx.x] = 0;
+    if (threadIdx.x < 4) dsp[threadIdx.x] = 0;
+}
+
 // ------------------------------------------------------------ host side
 static int grid_for(long long n, int block)
 {
@@ -534,6 +575,11 @@ void launch_row_finish(const Views &V, int mixed, int side, const int *old_slot,
             V, side, old_slot, old_up_off, old_ent_up, old_id, (const Hist4<double> *)old_hist, up_off, lo_off, ent_up,
             ent_lo, (Hist4<double> *)hist, bidx, erow, pdn, pfl, lfl, lo_of, wfo);
     k_copy_ids<<<grid_for(V.N, 256), 256, 0, st>>>(V, side);
+}
+
+void launch_rows_ready(int *status, int *nwork, unsigned *dsp, cudaStream_t st)
+{
+    k_rows_ready<<<1, 32, 0, st>>>(status, nwork, dsp);
 }
 
 }  // namespace godar

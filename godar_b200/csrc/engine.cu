@@ -237,7 +237,7 @@ void restart_bonds(const Inst &I, HostBonds &B)
 // RES_KEPT_BYTES of device memory; what is over is given back to the driver.
 // A set belongs to one engine at a time and comes back with its streams idle.
 constexpr size_t RES_KEPT = 4;
-constexpr size_t RES_KEPT_BYTES = 64u << 20;
+constexpr size_t RES_KEPT_BYTES = 256u << 20;
 constexpr int RES_RING = 16, RES_FRING = 4;
 constexpr size_t STAGE_SLOT = 128 << 10;      // one of two pinned read-back slots
 
@@ -1343,8 +1343,8 @@ struct Engine {
         launch_nbr_count(V, nxt, coff_b.as<int>(), cnt.as<int>(), row_off2.as<int>(), scan_scratch.as<int>(), st);
         // pairs, and entries of both rows (in the status mirror's spare ints)
         int *h_n = h_status + 2;
-        CK(cudaMemcpyAsync(h_n, row_off2.as<int>() + N, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(h_n + 1, row_off2.as<int>() + 2 * N, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpy2DAsync(h_n, sizeof(int), row_off2.as<int>() + N, (size_t)N * sizeof(int), sizeof(int), 2,
+                             cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         const int Pn = h_n[0], Enew = h_n[1];
         if (Enew < 0 || Pn < 0) { set_err("neighbour rows overflow int32"); return GODAR_ERR_CAPACITY; }
@@ -1409,7 +1409,6 @@ struct Engine {
             TRY(fp64_rows(nxt));
         }
         TRY(nwork_b.ensure(16, &bytes, &mp));
-        CK(cudaMemsetAsync(nwork_b.p, 0, 2 * sizeof(int), st));
         // per-floe sums: the FP64 path's ordered record sums, the mixed path's window partials
         TRY(fsum_b.ensure((size_t)N * (fp64 ? 8 * FP64_FLOE_SUMS : 32), &bytes, &mp));
         if (!fp64) {
@@ -1418,14 +1417,12 @@ struct Engine {
             launch_pack_snap(V, nxt, st);
             TRY(contact_list(nxt, Pn));
             TRY(mixed_bond_lists(nxt));
-            // the contact list holds the gaps at the rebuild: D starts at zero
-            CK(cudaMemsetAsync(dsp_b.p, 0, 4 * sizeof(unsigned), st));
         }
         E = Pn;
         cur = nxt;
         rebuilds++;
         gbase = 0;
-        TRY(reset_status());
+        launch_rows_ready(status.as<int>(), nwork_b.as<int>(), dsp_b.as<unsigned>(), st);
         have_rows = true;
         CK(cudaGetLastError());
         return GODAR_OK;
@@ -1440,7 +1437,7 @@ struct Engine {
         int *mark = dist2.as<int>(), *pos = mark + P;
         launch_contact_list(views(), side, P, erow_up.as<unsigned>(), pfl.as<unsigned char>(), mark, pos,
                             cscan_b.as<int>(), clist_b.as<int2>(), clist_b.as<int2>() + Ecap, st);
-        int ec = 0;
+        int &ec = h_status[2];
         CK(cudaMemcpyAsync(&ec, pos + P, sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         Ec = ec;
@@ -1456,7 +1453,7 @@ struct Engine {
         launch_fp64_rows(views(), side, (int)E, erow_up.as<unsigned>(), pfl.as<unsigned char>(), flisted_b.as<unsigned char>(),
                          fupn_b.as<int>(), flon_b.as<int>(), fpart_b.as<int2>(), fpos_b.as<int>(),
                          scan_scratch.as<int>(), fplist_b.as<int>(), st);
-        int lc = 0;
+        int &lc = h_status[2];
         CK(cudaMemcpyAsync(&lc, fpos_b.as<int>() + N, sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         CK(cudaGetLastError());

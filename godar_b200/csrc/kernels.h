@@ -29,17 +29,23 @@ inline void launch_step(bool pdl, void (*kern)(Params...), int grid, int block, 
     cudaLaunchKernelEx(&c, kern, args...);
 }
 
-// Launches a kernel of whole steps (k_steps_fp64, k_steps_mixed) as one
-// cluster of enough blocks to give every one of `items` a thread, at most
-// SMALL_CLUSTER.  False if the launch was refused.
+// Launches a kernel of whole steps (k_steps_fp64, k_steps_mixed) as one block
+// for at most `alone` items, else as one cluster of enough blocks to give
+// every item a thread, at most SMALL_CLUSTER.  One block finds what it wrote
+// in its own L1 and its barrier takes 28 cycles; across blocks every phase
+// starts from L2 behind a barrier of 380, so a few items a thread cost less
+// than a second block: 256 free floes 5.7 against 8.3 us a step FP64, 4.2
+// against 6.9 mixed; 200 bonded ones mixed 8.6 (one block), 12.4 (two), 10.0
+// (four).  False if the launch was refused.
 template <typename... Params, typename... Args>
-inline bool launch_cluster(bool pdl, void (*kern)(Params...), long long items, cudaStream_t st, Args... args)
+inline bool launch_cluster(bool pdl, void (*kern)(Params...), long long items, int alone, cudaStream_t st,
+                           Args... args)
 {
     static const bool wide =
         cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     const int most = wide ? SMALL_CLUSTER : 8;
     int blocks = 1;
-    while (blocks < most && (long long)blocks * SMALL_THREADS < items) blocks *= 2;
+    while (items > alone && blocks < most && (long long)blocks * SMALL_THREADS < items) blocks *= 2;
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3((unsigned)blocks);
     c.blockDim = dim3(SMALL_THREADS);
@@ -72,6 +78,7 @@ void launch_nbr_count(const Views &V, int side, const int *coff, int *cnt, int *
                       cudaStream_t st);
 void launch_nbr_fill(const Views &V, int side, const int *coff, const int *off2, int up_by_id, int *lo_off,
                      int *up_off, int2 *ent_lo, int2 *ent_up, double *dist, cudaStream_t st);
+void launch_rows_ready(int *status, int *nwork, unsigned *dsp, cudaStream_t st);
 void launch_row_finish(const Views &V, int mixed, int side, const int *old_slot, const int *old_up_off,
                        const int2 *old_ent_up, const int *old_id, const void *old_hist, const int *up_off,
                        const int *lo_off, const int2 *ent_up, int2 *ent_lo, void *hist, int *bidx, unsigned *erow,
@@ -108,9 +115,10 @@ void launch_fp64_bonds(const Views &V, int side, int *cnt, int *wfo, int *scan_s
 // shelter: some field of the batch has sheltering; drag: 8 N doubles; out:
 // pinned host memory for the status word and the first expired step; done: an
 // int that is zero): as one launch of one cluster up to ONE_CLUSTER_* items
-// (positions, bonds and floes), else as two launches a step.  False if the
-// launch was refused.
+// (positions, bonds and floes; one block up to ONE_BLOCK_*), else as two
+// launches a step.  False if the launch was refused.
 constexpr int ONE_CLUSTER_FP64 = 1024, ONE_CLUSTER_MIXED = 4096;
+constexpr int ONE_BLOCK_FP64 = 640, ONE_BLOCK_MIXED = 1024;
 bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int shelter,
                        const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
                        const int *up_n, double *drag, int *out, int *done, cudaStream_t st);

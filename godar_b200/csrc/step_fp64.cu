@@ -64,7 +64,7 @@ bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, 
     A.n = n; A.E = E; A.plist = plist; A.erow = erow; A.pfl = pfl; A.rec = (PairRec64 *)rec;
     A.lo_n = lo_n; A.up_n = up_n; A.drag = drag; A.out = out; A.done = done;
     const long long items = (long long)n + V.N;
-    if (!shelter && items <= ONE_CLUSTER_FP64) return launch_cluster(V.pdl != 0, k_steps_fp64, items, st, V, A);
+    if (!shelter && items <= ONE_CLUSTER_FP64) return launch_cluster(V.pdl != 0, k_steps_fp64, items, ONE_BLOCK_FP64, st, V, A);
     const int rounds = group_rounds(V.N, shelter);
     for (int k = 0; k < K; k++) {
         const int c = cur ^ (k & 1);

@@ -1322,7 +1322,7 @@ bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base,
     A.out = out;
     A.done = done;
     const long long all = (long long)n + NB + V.N;
-    if (!shelter && all <= ONE_CLUSTER_MIXED) return launch_cluster(V.pdl != 0, k_steps_mixed, all, st, V, A, B);
+    if (!shelter && all <= ONE_CLUSTER_MIXED) return launch_cluster(V.pdl != 0, k_steps_mixed, all, ONE_BLOCK_MIXED, st, V, A, B);
     const int rounds = group_rounds(V.N, shelter);
     for (int k = 0; k < K; k++) {
         const int c = cur ^ (k & 1);

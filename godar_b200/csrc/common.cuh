@@ -248,12 +248,12 @@ GD_DEV void cluster_sync()
 }
 
 // One thread: the status word and the first expired step into pinned host
-// memory.
+// memory.  The host reads them after an event or the stream's end, which the
+// kernel's own end makes them visible to: no fence.
 GD_DEV void publish_status(const Views &V, int *out)
 {
     ((volatile int *)out)[0] = *(volatile const int *)V.status;
     ((volatile int *)out)[1] = *(volatile const int *)V.expired_at;
-    __threadfence_system();
 }
 
 // The same by the last block of a grid to get here (every block calls it

@@ -455,8 +455,8 @@ struct Engine {
     double skin_frac = 0.01;
     double kernel_ms = 0.0;        // device time inside step kernels
     long long launches = 0;        // time steps launched
-    // the kernels of a time step: mixed [pair screen, pair work list, bonds,
-    // floe sums, floe update]; FP64 [pairs, pair work list, none, row sums,
+    // the kernels of a time step: mixed [pairs, pairs of a diagnostic step,
+    // bonds, floe sums, floe update]; FP64 [pairs, pair work list, none, row sums,
     // floe update]
     static constexpr int NPH = 5;
     static constexpr int NEV = NPH + 2;   // timing events per step
@@ -533,7 +533,7 @@ struct Engine {
     Buf up_off, lo_off, ent_up, ent_lo, bidx, hist[1], edist, pdn;
     // mixed path: row of every owner entry, partner index, flags, pair records;
     // bond records, bond slots and the partner-bond lists
-    Buf erow_up, lo_of, pfl, lfl, prec_b, prx_b, pdg_b, work_b, work_st_b, nwork_b, fsum_b, frex_b, fdg_b, clist_b, cscan_b;
+    Buf erow_up, lo_of, pfl, lfl, prec_b, prx_b, pdg_b, work_b, nwork_b, fsum_b, frex_b, fdg_b, clist_b, cscan_b;
     // FP64 path: the pair records and the bonds' geometry in working order (the
     // row of every owner entry, the pair flags, the work list and the bonds'
     // working state are the mixed path's erow_up, pfl, work_b and wdyn_b)
@@ -1356,7 +1356,7 @@ struct Engine {
             // what the previous rows hold in these does not outlive them
             const long long cap = (long long)(Pn * 1.25) + 1024;
             Buf *pb[] = {&edist, &pdn, &erow_up, &lo_of, &pfl, &lfl,
-                         &prec_b, &prx_b, &pdg_b, &work_b, &work_st_b, &clist_b, &cscan_b, &frec_b,
+                         &prec_b, &prx_b, &pdg_b, &work_b, &clist_b, &cscan_b, &frec_b,
                          &flisted_b, &fpart_b, &fplist_b};
             for (Buf *b : pb) b->release(&bytes);
             TRY(ens(pdn, cap * 4));
@@ -1369,7 +1369,7 @@ struct Engine {
             } else {
                 TRY(ens(erow_up, cap * 4)); TRY(ens(lo_of, cap * 4));
                 // flag bytes are read in aligned 8-byte words
-                TRY(ens(pfl, cap + 16)); TRY(ens(lfl, cap + 16)); TRY(ens(work_b, cap * 4)); TRY(ens(work_st_b, cap * 8));
+                TRY(ens(pfl, cap + 16)); TRY(ens(lfl, cap + 16));
                 // the contact list: {entry, bound} for every item, then {slots}
                 TRY(ens(clist_b, cap * 16)); TRY(ens(cscan_b, (cap / 2048 + 16) * 4));
                 TRY(ens(prec_b, cap * 32)); TRY(ens(prx_b, cap * 8)); TRY(ens(pdg_b, cap * 32));
@@ -1468,7 +1468,6 @@ struct Engine {
         B.rec = prec_b.as<float4>(); B.rx = prx_b.as<float2>(); B.pdg = pdg_b.as<float4>();
         B.brec = brec.as<float4>(); B.bdg = bdg.as<float4>(); B.bsp = wsp_b.as<int4>(); B.wdyn = wdyn_b.as<BondDyn>(); B.winv = winv_b.as<int>();
         
-        B.work = work_b.as<int>(); B.nwork = nwork_b.as<int>(); B.work_st = work_st_b.as<int2>();
         B.bfo = bfo.as<int>(); B.bst = bst32.as<BondGeom32>();
         B.fsum = fsum_b.as<float4>(); B.frex = frex_b.as<float>(); B.fdg = fdg_b.as<float4>();
         B.dsp = dsp_b.as<unsigned>();
@@ -1578,7 +1577,7 @@ struct Engine {
             launch_pairs_screen(V, side, diag, diag ? (int)E : (int)Ec, diag ? nullptr : clist_b.as<int2>(),
                                 clist_b.as<int2>() + Ecap, B, cfg_block(bs[0]), cfg_variant(bs[0]), st);
             if (ev) TRY(record(ev[1], capturing));
-            launch_pairs_work(V, side, diag, (int)E, erow_up.as<unsigned>(), B, cfg_block(bs[1]), st);
+            if (diag) launch_pairs_diag(V, side, (int)E, erow_up.as<unsigned>(), B, cfg_block(bs[1]), st);
             if (ev) TRY(record(ev[2], capturing));
             if (conc) CK(cudaStreamWaitEvent(st, ev_join, 0));
             else launch_bonds_mixed(V, side, diag, NB, B, cfg_block(bs[2]), cfg_variant(bs[2]), test_wait_spins, st);
@@ -1628,7 +1627,7 @@ struct Engine {
     }
 
     int kernels_per_step() const {
-        return prec == GODAR_PREC_FP64 ? 4 : (E > 0 ? 2 : 0) + (NB > 0 ? 1 : 0) + 2;
+        return prec == GODAR_PREC_FP64 ? 4 : (E > 0 ? 1 : 0) + (NB > 0 ? 1 : 0) + 2;
     }
 
     // The graph of K steps from side c0, captured on first use.  Returns

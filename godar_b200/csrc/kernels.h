@@ -149,8 +149,6 @@ struct MixedBufs {
     const unsigned char *bfl_rd;   // [NB] live-bond flags at the start of the step
     unsigned char *bfl_wr;         // [NB] ... at its end (the other side)
     int4 *bsp;                  // [NB] slots of the bond's two floes, positions of their records (working order)
-    int *work, *nwork;          // [P] owner entries for the full pair computation, and their count
-    int2 *work_st;              // [P] their row and partner slots (not on diagnostic steps)
     float4 *fsum;               // [2N] per floe: fcx fcy mc fbx | fby mb shelter(air) shelter(water)
     float *frex;                // [N] per floe: ridging excess
     float4 *fdg;                // [2N] per floe, diagnostic steps: tac pc tab pb | sxx syy sxy syx
@@ -170,7 +168,8 @@ void launch_pairs_screen(const Views &V, int cur, int diag, int P, int2 *eb, con
                          MixedBufs B, int block, int variant, cudaStream_t st);
 void launch_contact_list(const Views &V, int side, int P, const unsigned *erow, const unsigned char *pfl, int *mark,
                          int *pos, int *scan_scratch, int2 *eb, int2 *stl, cudaStream_t st);
-void launch_pairs_work(const Views &V, int cur, int diag, int P, const unsigned *erow_up, MixedBufs B, int block,
+// Diagnostic steps: the pair physics of every owner entry.
+void launch_pairs_diag(const Views &V, int cur, int P, const unsigned *erow_up, MixedBufs B, int block,
                        cudaStream_t st);
 void launch_floe_sums(const Views &V, int diag, MixedBufs B, int block, cudaStream_t st);
 void launch_bonds_mixed(const Views &V, int cur, int diag, int NB, MixedBufs B, int block, int variant,

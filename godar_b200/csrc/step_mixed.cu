@@ -312,91 +312,6 @@ GD_DEV float advance_bound(int cur, const MixedBufs &B)
     return Dk;
 }
 
-// Appends entry e of every lane with `heavy` to the work list, with its
-// slots st where known (st.x >= 0), one atomic per warp; every lane of the
-// warp must call it.
-GD_DEV void work_append(bool heavy, int e, int2 st, int lane, const MixedBufs &B)
-{
-    const unsigned m = __ballot_sync(0xffffffffu, heavy);
-    if (m) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(B.nwork, __popc(m));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (heavy) {
-            const int q = base + __popc(m & ((1u << lane) - 1u));
-            B.work[q] = e;
-            if (st.x >= 0) B.work_st[q] = st;
-        }
-    }
-}
-
-// SCREEN_U: contact-list items per lane per round (the screen's tile,
-// chosen per batch by the autotuner among 4, 8 and 16)
-template <int SCREEN_U>
-__global__ void __launch_bounds__(256) k_pairs_screen(Views V, int cur, int diag, int P, int2 *eb,
-                                                      const int2 *stl, MixedBufs B)
-{
-    step_kernel_entry();
-    if (*(volatile int *)V.status & ST_ABORT) return;
-    // items of a round that need the FP64 test, per warp
-    __shared__ int chk[256 / 32][SCREEN_U * 32];
-    const Snap *S = V.snap[cur];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int stride = gridDim.x * blockDim.x;
-    const int nit = (P + stride - 1) / stride;
-    const float Dk = advance_bound(cur, B);
-    // a diagnostic step computes every owner entry: the pair kernel walks
-    // them itself, without a work list
-    if (diag || !eb) return;
-    const float thr = __fadd_ru(2.f * Dk, 1e-6f);
-    const unsigned lt = (1u << lane) - 1u;
-    int k0 = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int it = 0; it < nit; it += SCREEN_U, k0 += SCREEN_U * stride) {
-        // the bound test of SCREEN_U items per lane, their loads issued
-        // together; the items that fail it are gathered per warp ...
-        //
-        // A pair with a contact history, or with a force record from its last
-        // computation, is in contact or was at that computation; conservative
-        // advancement keeps its bound at or below the threshold from then on
-        // (and the contact list is built with a bound of at most -1 for a pair
-        // with a history), so an item that passes the bound test carries
-        // neither: its flags need not be read.
-        int2 c[SCREEN_U];
-#pragma unroll
-        for (int u = 0; u < SCREEN_U; u++) {
-            const int k = k0 + u * stride;
-            c[u] = make_int2(-1, 0);
-            if (it + u < nit && k < P) c[u] = eb[k];
-        }
-        int cnt = 0;
-#pragma unroll
-        for (int u = 0; u < SCREEN_U; u++) {
-            const bool need = c[u].x >= 0 && !(__int_as_float(c[u].y) > thr);
-            // gathered per warp, then tested together
-            const unsigned m = __ballot_sync(0xffffffffu, need);
-            if (need) chk[warp][cnt + __popc(m & lt)] = k0 + u * stride;
-            cnt += __popc(m);
-        }
-        __syncwarp();
-        // ... one item per lane: a pair with a history goes on the work list
-        // at once, the others by the FP64 test
-        for (int j0 = 0; j0 < cnt; j0 += 32) {
-            bool heavy = false;
-            int e = 0;
-            int2 st = make_int2(-1, -1);
-            if (j0 + lane < cnt) {
-                const int k = chk[warp][j0 + lane];
-                const int2 ck = eb[k];
-                e = ck.x;
-                st = stl[k];
-                heavy = screen_test(V, S, eb, k, ck, st, (unsigned)B.pfl[e], Dk, B);
-            }
-            work_append(heavy, e, st, lane, B);
-        }
-        __syncwarp();
-    }
-}
-
 // The pair physics of owner entry e (slots s, t): contact forces, ridging
 // event, sheltering, history update, record and flags.
 GD_DEV void pair_mixed(const Views &V, const Snap *S, Hist4<float> *Hh, int diag, int e, int s, int t,
@@ -499,43 +414,119 @@ GD_DEV void pair_mixed(const Views &V, const Snap *S, Hist4<float> *Hh, int diag
     }
 }
 
-// Pairs of the work list: contact forces, ridging events, sheltering,
-// history updates and records.
-__global__ void __launch_bounds__(256, 3) k_pairs_mixed(Views V, int cur, int diag, int P, const unsigned *erow,
-                                                        MixedBufs B)
+// The contact list: the bound test, the FP64 test of the items that fail it,
+// and the pair physics of those that touch, have touched or shelter.
+//
+// The screen and the physics were two kernels with a work list between them
+// (an append of one atomic on one address a warp, both floes gathered twice, a
+// launch): 35-56 + 29 us on 2.2 M floes (growing with the bound), 54-71 us in
+// one.  One wave of blocks, so
+// that a warp meets enough heavy pairs to fill its lanes: they collect in
+// shared memory and go through the physics 32 at a time.
+//
+// SCREEN_U: contact-list items per lane per round (the screen's tile,
+// chosen per batch by the autotuner among 4, 8 and 16)
+template <int SCREEN_U>
+__global__ void __launch_bounds__(256, 3) k_pairs_screen(Views V, int cur, int diag, int P, int2 *eb,
+                                                         const int2 *stl, MixedBufs B)
+{
+    step_kernel_entry();
+    if (*(volatile int *)V.status & ST_ABORT) return;
+    // items of a round that need the FP64 test, per warp, and the heavy ones
+    // waiting for a full warp (entry, slots)
+    __shared__ int chk[256 / 32][SCREEN_U * 32];
+    __shared__ int heavy_e[256 / 32][64];
+    __shared__ int2 heavy_st[256 / 32][64];
+    const Snap *S = V.snap[cur];
+    Hist4<float> *Hh = (Hist4<float> *)V.hist[0];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int stride = gridDim.x * blockDim.x;
+    const int nit = (P + stride - 1) / stride;
+    const float Dk = advance_bound(cur, B);
+    // a diagnostic step computes every owner entry in k_pairs_mixed
+    if (diag || !eb) return;
+    const float thr = __fadd_ru(2.f * Dk, 1e-6f);
+    const unsigned lt = (1u << lane) - 1u;
+    unsigned long long none = 0;
+    int waiting = 0;
+    int k0 = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int it = 0; it < nit; it += SCREEN_U, k0 += SCREEN_U * stride) {
+        // the bound test of SCREEN_U items per lane, their loads issued
+        // together; the items that fail it are gathered per warp ...
+        //
+        // A pair with a contact history, or with a force record from its last
+        // computation, is in contact or was at that computation; conservative
+        // advancement keeps its bound at or below the threshold from then on
+        // (and the contact list is built with a bound of at most -1 for a pair
+        // with a history), so an item that passes the bound test carries
+        // neither: its flags need not be read.
+        int2 c[SCREEN_U];
+#pragma unroll
+        for (int u = 0; u < SCREEN_U; u++) {
+            const int k = k0 + u * stride;
+            c[u] = make_int2(-1, 0);
+            if (it + u < nit && k < P) c[u] = eb[k];
+        }
+        int cnt = 0;
+#pragma unroll
+        for (int u = 0; u < SCREEN_U; u++) {
+            const bool need = c[u].x >= 0 && !(__int_as_float(c[u].y) > thr);
+            // gathered per warp, then tested together
+            const unsigned m = __ballot_sync(0xffffffffu, need);
+            if (need) chk[warp][cnt + __popc(m & lt)] = k0 + u * stride;
+            cnt += __popc(m);
+        }
+        __syncwarp();
+        // ... one item per lane: a pair with a history is heavy at once, the
+        // others by the FP64 test
+        for (int j0 = 0; j0 < cnt; j0 += 32) {
+            bool heavy = false;
+            int e = 0;
+            int2 st = make_int2(-1, -1);
+            if (j0 + lane < cnt) {
+                const int k = chk[warp][j0 + lane];
+                const int2 ck = eb[k];
+                e = ck.x;
+                st = stl[k];
+                heavy = screen_test(V, S, eb, k, ck, st, (unsigned)B.pfl[e], Dk, B);
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, heavy);
+            if (heavy) {
+                const int q = waiting + __popc(m & lt);
+                heavy_e[warp][q] = e;
+                heavy_st[warp][q] = st;
+            }
+            waiting += __popc(m);
+            __syncwarp();
+            if (waiting >= 32) {
+                waiting -= 32;
+                const int2 h = heavy_st[warp][waiting + lane];
+                pair_mixed(V, S, Hh, 0, heavy_e[warp][waiting + lane], h.x, h.y, B, none, none, none);
+                __syncwarp();
+            }
+        }
+        __syncwarp();
+    }
+    if (lane < waiting) {
+        const int2 h = heavy_st[warp][lane];
+        pair_mixed(V, S, Hh, 0, heavy_e[warp][lane], h.x, h.y, B, none, none, none);
+    }
+}
+
+// The pair physics of a diagnostic step: every owner entry.
+__global__ void __launch_bounds__(256, 3) k_pairs_mixed(Views V, int cur, int P, const unsigned *erow, MixedBufs B)
 {
     step_kernel_entry();
     if (*(volatile int *)V.status & ST_ABORT) return;
     Hist4<float> *Hh = (Hist4<float> *)V.hist[0];
     const Snap *S = V.snap[cur];
     unsigned long long n_cand = 0, n_cont = 0, n_plast = 0;
-    // the work list of the screen, or on a diagnostic step every owner entry
-    const int n = diag ? P : *(volatile const int *)B.nwork;
-    const int stride = gridDim.x * blockDim.x;
-    // every lane of a warp runs the same number of iterations (the counters
-    // are reduced with full-warp shuffles at the end)
-    const int nit = (n + stride - 1) / stride;
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int it = 0; it < nit; it++, k += stride) {
-        if (k >= n) continue;
-        const int e = diag ? k : B.work[k];
-        // the screen passes the slots along, except on diagnostic steps
-        int s, t;
-        if (diag) {
-            s = (int)erow[e];
-            t = V.ent_up[e].x;
-        } else {
-            const int2 st = B.work_st[k];
-            s = st.x;
-            t = st.y;
-        }
-        pair_mixed(V, S, Hh, diag, e, s, t, B, n_cand, n_cont, n_plast);
-    }
-    if (diag) {
-        warp_count(n_cand, V.counters, 0);
-        warp_count(n_cont, V.counters, 1);
-        warp_count(n_plast, V.counters, 3);
-    }
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < P; e += gridDim.x * blockDim.x)
+        pair_mixed(V, S, Hh, 1, e, (int)erow[e], V.ent_up[e].x, B, n_cand, n_cont, n_plast);
+    __syncwarp();
+    warp_count(n_cand, V.counters, 0);
+    warp_count(n_cont, V.counters, 1);
+    warp_count(n_plast, V.counters, 3);
 }
 
 // One lane per bond.  A broken bond is skipped (its record was zeroed when it
@@ -892,9 +883,6 @@ template <bool DIAG>
 __global__ void __launch_bounds__(256, 8) k_floe_sums(Views V, MixedBufs B)
 {
     step_kernel_entry();
-    // the work list of the next step starts empty (the pair kernels of this
-    // step have completed)
-    if (blockIdx.x == 0 && threadIdx.x == 0) *B.nwork = 0;
     if (*(volatile int *)V.status & ST_ABORT) return;
     const int stride = gridDim.x * blockDim.x;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < V.N; g += stride) {
@@ -1554,8 +1542,9 @@ void launch_pairs_screen(const Views &V, int cur, int diag, int P, int2 *eb, con
                          MixedBufs B, int block, int variant, cudaStream_t st)
 {
     if (P <= 0) return;
-    // a diagnostic step only advances the displacement bound here
-    const int grid = diag ? 1 : grid_of(P, block);
+    // a diagnostic step only advances the displacement bound here; a plain one
+    // runs one wave (three blocks of 256 threads an SM)
+    const int grid = diag ? 1 : std::max(1, std::min((P + block - 1) / block, 148 * (768 / block)));
     if (variant == 1) launch_step(V.pdl != 0, k_pairs_screen<4>, grid, block, st, V, cur, diag, P, eb, stl, B);
     else if (variant == 2) launch_step(V.pdl != 0, k_pairs_screen<16>, grid, block, st, V, cur, diag, P, eb, stl, B);
     else launch_step(V.pdl != 0, k_pairs_screen<8>, grid, block, st, V, cur, diag, P, eb, stl, B);
@@ -1570,12 +1559,10 @@ bool step_pdl()
     return on;
 }
 
-void launch_pairs_work(const Views &V, int cur, int diag, int P, const unsigned *erow_up, MixedBufs B, int block,
+void launch_pairs_diag(const Views &V, int cur, int P, const unsigned *erow_up, MixedBufs B, int block,
                        cudaStream_t st)
 {
-    // the list length is only known on the device: a grid of a few CTAs per
-    // SM strides over it
-    if (P > 0) launch_step(V.pdl != 0, k_pairs_mixed, 148 * (1024 / block), block, st, V, cur, diag, P, erow_up, B);
+    if (P > 0) launch_step(V.pdl != 0, k_pairs_mixed, 148 * (1024 / block), block, st, V, cur, P, erow_up, B);
 }
 
 void launch_bonds_mixed(const Views &V, int cur, int diag, int NB, MixedBufs B, int block, int variant,

@@ -499,8 +499,9 @@ __global__ void __launch_bounds__(256) k_row_finish(Views V, int side, const int
     }
 }
 
-// Ids and rebuild positions on both sides (after the histories moved: they
-// are found by the previous layout's ids).
+// Ids, rebuild positions and shapes on both sides (after the histories moved:
+// they are found by the previous layout's ids); a batch whose shapes cannot
+// change does not write them again.
 __global__ void k_copy_ids(Views V, int from)
 {
     const int to = from ^ 1;
@@ -508,6 +509,8 @@ __global__ void k_copy_ids(Views V, int from)
         V.id[to][s] = V.id[from][s];
         V.x0[to][s] = V.x0[from][s];
         V.y0[to][s] = V.y0[from][s];
+        V.r[to][s] = V.r[from][s];
+        V.h[to][s] = V.h[from][s];
     }
 }
 

@@ -1540,6 +1540,7 @@ struct Engine {
         V.pdl = step_pdl() && N <= PDL_MAX_FLOES;
         if (ev) TRY(record(ev[0], capturing));
         if (NB > 0) wdirty = true;
+        const int light = !ridging_any && !shelter_any && !walls_any;
         if (prec == GODAR_PREC_FP64) {
             FP64List L;
             L.work = work_b.as<FP64Item>();
@@ -1553,10 +1554,10 @@ struct Engine {
             // (the third phase has no kernel of its own)
             if (ev) TRY(record(ev[2], capturing));
             if (ev) TRY(record(ev[3], capturing));
-            launch_row_sums_fp64(V, side, diag, pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
+            launch_row_sums_fp64(V, side, diag, light, pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
                                  fupn_b.as<int>(), fsum_b.as<double>(), cfg_block(bs[3]), st);
             if (ev) TRY(record(ev[4], capturing));
-            launch_floes_fp64(V, side, diag, sic, walls_any ? 1 : 0, fsum_b.as<double>(), nwork_b.as<int>(),
+            launch_floes_fp64(V, side, diag, sic, walls_any ? 1 : 0, light, fsum_b.as<double>(), nwork_b.as<int>(),
                               cfg_block(bs[4]), st);
             if (ev)
                 for (int q = 5; q < NEV; q++) TRY(record(ev[q], capturing));
@@ -1582,9 +1583,10 @@ struct Engine {
             if (conc) CK(cudaStreamWaitEvent(st, ev_join, 0));
             else launch_bonds_mixed(V, side, diag, NB, B, cfg_block(bs[2]), cfg_variant(bs[2]), test_wait_spins, st);
             if (ev) TRY(record(ev[3], capturing));
-            launch_floe_sums(V, diag, B, cfg_block(bs[3]), st);
+            launch_floe_sums(V, diag, light, B, cfg_block(bs[3]), st);
             if (ev) TRY(record(ev[4], capturing));
-            launch_floes_mixed(V, side, diag, sic, walls_any ? 1 : 0, B, cfg_block(bs[4]), st);
+            // (without a contact list only diagnostic steps would advance the bound)
+            launch_floes_mixed(V, side, diag, sic, walls_any ? 1 : 0, light, Ec > 0 ? 1 : 0, B, cfg_block(bs[4]), st);
             if (ev) TRY(record(ev[5], capturing));
         }
         return GODAR_OK;

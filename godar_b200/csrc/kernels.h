@@ -96,7 +96,8 @@ void launch_pairs_fp64(const Views &V, int cur, int diag, int n, const int *plis
                        unsigned char *pfl, FP64List L, void *rec, int block, cudaStream_t st);
 void launch_pairs_list_fp64(const Views &V, int cur, int diag, int E, unsigned char *pfl, FP64List L, void *rec,
                             int block, cudaStream_t st);
-void launch_row_sums_fp64(const Views &V, int cur, int diag, const unsigned char *pfl, const void *rec,
+// (light: no field of the batch has ridging, sheltering or walls)
+void launch_row_sums_fp64(const Views &V, int cur, int diag, int light, const unsigned char *pfl, const void *rec,
                           const int *lo_n, const int *up_n, double *fs, int block, cudaStream_t st);
 // At a rebuild: the pairs that can act on a step without diagnostics before
 // the next one marked (listed[p]), every row reordered to hold them first
@@ -105,7 +106,7 @@ void launch_row_sums_fp64(const Views &V, int cur, int diag, const unsigned char
 // Also sets the pairs' flags before the first step.
 void launch_fp64_rows(const Views &V, int side, int E, const unsigned *erow, unsigned char *pfl,
                       unsigned char *listed, int *up_n, int *lo_n, int2 *tmp, int *pos, int *scan_scratch, int *plist, cudaStream_t st);
-void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, const double *fs, int *nwork, int block,
+void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, int light, const double *fs, int *nwork, int block,
                        cudaStream_t st);
 // At a rebuild: the bonds' working order (perm; wfo: N + 1, its first index of
 // every slot) and working copies.  cnt: N.
@@ -171,11 +172,13 @@ void launch_contact_list(const Views &V, int side, int P, const unsigned *erow, 
 // Diagnostic steps: the pair physics of every owner entry.
 void launch_pairs_diag(const Views &V, int cur, int P, const unsigned *erow_up, MixedBufs B, int block,
                        cudaStream_t st);
-void launch_floe_sums(const Views &V, int diag, MixedBufs B, int block, cudaStream_t st);
+// light: no field of the batch has ridging, sheltering or walls; bounded: the
+// pair kernel advances the displacement bound in every step since the rebuild.
+void launch_floe_sums(const Views &V, int diag, int light, MixedBufs B, int block, cudaStream_t st);
 void launch_bonds_mixed(const Views &V, int cur, int diag, int NB, MixedBufs B, int block, int variant,
                         unsigned test_spins, cudaStream_t st);
-void launch_floes_mixed(const Views &V, int cur, int diag, int sic, int walls, MixedBufs B, int block,
-                        cudaStream_t st);
+void launch_floes_mixed(const Views &V, int cur, int diag, int sic, int walls, int light, int bounded, MixedBufs B,
+                        int block, cudaStream_t st);
 
 // The same on the mixed path (n contact-list items eb/stl, bfl: the live-bond
 // flags of both sides).

@@ -34,24 +34,26 @@ void launch_pairs_list_fp64(const Views &V, int cur, int diag, int E, unsigned c
     else launch_step(V.pdl != 0, k_pairs_list_fp64<false>, grid, block, st, V, cur, L, pfl, r);
 }
 
-void launch_row_sums_fp64(const Views &V, int cur, int diag, const unsigned char *pfl, const void *rec,
+void launch_row_sums_fp64(const Views &V, int cur, int diag, int light, const unsigned char *pfl, const void *rec,
                           const int *lo_n, const int *up_n, double *fs, int block, cudaStream_t st)
 {
     const PairRec64 *r = (const PairRec64 *)rec;
-    if (diag) launch_step(V.pdl != 0, k_row_sums_fp64<true>, fp64_grid(V.N, block), block, st, V, cur, pfl, r, lo_n, up_n, fs);
-    else launch_step(V.pdl != 0, k_row_sums_fp64<false>, fp64_grid(V.N, block), block, st, V, cur, pfl, r, lo_n, up_n, fs);
+    if (diag) launch_step(V.pdl != 0, k_row_sums_fp64<true, false>, fp64_grid(V.N, block), block, st, V, cur, pfl, r, lo_n, up_n, fs);
+    else if (light) launch_step(V.pdl != 0, k_row_sums_fp64<false, true>, fp64_grid(V.N, block), block, st, V, cur, pfl, r, lo_n, up_n, fs);
+    else launch_step(V.pdl != 0, k_row_sums_fp64<false, false>, fp64_grid(V.N, block), block, st, V, cur, pfl, r, lo_n, up_n, fs);
 }
 
-void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, const double *fs, int *nwork, int block,
+void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, int light, const double *fs, int *nwork, int block,
                        cudaStream_t st)
 {
     const int grid = fp64_grid(V.N, block);
     if (walls) {
-        if (diag) launch_step(V.pdl != 0, k_floes_fp64<true, true>, grid, block, st, V, cur, sic, fs, nwork);
-        else launch_step(V.pdl != 0, k_floes_fp64<false, true>, grid, block, st, V, cur, sic, fs, nwork);
+        if (diag) launch_step(V.pdl != 0, k_floes_fp64<true, true, false>, grid, block, st, V, cur, sic, fs, nwork);
+        else launch_step(V.pdl != 0, k_floes_fp64<false, true, false>, grid, block, st, V, cur, sic, fs, nwork);
     } else {
-        if (diag) launch_step(V.pdl != 0, k_floes_fp64<true, false>, grid, block, st, V, cur, sic, fs, nwork);
-        else launch_step(V.pdl != 0, k_floes_fp64<false, false>, grid, block, st, V, cur, sic, fs, nwork);
+        if (diag) launch_step(V.pdl != 0, k_floes_fp64<true, false, false>, grid, block, st, V, cur, sic, fs, nwork);
+        else if (light) launch_step(V.pdl != 0, k_floes_fp64<false, false, true>, grid, block, st, V, cur, sic, fs, nwork);
+        else launch_step(V.pdl != 0, k_floes_fp64<false, false, false>, grid, block, st, V, cur, sic, fs, nwork);
     }
 }
 

@@ -562,6 +562,7 @@ struct Engine {
     int gbase = 0;
     // (its second int counts the blocks of a chunk's last kernel, launch_small)
     Buf step_base_b;
+    int dev_base = -1;      // what step_base_b holds in stream order (-1: unknown)
     // asynchronous steps (godar_batch_step_async): chunks launched whose
     // status has not been read yet, oldest first.  Each has a pinned slot
     // that receives the status word and the first expired step after it.
@@ -1700,6 +1701,22 @@ struct Engine {
         return GODAR_OK;
     }
 
+    // The chunk's first step number in device memory, and after its steps the
+    // status word in the host's slot `hs` (pinned) with the next chunk's first
+    // number: one small kernel between two chunks of a batch that keeps
+    // stepping.  Between the last kernel of a queued step and the first of the
+    // next: 23 us with a copy of the status, a kernel for the number and a
+    // graph, 5 us now.
+    void begin_chunk() {
+        if (dev_base == gbase) return;
+        launch_set_int(step_base_b.as<int>(), gbase, st);
+        dev_base = gbase;
+    }
+    void end_chunk(int K, int *hs) {
+        dev_base = gbase + K;
+        launch_chunk_end(status.as<int>(), hs, step_base_b.as<int>(), dev_base, st);
+    }
+
     // Launches K steps from side c0 (diagnostics on the last one if
     // diag_last) directly or through a captured graph.
     // every > 0: steps k of the chunk with k % every == 0 record the timing
@@ -1711,7 +1728,9 @@ struct Engine {
             kev.push_back(e);
         }
         const bool pow2 = (K & (K - 1)) == 0;
-        if (graphs_on && !tuning && pow2) {
+        // (one step's launches are shorter than its kernels, and the first of
+        // them starts sooner than a graph)
+        if (graphs_on && !tuning && pow2 && K > 1) {
             if (graph_gen != rebuilds) {
                 drop_graphs();
                 graph_gen = rebuilds;
@@ -1780,7 +1799,7 @@ struct Engine {
             int bs[NPH];
             for (int q = 0; q < NPH; q++) bs[q] = blk[q];
             small = small && launch_small(K, cur, diag_last, h_status);
-            if (!small) launch_set_int(step_base_b.as<int>(), gbase, st);
+            if (!small) begin_chunk();
             if (small) {
                 // launched
             } else if (tuning) {
@@ -1804,7 +1823,7 @@ struct Engine {
             if (NB > 0) wdirty = true;
             CK(cudaGetLastError());
             // (a small batch's kernel has written the status word itself)
-            if (!small) CK(cudaMemcpyAsync(h_status, status.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+            if (!small) end_chunk(K, h_status);
             CK(cudaStreamSynchronize(st));
             const int stt = h_status[0];
             if (stt & ST_NAN) { set_err("non-finite floe state"); return GODAR_ERR_NAN; }
@@ -1927,10 +1946,10 @@ struct Engine {
             small = small && launch_small(K, cur, diag_last, hs);
             P.small = small;
             if (!small) {
-                launch_set_int(step_base_b.as<int>(), gbase, st);
+                begin_chunk();
                 // queued steps record no timing events: nothing reads them
                 TRY(launch_chunk(K, cur, diag_last, blk, false, 0));
-                CK(cudaMemcpyAsync(hs, status.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+                end_chunk(K, hs);
             }
             if (NB > 0) wdirty = true;
             CK(cudaGetLastError());
@@ -2132,9 +2151,8 @@ struct Engine {
             for (int k = 0; k < FRING; k++) CK(cudaMallocHost(&fring[k], fring_cap * sizeof(double)));
         }
         std::memcpy(fring[q], uvw, 4 * ni * sizeof(double));
-        // the four doubles are contiguous in InstParams: one strided copy
-        CK(cudaMemcpy2DAsync((char *)params_b.p + offsetof(InstParams, ua), sizeof(InstParams), fring[q],
-                             4 * sizeof(double), 4 * sizeof(double), ni, cudaMemcpyHostToDevice, st));
+        launch_set_forcing((InstParams *)params_b.p, (int)ni, fring[q], st);
+        CK(cudaGetLastError());
         CK(cudaEventRecord(fring_ev[q], st));
         fring_used[q] = true;
         return GODAR_OK;
@@ -2181,13 +2199,15 @@ struct Engine {
         CK(cudaEventRecord(ev_state, st));
         CK(cudaStreamWaitEvent(stg, ev_state, 0));
         Views V = views();
-        for (int k = 0; k < nf; k++) launch_gather_field(V, cur, -1, 0, N, fields[k], async_tmp[sl][k].as<double>(), stg);
-        CK(cudaEventRecord(ev_gath[sl], stg));
-        gath_rec[sl] = true;
         gath_side[sl] = cur;
-        CK(cudaStreamWaitEvent(stc, ev_gath[sl], 0));
-        for (int k = 0; k < nf; k++)
+        // a field's copy waits for its own gather only
+        for (int k = 0; k < nf; k++) {
+            launch_gather_field(V, cur, -1, 0, N, fields[k], async_tmp[sl][k].as<double>(), stg);
+            CK(cudaEventRecord(ev_gath[sl], stg));
+            gath_rec[sl] = true;
+            CK(cudaStreamWaitEvent(stc, ev_gath[sl], 0));
             CK(cudaMemcpyAsync(outs[k], async_tmp[sl][k].p, (size_t)N * 8, cudaMemcpyDeviceToHost, stc));
+        }
         CK(cudaEventRecord(ev_copy[sl], stc));
         copy_pend[sl] = true;
         // the previous call's outputs are complete when this call returns

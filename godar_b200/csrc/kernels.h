@@ -195,6 +195,7 @@ void launch_hist_inject(const Views &V, int cur, int off, int nh, const int *pi,
 // Output helpers.  Field codes GODAR_F_*; GATHER_DTB1 .. + 3: the wall
 // histories deltat_bc1, deltat_bc2, theta_bc1, theta_bc2.
 constexpr int GATHER_DTB1 = 100;
+void launch_set_forcing(InstParams *P, int ni, const double *uvw, cudaStream_t st);
 void launch_gather_field(const Views &V, int cur, int inst, int off, int n, int field, double *out, cudaStream_t st);
 // Several fields of the instance at slots [off, off + n) in id order, field q
 // at out + q n.
@@ -220,6 +221,8 @@ void launch_relayout_bonds(const int *old_bond_off, int *new_bond_off, const int
                            const BondStat *old_st, const BondDyn *old_dy, int *new_hi, BondStat *new_st,
                            BondDyn *new_dy, const RelayoutTable &T, int n, int nb, cudaStream_t st);
 void launch_set_int(int *p, int v, cudaStream_t st);
+// hs[0..1] = status[0..1] (hs: pinned host memory), *base = next.
+void launch_chunk_end(const int *status, int *hs, int *base, int next, cudaStream_t st);
 
 // Bond creation at admission (bonds_init.cu): per-floe bond counts of the
 // admitted floes [s0, s0 + n) on side `side` and their scan (coff, list: their

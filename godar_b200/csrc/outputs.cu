@@ -177,41 +177,87 @@ __global__ void __launch_bounds__(1024) k_list_pairs(Views V, int cur, int off, 
 // physics.f90:179-198), summed over a block-stride loop and a fixed tree in
 // shared memory: deterministic for a given state in a given memory order of
 // the floes (their cell order at the last neighbour rebuild).
+// It runs beside the next step, whose one-wave kernels wait for the slots its
+// blocks hold, so its latency counts: the chains of sums stay those of
+// SUM_THREADS threads, but four times as many threads load the floes and form
+// the terms (a round ahead of the sums), and each quarter adds one component.
+// 512 fields, 2.2 M floes: 60 -> 33 us (one field's block of 256 threads took
+// its loads one floe at a time; the largest field, 16,384 floes, is the tail).
 constexpr int SUM_THREADS = 256;
-__global__ void __launch_bounds__(SUM_THREADS) k_instance_summary(Views V, int cur, double4 *out)
+constexpr int SUM_U = 1;
+__global__ void __launch_bounds__(4 * SUM_THREADS, 2) k_instance_summary(Views V, int cur, double4 *out)
 {
-    __shared__ double4 red[SUM_THREADS];
+    constexpr int T = 4 * SUM_THREADS;
+    __shared__ double term[4][SUM_U * T];
     const InstParams &P = V.P[blockIdx.x];
-    double4 a = make_double4(0.0, 0.0, 0.0, 0.0);
-    for (int i = threadIdx.x; i < P.n; i += SUM_THREADS) {
-        const int g = P.off + i;
-        const double r = V.r[cur][g], h = V.h[cur][g];
-        const double u = V.u[cur][g], v = V.v[cur][g], om = V.om[cur][g];
-        const double m = ((P.rhoice * P.pi) * h) * (r * r);
-        const double in = (0.5 * m) * (r * r);
-        const double s2 = u * u + v * v;
-        a.x = a.x + m * u;
-        a.y = a.y + m * v;
-        a.z = a.z + ((0.5 * m) * s2 + (0.5 * in) * (om * om));
-        a.w = fmax(a.w, sqrt(s2));
-    }
-    red[threadIdx.x] = a;
-    __syncthreads();
-    for (int w = SUM_THREADS / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) {
-            const double4 b = red[threadIdx.x + w];
-            double4 c = red[threadIdx.x];
-            c.x = c.x + b.x; c.y = c.y + b.y; c.z = c.z + b.z; c.w = fmax(c.w, b.w);
-            red[threadIdx.x] = c;
+    const int n = P.n, off = P.off;
+    const double rp = P.rhoice * P.pi;
+    const int part = threadIdx.x / SUM_THREADS, t = threadIdx.x % SUM_THREADS;
+    double a = 0.0;
+    double r[SUM_U], h[SUM_U], u[SUM_U], v[SUM_U], om[SUM_U];
+    auto load = [&](int base) {
+#pragma unroll
+        for (int q = 0; q < SUM_U; q++) {
+            const int i = off + min(base + q * T + (int)threadIdx.x, n - 1);
+            r[q] = V.r[cur][i]; h[q] = V.h[cur][i];
+            u[q] = V.u[cur][i]; v[q] = V.v[cur][i]; om[q] = V.om[cur][i];
+        }
+    };
+    if (n > 0) load(0);
+    for (int base = 0; base < n; base += SUM_U * T) {
+#pragma unroll
+        for (int q = 0; q < SUM_U; q++) {
+            const double m = (rp * h[q]) * (r[q] * r[q]);
+            const double in = (0.5 * m) * (r[q] * r[q]);
+            const double s2 = u[q] * u[q] + v[q] * v[q];
+            const int at = q * T + threadIdx.x;
+            term[0][at] = m * u[q];
+            term[1][at] = m * v[q];
+            term[2][at] = (0.5 * m) * s2 + (0.5 * in) * (om[q] * om[q]);
+            term[3][at] = s2;
+        }
+        if (base + SUM_U * T < n) load(base + SUM_U * T);
+        __syncthreads();
+        const double *w = term[part] + t;
+        const int m = min((n - base - t + SUM_THREADS - 1) / SUM_THREADS, 4 * SUM_U);
+        if (part < 3) {
+            for (int k = 0; k < m; k++) a = a + w[k * SUM_THREADS];
+        } else {
+            for (int k = 0; k < m; k++) a = fmax(a, w[k * SUM_THREADS]);
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[blockIdx.x] = red[0];
+    // (monotone: the root of the largest is the largest root)
+    if (part == 3) a = sqrt(a);
+    double *red = term[part];
+    red[t] = a;
+    __syncthreads();
+    for (int w = SUM_THREADS / 2; w > 0; w >>= 1) {
+        if (t < w) red[t] = part < 3 ? red[t] + red[t + w] : fmax(red[t], red[t + w]);
+        __syncthreads();
+    }
+    if (t == 0) reinterpret_cast<double *>(out + blockIdx.x)[part] = red[0];
 }
 
 void launch_instance_summary(const Views &V, int cur, double *out, cudaStream_t st)
 {
-    if (V.ninst > 0) k_instance_summary<<<V.ninst, SUM_THREADS, 0, st>>>(V, cur, reinterpret_cast<double4 *>(out));
+    if (V.ninst > 0) k_instance_summary<<<V.ninst, 4 * SUM_THREADS, 0, st>>>(V, cur, reinterpret_cast<double4 *>(out));
+}
+
+// The four forcing numbers of every field into its parameters, read from
+// pinned host memory: one small kernel (a strided copy of 512 rows held the
+// stream longer).
+__global__ void k_set_forcing(InstParams *P, int ni, const double4 *uvw)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= ni) return;
+    const double4 f = uvw[k];
+    P[k].ua = f.x; P[k].va = f.y; P[k].uw = f.z; P[k].vw = f.w;
+}
+
+void launch_set_forcing(InstParams *P, int ni, const double *uvw, cudaStream_t st)
+{
+    k_set_forcing<<<(ni + 255) / 256, 256, 0, st>>>(P, ni, reinterpret_cast<const double4 *>(uvw));
 }
 
 void launch_gather_field(const Views &V, int cur, int inst, int off, int n, int field, double *out, cudaStream_t st)
@@ -331,6 +377,18 @@ __global__ void k_set_int(int *p, int v) { *p = v; }
 void launch_set_int(int *p, int v, cudaStream_t st)
 {
     k_set_int<<<1, 1, 0, st>>>(p, v);
+}
+
+__global__ void k_chunk_end(const int *status, int *hs, int *base, int next)
+{
+    hs[0] = status[0];
+    hs[1] = status[1];
+    *base = next;
+}
+
+void launch_chunk_end(const int *status, int *hs, int *base, int next, cudaStream_t st)
+{
+    k_chunk_end<<<1, 1, 0, st>>>(status, hs, base, next);
 }
 
 }  // namespace godar

@@ -1555,8 +1555,12 @@ struct Engine {
             // (the third phase has no kernel of its own)
             if (ev) TRY(record(ev[2], capturing));
             if (ev) TRY(record(ev[3], capturing));
-            launch_row_sums_fp64(V, side, diag, light, pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
-                                 fupn_b.as<int>(), fsum_b.as<double>(), cfg_block(bs[3]), st);
+            if (shelter_any && !diag)
+                launch_group_sums_fp64(V, side, pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(), fupn_b.as<int>(),
+                                       fsum_b.as<double>(), st);
+            else
+                launch_row_sums_fp64(V, side, diag, light, pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
+                                     fupn_b.as<int>(), fsum_b.as<double>(), cfg_block(bs[3]), st);
             if (ev) TRY(record(ev[4], capturing));
             launch_floes_fp64(V, side, diag, sic, walls_any ? 1 : 0, light, fsum_b.as<double>(), nwork_b.as<int>(),
                               cfg_block(bs[4]), st);
@@ -1584,7 +1588,8 @@ struct Engine {
             if (conc) CK(cudaStreamWaitEvent(st, ev_join, 0));
             else launch_bonds_mixed(V, side, diag, NB, B, cfg_block(bs[2]), cfg_variant(bs[2]), test_wait_spins, st);
             if (ev) TRY(record(ev[3], capturing));
-            launch_floe_sums(V, diag, light, B, cfg_block(bs[3]), st);
+            if (shelter_any && !diag) launch_group_sums_mixed(V, B, st);
+            else launch_floe_sums(V, diag, light, B, cfg_block(bs[3]), st);
             if (ev) TRY(record(ev[4], capturing));
             // (without a contact list only diagnostic steps would advance the bound)
             launch_floes_mixed(V, side, diag, sic, walls_any ? 1 : 0, light, Ec > 0 ? 1 : 0, B, cfg_block(bs[4]), st);

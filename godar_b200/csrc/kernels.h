@@ -106,6 +106,8 @@ void launch_row_sums_fp64(const Views &V, int cur, int diag, int light, const un
 // Also sets the pairs' flags before the first step.
 void launch_fp64_rows(const Views &V, int side, int E, const unsigned *erow, unsigned char *pfl,
                       unsigned char *listed, int *up_n, int *lo_n, int2 *tmp, int *pos, int *scan_scratch, int *plist, cudaStream_t st);
+void launch_group_sums_fp64(const Views &V, int cur, const unsigned char *pfl, const void *rec, const int *lo_n,
+                            const int *up_n, double *fs, cudaStream_t st);
 void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, int light, const double *fs, int *nwork, int block,
                        cudaStream_t st);
 // At a rebuild: the bonds' working order (perm; wfo: N + 1, its first index of
@@ -124,14 +126,15 @@ bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, 
                        const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
                        const int *up_n, double *drag, int *out, int *done, cudaStream_t st);
 
-// Rounds of GRP_FLOES floes that a block of the two-launch step sums by
-// groups of lanes; 0: one thread per floe.
-inline int group_rounds(int N, int shelter)
+// How a plain step of the merged kernels sums the pairs of a floe: one thread
+// a floe; by groups of lanes in the update's kernel, up to one wave of its
+// blocks; by groups of lanes in a kernel of their own (sheltering fields, whose
+// every candidate has a record).
+enum GroupSums { SUMS_THREAD, SUMS_GROUP, SUMS_GROUP_APART };
+inline GroupSums group_sums(int N, int shelter)
 {
-    const int wave = 148 * 2 * GRP_FLOES;     // floes of one round of every block that fits the GPU at once
-    int r = 1;
-    while (r < GRP && N > r * wave) r *= 2;
-    return shelter || r == 1 ? r : 0;
+    if (N <= 148 * 2 * GRP_FLOES) return SUMS_GROUP;
+    return shelter ? SUMS_GROUP_APART : SUMS_THREAD;
 }
 
 // Mixed precision: (b) one lane per pair with warp-segmented sums, (b') the
@@ -175,6 +178,7 @@ void launch_pairs_diag(const Views &V, int cur, int P, const unsigned *erow_up, 
 // light: no field of the batch has ridging, sheltering or walls; bounded: the
 // pair kernel advances the displacement bound in every step since the rebuild.
 void launch_floe_sums(const Views &V, int diag, int light, MixedBufs B, int block, cudaStream_t st);
+void launch_group_sums_mixed(const Views &V, MixedBufs B, cudaStream_t st);
 void launch_bonds_mixed(const Views &V, int cur, int diag, int NB, MixedBufs B, int block, int variant,
                         unsigned test_spins, cudaStream_t st);
 void launch_floes_mixed(const Views &V, int cur, int diag, int sic, int walls, int light, int bounded, MixedBufs B,

@@ -43,6 +43,14 @@ void launch_row_sums_fp64(const Views &V, int cur, int diag, int light, const un
     else launch_step(V.pdl != 0, k_row_sums_fp64<false, false>, fp64_grid(V.N, block), block, st, V, cur, pfl, r, lo_n, up_n, fs);
 }
 
+// Plain steps of sheltering batches too large for the merged steps.
+void launch_group_sums_fp64(const Views &V, int cur, const unsigned char *pfl, const void *rec, const int *lo_n,
+                            const int *up_n, double *fs, cudaStream_t st)
+{
+    launch_step(V.pdl != 0, k_group_sums_fp64, (V.N + GRP_FLOES - 1) / GRP_FLOES, SMALL_THREADS, st, V, cur, pfl,
+                (const PairRec64 *)rec, lo_n, up_n, fs);
+}
+
 void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, int light, const double *fs, int *nwork, int block,
                        cudaStream_t st)
 {
@@ -67,18 +75,28 @@ bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, 
     A.lo_n = lo_n; A.up_n = up_n; A.drag = drag; A.out = out; A.done = done;
     const long long items = (long long)n + V.N;
     if (!shelter && items <= ONE_CLUSTER_FP64) return launch_cluster(V.pdl != 0, k_steps_fp64, items, ONE_BLOCK_FP64, st, V, A);
-    const int rounds = group_rounds(V.N, shelter);
+    const GroupSums how = group_sums(V.N, shelter);
+    // the drag planes of floes out of sheltering fields, then the sums
+    double *fs = drag + 8 * (size_t)V.N;
     for (int k = 0; k < K; k++) {
         const int c = cur ^ (k & 1);
         const bool diag = diag_last && k == K - 1;
-        const int gp = fp64_grid((long long)(diag ? E : n) + 32 + V.N, 128);
-        if (diag) launch_step(V.pdl != 0, k_step_pairs_fp64<true>, gp, 128, st, V, A, c);
-        else launch_step(V.pdl != 0, k_step_pairs_fp64<false>, gp, 128, st, V, A, c);
-        if (diag) launch_step(V.pdl != 0, k_step_floes_fp64<true>, fp64_grid(V.N, 64), 64, st, V, A, c, k);
-        else if (rounds == 0) launch_step(V.pdl != 0, k_step_floes_fp64<false>, fp64_grid(V.N, 64), 64, st, V, A, c, k);
-        else
-            launch_step(V.pdl != 0, k_step_floes_grp_fp64, (V.N + rounds * GRP_FLOES - 1) / (rounds * GRP_FLOES),
-                        SMALL_THREADS, st, V, A, c, k, rounds);
+        const long long work = (long long)(diag ? E : n) + 32 + V.N;
+        const int gp = fp64_grid(work, 128);
+        const bool dense = work > 148 * 2 * 128;
+        if (diag) launch_step(V.pdl != 0, dense ? k_step_pairs_fp64<true, 4> : k_step_pairs_fp64<true, 2>, gp, 128, st, V, A, c);
+        else launch_step(V.pdl != 0, dense ? k_step_pairs_fp64<false, 4> : k_step_pairs_fp64<false, 2>, gp, 128, st, V, A, c);
+        const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
+        if (diag) {
+            launch_step(V.pdl != 0, k_step_floes_fp64<true>, fp64_grid(V.N, 64), 64, st, V, A, c, k);
+        } else if (how == SUMS_THREAD) {
+            launch_step(V.pdl != 0, k_step_floes_fp64<false>, fp64_grid(V.N, 64), 64, st, V, A, c, k);
+        } else if (how == SUMS_GROUP) {
+            launch_step(V.pdl != 0, k_step_floes_grp_fp64, groups, SMALL_THREADS, st, V, A, c, k);
+        } else {
+            launch_step(V.pdl != 0, k_group_sums_fp64, groups, SMALL_THREADS, st, V, c, pfl, A.rec, lo_n, up_n, fs);
+            launch_step(V.pdl != 0, k_step_update_fp64, fp64_grid(V.N, 64), 64, st, V, A, c, k, fs);
+        }
     }
     return true;
 }

@@ -221,7 +221,7 @@ GD_DEV void pair_work64(const Views &V, int cur, Hist4<double> *Hs, int p, int g
 // state in reference order, and every pair's history read and written back.
 // 529,113 floes, 0.82 M bonds: 41 + 84 us then, 77 us now.
 template <bool DIAG>
-__global__ void __launch_bounds__(128) k_pairs_fp64(Views V, int cur, int n, const int *plist, const unsigned *erow,
+__global__ void __launch_bounds__(128, DIAG ? 4 : 6) k_pairs_fp64(Views V, int cur, int n, const int *plist, const unsigned *erow,
                                                     unsigned char *pfl, FP64List L, PairRec64 *rec)
 {
     step_kernel_entry();
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(128) k_pairs_fp64(Views V, int cur, int n, con
 
 // The work list: contacts, and every candidate of a sheltering field.
 template <bool DIAG>
-__global__ void __launch_bounds__(128) k_pairs_list_fp64(Views V, int cur, FP64List L, unsigned char *pfl,
+__global__ void __launch_bounds__(128, 4) k_pairs_list_fp64(Views V, int cur, FP64List L, unsigned char *pfl,
                                                          PairRec64 *rec)
 {
     step_kernel_entry();
@@ -899,8 +899,12 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_steps_fp64(Views V, SmallA
 // The two halves of a step as ordinary grids, for batches with more work
 // than one cluster does quickly: two launches a step instead of five.  The
 // second one of a chunk's last step publishes the status word.
-template <bool DIAG>
-__global__ void __launch_bounds__(128) k_step_pairs_fp64(Views V, SmallArgs64 A, int cur)
+// MINB blocks an SM: a sheltering pair is a chain of dependent FP64
+// instructions and loads (the FP64 pipe 15% busy at 182 registers and two
+// blocks), so items that fill more than one wave of two blocks run four, at
+// the price of a few spills: 65,536 sheltering floes 195 -> 145 us.
+template <bool DIAG, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_step_pairs_fp64(Views V, SmallArgs64 A, int cur)
 {
     step_kernel_entry();
     if (*(volatile int *)V.status & ST_ABORT) return;
@@ -916,47 +920,89 @@ __global__ void __launch_bounds__(128) k_step_floes_fp64(Views V, SmallArgs64 A,
 }
 
 // The second half of a plain step with the floes' sums by groups of lanes: a
-// block sums GRP_FLOES floes at a time, `rounds` times (at most GRP), then
-// gives every floe's update a thread.
-__global__ void __launch_bounds__(SMALL_THREADS, 2) k_step_floes_grp_fp64(Views V, SmallArgs64 A, int cur, int sic,
-                                                                          int rounds)
+// block sums GRP_FLOES floes, then gives every floe's update a thread.
+__global__ void __launch_bounds__(SMALL_THREADS, 2) k_step_floes_grp_fp64(Views V, SmallArgs64 A, int cur, int sic)
 {
     __shared__ GroupList list[GRP_FLOES];
-    __shared__ double sum[10][SMALL_THREADS];
+    __shared__ double sum[10][GRP_FLOES];
     __shared__ int stopped;
     step_kernel_entry();
     // one answer per block: another block may raise an expiry meanwhile
     if (threadIdx.x == 0) stopped = floe_update_stopped(V, A.base, sic);
     __syncthreads();
-    const int grp = threadIdx.x / GRP, per = rounds * GRP_FLOES;
-    for (int g0 = blockIdx.x * per; !stopped && g0 < V.N; g0 += gridDim.x * per) {
-        for (int r = 0; r < rounds; r++) {
-            const int at = r * GRP_FLOES + grp;
-            const bool on = g0 + at < V.N;
-            Acc<double> S;
-            Shape run;
-            run.r = run.h = 0.0;
-            group_sums64(V, cur, on, g0 + at, A.pfl, A.rec, A.lo_n, A.up_n, list[grp], S, run);
-            if (on && threadIdx.x % GRP == 0) {
-                sum[0][at] = S.fcx; sum[1][at] = S.fcy; sum[2][at] = S.mc;
-                sum[3][at] = S.fbx; sum[4][at] = S.fby; sum[5][at] = S.mb;
-                sum[6][at] = S.hsfa; sum[7][at] = S.hsfw;
-                sum[8][at] = run.r; sum[9][at] = run.h;
-            }
+    const int grp = threadIdx.x / GRP;
+    for (int g0 = blockIdx.x * GRP_FLOES; !stopped && g0 < V.N; g0 += gridDim.x * GRP_FLOES) {
+        const bool on = g0 + grp < V.N;
+        Acc<double> S;
+        Shape run;
+        run.r = run.h = 0.0;
+        group_sums64(V, cur, on, g0 + grp, A.pfl, A.rec, A.lo_n, A.up_n, list[grp], S, run);
+        if (on && threadIdx.x % GRP == 0) {
+            sum[0][grp] = S.fcx; sum[1][grp] = S.fcy; sum[2][grp] = S.mc;
+            sum[3][grp] = S.fbx; sum[4][grp] = S.fby; sum[5][grp] = S.mb;
+            sum[6][grp] = S.hsfa; sum[7][grp] = S.hsfw;
+            sum[8][grp] = run.r; sum[9][grp] = run.h;
         }
         __syncthreads();
         const int q = threadIdx.x, g = g0 + q;
-        if (q < per && g < V.N) {
+        if (q < GRP_FLOES && g < V.N) {
             const InstParams &P = V.P[V.inst[g]];
-            Acc<double> S;
             S.fcx = sum[0][q]; S.fcy = sum[1][q]; S.mc = sum[2][q];
             S.fbx = sum[3][q]; S.fby = sum[4][q]; S.mb = sum[5][q];
             S.hsfa = sum[6][q]; S.hsfw = sum[7][q];
-            const Shape run = make_shape(P, sum[8][q], sum[9][q]);
+            run = make_shape(P, sum[8][q], sum[9][q]);
             floe_update64<false, true>(V, cur, A.base, sic, g, P, S, run, P.shelter != 0 ? nullptr : A.drag);
         }
         __syncthreads();
     }
+    if (sic == A.K - 1) publish_status_last(V, A.done, A.out);
+}
+
+// The sums of a plain step by groups of lanes as a kernel of their own, for
+// sheltering batches of more floes than one wave of the kernel above: they
+// wait for loads, and without the update's registers four blocks an SM wait
+// side by side instead of two.  18,945 sheltering floes: 93 -> 66 us a step;
+// 65,536: 253 -> 198, of which the pairs' denser blocks give 50.
+__global__ void __launch_bounds__(SMALL_THREADS, 4) k_group_sums_fp64(Views V, int cur, const unsigned char *pfl,
+                                                                      const PairRec64 *rec, const int *lo_n,
+                                                                      const int *up_n, double *fs)
+{
+    __shared__ GroupList list[GRP_FLOES];
+    step_kernel_entry();
+    if (*(volatile int *)V.status & ST_ABORT) return;
+    const size_t N = (size_t)V.N;
+    const int grp = threadIdx.x / GRP;
+    for (int g0 = blockIdx.x * GRP_FLOES; g0 < V.N; g0 += gridDim.x * GRP_FLOES) {
+        const int g = g0 + grp;
+        const bool on = g < V.N;
+        Acc<double> S;
+        Shape run;
+        run.r = run.h = 0.0;
+        group_sums64(V, cur, on, g, pfl, rec, lo_n, up_n, list[grp], S, run);
+        if (on && threadIdx.x % GRP == 0) {
+            fs[FS64_FCX * N + g] = S.fcx; fs[FS64_FCY * N + g] = S.fcy; fs[FS64_MC * N + g] = S.mc;
+            fs[FS64_FBX * N + g] = S.fbx; fs[FS64_FBY * N + g] = S.fby; fs[FS64_MB * N + g] = S.mb;
+            fs[FS64_HSFA * N + g] = S.hsfa; fs[FS64_HSFW * N + g] = S.hsfw;
+            fs[FS64_R * N + g] = run.r; fs[FS64_H * N + g] = run.h;
+        }
+    }
+}
+
+// ... and the update from them, as the last kernel of a small batch's step.
+__global__ void __launch_bounds__(64) k_step_update_fp64(Views V, SmallArgs64 A, int cur, int sic, const double *fs)
+{
+    step_kernel_entry();
+    const size_t N = (size_t)V.N;
+    if (!floe_update_stopped(V, A.base, sic))
+        for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < V.N; g += gridDim.x * blockDim.x) {
+            const InstParams &P = V.P[V.inst[g]];
+            Acc<double> S;
+            S.fcx = fs[FS64_FCX * N + g]; S.fcy = fs[FS64_FCY * N + g]; S.mc = fs[FS64_MC * N + g];
+            S.fbx = fs[FS64_FBX * N + g]; S.fby = fs[FS64_FBY * N + g]; S.mb = fs[FS64_MB * N + g];
+            S.hsfa = fs[FS64_HSFA * N + g]; S.hsfw = fs[FS64_HSFW * N + g];
+            const Shape run = make_shape(P, fs[FS64_R * N + g], fs[FS64_H * N + g]);
+            floe_update64<false, true>(V, cur, A.base, sic, g, P, S, run, P.shelter != 0 ? nullptr : A.drag);
+        }
     if (sic == A.K - 1) publish_status_last(V, A.done, A.out);
 }
 

@@ -1276,7 +1276,10 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_steps_mixed(Views V, Small
 // than one cluster does quickly: two launches a step instead of five (three
 // where the bonds follow the pairs).  The last one of a chunk's last step
 // publishes the status word.
-__global__ void __launch_bounds__(128) k_step_pairs_mixed(Views V, SmallArgs32 A, MixedBufs B, int cur, int diag)
+// MINB blocks an SM: as k_step_pairs_fp64 (65,536 sheltering floes: 117 -> 112
+// us a step).
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB) k_step_pairs_mixed(Views V, SmallArgs32 A, MixedBufs B, int cur, int diag)
 {
     step_kernel_entry();
     if (*(volatile int *)V.status & ST_ABORT) return;
@@ -1294,32 +1297,28 @@ __global__ void __launch_bounds__(128) k_step_floes_mixed(Views V, SmallArgs32 A
 // The second half of a plain step with the floes' sums by groups of lanes
 // (k_step_floes_grp_fp64).
 __global__ void __launch_bounds__(SMALL_THREADS, 2) k_step_floes_grp_mixed(Views V, SmallArgs32 A, MixedBufs B,
-                                                                           int cur, int sic, int rounds)
+                                                                           int cur, int sic)
 {
-    __shared__ float sum[9][SMALL_THREADS];
+    __shared__ float sum[9][GRP_FLOES];
     __shared__ int stopped;
     step_kernel_entry();
     // one answer per block: another block may raise an expiry meanwhile
     if (threadIdx.x == 0) stopped = floe_update_stopped(V, A.base, sic);
     __syncthreads();
-    const int grp = threadIdx.x / GRP, per = rounds * GRP_FLOES;
+    const int grp = threadIdx.x / GRP;
     unsigned dmx = 0;
-    for (int g0 = blockIdx.x * per; !stopped && g0 < V.N; g0 += gridDim.x * per) {
-        for (int r = 0; r < rounds; r++) {
-            const int at = r * GRP_FLOES + grp;
-            const bool on = g0 + at < V.N;
-            FloeSum32 F;
-            group_sum32(V, B, on, g0 + at, F);
-            if (on && threadIdx.x % GRP == 0) {
-                sum[0][at] = F.fcx; sum[1][at] = F.fcy; sum[2][at] = F.mc;
-                sum[3][at] = F.fbx; sum[4][at] = F.fby; sum[5][at] = F.mb;
-                sum[6][at] = F.sca; sum[7][at] = F.scw; sum[8][at] = F.rex;
-            }
+    for (int g0 = blockIdx.x * GRP_FLOES; !stopped && g0 < V.N; g0 += gridDim.x * GRP_FLOES) {
+        const bool on = g0 + grp < V.N;
+        FloeSum32 F;
+        group_sum32(V, B, on, g0 + grp, F);
+        if (on && threadIdx.x % GRP == 0) {
+            sum[0][grp] = F.fcx; sum[1][grp] = F.fcy; sum[2][grp] = F.mc;
+            sum[3][grp] = F.fbx; sum[4][grp] = F.fby; sum[5][grp] = F.mb;
+            sum[6][grp] = F.sca; sum[7][grp] = F.scw; sum[8][grp] = F.rex;
         }
         __syncthreads();
         const int q = threadIdx.x, g = g0 + q;
-        if (q < per && g < V.N) {
-            FloeSum32 F;
+        if (q < GRP_FLOES && g < V.N) {
             F.fcx = sum[0][q]; F.fcy = sum[1][q]; F.mc = sum[2][q];
             F.fbx = sum[3][q]; F.fby = sum[4][q]; F.mb = sum[5][q];
             F.sca = sum[6][q]; F.scw = sum[7][q]; F.rex = sum[8][q];
@@ -1330,6 +1329,54 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) k_step_floes_grp_mixed(Views
     }
     if (!stopped) raise_step(dmx, B.dsp + cur);
     if (sic == A.K - 1) publish_status_last(V, A.done, A.out);
+}
+
+// The sums as a kernel of their own (k_group_sums_fp64), two float4 a floe in
+// fs: 65,536 sheltering floes 112 -> 84 us a step.
+__global__ void __launch_bounds__(SMALL_THREADS, 8) k_group_sums_mixed(Views V, MixedBufs B, float4 *fs)
+{
+    step_kernel_entry();
+    if (*(volatile int *)V.status & ST_ABORT) return;
+    const int grp = threadIdx.x / GRP;
+    for (int g0 = blockIdx.x * GRP_FLOES; g0 < V.N; g0 += gridDim.x * GRP_FLOES) {
+        const int g = g0 + grp;
+        const bool on = g < V.N;
+        FloeSum32 F;
+        group_sum32(V, B, on, g, F);
+        if (on && threadIdx.x % GRP == 0) {
+            fs[2 * (size_t)g] = make_float4(F.fcx, F.fcy, F.mc, F.fbx);
+            fs[2 * (size_t)g + 1] = make_float4(F.fby, F.mb, F.sca, F.scw);
+            B.frex[g] = F.rex;
+        }
+    }
+}
+
+// ... and the update from them, as the last kernel of a small batch's step.
+__global__ void __launch_bounds__(128) k_step_update_mixed(Views V, SmallArgs32 A, MixedBufs B, int cur, int sic,
+                                                           const float4 *fs)
+{
+    step_kernel_entry();
+    if (!floe_update_stopped(V, A.base, sic)) {
+        unsigned dmx = 0;
+        for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < V.N; g += gridDim.x * blockDim.x) {
+            const float4 s0 = fs[2 * (size_t)g], s1 = fs[2 * (size_t)g + 1];
+            FloeSum32 F;
+            F.fcx = s0.x; F.fcy = s0.y; F.mc = s0.z; F.fbx = s0.w; F.fby = s1.x; F.mb = s1.y;
+            F.sca = s1.z; F.scw = s1.w;
+            F.rex = B.frex[g];
+            const bool shel = V.P[V.inst[g]].shelter != 0;
+            dmx = max(dmx, floe_update<false, true>(V, cur, A.base, sic, g, F, shel ? nullptr : A.drag));
+        }
+        __syncwarp();
+        raise_step(dmx, B.dsp + cur);
+    }
+    if (sic == A.K - 1) publish_status_last(V, A.done, A.out);
+}
+
+// Plain steps of sheltering batches too large for the merged steps.
+void launch_group_sums_mixed(const Views &V, MixedBufs B, cudaStream_t st)
+{
+    launch_step(V.pdl != 0, k_group_sums_mixed, (V.N + GRP_FLOES - 1) / GRP_FLOES, SMALL_THREADS, st, V, B, B.fsum);
 }
 
 bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
@@ -1345,23 +1392,30 @@ bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base,
     A.done = done;
     const long long all = (long long)n + NB + V.N;
     if (!shelter && all <= ONE_CLUSTER_MIXED) return launch_cluster(V.pdl != 0, k_steps_mixed, all, ONE_BLOCK_MIXED, st, V, A, B);
-    const int rounds = group_rounds(V.N, shelter);
+    const GroupSums how = group_sums(V.N, shelter);
+    const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
+    float4 *fs = B.fdg;   // (a plain step has no diagnostic sums)
     for (int k = 0; k < K; k++) {
         const int c = cur ^ (k & 1);
         const int diag = diag_last && k == K - 1;
         B.bfl_rd = A.bfl + (size_t)c * NB;
         B.bfl_wr = A.bfl + (size_t)(c ^ 1) * NB;
         const long long items = (long long)(diag ? E : n) + (ridging ? 0 : NB) + 64 + V.N;
-        launch_step(V.pdl != 0, k_step_pairs_mixed, grid_of(items, 128), 128, st, V, A, B, c, diag);
+        launch_step(V.pdl != 0, items > 148 * 5 * 128 ? k_step_pairs_mixed<8> : k_step_pairs_mixed<5>, grid_of(items, 128),
+                    128, st, V, A, B, c, diag);
         if (ridging && NB > 0)
             launch_step(V.pdl != 0, k_bonds_mixed, grid_of(NB, 128), 128, st, V, c, diag, NB, B.bsp, B.bst, B.brec,
                         B.bdg, B.bfl_wr, B.wdyn);
-        if (diag) launch_step(V.pdl != 0, k_step_floes_mixed<true>, grid_of(V.N, 64), 64, st, V, A, B, c, k);
-        else if (rounds == 0)
+        if (diag) {
+            launch_step(V.pdl != 0, k_step_floes_mixed<true>, grid_of(V.N, 64), 64, st, V, A, B, c, k);
+        } else if (how == SUMS_THREAD) {
             launch_step(V.pdl != 0, k_step_floes_mixed<false>, grid_of(V.N, 64), 64, st, V, A, B, c, k);
-        else
-            launch_step(V.pdl != 0, k_step_floes_grp_mixed, (V.N + rounds * GRP_FLOES - 1) / (rounds * GRP_FLOES),
-                        SMALL_THREADS, st, V, A, B, c, k, rounds);
+        } else if (how == SUMS_GROUP) {
+            launch_step(V.pdl != 0, k_step_floes_grp_mixed, groups, SMALL_THREADS, st, V, A, B, c, k);
+        } else {
+            launch_step(V.pdl != 0, k_group_sums_mixed, groups, SMALL_THREADS, st, V, B, fs);
+            launch_step(V.pdl != 0, k_step_update_mixed, grid_of(V.N, 64), 64, st, V, A, B, c, k, fs);
+        }
     }
     return true;
 }

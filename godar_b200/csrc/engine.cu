@@ -1548,10 +1548,16 @@ struct Engine {
             L.n = nwork_b.as<int>();
             // a plain step visits the pairs that can act before the next
             // rebuild; a diagnostic step every owner entry
-            launch_pairs_fp64(V, side, diag, diag ? (int)E : (int)Lc, diag ? nullptr : fplist_b.as<int>(),
-                              erow_up.as<unsigned>(), pfl.as<unsigned char>(), L, frec_b.p, cfg_block(bs[0]), st);
-            if (ev) TRY(record(ev[1], capturing));
-            launch_pairs_list_fp64(V, side, diag, (int)E, pfl.as<unsigned char>(), L, frec_b.p, cfg_block(bs[1]), st);
+            if (shelter_any && !diag) {
+                launch_pairs_shel_fp64(V, side, (int)Lc, fplist_b.as<int>(), erow_up.as<unsigned>(),
+                                       pfl.as<unsigned char>(), frec_b.p, st);
+                if (ev) TRY(record(ev[1], capturing));
+            } else {
+                launch_pairs_fp64(V, side, diag, diag ? (int)E : (int)Lc, diag ? nullptr : fplist_b.as<int>(),
+                                  erow_up.as<unsigned>(), pfl.as<unsigned char>(), L, frec_b.p, cfg_block(bs[0]), st);
+                if (ev) TRY(record(ev[1], capturing));
+                launch_pairs_list_fp64(V, side, diag, (int)E, pfl.as<unsigned char>(), L, frec_b.p, cfg_block(bs[1]), st);
+            }
             // (the third phase has no kernel of its own)
             if (ev) TRY(record(ev[2], capturing));
             if (ev) TRY(record(ev[3], capturing));

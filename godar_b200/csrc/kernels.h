@@ -106,6 +106,8 @@ void launch_row_sums_fp64(const Views &V, int cur, int diag, int light, const un
 // Also sets the pairs' flags before the first step.
 void launch_fp64_rows(const Views &V, int side, int E, const unsigned *erow, unsigned char *pfl,
                       unsigned char *listed, int *up_n, int *lo_n, int2 *tmp, int *pos, int *scan_scratch, int *plist, cudaStream_t st);
+void launch_pairs_shel_fp64(const Views &V, int cur, int n, const int *plist, const unsigned *erow,
+                            unsigned char *pfl, void *rec, cudaStream_t st);
 void launch_group_sums_fp64(const Views &V, int cur, const unsigned char *pfl, const void *rec, const int *lo_n,
                             const int *up_n, double *fs, cudaStream_t st);
 void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, int light, const double *fs, int *nwork, int block,

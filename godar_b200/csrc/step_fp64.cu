@@ -44,6 +44,14 @@ void launch_row_sums_fp64(const Views &V, int cur, int diag, int light, const un
 }
 
 // Plain steps of sheltering batches too large for the merged steps.
+void launch_pairs_shel_fp64(const Views &V, int cur, int n, const int *plist, const unsigned *erow,
+                            unsigned char *pfl, void *rec, cudaStream_t st)
+{
+    SmallArgs64 A{};
+    A.n = n; A.plist = plist; A.erow = erow; A.pfl = pfl; A.rec = (PairRec64 *)rec;
+    if (n > 0) launch_step(V.pdl != 0, k_step_pairs_shel_fp64, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, cur);
+}
+
 void launch_group_sums_fp64(const Views &V, int cur, const unsigned char *pfl, const void *rec, const int *lo_n,
                             const int *up_n, double *fs, cudaStream_t st)
 {
@@ -85,6 +93,7 @@ bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, 
         const int gp = fp64_grid(work, 128);
         const bool dense = work > 148 * 2 * 128;
         if (diag) launch_step(V.pdl != 0, dense ? k_step_pairs_fp64<true, 4> : k_step_pairs_fp64<true, 2>, gp, 128, st, V, A, c);
+        else if (shelter && n > SHEL_WAVE) launch_step(V.pdl != 0, k_step_pairs_shel_fp64, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, c);
         else launch_step(V.pdl != 0, dense ? k_step_pairs_fp64<false, 4> : k_step_pairs_fp64<false, 2>, gp, 128, st, V, A, c);
         const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
         if (diag) {

@@ -1586,7 +1586,9 @@ struct Engine {
                 CK(cudaEventRecord(ev_join, st2));
             }
             // the screen walks the contact list, or every entry on a diagnostic step
-            launch_pairs_screen(V, side, diag, diag ? (int)E : (int)Ec, diag ? nullptr : clist_b.as<int2>(),
+            if (shelter_any && !diag)
+                launch_pairs_shel_mixed(V, side, (int)Ec, clist_b.as<int2>(), clist_b.as<int2>() + Ecap, B, st);
+            else launch_pairs_screen(V, side, diag, diag ? (int)E : (int)Ec, diag ? nullptr : clist_b.as<int2>(),
                                 clist_b.as<int2>() + Ecap, B, cfg_block(bs[0]), cfg_variant(bs[0]), st);
             if (ev) TRY(record(ev[1], capturing));
             if (diag) launch_pairs_diag(V, side, (int)E, erow_up.as<unsigned>(), B, cfg_block(bs[1]), st);

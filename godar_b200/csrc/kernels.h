@@ -180,6 +180,7 @@ void launch_pairs_diag(const Views &V, int cur, int P, const unsigned *erow_up, 
 // light: no field of the batch has ridging, sheltering or walls; bounded: the
 // pair kernel advances the displacement bound in every step since the rebuild.
 void launch_floe_sums(const Views &V, int diag, int light, MixedBufs B, int block, cudaStream_t st);
+void launch_pairs_shel_mixed(const Views &V, int cur, int n, int2 *eb, const int2 *stl, MixedBufs B, cudaStream_t st);
 void launch_group_sums_mixed(const Views &V, MixedBufs B, cudaStream_t st);
 void launch_bonds_mixed(const Views &V, int cur, int diag, int NB, MixedBufs B, int block, int variant,
                         unsigned test_spins, cudaStream_t st);

@@ -1101,6 +1101,20 @@ struct SmallArgs32 {
     int *done;                     // blocks of k_step_floes_mixed that have finished
 };
 
+// The drag and Coriolis terms of floe g with its start-of-step shape, unless
+// its field has sheltering (which needs the pairs first).
+GD_DEV void drag_ahead32(const Views &V, int cur, int g, float4 *drag)
+{
+    const InstParams &P = V.P[V.inst[g]];
+    if (P.shelter != 0) return;
+    double ua, va, uw, vw;
+    wind_at(P, V.field, V.x[cur][g], V.y[cur][g], ua, va, uw, vw);
+    const Drag<float> D = forcing<float>(P, shape_mixed(P, V.r[cur][g], V.h[cur][g]), V.u[cur][g], V.v[cur][g],
+                                         V.om[cur][g], ua, va, uw, vw, 0.f, 0.f);
+    drag[2 * (size_t)g] = make_float4(D.fax, D.fay, D.fwx, D.fwy);
+    drag[2 * (size_t)g + 1] = make_float4(D.ma, D.mw, D.fcorx, D.fcory);
+}
+
 GD_DEV void small_pairs32(const Views &V, const SmallArgs32 &A, const MixedBufs &B, int cur, int diag,
                           int first, int nthr)
 {
@@ -1134,15 +1148,7 @@ GD_DEV void small_pairs32(const Views &V, const SmallArgs32 &A, const MixedBufs 
             const int b = i - n0;
             n_bond += bond_step(V, S, diag, b, B.bsp[b], B.wdyn[b], B.bst[b], B.brec, B.bdg, B.bfl_wr, B.wdyn);
         } else if (i >= n1) {
-            const int g = i - n1;
-            const InstParams &P = V.P[V.inst[g]];
-            if (P.shelter != 0) continue;
-            double ua, va, uw, vw;
-            wind_at(P, V.field, V.x[cur][g], V.y[cur][g], ua, va, uw, vw);
-            const Drag<float> D = forcing<float>(P, shape_mixed(P, V.r[cur][g], V.h[cur][g]), V.u[cur][g],
-                                                 V.v[cur][g], V.om[cur][g], ua, va, uw, vw, 0.f, 0.f);
-            A.drag[2 * (size_t)g] = make_float4(D.fax, D.fay, D.fwx, D.fwy);
-            A.drag[2 * (size_t)g + 1] = make_float4(D.ma, D.mw, D.fcorx, D.fcory);
+            drag_ahead32(V, cur, i - n1, A.drag);
         }
     }
     __syncwarp();
@@ -1286,6 +1292,95 @@ __global__ void __launch_bounds__(128, MINB) k_step_pairs_mixed(Views V, SmallAr
     small_pairs32(V, A, B, cur, diag, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
+// The pairs of a plain step of a sheltering batch whose items fill several
+// rounds of one wave, as k_step_pairs_shel_fp64: a pair out of contact computes
+// its shelter factors (pair_mixed's expressions) on its lane, the others
+// collect and go through the physics 32 at a time.  The bonds (NB: 0 where they
+// have a kernel of their own) and the floes' drag (drag: null, not wanted)
+// follow.  65,536 floes: 83 -> 78 us a step, 160,000: 179 -> 163 (five blocks an
+// SM 80 and 172, eight 85 and 155).
+constexpr int SHEL_THREADS = 128, SHEL_BLOCKS = 6, SHEL_WAVE = 148 * SHEL_BLOCKS * SHEL_THREADS;
+__global__ void __launch_bounds__(SHEL_THREADS, SHEL_BLOCKS) k_step_pairs_shel_mixed(Views V, SmallArgs32 A,
+                                                                                     MixedBufs B, int cur)
+{
+    struct Item { int e, s, t; };
+    __shared__ Item list[SHEL_THREADS / 32][64];
+    step_kernel_entry();
+    if (*(volatile int *)V.status & ST_ABORT) return;
+    const Snap *S = V.snap[cur];
+    Hist4<float> *Hh = (Hist4<float> *)V.hist[0];
+    const float Dk = advance_bound(cur, B);
+    const float thr = __fadd_ru(2.f * Dk, 1e-6f);
+    Item *const L = list[threadIdx.x / 32];
+    const int lane = threadIdx.x & 31, nthr = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned lt = (1u << lane) - 1u;
+    unsigned long long none = 0;
+    int waiting = 0;
+    // every lane of a warp runs the same iterations
+    for (int i0 = first - lane; i0 < A.n; i0 += nthr) {
+        const int i = i0 + lane;
+        bool heavy = false;
+        Item it;
+        int2 c = make_int2(-1, __float_as_int(INFINITY));
+        if (i < A.n) c = A.eb[i];
+        if (!(__int_as_float(c.y) > thr)) {
+            const int2 st = A.stl[i];
+            it.e = c.x; it.s = st.x; it.t = st.y;
+            const unsigned f0 = B.pfl[it.e];
+            const Snap Si = S[it.s], Sj = S[it.t];
+            const InstParams &P = V.P[Si.inst];
+            if (P.shelter == 0) {
+                heavy = screen_test(V, S, A.eb, i, c, st, f0, Dk, B);
+            } else {
+                const bool px = P.boundary & BC_PERIODIC_X, py = P.boundary & BC_PERIODIC_Y;
+                const double dx = wrap_d(Si.x - Sj.x, P.nx, px), dy = wrap_d(Si.y - Sj.y, P.ny, py);
+                const double dist = sqrt(dx * dx + dy * dy);
+                const double deltan = (Si.r + Sj.r) - dist;
+                const bool cand = dist <= Si.r + P.rtree;
+                heavy = cand && (deltan > 0.0 || (f0 & PF_HIST));
+                if (!heavy) {
+                    unsigned f1 = f0 & PF_HIST;
+                    if (cand) {
+                        const float fd = (float)dist;
+                        const float cosa = (float)(-dx) / fd, sina = (float)(-dy) / fd;
+                        double a0, a1, a2, a3;
+                        wind_at(P, V.field, Si.x, Si.y, a0, a1, a2, a3);
+                        const float ua = (float)a0, va = (float)a1, uw = (float)a2, vw = (float)a3;
+                        const float dn = (float)deltan;
+                        float a_ij, a_ji, w_ij, w_ji;
+                        shelter_pair<float>(P.f_hfa * Si.h, P.f_hfa * Sj.h, dn, cosa, sina, ua, va, a_ij, a_ji);
+                        shelter_pair<float>(P.f_hfw * Si.h, P.f_hfw * Sj.h, dn, cosa, sina, uw, vw, w_ij, w_ji);
+                        B.rec[2 * (size_t)it.e] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        B.rec[2 * (size_t)it.e + 1] = make_float4(a_ji, w_ji, a_ij, w_ij);
+                        f1 |= PF_REC;
+                    }
+                    if (f1 != f0) {
+                        B.pfl[it.e] = (unsigned char)f1;
+                        B.lfl[B.lo_of[it.e]] = (unsigned char)(f1 & ~PF_HIST);
+                    }
+                }
+            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, heavy);
+        if (heavy) L[waiting + __popc(m & lt)] = it;
+        waiting += __popc(m);
+        __syncwarp();
+        if (waiting >= 32) {
+            waiting -= 32;
+            it = L[waiting + lane];
+            pair_mixed(V, S, Hh, 0, it.e, it.s, it.t, B, none, none, none);
+            __syncwarp();
+        }
+    }
+    if (lane < waiting) pair_mixed(V, S, Hh, 0, L[lane].e, L[lane].s, L[lane].t, B, none, none, none);
+    __syncwarp();
+    if (!A.ridging)
+        for (int b = first; b < A.NB; b += nthr)
+            bond_step(V, S, 0, b, B.bsp[b], B.wdyn[b], B.bst[b], B.brec, B.bdg, B.bfl_wr, B.wdyn);
+    if (A.drag)
+        for (int g = first; g < V.N; g += nthr) drag_ahead32(V, cur, g, A.drag);
+}
+
 template <bool DIAG>
 __global__ void __launch_bounds__(128) k_step_floes_mixed(Views V, SmallArgs32 A, MixedBufs B, int cur, int sic)
 {
@@ -1374,6 +1469,13 @@ __global__ void __launch_bounds__(128) k_step_update_mixed(Views V, SmallArgs32 
 }
 
 // Plain steps of sheltering batches too large for the merged steps.
+void launch_pairs_shel_mixed(const Views &V, int cur, int n, int2 *eb, const int2 *stl, MixedBufs B, cudaStream_t st)
+{
+    SmallArgs32 A{};
+    A.n = n; A.eb = eb; A.stl = stl;
+    if (n > 0) launch_step(V.pdl != 0, k_step_pairs_shel_mixed, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, B, cur);
+}
+
 void launch_group_sums_mixed(const Views &V, MixedBufs B, cudaStream_t st)
 {
     launch_step(V.pdl != 0, k_group_sums_mixed, (V.N + GRP_FLOES - 1) / GRP_FLOES, SMALL_THREADS, st, V, B, B.fsum);
@@ -1401,7 +1503,9 @@ bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base,
         B.bfl_rd = A.bfl + (size_t)c * NB;
         B.bfl_wr = A.bfl + (size_t)(c ^ 1) * NB;
         const long long items = (long long)(diag ? E : n) + (ridging ? 0 : NB) + 64 + V.N;
-        launch_step(V.pdl != 0, items > 148 * 5 * 128 ? k_step_pairs_mixed<8> : k_step_pairs_mixed<5>, grid_of(items, 128),
+        if (shelter && !diag && n > SHEL_WAVE)
+            launch_step(V.pdl != 0, k_step_pairs_shel_mixed, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, B, c);
+        else launch_step(V.pdl != 0, items > 148 * 5 * 128 ? k_step_pairs_mixed<8> : k_step_pairs_mixed<5>, grid_of(items, 128),
                     128, st, V, A, B, c, diag);
         if (ridging && NB > 0)
             launch_step(V.pdl != 0, k_bonds_mixed, grid_of(NB, 128), 128, st, V, c, diag, NB, B.bsp, B.bst, B.brec,

@@ -414,17 +414,18 @@ struct Engine {
     bool overlap_bonds = false;
     bool shelter_any = false;      // some field of the batch has sheltering
     bool walls_any = false;        // some field of the batch has a solid wall
-    // Batches of at most SMALL_FLOES_* floes run their steps as one or two
-    // launches (launch_small): below these sizes the five kernels of a step
+    // Batches of at most SMALL_FLOES_* floes run their steps as one to three
+    // launches (launch_small): below these sizes the four kernels of a step
     // are mostly gaps and one thread's latency; above them the registers of
     // the merged kernels cost more than the launches.  Measured, us a step
-    // (merged / five kernels): FP64 bonded fields 43.8 / 46.8 at 65,536 floes,
-    // 95 / 84 at 140,000; mixed 37.9 / 43.4 at 140,000, 600 / 340 at 2.2 M.
+    // (merged / separate kernels), bonded fields: FP64 31.8 / 40.3 at 66,000
+    // floes, 50.1 / 51.4 at 100,000, 58.0 / 57.2 at 115,000; mixed 25.1 / 31.5
+    // at 100,000, 30.5 / 33.7 at 115,000, 34.8 / 33.3 at 131,000.
     // GODAR_FUSED=0 turns it off, as does any switch that asks for a
-    // particular launch of the five step kernels.
+    // particular launch of the separate kernels.
     bool fused_on = true;
-    static constexpr int SMALL_FLOES_FP64 = 64 * 1024;
-    static constexpr int SMALL_FLOES_MIXED = 148 * 1024;
+    static constexpr int SMALL_FLOES_FP64 = 100 * 1024;
+    static constexpr int SMALL_FLOES_MIXED = 120 * 1024;
 
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::atomic<size_t> bytes{0};
@@ -1620,11 +1621,11 @@ struct Engine {
         V.pdl = step_pdl();
         bool ok;
         if (prec == GODAR_PREC_FP64)
-            ok = launch_steps_fp64(V, c0, K, diag_last, gbase, (int)Lc, (int)E, shelter_any ? 1 : 0, fplist_b.as<int>(),
+            ok = launch_steps_fp64(V, c0, K, diag_last, gbase, (int)Lc, (int)E, shelter_any ? 1 : 0, walls_any ? 1 : 0, fplist_b.as<int>(),
                                    erow_up.as<unsigned>(), pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
                                    fupn_b.as<int>(), fsum_b.as<double>(), out, step_base_b.as<int>() + 1, st);
         else
-            ok = launch_steps_mixed(V, c0, K, diag_last, gbase, (int)Ec, (int)E, NB, shelter_any ? 1 : 0, ridging_any ? 1 : 0,
+            ok = launch_steps_mixed(V, c0, K, diag_last, gbase, (int)Ec, (int)E, NB, shelter_any ? 1 : 0, walls_any ? 1 : 0, ridging_any ? 1 : 0,
                                     clist_b.as<int2>(), clist_b.as<int2>() + Ecap, erow_up.as<unsigned>(),
                                     bflag_b.as<unsigned char>(), mixed_bufs(), out, step_base_b.as<int>() + 1, st);
         if (!ok) {

@@ -124,7 +124,7 @@ void launch_fp64_bonds(const Views &V, int side, int *cnt, int *wfo, int *scan_s
 // launches a step.  False if the launch was refused.
 constexpr int ONE_CLUSTER_FP64 = 1024, ONE_CLUSTER_MIXED = 4096;
 constexpr int ONE_BLOCK_FP64 = 640, ONE_BLOCK_MIXED = 1024;
-bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int shelter,
+bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
                        const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
                        const int *up_n, double *drag, int *out, int *done, cudaStream_t st);
 
@@ -190,7 +190,7 @@ void launch_floes_mixed(const Views &V, int cur, int diag, int sic, int walls, i
 // The same on the mixed path (n contact-list items eb/stl, bfl: the live-bond
 // flags of both sides).
 bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
-                        int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
+                        int walls, int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
                         int *done, cudaStream_t st);
 
 // Checkpoints: pair histories out and back in.

@@ -73,7 +73,7 @@ void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, in
     }
 }
 
-bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int shelter,
+bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
                        const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
                        const int *up_n, double *drag, int *out, int *done, cudaStream_t st)
 {
@@ -97,14 +97,14 @@ bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, 
         else launch_step(V.pdl != 0, dense ? k_step_pairs_fp64<false, 4> : k_step_pairs_fp64<false, 2>, gp, 128, st, V, A, c);
         const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
         if (diag) {
-            launch_step(V.pdl != 0, k_step_floes_fp64<true>, fp64_grid(V.N, 64), 64, st, V, A, c, k);
+            launch_step(V.pdl != 0, walls ? k_step_floes_fp64<true, true> : k_step_floes_fp64<true, false>, fp64_grid(V.N, 64), 64, st, V, A, c, k);
         } else if (how == SUMS_THREAD) {
-            launch_step(V.pdl != 0, k_step_floes_fp64<false>, fp64_grid(V.N, 64), 64, st, V, A, c, k);
+            launch_step(V.pdl != 0, walls ? k_step_floes_fp64<false, true> : k_step_floes_fp64<false, false>, fp64_grid(V.N, 64), 64, st, V, A, c, k);
         } else if (how == SUMS_GROUP) {
             launch_step(V.pdl != 0, k_step_floes_grp_fp64, groups, SMALL_THREADS, st, V, A, c, k);
         } else {
             launch_step(V.pdl != 0, k_group_sums_fp64, groups, SMALL_THREADS, st, V, c, pfl, A.rec, lo_n, up_n, fs);
-            launch_step(V.pdl != 0, k_step_update_fp64, fp64_grid(V.N, 64), 64, st, V, A, c, k, fs);
+            launch_step(V.pdl != 0, walls ? k_step_update_fp64<true> : k_step_update_fp64<false>, fp64_grid(V.N, 64), 64, st, V, A, c, k, fs);
         }
     }
     return true;

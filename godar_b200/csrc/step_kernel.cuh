@@ -889,7 +889,7 @@ GD_DEV void small_pairs64(const Views &V, const SmallArgs64 &A, int cur)
 }
 
 // The floes' sums and update, one thread per floe.
-template <bool DIAG>
+template <bool DIAG, bool WALLS>
 GD_DEV void small_floes64(const Views &V, const SmallArgs64 &A, int cur, int sic)
 {
     const int nthr = gridDim.x * blockDim.x;
@@ -898,7 +898,7 @@ GD_DEV void small_floes64(const Views &V, const SmallArgs64 &A, int cur, int sic
         const InstParams &P = V.P[V.inst[g]];
         Acc<double> S;
         const Shape run = row_sums64<DIAG>(V, cur, g, P, A.pfl, A.rec, A.lo_n, A.up_n, S);
-        C.plast += floe_update64<DIAG, true>(V, cur, A.base, sic, g, P, S, run, P.shelter != 0 ? nullptr : A.drag);
+        C.plast += floe_update64<DIAG, WALLS>(V, cur, A.base, sic, g, P, S, run, P.shelter != 0 ? nullptr : A.drag);
     }
     __syncwarp();
     if (DIAG) add_counts(C, V.counters);
@@ -916,8 +916,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_steps_fp64(Views V, SmallA
         if (diag) small_pairs64<true>(V, A, cur);
         else small_pairs64<false>(V, A, cur);
         cluster_sync();
-        if (diag) small_floes64<true>(V, A, cur, k);
-        else small_floes64<false>(V, A, cur, k);
+        if (diag) small_floes64<true, true>(V, A, cur, k);
+        else small_floes64<false, true>(V, A, cur, k);
         cluster_sync();
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) publish_status(V, A.out);
@@ -1015,11 +1015,11 @@ __global__ void __launch_bounds__(SHEL_THREADS, 4) k_step_pairs_shel_fp64(Views 
         drag_ahead64(V, cur, g, A.drag);
 }
 
-template <bool DIAG>
+template <bool DIAG, bool WALLS>
 __global__ void __launch_bounds__(128) k_step_floes_fp64(Views V, SmallArgs64 A, int cur, int sic)
 {
     step_kernel_entry();
-    if (!floe_update_stopped(V, A.base, sic)) small_floes64<DIAG>(V, A, cur, sic);
+    if (!floe_update_stopped(V, A.base, sic)) small_floes64<DIAG, WALLS>(V, A, cur, sic);
     if (sic == A.K - 1) publish_status_last(V, A.done, A.out);
 }
 
@@ -1093,6 +1093,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4) k_group_sums_fp64(Views V, i
 }
 
 // ... and the update from them, as the last kernel of a small batch's step.
+template <bool WALLS>
 __global__ void __launch_bounds__(64) k_step_update_fp64(Views V, SmallArgs64 A, int cur, int sic, const double *fs)
 {
     step_kernel_entry();
@@ -1105,7 +1106,7 @@ __global__ void __launch_bounds__(64) k_step_update_fp64(Views V, SmallArgs64 A,
             S.fbx = fs[FS64_FBX * N + g]; S.fby = fs[FS64_FBY * N + g]; S.mb = fs[FS64_MB * N + g];
             S.hsfa = fs[FS64_HSFA * N + g]; S.hsfw = fs[FS64_HSFW * N + g];
             const Shape run = make_shape(P, fs[FS64_R * N + g], fs[FS64_H * N + g]);
-            floe_update64<false, true>(V, cur, A.base, sic, g, P, S, run, P.shelter != 0 ? nullptr : A.drag);
+            floe_update64<false, WALLS>(V, cur, A.base, sic, g, P, S, run, P.shelter != 0 ? nullptr : A.drag);
         }
     if (sic == A.K - 1) publish_status_last(V, A.done, A.out);
 }

@@ -1233,7 +1233,7 @@ GD_DEV void group_sum32(const Views &V, const MixedBufs &B, bool on, int g, Floe
 }
 
 // The floes' sums and update, one thread per floe.
-template <bool DIAG>
+template <bool DIAG, bool WALLS>
 GD_DEV void small_floes32(const Views &V, const SmallArgs32 &A, const MixedBufs &B, int cur, int sic)
 {
     const int nthr = gridDim.x * blockDim.x;
@@ -1242,7 +1242,7 @@ GD_DEV void small_floes32(const Views &V, const SmallArgs32 &A, const MixedBufs 
         FloeSum32 F;
         floe_sum<DIAG>(V, B, g, F);
         const bool shel = V.P[V.inst[g]].shelter != 0;
-        dmx = max(dmx, floe_update<DIAG, true>(V, cur, A.base, sic, g, F, shel ? nullptr : A.drag));
+        dmx = max(dmx, floe_update<DIAG, WALLS>(V, cur, A.base, sic, g, F, shel ? nullptr : A.drag));
     }
     __syncwarp();
     raise_step(dmx, B.dsp + cur);
@@ -1271,8 +1271,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_steps_mixed(Views V, Small
             if (diag) warp_count(n_bond, V.counters, 2);
             cluster_sync();
         }
-        if (diag) small_floes32<true>(V, A, B, cur, k);
-        else small_floes32<false>(V, A, B, cur, k);
+        if (diag) small_floes32<true, true>(V, A, B, cur, k);
+        else small_floes32<false, true>(V, A, B, cur, k);
         cluster_sync();
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) publish_status(V, A.out);
@@ -1381,11 +1381,14 @@ __global__ void __launch_bounds__(SHEL_THREADS, SHEL_BLOCKS) k_step_pairs_shel_m
         for (int g = first; g < V.N; g += nthr) drag_ahead32(V, cur, g, A.drag);
 }
 
-template <bool DIAG>
-__global__ void __launch_bounds__(128) k_step_floes_mixed(Views V, SmallArgs32 A, MixedBufs B, int cur, int sic)
+// A batch without walls runs the instance without their code, whose 80
+// registers let six blocks an SM wait for loads side by side (128 and four
+// before: 103,567 floes 30.4 -> 25.4 us a step).
+template <bool DIAG, bool WALLS>
+__global__ void __launch_bounds__(128, WALLS ? 3 : 6) k_step_floes_mixed(Views V, SmallArgs32 A, MixedBufs B, int cur, int sic)
 {
     step_kernel_entry();
-    if (!floe_update_stopped(V, A.base, sic)) small_floes32<DIAG>(V, A, B, cur, sic);
+    if (!floe_update_stopped(V, A.base, sic)) small_floes32<DIAG, WALLS>(V, A, B, cur, sic);
     if (sic == A.K - 1) publish_status_last(V, A.done, A.out);
 }
 
@@ -1447,7 +1450,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 8) k_group_sums_mixed(Views V, 
 }
 
 // ... and the update from them, as the last kernel of a small batch's step.
-__global__ void __launch_bounds__(128) k_step_update_mixed(Views V, SmallArgs32 A, MixedBufs B, int cur, int sic,
+template <bool WALLS>
+__global__ void __launch_bounds__(128, WALLS ? 4 : 6) k_step_update_mixed(Views V, SmallArgs32 A, MixedBufs B, int cur, int sic,
                                                            const float4 *fs)
 {
     step_kernel_entry();
@@ -1460,7 +1464,7 @@ __global__ void __launch_bounds__(128) k_step_update_mixed(Views V, SmallArgs32 
             F.sca = s1.z; F.scw = s1.w;
             F.rex = B.frex[g];
             const bool shel = V.P[V.inst[g]].shelter != 0;
-            dmx = max(dmx, floe_update<false, true>(V, cur, A.base, sic, g, F, shel ? nullptr : A.drag));
+            dmx = max(dmx, floe_update<false, WALLS>(V, cur, A.base, sic, g, F, shel ? nullptr : A.drag));
         }
         __syncwarp();
         raise_step(dmx, B.dsp + cur);
@@ -1482,7 +1486,7 @@ void launch_group_sums_mixed(const Views &V, MixedBufs B, cudaStream_t st)
 }
 
 bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
-                        int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
+                        int walls, int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
                         int *done, cudaStream_t st)
 {
     SmallArgs32 A;
@@ -1511,14 +1515,14 @@ bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base,
             launch_step(V.pdl != 0, k_bonds_mixed, grid_of(NB, 128), 128, st, V, c, diag, NB, B.bsp, B.bst, B.brec,
                         B.bdg, B.bfl_wr, B.wdyn);
         if (diag) {
-            launch_step(V.pdl != 0, k_step_floes_mixed<true>, grid_of(V.N, 64), 64, st, V, A, B, c, k);
+            launch_step(V.pdl != 0, walls ? k_step_floes_mixed<true, true> : k_step_floes_mixed<true, false>, grid_of(V.N, 64), 64, st, V, A, B, c, k);
         } else if (how == SUMS_THREAD) {
-            launch_step(V.pdl != 0, k_step_floes_mixed<false>, grid_of(V.N, 64), 64, st, V, A, B, c, k);
+            launch_step(V.pdl != 0, walls ? k_step_floes_mixed<false, true> : k_step_floes_mixed<false, false>, grid_of(V.N, 64), 64, st, V, A, B, c, k);
         } else if (how == SUMS_GROUP) {
             launch_step(V.pdl != 0, k_step_floes_grp_mixed, groups, SMALL_THREADS, st, V, A, B, c, k);
         } else {
             launch_step(V.pdl != 0, k_group_sums_mixed, groups, SMALL_THREADS, st, V, B, fs);
-            launch_step(V.pdl != 0, k_step_update_mixed, grid_of(V.N, 64), 64, st, V, A, B, c, k, fs);
+            launch_step(V.pdl != 0, walls ? k_step_update_mixed<true> : k_step_update_mixed<false>, grid_of(V.N, 64), 64, st, V, A, B, c, k, fs);
         }
     }
     return true;

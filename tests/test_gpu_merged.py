@@ -67,7 +67,7 @@ def _same(f, precision, monkeypatch):
 
 
 @pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
-@pytest.mark.parametrize("n", [64, 390, 420, 970, 1010, 9472, 9473, 65536, 65537])
+@pytest.mark.parametrize("n", [64, 390, 420, 970, 1010, 9472, 9473, 65536, 65537, 102400, 102401, 122880, 122881])
 def test_bonded_fields(n, precision, monkeypatch):
     _same(gen.bonded_field(n=n, seed=n, device="gpu" if n > 9000 else "cpu"), precision, monkeypatch)
 

@@ -5,7 +5,7 @@ Workload: the batched ensemble of 512 independent floe fields (floe counts
 log-uniform in [256, 16384], bonded-field generator with seeds 10+i, 80%
 target area fraction, uniform wind of random direction U[0,360) deg and speed
 U[8,16] m/s), advanced with FP32 pair forces and FP64 integration, bond and
-ridging state: per time step a candidate screen, the contact work list, the
+ridging state: per time step the candidate screen with the contacts, the
 bonds, the per-floe force sums and the floe update (forcing, integration),
 replayed as CUDA graphs.  A "step" is one time step of every instance.  Under
 torchrun each rank runs its share of the one ensemble (split by floe count):
@@ -416,21 +416,22 @@ def run_godar(args, ws, rank, local):
 
     # roofline of the dominant kernel: algorithmic bytes per launch over the
     # kernel's mean CUDA-event duration in the timed region.  Per kernel:
-    # pair screen 36 B/floe own state + 4 B per candidate pair (CSR read);
-    # pair work list 40 B per contact (history read+write); bonds 128 B per
-    # bond; floe sums 20 B/floe; floe update 132 B/floe
+    # pair screen and contacts 36 B/floe own state + 4 B per candidate pair
+    # (CSR read) + 40 B per contact (history read+write); bonds 128 B per
+    # bond; floe sums 20 B/floe; floe update 132 B/floe (the second phase has
+    # a kernel on diagnostic steps only)
     launches = st1["launches"] - st0["launches"]
     klaunch = st1["kernel_launches"] - st0["kernel_launches"]
     timed = st1["timed_steps"] - st0["timed_steps"]
     ph_ms = [(a - b) / max(1, timed) for a, b in zip(st1["phase_ms"], st0["phase_ms"])]
     step_ms = (st1["kernel_ms"] - st0["kernel_ms"]) / max(1, timed)
     P, C, B = st1["candidates"], st1["contacts"], st1["bonds"]
-    names = ["k_pairs_screen (candidate screening)",
-             "k_pairs_mixed (contact forces, ridging events, sheltering)",
+    names = ["k_pairs_screen (candidate screening, contact forces, ridging events, sheltering)",
+             "k_pairs_mixed (the same of every candidate, on diagnostic steps)",
              "k_bonds_mixed (bond forces and breaking)",
              "k_floe_sums (pair and bond record sums)",
              "k_floes_mixed (walls, ridging, drag, Coriolis, integration)"]
-    algos = [36 * nf + 4 * P, 40 * C, 128 * B, 20 * nf, 132 * nf]
+    algos = [36 * nf + 4 * P + 40 * C, 0, 128 * B, 20 * nf, 132 * nf]
     peak, kind = peaks()
     phases = []
     for q in range(len(names)):
@@ -472,7 +473,7 @@ def run_godar(args, ws, rank, local):
                               "graph_launches": st1["graph_launches"] - st0["graph_launches"]},
             "gpu_launches": int(klaunch + 24 * (st1["rebuilds"] - st0["rebuilds"])),
             "rebuilds_in_timed_region": st1["rebuilds"] - st0["rebuilds"],
-            # the neighbour search (cell keys, radix sort, Verlet superset,
+            # the neighbour search (cell lists, Verlet superset,
             # contact list, bond lists) of the set-up: host wall time per
             # rebuild, each to its end on the device
             "neighbour_rebuild": {"ms_per_rebuild": st0["rebuild_ms"] / max(1, st0["rebuilds"]),

@@ -1806,7 +1806,7 @@ struct Engine {
             bool small = small_batch(phase_every);
             const bool tuning = tune_left > 0 && !small;
             // a tuning chunk runs one step per candidate; otherwise chunks of
-            // the five kernels are powers of two so that their graphs are reused
+            // the separate kernels are powers of two so that their graphs are reused
             int K = tuning ? std::min(remaining, max_cfg()) : std::min(remaining, chunk);
             if (!tuning && !small) while (K & (K - 1)) K &= K - 1;
             const int diag_last = (diagnostics && remaining == K) ? 1 : 0;

@@ -139,8 +139,7 @@ inline GroupSums group_sums(int N, int shelter)
     return shelter ? SUMS_GROUP_APART : SUMS_THREAD;
 }
 
-// Mixed precision: (b) one lane per pair with warp-segmented sums, (b') the
-// partners' shares gathered the same way, (c)-(e) one thread per floe.
+// Mixed precision: pair and bond records (b, b'), summed per floe (c)-(e).
 struct MixedBufs {
     unsigned char *pfl, *lfl;   // flags of the owner entries and of their mirror partner entries
     int *lo_of;                 // partner-row index of every owner entry

@@ -807,8 +807,8 @@ __global__ void __launch_bounds__(128) k_floes_fp64(Views V, int cur, int sic, c
 // beside the drag and Coriolis terms of every floe (they need the pairs only
 // where an event changes the shape or in a sheltering field, where the update
 // computes them again); a cluster barrier; the ordered sums and the update of
-// every floe; a cluster barrier.  Two barriers a step stand in for five
-// kernels.  Every value is computed by the functions the five kernels use.
+// every floe; a cluster barrier.  Two barriers a step stand in for four
+// kernels.  Every value is computed by the functions the four kernels use.
 struct SmallArgs64 {
     int cur, K, diag_last, base;   // first side, steps, diagnostics on the last one, global number of the first
     int n, E;                      // marked positions (plist), owner entries
@@ -924,7 +924,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_steps_fp64(Views V, SmallA
 }
 
 // The two halves of a step as ordinary grids, for batches with more work
-// than one cluster does quickly: two launches a step instead of five.  The
+// than one cluster does quickly: two launches a step instead of four.  The
 // second one of a chunk's last step publishes the status word.
 // MINB blocks an SM: a sheltering pair is a chain of dependent FP64
 // instructions and loads (the FP64 pipe 15% busy at 182 registers and two

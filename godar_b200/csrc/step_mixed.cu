@@ -1,20 +1,21 @@
-// The mixed-precision time step as three kernels.
+// The mixed-precision time step as four kernels (small batches merge them, see
+// k_steps_mixed; sheltering batches take k_step_pairs_shel_mixed and
+// k_group_sums_mixed).
 //
-// (b) k_pairs_mixed: one lane per owner-row entry (each unordered pair once,
-//     stepper.f90:89-271 without the bond terms).  Most candidates are not in
-//     contact: a lane that can see from the squared distance that the pair
-//     neither touches nor carries a contact history does nothing beyond
-//     clearing its flags.  A contact, a pair with history, every candidate of
-//     a sheltering field and every candidate on a diagnostic step leaves a
-//     32-byte record at its own index (force on the lower-id floe, both
-//     moments, shelter factors) and sets a flag byte in both rows; histories
-//     are updated in place.  No reductions and no atomics.
+// (b) k_pairs_screen: the contact list (each unordered pair that can touch
+//     before the next rebuild once, stepper.f90:89-271 without the bond
+//     terms).  A pair that its distance bound proves apart is skipped; a
+//     contact, a pair with a history and every candidate of a sheltering field
+//     leaves a 32-byte record at its own index (force on the lower-id floe,
+//     both moments, shelter factors) and sets a flag byte in both rows;
+//     histories are updated in place.  No reductions and no atomics.  On a
+//     diagnostic step k_pairs_mixed does this for every owner entry.
 // (b') k_bonds_mixed: one lane per bond (bonds.f90:74-212), in bond order, so
 //     the bond state is read and written contiguously; it leaves a 16-byte
-//     record per bond.
-// (c)-(e) k_floes_mixed: one thread per floe; sums the flagged records of its
-//     two rows and of its bonds, then walls, ridging, drag, Coriolis and the
-//     FP64 update.
+//     record per floe of a bond.
+// (c)-(e) k_floe_sums: one thread per floe sums the flagged records of its two
+//     rows and of its bonds; k_floes_mixed: walls, ridging, drag, Coriolis and
+//     the FP64 update.
 // Pair forces, sheltering and drag are FP32; geometry that cancels, bond
 // strain/damage, ridging bookkeeping and integration are FP64.
 #include <algorithm>
@@ -1279,7 +1280,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_steps_mixed(Views V, Small
 }
 
 // The two halves of a step as ordinary grids, for batches with more work
-// than one cluster does quickly: two launches a step instead of five (three
+// than one cluster does quickly: two launches a step instead of four (three
 // where the bonds follow the pairs).  The last one of a chunk's last step
 // publishes the status word.
 // MINB blocks an SM: as k_step_pairs_fp64 (65,536 sheltering floes: 117 -> 112

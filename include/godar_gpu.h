@@ -343,9 +343,10 @@ int godar_batch_wait(godar_batch *b);
 int godar_batch_stats(godar_batch *b, double *kernel_ms, int64_t *launches,
                       int64_t *rebuilds, int64_t *counts4);
 /* The same device time split by kernel (CUDA events between the kernels of
- * each timed step), up to nphase entries: GODAR_PREC_MIXED [pair screen, pair
- * work list, bonds, floe sums, floe update], GODAR_PREC_FP64 [entry screen,
- * general work list, bond work list, row sums, floe update]; the number of
+ * each timed step), up to nphase entries: GODAR_PREC_MIXED [pair screen and
+ * physics, every candidate (diagnostic steps only), bonds, floe sums, floe
+ * update], GODAR_PREC_FP64 [entry screen and bonded pairs (sheltering fields:
+ * every pair), work list, none, row sums, floe update]; the number of
  * step kernels launched; and the number of steps timed.  No counterpart in
  * the reference (its timers are the wall-clock prints of godar.f90). */
 #define GODAR_NPHASES 5
@@ -365,7 +366,7 @@ int godar_batch_set_phase_timing(godar_batch *b, int every);
  * of a batch (or the block size of GODAR_BLOCK, variant 0); whether chunks of
  * steps run as captured CUDA graphs, and how many chunks ran as a whole (a
  * graph launch, or on small batches the merged step kernels, which have no
- * configuration to choose: GODAR_FUSED=0 runs the five kernels instead).
+ * configuration to choose: GODAR_FUSED=0 runs the separate kernels).
  * Environment: GODAR_TUNE=0 disables the tuner, GODAR_TUNE_LOG=1
  * prints its measurements, GODAR_BOND_VARIANT=v fixes the bond kernel's
  * variant, GODAR_GRAPHS=0 disables the graphs; GODAR_OVERLAP_BONDS=1 runs

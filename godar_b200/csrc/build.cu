@@ -113,7 +113,8 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(const uint32_t *ke
 
 // ------------------------------------------------------------ exclusive scan
 // out[i] = sum_{k<i} in[i]; out[n] = total.  Three phases: per-block scan,
-// scan of block sums by one block, add.
+// scan of block sums by one block, add.  n may be any int: a batch of sparse
+// fields has up to 2^31 - 1 cells, so a stride past the end is not an int.
 constexpr int SC_THREADS = 512;
 constexpr int SC_ITEMS = 4;
 constexpr int SC_TILE = SC_THREADS * SC_ITEMS;
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(1024) k_scan_sums(int *tile_sums, int ntiles, 
 
 __global__ void k_scan_add(int *out, int n, const int *tile_sums, const int *total, int *out_n)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] += tile_sums[i / SC_TILE];
     if (blockIdx.x == 0 && threadIdx.x == 0 && out_n) *out_n = *total;
 }
@@ -219,10 +220,10 @@ void scan_excl(const int *in, int *out, int n, int *scratch, cudaStream_t st)
         k_scan_short<<<1, 1024, 0, st>>>(in, out, n);
         return;
     }
-    const int ntiles = (n + SC_TILE - 1) / SC_TILE;
+    const int ntiles = (int)(((long long)n + SC_TILE - 1) / SC_TILE);
     k_scan_tiles<<<ntiles, SC_THREADS, 0, st>>>(in, out, n, scratch + 1);
     k_scan_sums<<<1, 1024, 0, st>>>(scratch + 1, ntiles, scratch);
-    k_scan_add<<<(n + 255) / 256, 256, 0, st>>>(out, n, scratch + 1, scratch, out + n);
+    k_scan_add<<<(int)(((long long)n + 255) / 256), 256, 0, st>>>(out, n, scratch + 1, scratch, out + n);
 }
 
 void radix_sort(uint32_t *keys, int *vals, uint32_t *keys_alt, int *vals_alt, int n, int bits,

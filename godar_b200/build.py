@@ -47,7 +47,7 @@ UNITS = {
     "posts.cu": EXACT,
     "place.cu": [],
 }
-HEADERS = ["common.cuh", "physics.cuh", "detmath.cuh", "step_kernel.cuh", "kernels.h", "cells.cuh"]
+HEADERS = ["common.cuh", "physics.cuh", "detmath.cuh", "step_kernel.cuh", "kernels.h", "cells.cuh", "cover.h"]
 
 
 def _newer(target: str, deps) -> bool:

@@ -37,6 +37,7 @@
 
 #include "../../include/godar_gpu.h"
 #include "common.cuh"
+#include "cover.h"
 #include "kernels.h"
 
 namespace godar {
@@ -67,20 +68,6 @@ GD_DEV double pwrap(double d, double L, int per)
     if (d > 0.5 * L) d -= L;
     else if (d < -0.5 * L) d += L;
     return d;
-}
-
-// Cell index range [a, b] of the interval [lo, hi] on one axis; a periodic
-// range longer than the axis becomes the whole axis.
-GD_DEV void cell_span(double lo, double hi, double cw, int nc, int per, int &a, int &b)
-{
-    a = (int)floor(lo / cw);
-    b = (int)floor(hi / cw);
-    if (per) {
-        if (b - a + 1 >= nc) { a = 0; b = nc - 1; }
-    } else {
-        a = max(a, 0);
-        b = min(b, nc - 1);
-    }
 }
 
 GD_DEV int wrapc(int c, int nc, int per) { return per ? ((c % nc) + nc) % nc : c; }
@@ -381,8 +368,7 @@ int place_disks(int n, const double *r_in, double Lx, double Ly, int px, int py,
         double met = 0.0;
         C.big = 0;
         for (int k = 0; k < k1; k++) {
-            const double own = std::min((double)G.ncx, std::floor(2.0 * rs[k] / G.cwx) + 2.0) *
-                               std::min((double)G.ncy, std::floor(2.0 * rs[k] / G.cwy) + 2.0);
+            const double own = cells_met(rs[k], G.cwx, G.ncx) * cells_met(rs[k], G.cwy, G.ncy);
             met += own;
             if (own > COVER_ALONE) C.big = k + 1;
         }

@@ -161,12 +161,13 @@ __global__ void __launch_bounds__(256) k_trial(int c0, int c1, const double *r, 
     const int lane = threadIdx.x & 31, sub = lane & 3, att = lane >> 2, quad = lane & ~3;
     const int warps = gridDim.x * (blockDim.x >> 5);
     for (int i = c0 + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < c1; i += warps) {
-        if (lane == 0) cand[i] = 0;
-        if (placed[i]) continue;
         const double rad = r[i];
         const double xlo = G.px ? 0.0 : rad, xhi = G.px ? G.Lx : G.Lx - rad;
         const double ylo = G.py ? 0.0 : rad, yhi = G.py ? G.Ly : G.Ly - rad;
-        if (!(xhi > xlo && yhi > ylo)) continue;
+        if (placed[i] || !(xhi > xlo && yhi > ylo)) {
+            if (lane == 0) cand[i] = 0;
+            continue;
+        }
         uint64_t s = mix64(seed ^ (0x632be59bd9b4e019ULL * (uint64_t)(i + 1))) ^ mix64((uint64_t)round + 1);
         // attempt a takes the generator's values 2 a and 2 a + 1
         s += 2 * (uint64_t)att * 0x9e3779b97f4a7c15ULL;
@@ -250,10 +251,12 @@ __global__ void __launch_bounds__(256) k_trial(int c0, int c1, const double *r, 
             }
         }
         const unsigned ok = __ballot_sync(full, found);
-        if (ok && lane == __ffs(ok) - 1) {
-            cand[i] = 1;
-            tx[i] = cx;
-            ty[i] = cy;
+        if (lane == (ok ? __ffs(ok) - 1 : 0)) {
+            cand[i] = ok != 0;
+            if (ok) {
+                tx[i] = cx;
+                ty[i] = cy;
+            }
         }
     }
 }

@@ -424,6 +424,7 @@ struct Engine {
     // GODAR_FUSED=0 turns it off, as does any switch that asks for a
     // particular launch of the separate kernels.
     bool fused_on = true;
+    ClusterLimit cluster;
     static constexpr int SMALL_FLOES_FP64 = 100 * 1024;
     static constexpr int SMALL_FLOES_MIXED = 120 * 1024;
 
@@ -570,7 +571,7 @@ struct Engine {
     struct Pending {
         int base, K, c0, slot;
         bool diag;                 // its last step produced the diagnostics
-        bool small;                // it was one launch (launch_small)
+        bool small;                // it ran as merged steps (launch_small)
         std::vector<double> uvw;   // the uniform forcing it ran with (empty: as admitted)
     };
     static constexpr int RING = RES_RING;
@@ -1607,34 +1608,26 @@ struct Engine {
         return GODAR_OK;
     }
 
-    // Whether this batch's chunks run as one launch.  A call whose steps are
+    // Whether this batch's chunks run as merged steps.  A call whose steps are
     // timed kernel by kernel runs the kernels.
     bool small_batch(int every) const {
         return fused_on && every == 0 && N > 0 && N <= (prec == GODAR_PREC_FP64 ? SMALL_FLOES_FP64 : SMALL_FLOES_MIXED);
     }
 
-    // K steps from side c0 in one launch; out receives the status word and
-    // the first expired step.  False (and off from then on) where a cluster
-    // launch is not available.
-    bool launch_small(int K, int c0, int diag_last, int *out) {
+    // K steps from side c0 as merged steps; out receives the status word and
+    // the first expired step.
+    void launch_small(int K, int c0, int diag_last, int *out) {
         Views V = views();
         V.pdl = step_pdl();
-        bool ok;
         if (prec == GODAR_PREC_FP64)
-            ok = launch_steps_fp64(V, c0, K, diag_last, gbase, (int)Lc, (int)E, shelter_any ? 1 : 0, walls_any ? 1 : 0, fplist_b.as<int>(),
-                                   erow_up.as<unsigned>(), pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
-                                   fupn_b.as<int>(), fsum_b.as<double>(), out, step_base_b.as<int>() + 1, st);
+            launch_steps_fp64(V, cluster, c0, K, diag_last, gbase, (int)Lc, (int)E, shelter_any ? 1 : 0, walls_any ? 1 : 0, fplist_b.as<int>(),
+                              erow_up.as<unsigned>(), pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
+                              fupn_b.as<int>(), fsum_b.as<double>(), out, step_base_b.as<int>() + 1, st);
         else
-            ok = launch_steps_mixed(V, c0, K, diag_last, gbase, (int)Ec, (int)E, NB, shelter_any ? 1 : 0, walls_any ? 1 : 0, ridging_any ? 1 : 0,
-                                    clist_b.as<int2>(), clist_b.as<int2>() + Ecap, erow_up.as<unsigned>(),
-                                    bflag_b.as<unsigned char>(), mixed_bufs(), out, step_base_b.as<int>() + 1, st);
-        if (!ok) {
-            cudaGetLastError();
-            fused_on = false;
-            return false;
-        }
+            launch_steps_mixed(V, cluster, c0, K, diag_last, gbase, (int)Ec, (int)E, NB, shelter_any ? 1 : 0, walls_any ? 1 : 0, ridging_any ? 1 : 0,
+                               clist_b.as<int2>(), clist_b.as<int2>() + Ecap, erow_up.as<unsigned>(),
+                               bflag_b.as<unsigned char>(), mixed_bufs(), out, step_base_b.as<int>() + 1, st);
         graph_launches++;
-        return true;
     }
 
     int max_cfg() const {
@@ -1803,7 +1796,7 @@ struct Engine {
         }
         int remaining = nsteps;
         while (remaining > 0) {
-            bool small = small_batch(phase_every);
+            const bool small = small_batch(phase_every);
             const bool tuning = tune_left > 0 && !small;
             // a tuning chunk runs one step per candidate; otherwise chunks of
             // the separate kernels are powers of two so that their graphs are reused
@@ -1812,10 +1805,9 @@ struct Engine {
             const int diag_last = (diagnostics && remaining == K) ? 1 : 0;
             int bs[NPH];
             for (int q = 0; q < NPH; q++) bs[q] = blk[q];
-            small = small && launch_small(K, cur, diag_last, h_status);
             if (!small) begin_chunk();
             if (small) {
-                // launched
+                launch_small(K, cur, diag_last, h_status);
             } else if (tuning) {
                 // each tuning step uses the next candidate for every kernel
                 for (int k = 0; k < K; k++) {
@@ -1948,7 +1940,7 @@ struct Engine {
         while (remaining > 0) {
             if ((int)pend.size() >= RING) TRY(resolve_front(pend.size()));
             int K = std::min(remaining, chunk);
-            bool small = small_batch(0);
+            const bool small = small_batch(0);
             if (!small) while (K & (K - 1)) K &= K - 1;
             const int diag_last = (diagnostics && remaining == K) ? 1 : 0;
             Pending P;
@@ -1957,9 +1949,10 @@ struct Engine {
             P.uvw = cur_uvw;
             ring_next = (ring_next + 1) % RING;
             int *hs = h_ring + 4 * P.slot;
-            small = small && launch_small(K, cur, diag_last, hs);
             P.small = small;
-            if (!small) {
+            if (small) {
+                launch_small(K, cur, diag_last, hs);
+            } else {
                 begin_chunk();
                 // queued steps record no timing events: nothing reads them
                 TRY(launch_chunk(K, cur, diag_last, blk, false, 0));

@@ -29,6 +29,12 @@ inline void launch_step(bool pdl, void (*kern)(Params...), int grid, int block, 
     cudaLaunchKernelEx(&c, kern, args...);
 }
 
+// The largest cluster an engine's kernels of whole steps may ask for: -1 before
+// the first one (the attribute that allows more than eight blocks belongs to
+// the kernel on one device, so every engine sets it), 0 where even eight were
+// refused.
+struct ClusterLimit { int blocks = -1; };
+
 // Launches a kernel of whole steps (k_steps_fp64, k_steps_mixed) as one block
 // for at most `alone` items, else as one cluster of enough blocks to give
 // every item a thread, at most SMALL_CLUSTER.  One block finds what it wrote
@@ -36,30 +42,39 @@ inline void launch_step(bool pdl, void (*kern)(Params...), int grid, int block, 
 // starts from L2 behind a barrier of 380, so a few items a thread cost less
 // than a second block: 256 free floes 5.7 against 8.3 us a step FP64, 4.2
 // against 6.9 mixed; 200 bonded ones mixed 8.6 (one block), 12.4 (two), 10.0
-// (four).  False if the launch was refused.
+// (four).  A cluster that is refused is asked for with eight blocks, and then
+// no more: false, with nothing launched.
 template <typename... Params, typename... Args>
-inline bool launch_cluster(bool pdl, void (*kern)(Params...), long long items, int alone, cudaStream_t st,
-                           Args... args)
+inline bool launch_cluster(ClusterLimit &most, bool pdl, void (*kern)(Params...), long long items, int alone,
+                           cudaStream_t st, Args... args)
 {
-    static const bool wide =
-        cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-    const int most = wide ? SMALL_CLUSTER : 8;
-    int blocks = 1;
-    while (items > alone && blocks < most && (long long)blocks * SMALL_THREADS < items) blocks *= 2;
-    cudaLaunchConfig_t c = {};
-    c.gridDim = dim3((unsigned)blocks);
-    c.blockDim = dim3(SMALL_THREADS);
-    c.stream = st;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)blocks;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = at;
-    c.numAttrs = pdl ? 2 : 1;
-    return cudaLaunchKernelEx(&c, kern, args...) == cudaSuccess;
+    if (items > alone && most.blocks < 0)
+        most.blocks = cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                              cudaSuccess
+                          ? SMALL_CLUSTER
+                          : 8;
+    while (items <= alone || most.blocks > 1) {
+        int blocks = 1;
+        while (items > alone && blocks < most.blocks && (long long)blocks * SMALL_THREADS < items) blocks *= 2;
+        cudaLaunchConfig_t c = {};
+        c.gridDim = dim3((unsigned)blocks);
+        c.blockDim = dim3(SMALL_THREADS);
+        c.stream = st;
+        cudaLaunchAttribute at[2];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)blocks;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
+        c.attrs = at;
+        c.numAttrs = pdl ? 2 : 1;
+        if (cudaLaunchKernelEx(&c, kern, args...) == cudaSuccess) return true;
+        cudaGetLastError();
+        if (blocks == 1) return false;
+        most.blocks = blocks > 8 ? 8 : 0;
+    }
+    return false;
 }
 
 void scan_excl(const int *in, int *out, int n, int *scratch, cudaStream_t st);
@@ -120,11 +135,11 @@ void launch_fp64_bonds(const Views &V, int side, int *cnt, int *wfo, int *scan_s
 // shelter: some field of the batch has sheltering; drag: 8 N doubles; out:
 // pinned host memory for the status word and the first expired step; done: an
 // int that is zero): as one launch of one cluster up to ONE_CLUSTER_* items
-// (positions, bonds and floes; one block up to ONE_BLOCK_*), else as two
-// launches a step.  False if the launch was refused.
+// (positions, bonds and floes; one block up to ONE_BLOCK_*), else, or where
+// the cluster is refused, as two launches a step.
 constexpr int ONE_CLUSTER_FP64 = 1024, ONE_CLUSTER_MIXED = 4096;
 constexpr int ONE_BLOCK_FP64 = 640, ONE_BLOCK_MIXED = 1024;
-bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
+void launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
                        const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
                        const int *up_n, double *drag, int *out, int *done, cudaStream_t st);
 
@@ -188,7 +203,7 @@ void launch_floes_mixed(const Views &V, int cur, int diag, int sic, int walls, i
 
 // The same on the mixed path (n contact-list items eb/stl, bfl: the live-bond
 // flags of both sides).
-bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
+void launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
                         int walls, int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
                         int *done, cudaStream_t st);
 

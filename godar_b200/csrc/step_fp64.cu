@@ -73,7 +73,7 @@ void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, in
     }
 }
 
-bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
+void launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
                        const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
                        const int *up_n, double *drag, int *out, int *done, cudaStream_t st)
 {
@@ -82,7 +82,9 @@ bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, 
     A.n = n; A.E = E; A.plist = plist; A.erow = erow; A.pfl = pfl; A.rec = (PairRec64 *)rec;
     A.lo_n = lo_n; A.up_n = up_n; A.drag = drag; A.out = out; A.done = done;
     const long long items = (long long)n + V.N;
-    if (!shelter && items <= ONE_CLUSTER_FP64) return launch_cluster(V.pdl != 0, k_steps_fp64, items, ONE_BLOCK_FP64, st, V, A);
+    if (!shelter && items <= ONE_CLUSTER_FP64 &&
+        launch_cluster(most, V.pdl != 0, k_steps_fp64, items, ONE_BLOCK_FP64, st, V, A))
+        return;
     const GroupSums how = group_sums(V.N, shelter);
     // the drag planes of floes out of sheltering fields, then the sums
     double *fs = drag + 8 * (size_t)V.N;
@@ -107,7 +109,6 @@ bool launch_steps_fp64(const Views &V, int cur, int K, int diag_last, int base, 
             launch_step(V.pdl != 0, walls ? k_step_update_fp64<true> : k_step_update_fp64<false>, fp64_grid(V.N, 64), 64, st, V, A, c, k, fs);
         }
     }
-    return true;
 }
 
 // Owner entries [0, E) at a rebuild (floes on side `side`, at the rebuild

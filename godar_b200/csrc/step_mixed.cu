@@ -1486,7 +1486,7 @@ void launch_group_sums_mixed(const Views &V, MixedBufs B, cudaStream_t st)
     launch_step(V.pdl != 0, k_group_sums_mixed, (V.N + GRP_FLOES - 1) / GRP_FLOES, SMALL_THREADS, st, V, B, B.fsum);
 }
 
-bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
+void launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
                         int walls, int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
                         int *done, cudaStream_t st)
 {
@@ -1498,7 +1498,9 @@ bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base,
     A.out = out;
     A.done = done;
     const long long all = (long long)n + NB + V.N;
-    if (!shelter && all <= ONE_CLUSTER_MIXED) return launch_cluster(V.pdl != 0, k_steps_mixed, all, ONE_BLOCK_MIXED, st, V, A, B);
+    if (!shelter && all <= ONE_CLUSTER_MIXED &&
+        launch_cluster(most, V.pdl != 0, k_steps_mixed, all, ONE_BLOCK_MIXED, st, V, A, B))
+        return;
     const GroupSums how = group_sums(V.N, shelter);
     const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
     float4 *fs = B.fdg;   // (a plain step has no diagnostic sums)
@@ -1526,7 +1528,6 @@ bool launch_steps_mixed(const Views &V, int cur, int K, int diag_last, int base,
             launch_step(V.pdl != 0, walls ? k_step_update_mixed<true> : k_step_update_mixed<false>, grid_of(V.N, 64), 64, st, V, A, B, c, k, fs);
         }
     }
-    return true;
 }
 
 __global__ void k_pack_snap(Views V, int side)

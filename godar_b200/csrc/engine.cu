@@ -571,7 +571,7 @@ struct Engine {
     struct Pending {
         int base, K, c0, slot;
         bool diag;                 // its last step produced the diagnostics
-        bool small;                // it ran as merged steps (launch_small)
+        int merged;                // kernels it ran as merged steps (0: the separate kernels)
         std::vector<double> uvw;   // the uniform forcing it ran with (empty: as admitted)
     };
     static constexpr int RING = RES_RING;
@@ -1615,19 +1615,18 @@ struct Engine {
     }
 
     // K steps from side c0 as merged steps; out receives the status word and
-    // the first expired step.
-    void launch_small(int K, int c0, int diag_last, int *out) {
+    // the first expired step.  Returns the kernels launched.
+    int launch_small(int K, int c0, int diag_last, int *out) {
         Views V = views();
         V.pdl = step_pdl();
-        if (prec == GODAR_PREC_FP64)
-            launch_steps_fp64(V, cluster, c0, K, diag_last, gbase, (int)Lc, (int)E, shelter_any ? 1 : 0, walls_any ? 1 : 0, fplist_b.as<int>(),
-                              erow_up.as<unsigned>(), pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
-                              fupn_b.as<int>(), fsum_b.as<double>(), out, step_base_b.as<int>() + 1, st);
-        else
-            launch_steps_mixed(V, cluster, c0, K, diag_last, gbase, (int)Ec, (int)E, NB, shelter_any ? 1 : 0, walls_any ? 1 : 0, ridging_any ? 1 : 0,
-                               clist_b.as<int2>(), clist_b.as<int2>() + Ecap, erow_up.as<unsigned>(),
-                               bflag_b.as<unsigned char>(), mixed_bufs(), out, step_base_b.as<int>() + 1, st);
         graph_launches++;
+        if (prec == GODAR_PREC_FP64)
+            return launch_steps_fp64(V, cluster, c0, K, diag_last, gbase, (int)Lc, (int)E, shelter_any ? 1 : 0, walls_any ? 1 : 0, fplist_b.as<int>(),
+                                     erow_up.as<unsigned>(), pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
+                                     fupn_b.as<int>(), fsum_b.as<double>(), out, step_base_b.as<int>() + 1, st);
+        return launch_steps_mixed(V, cluster, c0, K, diag_last, gbase, (int)Ec, (int)E, NB, shelter_any ? 1 : 0, walls_any ? 1 : 0, ridging_any ? 1 : 0,
+                                  clist_b.as<int2>(), clist_b.as<int2>() + Ecap, erow_up.as<unsigned>(),
+                                  bflag_b.as<unsigned char>(), mixed_bufs(), out, step_base_b.as<int>() + 1, st);
     }
 
     int max_cfg() const {
@@ -1636,8 +1635,10 @@ struct Engine {
         return m;
     }
 
-    int kernels_per_step() const {
-        return prec == GODAR_PREC_FP64 ? 4 : (E > 0 ? 1 : 0) + (NB > 0 ? 1 : 0) + 2;
+    // The separate kernels of a plain or of a diagnostic step (launch_one).
+    int step_kernels(bool diag) const {
+        if (prec == GODAR_PREC_FP64) return shelter_any && !diag ? (Lc > 0) + 2 : 4;
+        return (diag ? (E > 0 ? 2 : 0) : (Ec > 0)) + (NB > 0) + 2;
     }
 
     // The graph of K steps from side c0, captured on first use.  Returns
@@ -1787,7 +1788,7 @@ struct Engine {
         TRY(open_counters());
         if (!timing_open) { CK(cudaEventRecord(ev0, st)); timing_open = true; }
         // tune once, and again only if the batch grew more than 4x since (a
-        // batch whose chunks are one launch has nothing to tune)
+        // batch of merged steps has nothing to tune)
         if (tune_on && !small_batch(phase_every) && (tuned_n == 0 || N > 4 * tuned_n) && tune_left == 0) {
             tune_left = TUNE_ROUNDS * max_cfg();
             tuned_n = N;
@@ -1806,8 +1807,9 @@ struct Engine {
             int bs[NPH];
             for (int q = 0; q < NPH; q++) bs[q] = blk[q];
             if (!small) begin_chunk();
+            int merged = 0;
             if (small) {
-                launch_small(K, cur, diag_last, h_status);
+                merged = launch_small(K, cur, diag_last, h_status);
             } else if (tuning) {
                 // each tuning step uses the next candidate for every kernel
                 for (int k = 0; k < K; k++) {
@@ -1892,7 +1894,7 @@ struct Engine {
                     drop_graphs();
                 }
             }
-            account(done, small);
+            account(done, K, diag_last != 0, merged);
             cur ^= (done & 1);
             remaining -= done;
             if (stt & ST_EXPIRED) {
@@ -1949,9 +1951,9 @@ struct Engine {
             P.uvw = cur_uvw;
             ring_next = (ring_next + 1) % RING;
             int *hs = h_ring + 4 * P.slot;
-            P.small = small;
+            P.merged = 0;
             if (small) {
-                launch_small(K, cur, diag_last, hs);
+                P.merged = launch_small(K, cur, diag_last, hs);
             } else {
                 begin_chunk();
                 // queued steps record no timing events: nothing reads them
@@ -1969,10 +1971,15 @@ struct Engine {
         return resolve_front(std::min(before, pend.size()));
     }
 
-    // Time steps counted as done.
-    void account(int done, bool small) {
+    // The first `done` of a chunk's K steps counted as done (diag: the K-th
+    // produced the diagnostics; merged: its kernels as merged steps).
+    void account(int done, int K, bool diag, int merged) {
         launches += done;
-        kernel_launches += small ? 1 : (long long)done * kernels_per_step();
+        if (merged)
+            kernel_launches += ((long long)merged * done + K - 1) / K;
+        else
+            kernel_launches += (long long)done * step_kernels(false) +
+                               (diag && done == K ? step_kernels(true) - step_kernels(false) : 0);
         for (auto &I : insts) I.steps += done;
     }
 
@@ -1992,7 +1999,7 @@ struct Engine {
                 return GODAR_ERR_TIMEOUT;
             }
             if (stt & ST_EXPIRED) return redo_after_expiry();
-            account(P.K, P.small);
+            account(P.K, P.K, P.diag, P.merged);
             chunk = std::min(chunk * 2, 256);
             pend.pop_front();
             n--;
@@ -2012,7 +2019,7 @@ struct Engine {
         std::vector<Redo> redo;
         if (P.K > done) redo.push_back({P.K - done, P.diag, P.uvw});
         for (size_t i = 1; i < pend.size(); i++) redo.push_back({pend[i].K, pend[i].diag, pend[i].uvw});
-        account(done, P.small);
+        account(done, P.K, P.diag, P.merged);
         cur = P.c0 ^ (done & 1);
         pend.clear();
         for (int q = 0; q < 2; q++)

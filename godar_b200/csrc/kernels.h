@@ -136,10 +136,11 @@ void launch_fp64_bonds(const Views &V, int side, int *cnt, int *wfo, int *scan_s
 // pinned host memory for the status word and the first expired step; done: an
 // int that is zero): as one launch of one cluster up to ONE_CLUSTER_* items
 // (positions, bonds and floes; one block up to ONE_BLOCK_*), else, or where
-// the cluster is refused, as two launches a step.
+// the cluster is refused, as two to four launches a step.  Returns the kernels
+// launched.
 constexpr int ONE_CLUSTER_FP64 = 1024, ONE_CLUSTER_MIXED = 4096;
 constexpr int ONE_BLOCK_FP64 = 640, ONE_BLOCK_MIXED = 1024;
-void launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
+int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
                        const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
                        const int *up_n, double *drag, int *out, int *done, cudaStream_t st);
 
@@ -203,7 +204,7 @@ void launch_floes_mixed(const Views &V, int cur, int diag, int sic, int walls, i
 
 // The same on the mixed path (n contact-list items eb/stl, bfl: the live-bond
 // flags of both sides).
-void launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
+int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
                         int walls, int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
                         int *done, cudaStream_t st);
 

@@ -73,7 +73,7 @@ void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, in
     }
 }
 
-void launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
+int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
                        const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
                        const int *up_n, double *drag, int *out, int *done, cudaStream_t st)
 {
@@ -84,31 +84,37 @@ void launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int d
     const long long items = (long long)n + V.N;
     if (!shelter && items <= ONE_CLUSTER_FP64 &&
         launch_cluster(most, V.pdl != 0, k_steps_fp64, items, ONE_BLOCK_FP64, st, V, A))
-        return;
+        return 1;
     const GroupSums how = group_sums(V.N, shelter);
     // the drag planes of floes out of sheltering fields, then the sums
     double *fs = drag + 8 * (size_t)V.N;
+    int kernels = 0;
+    const auto launch = [&](auto kern, int grid, int block, auto... args) {
+        launch_step(V.pdl != 0, kern, grid, block, st, args...);
+        kernels++;
+    };
     for (int k = 0; k < K; k++) {
         const int c = cur ^ (k & 1);
         const bool diag = diag_last && k == K - 1;
         const long long work = (long long)(diag ? E : n) + 32 + V.N;
         const int gp = fp64_grid(work, 128);
         const bool dense = work > 148 * 2 * 128;
-        if (diag) launch_step(V.pdl != 0, dense ? k_step_pairs_fp64<true, 4> : k_step_pairs_fp64<true, 2>, gp, 128, st, V, A, c);
-        else if (shelter && n > SHEL_WAVE) launch_step(V.pdl != 0, k_step_pairs_shel_fp64, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, c);
-        else launch_step(V.pdl != 0, dense ? k_step_pairs_fp64<false, 4> : k_step_pairs_fp64<false, 2>, gp, 128, st, V, A, c);
+        if (diag) launch(dense ? k_step_pairs_fp64<true, 4> : k_step_pairs_fp64<true, 2>, gp, 128, V, A, c);
+        else if (shelter && n > SHEL_WAVE) launch(k_step_pairs_shel_fp64, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, A, c);
+        else launch(dense ? k_step_pairs_fp64<false, 4> : k_step_pairs_fp64<false, 2>, gp, 128, V, A, c);
         const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
         if (diag) {
-            launch_step(V.pdl != 0, walls ? k_step_floes_fp64<true, true> : k_step_floes_fp64<true, false>, fp64_grid(V.N, 64), 64, st, V, A, c, k);
+            launch(walls ? k_step_floes_fp64<true, true> : k_step_floes_fp64<true, false>, fp64_grid(V.N, 64), 64, V, A, c, k);
         } else if (how == SUMS_THREAD) {
-            launch_step(V.pdl != 0, walls ? k_step_floes_fp64<false, true> : k_step_floes_fp64<false, false>, fp64_grid(V.N, 64), 64, st, V, A, c, k);
+            launch(walls ? k_step_floes_fp64<false, true> : k_step_floes_fp64<false, false>, fp64_grid(V.N, 64), 64, V, A, c, k);
         } else if (how == SUMS_GROUP) {
-            launch_step(V.pdl != 0, k_step_floes_grp_fp64, groups, SMALL_THREADS, st, V, A, c, k);
+            launch(k_step_floes_grp_fp64, groups, SMALL_THREADS, V, A, c, k);
         } else {
-            launch_step(V.pdl != 0, k_group_sums_fp64, groups, SMALL_THREADS, st, V, c, pfl, A.rec, lo_n, up_n, fs);
-            launch_step(V.pdl != 0, walls ? k_step_update_fp64<true> : k_step_update_fp64<false>, fp64_grid(V.N, 64), 64, st, V, A, c, k, fs);
+            launch(k_group_sums_fp64, groups, SMALL_THREADS, V, c, pfl, A.rec, lo_n, up_n, fs);
+            launch(walls ? k_step_update_fp64<true> : k_step_update_fp64<false>, fp64_grid(V.N, 64), 64, V, A, c, k, fs);
         }
     }
+    return kernels;
 }
 
 // Owner entries [0, E) at a rebuild (floes on side `side`, at the rebuild

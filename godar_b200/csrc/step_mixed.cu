@@ -1486,7 +1486,7 @@ void launch_group_sums_mixed(const Views &V, MixedBufs B, cudaStream_t st)
     launch_step(V.pdl != 0, k_group_sums_mixed, (V.N + GRP_FLOES - 1) / GRP_FLOES, SMALL_THREADS, st, V, B, B.fsum);
 }
 
-void launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
+int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
                         int walls, int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
                         int *done, cudaStream_t st)
 {
@@ -1500,10 +1500,15 @@ void launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int 
     const long long all = (long long)n + NB + V.N;
     if (!shelter && all <= ONE_CLUSTER_MIXED &&
         launch_cluster(most, V.pdl != 0, k_steps_mixed, all, ONE_BLOCK_MIXED, st, V, A, B))
-        return;
+        return 1;
     const GroupSums how = group_sums(V.N, shelter);
     const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
     float4 *fs = B.fdg;   // (a plain step has no diagnostic sums)
+    int kernels = 0;
+    const auto launch = [&](auto kern, int grid, int block, auto... args) {
+        launch_step(V.pdl != 0, kern, grid, block, st, args...);
+        kernels++;
+    };
     for (int k = 0; k < K; k++) {
         const int c = cur ^ (k & 1);
         const int diag = diag_last && k == K - 1;
@@ -1511,23 +1516,24 @@ void launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int 
         B.bfl_wr = A.bfl + (size_t)(c ^ 1) * NB;
         const long long items = (long long)(diag ? E : n) + (ridging ? 0 : NB) + 64 + V.N;
         if (shelter && !diag && n > SHEL_WAVE)
-            launch_step(V.pdl != 0, k_step_pairs_shel_mixed, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, B, c);
-        else launch_step(V.pdl != 0, items > 148 * 5 * 128 ? k_step_pairs_mixed<8> : k_step_pairs_mixed<5>, grid_of(items, 128),
-                    128, st, V, A, B, c, diag);
+            launch(k_step_pairs_shel_mixed, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, A, B, c);
+        else launch(items > 148 * 5 * 128 ? k_step_pairs_mixed<8> : k_step_pairs_mixed<5>, grid_of(items, 128),
+                    128, V, A, B, c, diag);
         if (ridging && NB > 0)
-            launch_step(V.pdl != 0, k_bonds_mixed, grid_of(NB, 128), 128, st, V, c, diag, NB, B.bsp, B.bst, B.brec,
+            launch(k_bonds_mixed, grid_of(NB, 128), 128, V, c, diag, NB, B.bsp, B.bst, B.brec,
                         B.bdg, B.bfl_wr, B.wdyn);
         if (diag) {
-            launch_step(V.pdl != 0, walls ? k_step_floes_mixed<true, true> : k_step_floes_mixed<true, false>, grid_of(V.N, 64), 64, st, V, A, B, c, k);
+            launch(walls ? k_step_floes_mixed<true, true> : k_step_floes_mixed<true, false>, grid_of(V.N, 64), 64, V, A, B, c, k);
         } else if (how == SUMS_THREAD) {
-            launch_step(V.pdl != 0, walls ? k_step_floes_mixed<false, true> : k_step_floes_mixed<false, false>, grid_of(V.N, 64), 64, st, V, A, B, c, k);
+            launch(walls ? k_step_floes_mixed<false, true> : k_step_floes_mixed<false, false>, grid_of(V.N, 64), 64, V, A, B, c, k);
         } else if (how == SUMS_GROUP) {
-            launch_step(V.pdl != 0, k_step_floes_grp_mixed, groups, SMALL_THREADS, st, V, A, B, c, k);
+            launch(k_step_floes_grp_mixed, groups, SMALL_THREADS, V, A, B, c, k);
         } else {
-            launch_step(V.pdl != 0, k_group_sums_mixed, groups, SMALL_THREADS, st, V, B, fs);
-            launch_step(V.pdl != 0, walls ? k_step_update_mixed<true> : k_step_update_mixed<false>, grid_of(V.N, 64), 64, st, V, A, B, c, k, fs);
+            launch(k_group_sums_mixed, groups, SMALL_THREADS, V, B, fs);
+            launch(walls ? k_step_update_mixed<true> : k_step_update_mixed<false>, grid_of(V.N, 64), 64, V, A, B, c, k, fs);
         }
     }
+    return kernels;
 }
 
 __global__ void k_pack_snap(Views V, int side)

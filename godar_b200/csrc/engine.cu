@@ -233,7 +233,7 @@ void restart_bonds(const Inst &I, HostBonds &B)
 // pinned memory and the memory pool.  Creating and destroying them takes
 // 1.5-8 ms, more than the whole first step of a field of a few thousand
 // floes, so a destroyed engine's set is kept for the next one on the same
-// device and context: at most RES_KEPT sets, each holding at most
+// device and context: at most RES_KEPT sets a context, each holding at most
 // RES_KEPT_BYTES of device memory; what is over is given back to the driver.
 // A set belongs to one engine at a time and comes back with its streams idle.
 constexpr size_t RES_KEPT = 4;
@@ -352,10 +352,11 @@ struct EngineRes {
         if (ok && r->ctx != 0 && r->ctx == context_id()) {
             std::lock_guard<std::mutex> lk(lock());
             auto &v = kept();
-            // sets of a context that is gone went with it
-            for (size_t k = v.size(); k-- > 0;)
-                if (v[k]->dev == r->dev && v[k]->ctx != r->ctx) v.erase(v.begin() + k);
-            if (v.size() < RES_KEPT) {
+            // (sets of other contexts are theirs: a context's id does not tell
+            // whether it is still there, and one that is gone took what the
+            // set holds with it)
+            const size_t mine = std::count_if(v.begin(), v.end(), [&](const EngineRes *k) { return k->ctx == r->ctx; });
+            if (mine < RES_KEPT) {
                 v.push_back(r);
                 return;
             }

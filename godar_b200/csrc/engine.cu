@@ -108,6 +108,11 @@ struct Buf {
         size_t nb = std::max<size_t>(grown, 256);
         pooled = pl && pl->pool;
         cudaError_t e = pooled ? cudaMallocFromPoolAsync(&p, nb, pl->pool, pl->st) : cudaMalloc(&p, nb);
+        if (e == cudaErrorMemoryAllocation && godar::release_kept()) {
+            // what destroyed engines left behind is back with the driver
+            cudaGetLastError();
+            e = pooled ? cudaMallocFromPoolAsync(&p, nb, pl->pool, pl->st) : cudaMalloc(&p, nb);
+        }
         if (e != cudaSuccess) { g_last_error = std::string("device allocation: ") + cudaGetErrorString(e); p = nullptr; return GODAR_ERR_NOMEM; }
         bytes = nb;
         if (acct) *acct += bytes;
@@ -234,8 +239,10 @@ void restart_bonds(const Inst &I, HostBonds &B)
 // 1.5-8 ms, more than the whole first step of a field of a few thousand
 // floes, so a destroyed engine's set is kept for the next one on the same
 // device and context: at most RES_KEPT sets a context, each holding at most
-// RES_KEPT_BYTES of device memory; what is over is given back to the driver.
-// A set belongs to one engine at a time and comes back with its streams idle.
+// RES_KEPT_BYTES of device memory; what is over is given back to the driver,
+// and so are the sets where an allocation finds no memory, or on request
+// (release_kept).  A set belongs to one engine at a time and comes back with
+// its streams idle.
 constexpr size_t RES_KEPT = 4;
 constexpr size_t RES_KEPT_BYTES = 256u << 20;
 constexpr int RES_RING = 16, RES_FRING = 4;
@@ -362,6 +369,28 @@ struct EngineRes {
             }
         }
         delete r;
+    }
+
+    // Every set kept for the calling thread's context back to the driver;
+    // whether there was one.
+    static bool release_all() {
+        std::vector<EngineRes *> mine;
+        {
+            std::lock_guard<std::mutex> lk(lock());
+            if (kept().empty()) return false;
+        }
+        const unsigned long long ctx = context_id();
+        {
+            std::lock_guard<std::mutex> lk(lock());
+            auto &v = kept();
+            for (size_t k = v.size(); k-- > 0;)
+                if (ctx != 0 && v[k]->ctx == ctx) {
+                    mine.push_back(v[k]);
+                    v.erase(v.begin() + k);
+                }
+        }
+        for (EngineRes *r : mine) delete r;
+        return !mine.empty();
     }
 };
 
@@ -1689,6 +1718,10 @@ struct Engine {
         if (held >= want) return GODAR_OK;
         void *p = nullptr;
         cudaError_t e = cudaMallocFromPoolAsync(&p, want - held, mp.pool, st);
+        if (e == cudaErrorMemoryAllocation && godar::release_kept()) {
+            cudaGetLastError();
+            e = cudaMallocFromPoolAsync(&p, want - held, mp.pool, st);
+        }
         if (e != cudaSuccess) { cudaGetLastError(); g_last_error = std::string("reserve: ") + cudaGetErrorString(e); return GODAR_ERR_NOMEM; }
         CK(cudaFreeAsync(p, st));
         CK(cudaStreamSynchronize(st));
@@ -2352,8 +2385,9 @@ struct godar_batch {
     Engine eng;
 };
 
-// for the output writer (posts.cu)
 namespace godar {
+bool release_kept() { return EngineRes::release_all(); }
+// for the output writer (posts.cu)
 int ctx_floe_count(const godar_ctx *c) { return c ? c->n : 0; }
 void set_last_error(const std::string &msg) { g_last_error = msg; }
 }  // namespace godar
@@ -2651,6 +2685,12 @@ int godar_gpu_stats(godar_ctx *c, double *ms, int64_t *counts4)
 }
 
 void godar_gpu_destroy(godar_ctx *c) { delete c; }
+
+int godar_gpu_release_kept(void)
+{
+    release_kept();
+    return GODAR_OK;
+}
 
 // ---------------------------------------------------------------- batches
 int godar_batch_create(int precision, size_t hbm_budget_bytes, godar_batch **out)

@@ -29,6 +29,11 @@ inline void launch_step(bool pdl, void (*kern)(Params...), int grid, int block, 
     cudaLaunchKernelEx(&c, kern, args...);
 }
 
+// What destroyed engines left for later ones on the calling thread's context
+// (streams, pinned memory, memory pools) back to the driver; whether there was
+// any (engine.cu).
+bool release_kept();
+
 // The largest cluster an engine's kernels of whole steps may ask for: -1 before
 // the first one (the attribute that allows more than eight blocks belongs to
 // the kernel on one device, so every engine sets it), 0 where even eight were

@@ -388,7 +388,12 @@ int place_disks(int n, const double *r_in, double Lx, double Ly, int px, int py,
     const size_t want = 5 * up((size_t)n * 8) + 2 * up((size_t)n) + 2 * up((nc + 1) * 4) + 2 * up(nc * 4) +
                         up((nc / 2048 + 64) * 4) + up((size_t)covers * 4) + up((size_t)covers * sizeof(Cover)) +
                         up((size_t)widest * 4) + up(16);
-    if (cudaMalloc(&M.base, want) != cudaSuccess) {
+    cudaError_t got_mem = cudaMalloc(&M.base, want);
+    if (got_mem == cudaErrorMemoryAllocation && release_kept()) {
+        cudaGetLastError();
+        got_mem = cudaMalloc(&M.base, want);
+    }
+    if (got_mem != cudaSuccess) {
         cudaGetLastError();
         M.base = nullptr;
         set_last_error("device allocation failed");

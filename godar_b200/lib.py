@@ -28,7 +28,7 @@ EXPORTS = [
     "godar_gpu_default_params", "godar_gpu_derive_params", "godar_gpu_create", "godar_gpu_upload",
     "godar_gpu_set_field", "godar_gpu_step", "godar_gpu_step_async", "godar_gpu_get_floe_field", "godar_gpu_get_pairs",
     "godar_gpu_download", "godar_gpu_place", "godar_gpu_write_posts", "godar_gpu_clear_posts", "godar_posts_format_reals",
-    "godar_gpu_set_precision", "godar_gpu_checkpoint", "godar_gpu_restore", "godar_gpu_stats", "godar_gpu_destroy", "godar_batch_create", "godar_batch_instance_bytes",
+    "godar_gpu_set_precision", "godar_gpu_checkpoint", "godar_gpu_restore", "godar_gpu_stats", "godar_gpu_destroy", "godar_gpu_release_kept", "godar_batch_create", "godar_batch_instance_bytes",
     "godar_batch_add", "godar_batch_remove", "godar_batch_step", "godar_batch_step_async", "godar_batch_sync",
     "godar_batch_get_floe_field", "godar_batch_steps_done", "godar_batch_count",
     "godar_batch_bytes_in_use", "godar_batch_set_uniform_forcing", "godar_batch_get_all",
@@ -164,6 +164,12 @@ def _field_array(params: GodarParams, field):
     if f.size != 4 * params.field_nx * params.field_ny:
         raise ValueError("forcing grid size does not match field_nx * field_ny")
     return f
+
+
+def release_kept():
+    """Gives back what destroyed steppers and batches left on the GPU for later
+    ones (godar_gpu_release_kept)."""
+    _check(load().godar_gpu_release_kept())
 
 
 class Stepper:

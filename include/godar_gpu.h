@@ -252,7 +252,15 @@ int godar_gpu_set_precision(godar_ctx *ctx, int mode);
  * step: candidate pairs, contacts, bonds, plastic events. */
 int godar_gpu_stats(godar_ctx *c, double *ms, int64_t *counts4);
 
+/* A destroyed context or batch leaves its streams, events, pinned memory and
+ * memory pool (at most 256 MB of device memory) for later ones, at most four
+ * such sets for each CUDA context; godar_batch_bytes_in_use does not count
+ * them.  An allocation of the library that finds no memory releases them and
+ * tries again. */
 void godar_gpu_destroy(godar_ctx *c);
+/* Releases what destroyed contexts and batches left on the calling thread's
+ * CUDA context (for a caller that needs the memory itself). */
+int godar_gpu_release_kept(void);
 
 /*
  * ---------------------------------------------------------------- batches
@@ -394,8 +402,8 @@ int godar_batch_prepare(godar_batch *b, int nsteps);
 /* Grows the batch's device memory pool to hold at least `bytes` (device
  * memory that the batch's buffers then draw on without the CUDA driver's
  * allocator), so that admissions and relayouts of a serving loop do not
- * allocate.  The pool keeps what it holds until the batch is destroyed and
- * grows past it on demand. */
+ * allocate.  The pool keeps what it holds until the batch is destroyed (of
+ * which see godar_gpu_destroy) and grows past it on demand. */
 int godar_batch_reserve(godar_batch *b, size_t bytes);
 void godar_batch_destroy(godar_batch *b);
 

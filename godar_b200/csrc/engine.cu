@@ -943,7 +943,11 @@ struct Engine {
         // scans over 2 n counts and over the cells
         TRY(ens(scan_scratch, ((2 * (size_t)n + (size_t)C) / 2048 + 64) * 4));
         TRY(ens(coff_b, (size_t)(C + 1) * 4)); TRY(ens(ccnt_b, (size_t)std::max<long long>(C, 1) * 4));
+        // (zero before the first diagnostic step: the pool's memory may have
+        // been another engine's)
+        const size_t had = diag.bytes;
         TRY(ens(diag, (size_t)14 * n * 8));
+        if (diag.bytes != had) CK(cudaMemsetAsync(diag.p, 0, diag.bytes, st));
         TRY(ens(tmp_out, (size_t)n * 8));
         return GODAR_OK;
     }

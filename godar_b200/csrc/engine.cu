@@ -777,9 +777,20 @@ struct Engine {
                                      : (8 + 8 + 4 + 16 + 4 + 4 + 4 + 1 + 1 + 32 + 8 + 32) +
                                            (16 + 16 + 8 + 8 + 4 + 16);
         const size_t per_floe = 2 * (2 * 15 * 8 + 2 * 48) + 64 + 12 * per_pair + (fp64 ? 8 * FP64_FLOE_SUMS : 12 + 68);
-        const size_t per_bond = 2 * (4 + sizeof(BondStat) + sizeof(BondDyn)) + 8 +
-                                (fp64 ? 0 : 32 + 64 + 8 + 8 + 16 + 32 + 2);
-        return (size_t)n * per_floe + (size_t)nb * per_bond + 4096;
+        const size_t bond_sets = 2 * (4 + sizeof(BondStat) + sizeof(BondDyn));
+        const size_t per_bond = bond_sets + 8 + (fp64 ? 0 : 32 + 64 + 8 + 8 + 16 + 32 + 2);
+        size_t sum = (size_t)n * per_floe + (size_t)nb * per_bond;
+        if (fp64) {
+            // what is allocated today: less a pair and a floe than the terms
+            // above (a batch's use stays well below them: 4.0 of 6.0 KB a floe
+            // on bonded fields), but the bonds have working copies, which count
+            // for more from about nine bonds a floe on
+            const size_t pair = (8 + 4 + 4 + 1 + 32 + FP64_PAIR_REC_BYTES + 1 + 16 + 4) + 2 * (8 + 8 + 4 + 32) + 8;
+            const size_t floe = 2 * 2 * (14 * 8 + 4) + 180 + 12 * pair + 16 + 8 * FP64_FLOE_SUMS;
+            const size_t bond = bond_sets + sizeof(BondDyn) + sizeof(BondGeom64) + 4;
+            sum = std::max(sum, (size_t)n * floe + (size_t)nb * bond);
+        }
+        return sum + 4096;
     }
 
     // bonds of a field not yet on the device: its restart list, or an upper

@@ -2346,20 +2346,19 @@ struct Engine {
         auto launch = [&](int m) {
             double *v = tmp_v.as<double>();
             int *i = (int *)(v + m);
-            launch_list_pairs(views(), cur, I->off, I->n, which, m, i, i + m, v, tmp_cnt.as<int>(), cnt.as<int>(),
-                              row_off2.as<int>(), scan_scratch.as<int>(), st);
+            return launch_list_pairs(views(), cur, I->off, I->n, bound, which, m, i, i + m, v, tmp_cnt.as<int>(),
+                                     cnt.as<int>(), row_off2.as<int>(), scan_scratch.as<int>(), st);
         };
         int *h_total = h_status + 2;
         if ((size_t)want * 16 > STAGE_SLOT) {
-            launch(0);
-            CK(cudaMemcpyAsync(h_total, tmp_cnt.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+            CK(cudaMemcpyAsync(h_total, launch(0), sizeof(int), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
             want = std::min(want, *h_total);
         }
         TRY(tmp_v.ensure(std::max<size_t>((size_t)want * 16, 16), &bytes, &mp));
-        launch(want);
+        const int *d_total = launch(want);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(h_total, tmp_cnt.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(h_total, d_total, sizeof(int), cudaMemcpyDeviceToHost, st));
         if ((size_t)want * 16 <= STAGE_SLOT) {
             if (want > 0) CK(cudaMemcpyAsync(h_stage, tmp_v.p, (size_t)want * 16, cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));

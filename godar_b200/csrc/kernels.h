@@ -231,10 +231,12 @@ void launch_gather_fields(const Views &V, int cur, int off, int n, const FieldLi
 // Per instance: momentum x, y, kinetic energy, largest speed (4 doubles).
 void launch_instance_summary(const Views &V, int cur, double *out, cudaStream_t st);
 // A pair list (0 candidates, 1 contacts, 2 live bonds) of the instance at
-// slots [off, off + n), ascending in (i, j): its first cap pairs and, in
-// total, its length.  cnt, base: n + 1 ints each.
-void launch_list_pairs(const Views &V, int cur, int off, int n, int which, int cap, int *pi, int *pj, double *val,
-                       int *total, int *cnt, int *base, int *scan_scratch, cudaStream_t st);
+// slots [off, off + n), ascending in (i, j): its first cap pairs.  Returns where
+// its length is written (total, or the end of base).  entries: of all the
+// batch's rows that the list is made from; cnt, base: n + 1 ints each.
+const int *launch_list_pairs(const Views &V, int cur, int off, int n, long long entries, int which, int cap, int *pi,
+                             int *pj, double *val, int *total, int *cnt, int *base, int *scan_scratch,
+                             cudaStream_t st);
 
 // Batch relayout (membership changes), per field: its first new slot and bond,
 // its first old ones (-1: admitted now).

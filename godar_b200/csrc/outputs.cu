@@ -1,6 +1,8 @@
 // Device-to-host outputs: per-floe fields back in reference index order, and
 // the pair lists the reference writes at output steps
 // (diagnostics_outputs.f90:157-167, mpi_coms.f90:691-796).
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -49,101 +51,167 @@ __global__ void k_gather_fields(Views V, int cur, int off, int n, FieldList F, d
 
 // The pair lists.  which: 0 candidates, 1 contacts (pdn of the last
 // diagnostic step), 2 live bonds.  A list is in ascending (i, j): the pairs
-// are counted by their lower id, the counts scanned, and every floe writes its
-// own pairs at its place, ascending in j, so the host has nothing to sort
-// (sorting there took most of a read-back: 0.4 ms for 5,300 bonds).
+// are counted by their lower id, the counts scanned, and every row's pairs
+// written at their place, ascending in j, so the host has nothing to sort
+// (sorting there took most of a read-back: 0.4 ms for 5,300 bonds).  A group
+// of lanes takes a row and places its pairs by their rank; a row of more than
+// CAP pairs is ranked by its whole block, since a large floe among small ones
+// has thousands (one thread inserting 3,272 of them by distance took 100 ms).
 
-// The pairs of row item k (0 .. n-1) of the instance at [off, off + n): for
-// lists 0 and 1 those of slot off + k, for bonds those of reference id k.
-// Calls f(j, value); returns the lower id.
-template <class F>
-GD_DEV int row_pairs(const Views &V, int cur, int off, int which, int k, F f)
+// Row item k (0 .. n-1) of the instance at [off, off + n): for lists 0 and 1
+// the owner entries of slot off + k, for bonds those of reference id k.
+// Returns the lower id.
+GD_DEV int list_row(const Views &V, int cur, int off, int which, int k, int &e0, int &e1)
+{
+    const int *first = which == 2 ? V.bond_off : V.up_off;
+    e0 = first[off + k];
+    e1 = first[off + k + 1];
+    return which == 2 ? k : V.id[cur][off + k];
+}
+
+// Whether entry e of a row is in the list, its higher id and value.
+GD_DEV bool list_entry(const Views &V, int cur, int which, int e, int &j, double &v)
 {
     if (which == 2) {
-        for (int b = V.bond_off[off + k]; b < V.bond_off[off + k + 1]; b++) {
-            const BondDyn d = V.bdyn[cur][b];
-            if (d.flag == 1) f(V.bond_hi[b], d.dmg);
+        const BondDyn d = V.bdyn[cur][e];
+        j = V.bond_hi[e];
+        v = d.dmg;
+        return d.flag == 1;
+    }
+    const int2 en = V.ent_up[e];
+    const float dn = V.pdn[en.y];
+    if (dn != dn || (which == 1 && !(dn > 0.0f))) return false;
+    j = V.id[cur][en.x];
+    v = (double)dn;
+    return true;
+}
+
+// cnt[lower id]: the pairs of every row.
+__global__ void __launch_bounds__(256) k_list_counts(Views V, int cur, int off, int n, int which, int *cnt)
+{
+    const int sub = threadIdx.x & (GRP - 1), step = gridDim.x * (blockDim.x / GRP);
+    // every lane of a warp runs the same rounds
+    for (int w = blockIdx.x * (blockDim.x / GRP) + (threadIdx.x & ~31) / GRP; w < n; w += step) {
+        const int k = w + (threadIdx.x & 31) / GRP;
+        int e0 = 0, e1 = 0, c = 0, id = 0;
+        if (k < n) id = list_row(V, cur, off, which, k, e0, e1);
+        for (int e = e0 + sub; e < e1; e += GRP) {
+            int j;
+            double v;
+            c += list_entry(V, cur, which, e, j, v);
         }
-        return k;
+#pragma unroll
+        for (int o = GRP / 2; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+        if (k < n && sub == 0) cnt[id] = c;
     }
-    const int s = off + k;
-    for (int e = V.up_off[s]; e < V.up_off[s + 1]; e++) {
-        const int2 en = V.ent_up[e];
-        const float dn = V.pdn[en.y];
-        if (dn != dn || (which == 1 && !(dn > 0.0f))) continue;
-        f(V.id[cur][en.x], (double)dn);
-    }
-    return V.id[cur][s];
 }
 
-GD_DEV int count_row(const Views &V, int cur, int off, int which, int k, int &id)
+// Every pair at base[lower id] + its rank in its row, up to cap of them (base:
+// n + 1).
+constexpr int LIST_THREADS = 128, LIST_CAP = 64;
+__global__ void __launch_bounds__(LIST_THREADS) k_list_fill(Views V, int cur, int off, int n, int which,
+                                                            const int *base, int cap, int *pi, int *pj, double *val)
 {
-    int c = 0;
-    id = row_pairs(V, cur, off, which, k, [&](int, double) { c++; });
-    return c;
-}
-
-// Row item k's pairs at their place: base[id], each inserted in ascending j
-// among those already there.
-GD_DEV void write_row(const Views &V, int cur, int off, int which, int k, const int *base, int cap, int *pi, int *pj,
-                      double *val)
-{
-    const int i = which == 2 ? k : V.id[cur][off + k];
-    const int a = base[i];
-    int m = a;
-    row_pairs(V, cur, off, which, k, [&](int j, double v) {
-        if (m < cap) {
-            int q = m;
-            while (q > a && pj[q - 1] > j) {
-                pj[q] = pj[q - 1];
-                val[q] = val[q - 1];
-                q--;
-            }
-            pi[m] = i;
-            pj[q] = j;
-            val[q] = v;
-        } else {
-            // past the caller's capacity: the largest j of this row leaves
-            int q = cap;
-            while (q > a && pj[q - 1] > j) {
-                if (q < cap) { pj[q] = pj[q - 1]; val[q] = val[q - 1]; }
-                q--;
-            }
-            if (q < cap) { pj[q] = j; val[q] = v; }
+    constexpr int T = LIST_THREADS;
+    __shared__ double bag_v[T / GRP][LIST_CAP];
+    __shared__ int bag_j[T / GRP][LIST_CAP];
+    __shared__ int tile[T];
+    __shared__ int whole[T / GRP];            // rows for the whole block (-1: none)
+    const int sub = threadIdx.x & (GRP - 1), grp = threadIdx.x / GRP;
+    const unsigned below = (1u << (threadIdx.x & 31)) - 1u;
+    const unsigned gmask = ((1u << GRP) - 1u) << (threadIdx.x & 31 & ~(GRP - 1));
+    for (int b = blockIdx.x * (T / GRP); b < n; b += gridDim.x * (T / GRP)) {
+        int e0 = 0, e1 = 0, id = 0, m = 0, at = 0;
+        if (b + grp < n) {
+            id = list_row(V, cur, off, which, b + grp, e0, e1);
+            at = base[id];
+            m = at < cap ? base[id + 1] - at : 0;
         }
-        m++;
-    });
-}
-
-__global__ void k_list_counts(Views V, int cur, int off, int n, int which, int *cnt)
-{
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        int id;
-        const int c = count_row(V, cur, off, which, k, id);
-        cnt[id] = c;
+        const bool lng = m > LIST_CAP;
+        if (lng || m == 0) e1 = e0;
+        int c = 0;
+        for (int e = e0; __any_sync(0xffffffffu, e < e1); e += GRP) {
+            int j = 0;
+            double v = 0.0;
+            const bool in = e + sub < e1 && list_entry(V, cur, which, e + sub, j, v);
+            const unsigned bal = __ballot_sync(0xffffffffu, in) & gmask;
+            if (in) {
+                const int q = c + __popc(bal & below);
+                bag_j[grp][q] = j;
+                bag_v[grp][q] = v;
+            }
+            c += __popc(bal);
+        }
+        __syncwarp();
+        for (int q = sub; q < c; q += GRP) {
+            const int j = bag_j[grp][q];
+            int r = at;
+            for (int k = 0; k < c; k++) r += bag_j[grp][k] < j;
+            if (r < cap) {
+                pi[r] = id;
+                pj[r] = j;
+                val[r] = bag_v[grp][q];
+            }
+        }
+        if (sub == 0) whole[grp] = lng ? b + grp : -1;
+        if (!__syncthreads_or(lng)) continue;
+        for (int g = 0; g < T / GRP; g++) {
+            if (whole[g] < 0) continue;
+            id = list_row(V, cur, off, which, whole[g], e0, e1);
+            at = base[id];
+            for (int e = e0; e < e1; e += T) {
+                int j = 0, r = at;
+                double v = 0.0;
+                const bool in = e + (int)threadIdx.x < e1 && list_entry(V, cur, which, e + threadIdx.x, j, v);
+                for (int t = e0; t < e1; t += T) {
+                    int tj = 0x7fffffff;
+                    double tv;
+                    if (t + (int)threadIdx.x < e1 && !list_entry(V, cur, which, t + threadIdx.x, tj, tv)) tj = 0x7fffffff;
+                    __syncthreads();
+                    tile[threadIdx.x] = tj;
+                    __syncthreads();
+                    if (in) {
+                        const int top = min(T, e1 - t);
+#pragma unroll 8
+                        for (int k = 0; k < top; k++) r += tile[k] < j;
+                    }
+                }
+                if (in && r < cap) {
+                    pi[r] = id;
+                    pj[r] = j;
+                    val[r] = v;
+                }
+            }
+        }
+        __syncthreads();          // (the rows' marks are read until here)
     }
 }
 
-__global__ void k_list_fill(Views V, int cur, int off, int n, int which, const int *base, int cap, int *pi, int *pj,
-                            double *val)
-{
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-        write_row(V, cur, off, which, k, base, cap, pi, pj, val);
-}
-
-// The whole list of a field of up to LIST_ONE_BLOCK floes by one block, the
-// counts in shared memory: one launch instead of six (count, three of the
-// scan, fill), which is what a list of a few thousand pairs costs.
-constexpr int LIST_ONE_BLOCK = 8192;
+// The whole list of a small field of short rows by one block, the counts in
+// shared memory: one launch instead of three (count, scan, fill).  A thread
+// takes a row and inserts up to LIST_SHORT pairs at their place; the block's
+// warps rank longer rows.  n floes, entries of all rows: bonds of 1,021 floes
+// 57 us a call against 78 by groups of lanes and 73 in three launches, of 4,096
+// 81 and 79.  Lists made from the neighbour rows end sooner, at half as many
+// floes or more than LIST_ONE_ROW entries a floe (4,096 floes, 23,000
+// candidates: 288 us, and 121 in three launches).
+constexpr int LIST_ONE_BLOCK = 4096, LIST_ONE_ROW = 8, LIST_SHORT = 16;
 __global__ void __launch_bounds__(1024) k_list_pairs(Views V, int cur, int off, int n, int which, int cap, int *pi,
                                                      int *pj, double *val, int *total)
 {
-    __shared__ int cnt[LIST_ONE_BLOCK];
+    __shared__ int cnt[LIST_ONE_BLOCK + 1];
     __shared__ int sums[32];
+    __shared__ int longs[LIST_ONE_BLOCK], nlong;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) nlong = 0;
     for (int k = tid; k < n; k += 1024) {
-        int id;
-        const int c = count_row(V, cur, off, which, k, id);
+        int e0, e1, c = 0;
+        const int id = list_row(V, cur, off, which, k, e0, e1);
+        for (int e = e0; e < e1; e++) {
+            int j;
+            double v;
+            c += list_entry(V, cur, which, e, j, v);
+        }
         cnt[id] = c;
     }
     __syncthreads();
@@ -160,15 +228,61 @@ __global__ void __launch_bounds__(1024) k_list_pairs(Views V, int cur, int off, 
     int before = 0;
     for (int w = 0; w < warp; w++) before += sums[w];
     int at = before + pre - own;
-    if (tid == 1023) *total = before + pre;
+    if (tid == 1023) *total = cnt[n] = before + pre;
     for (int k = k0; k < k1; k++) {
         const int c = cnt[k];
         cnt[k] = at;
         at += c;
     }
     __syncthreads();
-    if (cap > 0)
-        for (int k = tid; k < n; k += 1024) write_row(V, cur, off, which, k, cnt, cap, pi, pj, val);
+    if (cap <= 0) return;
+    for (int k = tid; k < n; k += 1024) {
+        int e0, e1;
+        const int id = list_row(V, cur, off, which, k, e0, e1);
+        const int a = cnt[id], m = cnt[id + 1] - a;
+        if (m == 0 || a >= cap) continue;
+        if (m > LIST_SHORT || a + m > cap) {
+            longs[atomicAdd(&nlong, 1)] = k;
+            continue;
+        }
+        int top = a;
+        for (int e = e0; e < e1; e++) {
+            int j;
+            double v;
+            if (!list_entry(V, cur, which, e, j, v)) continue;
+            int q = top++;
+            while (q > a && pj[q - 1] > j) {
+                pj[q] = pj[q - 1];
+                val[q] = val[q - 1];
+                q--;
+            }
+            pi[top - 1] = id;
+            pj[q] = j;
+            val[q] = v;
+        }
+    }
+    __syncthreads();
+    for (int w = warp; w < nlong; w += 32) {
+        int e0, e1;
+        const int id = list_row(V, cur, off, which, longs[w], e0, e1);
+        for (int e = e0; e < e1; e += 32) {
+            int j = 0, r = cnt[id];
+            double v = 0.0;
+            const bool in = e + lane < e1 && list_entry(V, cur, which, e + lane, j, v);
+            for (int t = e0; t < e1; t += 32) {
+                int tj = 0x7fffffff;
+                double tv;
+                if (t + lane < e1 && !list_entry(V, cur, which, t + lane, tj, tv)) tj = 0x7fffffff;
+#pragma unroll
+                for (int q = 0; q < 32; q++) r += __shfl_sync(0xffffffffu, tj, q) < j;
+            }
+            if (in && r < cap) {
+                pi[r] = id;
+                pj[r] = j;
+                val[r] = v;
+            }
+        }
+    }
 }
 
 // Per instance (one block each): total momentum (x, y), kinetic energy of
@@ -272,18 +386,20 @@ void launch_gather_fields(const Views &V, int cur, int off, int n, const FieldLi
     k_gather_fields<<<dim3(grid < 1024 ? grid : 1024, F.n), 256, 0, st>>>(V, cur, off, n, F, out);
 }
 
-void launch_list_pairs(const Views &V, int cur, int off, int n, int which, int cap, int *pi, int *pj, double *val,
-                       int *total, int *cnt, int *base, int *scan_scratch, cudaStream_t st)
+const int *launch_list_pairs(const Views &V, int cur, int off, int n, long long entries, int which, int cap, int *pi,
+                             int *pj, double *val, int *total, int *cnt, int *base, int *scan_scratch,
+                             cudaStream_t st)
 {
-    if (n <= LIST_ONE_BLOCK) {
+    if (which == 2 ? n <= LIST_ONE_BLOCK : n <= LIST_ONE_BLOCK / 2 && entries <= (long long)LIST_ONE_ROW * n) {
         k_list_pairs<<<1, 1024, 0, st>>>(V, cur, off, n, which, cap, pi, pj, val, total);
-        return;
+        return total;
     }
-    const int grid = (n + 127) / 128 < 2048 ? (n + 127) / 128 : 2048;
-    k_list_counts<<<grid, 128, 0, st>>>(V, cur, off, n, which, cnt);
+    const auto grid = [&](int per) { return (int)std::min<long long>(((long long)n + per - 1) / per, 148 * 16); };
+    k_list_counts<<<grid(256 / GRP), 256, 0, st>>>(V, cur, off, n, which, cnt);
     scan_excl(cnt, base, n, scan_scratch, st);
-    cudaMemcpyAsync(total, base + n, sizeof(int), cudaMemcpyDeviceToDevice, st);
-    if (cap > 0) k_list_fill<<<grid, 128, 0, st>>>(V, cur, off, n, which, base, cap, pi, pj, val);
+    if (cap > 0)
+        k_list_fill<<<grid(LIST_THREADS / GRP), LIST_THREADS, 0, st>>>(V, cur, off, n, which, base, cap, pi, pj, val);
+    return base + n;
 }
 
 }  // namespace godar

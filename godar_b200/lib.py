@@ -249,7 +249,7 @@ class Stepper:
             outs = {k: np.empty(self.n, dtype=np.float64) for k in names}
         ptrs = (ctypes.c_void_p * len(FLOE_FIELDS))()
         for k, a in outs.items():
-            ptrs[FIELD_ID[k]] = a.ctypes.data
+            ptrs[FIELD_ID[k]] = ctypes.addressof(ctypes.c_double.from_buffer(a))
         cnt = ctypes.c_int(0)
         L = load()
         if which < 0:

@@ -359,27 +359,43 @@ GD_DEV bool row_before(double da, int ida, double db, int idb, bool by_dist)
     return by_dist ? da < db || (da == db && ida < idb) : ida < idb;
 }
 
+// An entry of a row longer than a group keeps, before it is ranked.
+struct __align__(16) RowEntry {
+    double d;
+    int t, id;
+};
+
+static_assert(sizeof(RowEntry) <= sizeof(Hist4<float>), "raw owner rows lie where the histories go");
+
 // The rows of every floe: off2 is the scan of k_nbr_count's counts (partner
 // rows from off2[s], owner rows from off2[N + s] - off2[N]).  A group collects
-// its floe's entries in shared memory and places each by its rank; a floe with
-// more than ROW_CAP partners is written unordered and its rows sorted in
-// place by one lane (dist: their distances, owner rows).
-constexpr int ROW_CAP = 112;
-__global__ void __launch_bounds__(128) k_nbr_fill(Views V, int side, const int *coff, const int *off2, int up_by_id,
-                                                  int *lo_off, int *up_off, int2 *ent_lo, int2 *ent_up, double *dist)
+// its floe's entries in shared memory and places each by its rank.  The rows of
+// a floe with more than ROW_CAP partners are collected in global memory (lo_raw,
+// up_raw) and ranked by the whole block, a tile of entries in shared memory at
+// a time: one lane inserting the 3,272 entries of a large floe among small ones
+// took 480 ms, the block 3.
+constexpr int ROW_THREADS = 128, ROW_CAP = 112;
+__global__ void __launch_bounds__(ROW_THREADS) k_nbr_fill(Views V, int side, const int *coff, const int *off2,
+                                                          int up_by_id, int *lo_off, int *up_off, int2 *ent_lo,
+                                                          int2 *ent_up, int2 *lo_raw, RowEntry *up_raw)
 {
-    __shared__ GroupBag<ROW_CAP> bags[128 / GRP];
-    const int sub = threadIdx.x & (GRP - 1);
-    GroupBag<ROW_CAP> &B = bags[threadIdx.x / GRP];
-    const int groups = gridDim.x * (blockDim.x / GRP), N = V.N, P = off2[N];
-    for (int s0 = blockIdx.x * (blockDim.x / GRP) + (threadIdx.x & ~31) / GRP; s0 < N; s0 += groups) {
-        const int s = s0 + (threadIdx.x & 31) / GRP;
+    constexpr int T = ROW_THREADS;
+    __shared__ GroupBag<ROW_CAP> bags[T / GRP];
+    __shared__ int whole[T / GRP];                // floes for the whole block (-1: none)
+    __shared__ double tile_d[T];
+    __shared__ int tile_id[T];
+    const int sub = threadIdx.x & (GRP - 1), grp = threadIdx.x / GRP;
+    GroupBag<ROW_CAP> &B = bags[grp];
+    const int N = V.N, P = off2[N];
+    for (int b = blockIdx.x * (T / GRP); b < N; b += gridDim.x * (T / GRP)) {
+        const int s = b + grp;
         if (sub == 0) B.n[0] = B.n[1] = 0;
         __syncwarp();
         const bool on = s < N;
         const int ids = on ? V.id[side][s] : 0;
         const int lo = on ? off2[s] : 0, up = on ? off2[N + s] - P : 0;
         const int m = on ? off2[s + 1] - lo + (off2[N + s + 1] - P) - up : 0;
+        const bool lng = m > ROW_CAP;
         if (on && sub == 0) {
             lo_off[s] = lo;
             up_off[s] = up;
@@ -388,7 +404,7 @@ __global__ void __launch_bounds__(128) k_nbr_fill(Views V, int side, const int *
                 up_off[N] = P;
             }
         }
-        if (on && m <= ROW_CAP) {
+        if (on && !lng) {
             for_superset(V, side, coff, s, sub, [&](int t, double d, int idt) {
                 const int k = atomicAdd(&B.n[0], 1);
                 B.t[k] = t;
@@ -398,13 +414,17 @@ __global__ void __launch_bounds__(128) k_nbr_fill(Views V, int side, const int *
         } else if (on) {
             for_superset(V, side, coff, s, sub, [&](int t, double d, int idt) {
                 const int u = idt > ids, k = atomicAdd(&B.n[u], 1);
-                // .y holds the partner's id while the row is sorted
-                (u ? ent_up : ent_lo)[(u ? up : lo) + k] = make_int2(t, idt);
-                if (u) dist[up + k] = d;
+                if (u) {
+                    RowEntry e;
+                    e.d = d; e.t = t; e.id = idt;
+                    up_raw[up + k] = e;
+                } else {
+                    lo_raw[lo + k] = make_int2(t, idt);
+                }
             });
         }
         __syncwarp();
-        if (on && m <= ROW_CAP) {
+        if (on && !lng) {
             for (int k = sub; k < m; k += GRP) {
                 const int idk = B.id[k];
                 const double dk = B.d[k];
@@ -415,27 +435,44 @@ __global__ void __launch_bounds__(128) k_nbr_fill(Views V, int side, const int *
                 if (u) ent_up[up + at] = make_int2(B.t[k], up + at);      // the pair's index: its own place
                 else ent_lo[lo + at] = make_int2(B.t[k], -1);
             }
-        } else if (on && sub == 0) {
+        }
+        if (sub == 0) whole[grp] = lng ? s : -1;
+        if (!__syncthreads_or(lng)) continue;
+        for (int g = 0; g < T / GRP; g++) {
+            if (whole[g] < 0) continue;
+            const int lo_g = off2[whole[g]], up_g = off2[N + whole[g]] - P;
             for (int u = 0; u < 2; u++) {
-                int2 *e = u ? ent_up + up : ent_lo + lo;
-                double *d = dist + up;
-                const int n = B.n[u];
-                for (int a = 1; a < n; a++) {
-                    const int2 ea = e[a];
-                    const double da = u ? d[a] : 0.0;
-                    int b = a - 1;
-                    while (b >= 0 && row_before(da, ea.y, u ? d[b] : 0.0, e[b].y, u && !up_by_id)) {
-                        e[b + 1] = e[b];
-                        if (u) d[b + 1] = d[b];
-                        b--;
+                const int n = bags[g].n[u];
+                for (int c = 0; c < n; c += T) {
+                    const bool in = c + (int)threadIdx.x < n;
+                    RowEntry own;
+                    own.d = 0.0; own.t = own.id = 0;
+                    if (in && u) {
+                        own = up_raw[up_g + c + threadIdx.x];
+                    } else if (in) {
+                        const int2 e = lo_raw[lo_g + c + threadIdx.x];
+                        own.t = e.x; own.id = e.y;
                     }
-                    e[b + 1] = ea;
-                    if (u) d[b + 1] = da;
+                    int at = 0;
+                    for (int t0 = 0; t0 < n; t0 += T) {
+                        const int k = t0 + threadIdx.x;
+                        __syncthreads();
+                        if (k < n) {
+                            tile_d[threadIdx.x] = u ? up_raw[up_g + k].d : 0.0;
+                            tile_id[threadIdx.x] = u ? up_raw[up_g + k].id : lo_raw[lo_g + k].y;
+                        }
+                        __syncthreads();
+                        const int top = min(T, n - t0);
+#pragma unroll 4
+                        for (int j = 0; j < top; j++)
+                            at += row_before(tile_d[j], tile_id[j], own.d, own.id, u && !up_by_id);
+                    }
+                    if (in && u) ent_up[up_g + at] = make_int2(own.t, up_g + at);
+                    else if (in) ent_lo[lo_g + at] = make_int2(own.t, -1);
                 }
-                for (int a = 0; a < n; a++) e[a].y = u ? up + a : -1;
             }
         }
-        __syncwarp();
+        __syncthreads();          // (the bags and marks are read until here)
     }
 }
 
@@ -557,10 +594,10 @@ void launch_nbr_count(const Views &V, int side, const int *coff, int *cnt, int *
 }
 
 void launch_nbr_fill(const Views &V, int side, const int *coff, const int *off2, int up_by_id, int *lo_off,
-                     int *up_off, int2 *ent_lo, int2 *ent_up, double *dist, cudaStream_t st)
+                     int *up_off, int2 *ent_lo, int2 *ent_up, void *lo_raw, void *up_raw, cudaStream_t st)
 {
-    k_nbr_fill<<<grid_for((long long)V.N * GRP, 128), 128, 0, st>>>(V, side, coff, off2, up_by_id, lo_off, up_off,
-                                                                    ent_lo, ent_up, dist);
+    k_nbr_fill<<<grid_for((long long)V.N * GRP, ROW_THREADS), ROW_THREADS, 0, st>>>(
+        V, side, coff, off2, up_by_id, lo_off, up_off, ent_lo, ent_up, (int2 *)lo_raw, (RowEntry *)up_raw);
 }
 
 void launch_row_finish(const Views &V, int mixed, int side, const int *old_slot, const int *old_up_off,

@@ -1425,12 +1425,13 @@ struct Engine {
             Ecap = cap;
         }
         TRY(ens(up_off2, (size_t)(N + 1) * 4)); TRY(ens(lo_off2, (size_t)(N + 1) * 4));
-        // (two ints an entry also serve the contact list's marks and positions)
+        // (two ints an entry serve the raw partner rows, then the contact list's
+        // marks and positions; the histories' place the raw owner rows)
         TRY(ens(dist2, (size_t)(Ecap + 2) * 8));
         TRY(ens(ent_up2, (size_t)Ecap * 8)); TRY(ens(ent_lo2, (size_t)Ecap * 8));
         TRY(ens(bidx2, (size_t)Ecap * 4)); TRY(ens(hist2, (size_t)Ecap * he));
         launch_nbr_fill(V, nxt, coff_b.as<int>(), row_off2.as<int>(), fp64 ? 0 : 1, lo_off2.as<int>(),
-                        up_off2.as<int>(), ent_lo2.as<int2>(), ent_up2.as<int2>(), dist2.as<double>(), st);
+                        up_off2.as<int>(), ent_lo2.as<int2>(), ent_up2.as<int2>(), dist2.p, hist2.p, st);
         if (fp64 && NB > 0) {
             // the bonds' working order, which the pairs' bond indices count in
             TRY(ens(wdyn_b, (size_t)NB * sizeof(BondDyn))); TRY(ens(wgeo_b, (size_t)NB * sizeof(BondGeom64)));

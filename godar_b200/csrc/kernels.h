@@ -93,11 +93,11 @@ void launch_cell_list(const Views &V, int cur, int s0, int n, long long C, uint3
 void launch_cell_place(const Views &V, int cur, const uint32_t *keys, const int *coff, const int *list,
                        const int *repack, int *old_slot, cudaStream_t st);
 // The counts of every floe's partners (cnt: 2 N) and their scan (off2: 2 N + 1;
-// off2[N] pairs), then the rows.
+// off2[N] pairs), then the rows (lo_raw, up_raw: 8 and 16 bytes for every pair).
 void launch_nbr_count(const Views &V, int side, const int *coff, int *cnt, int *off2, int *scan_scratch,
                       cudaStream_t st);
 void launch_nbr_fill(const Views &V, int side, const int *coff, const int *off2, int up_by_id, int *lo_off,
-                     int *up_off, int2 *ent_lo, int2 *ent_up, double *dist, cudaStream_t st);
+                     int *up_off, int2 *ent_lo, int2 *ent_up, void *lo_raw, void *up_raw, cudaStream_t st);
 void launch_rows_ready(int *status, int *nwork, unsigned *dsp, cudaStream_t st);
 void launch_row_finish(const Views &V, int mixed, int side, const int *old_slot, const int *old_up_off,
                        const int2 *old_ent_up, const int *old_id, const void *old_hist, const int *up_off,

@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(const uint32_t *ke
 // ------------------------------------------------------------ exclusive scan
 // out[i] = sum_{k<i} in[i]; out[n] = total.  Three phases: per-block scan,
 // scan of block sums by one block, add.  n may be any int: a batch of sparse
-// fields has up to 2^31 - 1 cells, so a stride past the end is not an int.
+// fields has up to 2^31 - 1 cells, so an index past the end is not an int.
 constexpr int SC_THREADS = 512;
 constexpr int SC_ITEMS = 4;
 constexpr int SC_TILE = SC_THREADS * SC_ITEMS;
@@ -184,8 +184,9 @@ __global__ void __launch_bounds__(1024) k_scan_sums(int *tile_sums, int ntiles, 
 
 __global__ void k_scan_add(int *out, int n, const int *tile_sums, const int *total, int *out_n)
 {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        out[i] += tile_sums[i / SC_TILE];
+    // (an element a thread)
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < (unsigned)n) out[i] += tile_sums[i / SC_TILE];
     if (blockIdx.x == 0 && threadIdx.x == 0 && out_n) *out_n = *total;
 }
 

@@ -925,6 +925,56 @@ struct Engine {
         return P;
     }
 
+    // Uploads of a commit, in stream order: ranges of up to a quarter of a
+    // megabyte through the two pinned read-back slots (idle here), one filling
+    // while the other is copied, larger ones directly.  Ranges that follow one
+    // another on the device leave as one copy: thousands of small fields have
+    // eight arrays each, and every copy from pinned memory takes 1.4 us longer
+    // than a small one that the driver inlines.
+    struct Upload {
+        Engine &E;
+        char *dst = nullptr, *src = nullptr;      // the range being gathered
+        size_t len = 0, at = 0;                   // ... and the slot's end
+        int slot = 0;
+        bool used[2] = {false, false};
+
+        int put(void *to, const void *from, size_t nbytes) {
+            cudaStream_t st = E.st;
+            if (nbytes > 2 * STAGE_SLOT) {
+                TRY(flush());
+                CK(cudaMemcpyAsync(to, from, nbytes, cudaMemcpyHostToDevice, st));
+                return GODAR_OK;
+            }
+            const char *f = (const char *)from;
+            char *t = (char *)to;
+            while (nbytes > 0) {
+                if (len > 0 && t != dst + len) TRY(flush());
+                if (at == STAGE_SLOT) {
+                    TRY(flush());
+                    CK(cudaEventRecord(E.stage_ev[slot], st));
+                    used[slot] = true;
+                    slot ^= 1;
+                    if (used[slot]) CK(cudaEventSynchronize(E.stage_ev[slot]));
+                    at = 0;
+                }
+                if (len == 0) { dst = t; src = E.h_stage + slot * STAGE_SLOT + at; }
+                const size_t n = std::min(nbytes, STAGE_SLOT - at);
+                std::memcpy(src + len, f, n);
+                len += n; at += n; f += n; t += n; nbytes -= n;
+            }
+            return GODAR_OK;
+        }
+
+        // What is gathered so far leaves (before a kernel that reads it).
+        int flush() {
+            if (len == 0) return GODAR_OK;
+            CK(cudaMemcpyAsync(dst, src, len, cudaMemcpyHostToDevice, E.st));
+            len = 0;
+            at = std::min(STAGE_SLOT, (at + 15) & ~(size_t)15);
+            return GODAR_OK;
+        }
+    };
+
     int alloc_floe_set(FloeSet &f, int n) {
         const auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
         const size_t one = up((size_t)n * 8), snap = prec == GODAR_PREC_FP64 ? 0 : up((size_t)n * sizeof(Snap));
@@ -1113,23 +1163,8 @@ struct Engine {
         TRY(alloc_floe_set(*F, n_tot));
         TRY(alloc_scratch(n_tot));
         const int sn = 0;
-        // uploads of up to a quarter of a megabyte go through the pinned
-        // read-back slots (idle here), the larger ones directly
-        size_t staged = 0;
-        auto up = [&](void *dst, const void *src, size_t nbytes) -> int {
-            if (nbytes == 0) return GODAR_OK;
-            if (nbytes <= 2 * STAGE_SLOT) {
-                if (staged + nbytes > 2 * STAGE_SLOT) {
-                    CK(cudaStreamSynchronize(st));
-                    staged = 0;
-                }
-                std::memcpy(h_stage + staged, src, nbytes);
-                src = h_stage + staged;
-                staged += (nbytes + 15) & ~(size_t)15;
-            }
-            CK(cudaMemcpyAsync(dst, src, nbytes, cudaMemcpyHostToDevice, st));
-            return GODAR_OK;
-        };
+        Upload U{*this};
+        auto up = [&](void *dst, const void *src, size_t nbytes) { return U.put(dst, src, nbytes); };
         TRY(params_b.ensure(std::max<size_t>(hp.size(), 1) * sizeof(InstParams), &bytes, &mp));
         TRY(up(params_b.p, hp.data(), hp.size() * sizeof(InstParams)));
         hparams = hp;
@@ -1149,25 +1184,29 @@ struct Engine {
         RelayoutTable T;
         T.ni = ni;
         T.off = layout_b.as<int>(); T.old_off = T.off + ni; T.boff = T.off + 2 * ni; T.old_boff = T.off + 3 * ni;
+        TRY(U.flush());
         Views Vn = views();
         if (N > 0)
             launch_relayout_floes(oldF && oldN > 0 ? make_views(*oldF, *oldB) : Vn, old_cur, Vn, sn, T, inst_b.as<int>(),
                                   repack_b.as<int>(), N, st);
-        // admitted floes, host to device
+        // admitted floes, host to device, an array of every field after the other
+        const auto upload = [&](Piece &to, std::vector<double> Inst::*from) -> int {
+            for (const Inst &I : insts)
+                if (I.pending) TRY(up(to.as<double>() + I.off, (I.*from).data(), (size_t)I.n * 8));
+            return GODAR_OK;
+        };
+        TRY(upload(F->x[sn], &Inst::x)); TRY(upload(F->y[sn], &Inst::y)); TRY(upload(F->th[sn], &Inst::th));
+        TRY(upload(F->u[sn], &Inst::u)); TRY(upload(F->v[sn], &Inst::v)); TRY(upload(F->om[sn], &Inst::om));
+        TRY(upload(F->r[sn], &Inst::r)); TRY(upload(F->h[sn], &Inst::h));
         for (Inst &I : insts) {
-            if (!I.pending) continue;
+            if (!I.pending || !I.rx) continue;
             const size_t o = (size_t)I.off, nb8 = (size_t)I.n * 8;
-            TRY(up(F->x[sn].as<double>() + o, I.x.data(), nb8)); TRY(up(F->y[sn].as<double>() + o, I.y.data(), nb8));
-            TRY(up(F->th[sn].as<double>() + o, I.th.data(), nb8)); TRY(up(F->u[sn].as<double>() + o, I.u.data(), nb8));
-            TRY(up(F->v[sn].as<double>() + o, I.v.data(), nb8)); TRY(up(F->om[sn].as<double>() + o, I.om.data(), nb8));
-            TRY(up(F->r[sn].as<double>() + o, I.r.data(), nb8)); TRY(up(F->h[sn].as<double>() + o, I.h.data(), nb8));
-            if (I.rx) {
-                TRY(up(F->dtb1[sn].as<double>() + o, I.rx->dtb1.data(), nb8));
-                TRY(up(F->dtb2[sn].as<double>() + o, I.rx->dtb2.data(), nb8));
-                TRY(up(F->thb1[sn].as<double>() + o, I.rx->thb1.data(), nb8));
-                TRY(up(F->thb2[sn].as<double>() + o, I.rx->thb2.data(), nb8));
-            }
+            TRY(up(F->dtb1[sn].as<double>() + o, I.rx->dtb1.data(), nb8));
+            TRY(up(F->dtb2[sn].as<double>() + o, I.rx->dtb2.data(), nb8));
+            TRY(up(F->thb1[sn].as<double>() + o, I.rx->thb1.data(), nb8));
+            TRY(up(F->thb2[sn].as<double>() + o, I.rx->thb2.data(), nb8));
         }
+        TRY(U.flush());
         // bonds: the fresh fields' counts from the device, then every
         // field's place in the table (instances in layout order)
         if (std::any_of(gpu_bonds.begin(), gpu_bonds.end(), [](char c) { return c != 0; }))
@@ -1186,6 +1225,7 @@ struct Engine {
         if (oldB && oldN > 0) {
             for (int k = 0; k < ni; k++) tab[k] = insts[k].boff;
             TRY(up(layout_b.as<int>() + 2 * ni, tab.data(), (size_t)ni * 4));
+            TRY(U.flush());
             launch_relayout_bonds(oldB->bond_off.as<int>(), BS->bond_off.as<int>(), inst_b.as<int>(),
                                   oldB->bond_hi.as<int>(), oldB->bstat.as<BondStat>(), oldB->bdyn[0].as<BondDyn>(),
                                   BS->bond_hi.as<int>(), BS->bstat.as<BondStat>(), BS->bdyn[sn].as<BondDyn>(), T, N,
@@ -1193,21 +1233,18 @@ struct Engine {
         }
         if (std::any_of(gpu_bonds.begin(), gpu_bonds.end(), [](char c) { return c != 0; }))
             TRY(fill_fresh_bonds(first_pending, gpu_bonds));
-        for (int k = 0; k < ni; k++) {
-            Inst &I = insts[k];
-            if (!I.pending || gpu_bonds[k]) continue;
-            const HostBonds &B = bonds[k];
-            std::vector<int> off(I.n);
-            for (int i = 0; i < I.n; i++) off[i] = I.boff + (B.off.empty() ? 0 : B.off[i]);
-            TRY(up(BS->bond_off.as<int>() + I.off, off.data(), (size_t)I.n * 4));
-            if (I.nb == 0) continue;
-            std::vector<BondStat> hbs(I.nb);
-            std::vector<BondDyn> hbd(I.nb);
+        // the other admitted fields' bonds, likewise
+        const auto each = [&](auto part) -> int {
+            for (int k = 0; k < ni; k++)
+                if (insts[k].pending && !gpu_bonds[k]) TRY(part(insts[k], bonds[k]));
+            return GODAR_OK;
+        };
+        TRY(each([&](const Inst &I, const HostBonds &B) {
+            return up(BS->bond_hi.as<int>() + I.boff, B.hi.data(), (size_t)I.nb * 4);
+        }));
+        TRY(each([&](const Inst &I, const HostBonds &B) {
+            std::vector<BondStat> st_(I.nb);
             for (int q = 0; q < I.nb; q++) {
-                BondDyn bd{};
-                bd.dnb = B.dnb[q]; bd.dtb = B.dtb[q]; bd.thji = B.thji[q]; bd.thij = B.thij[q]; bd.dmg = B.dmg[q];
-                bd.flag = B.flag[q];
-                hbd[q] = bd;
                 BondStat bs{};
                 bs.rb = B.rb[q]; bs.hb = B.hb[q]; bs.lb = B.lb[q]; bs.sb = B.sb[q]; bs.ib = B.ib[q];
                 const double EA = I.prm.eb * bs.sb, EI = I.prm.eb * bs.ib, L = bs.lb;
@@ -1219,13 +1256,27 @@ struct Engine {
                 bs.ei_l = (float)(EI / L);
                 bs.ea_l = (float)(EA * L);
                 bs.inv_l = (float)(1.0 / L);
-                hbs[q] = bs;
+                st_[q] = bs;
             }
-            TRY(up(BS->bond_hi.as<int>() + I.boff, B.hi.data(), (size_t)I.nb * 4));
-            TRY(up(BS->bstat.as<BondStat>() + I.boff, hbs.data(), (size_t)I.nb * sizeof(BondStat)));
-            TRY(up(BS->bdyn[sn].as<BondDyn>() + I.boff, hbd.data(), (size_t)I.nb * sizeof(BondDyn)));
-        }
+            return up(BS->bstat.as<BondStat>() + I.boff, st_.data(), (size_t)I.nb * sizeof(BondStat));
+        }));
+        TRY(each([&](const Inst &I, const HostBonds &B) {
+            std::vector<BondDyn> dyn(I.nb);
+            for (int q = 0; q < I.nb; q++) {
+                BondDyn bd{};
+                bd.dnb = B.dnb[q]; bd.dtb = B.dtb[q]; bd.thji = B.thji[q]; bd.thij = B.thij[q]; bd.dmg = B.dmg[q];
+                bd.flag = B.flag[q];
+                dyn[q] = bd;
+            }
+            return up(BS->bdyn[sn].as<BondDyn>() + I.boff, dyn.data(), (size_t)I.nb * sizeof(BondDyn));
+        }));
+        TRY(each([&](const Inst &I, const HostBonds &B) {
+            std::vector<int> off(I.n);
+            for (int i = 0; i < I.n; i++) off[i] = I.boff + (B.off.empty() ? 0 : B.off[i]);
+            return up(BS->bond_off.as<int>() + I.off, off.data(), (size_t)I.n * 4);
+        }));
         TRY(up(BS->bond_off.as<int>() + N, &NB, sizeof(int)));
+        TRY(U.flush());
         CK(cudaStreamSynchronize(st));
         for (auto &I : insts) {
             if (I.pending) {

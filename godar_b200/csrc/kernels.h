@@ -40,27 +40,35 @@ bool release_kept();
 // refused.
 struct ClusterLimit { int blocks = -1; };
 
-// Launches a kernel of whole steps (k_steps_fp64, k_steps_mixed) as one block
-// for at most `alone` items, else as one cluster of enough blocks to give
-// every item a thread, at most SMALL_CLUSTER.  One block finds what it wrote
-// in its own L1 and its barrier takes 28 cycles; across blocks every phase
-// starts from L2 behind a barrier of 380, so a few items a thread cost less
-// than a second block: 256 free floes 5.7 against 8.3 us a step FP64, 4.2
-// against 6.9 mixed; 200 bonded ones mixed 8.6 (one block), 12.4 (two), 10.0
-// (four).  A cluster that is refused is asked for with eight blocks, and then
-// no more: false, with nothing launched.
-template <typename... Params, typename... Args>
-inline bool launch_cluster(ClusterLimit &most, bool pdl, void (*kern)(Params...), long long items, int alone,
-                           cudaStream_t st, Args... args)
+// The blocks of a kernel of whole steps (k_steps_fp64, k_steps_mixed): one, or
+// a cluster of enough blocks to give every item a thread, at most SMALL_CLUSTER.
+// One block finds what it wrote in its own L1 and its barrier takes 28 cycles;
+// across blocks every phase starts from L2 behind a barrier of 380, and that
+// costs less than another round of a block's threads over the pairs or the
+// floes.  Us a step, one block against a cluster: 256 free floes FP64 5.0 and
+// 7.5, mixed 4.2 and 6.5; 1,000 free mixed 11.0 and 6.5; 215 bonded FP64 (256
+// pairs) 14.4 and 14.9, 230: 19.7 and 16.0; 256 bonded mixed 9.6 and 10.3, 270:
+// 12.7 and 10.7.
+inline int cluster_blocks(long long items, bool one)
 {
-    if (items > alone && most.blocks < 0)
+    int blocks = 1;
+    while (!one && blocks < SMALL_CLUSTER && (long long)blocks * SMALL_THREADS < items) blocks *= 2;
+    return blocks;
+}
+
+// Launches it so.  A cluster that is refused is asked for with eight blocks,
+// and then no more: false, with nothing launched.
+template <typename... Params, typename... Args>
+inline bool launch_cluster(ClusterLimit &most, bool pdl, void (*kern)(Params...), int want, cudaStream_t st,
+                           Args... args)
+{
+    if (want > 1 && most.blocks < 0)
         most.blocks = cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
                               cudaSuccess
                           ? SMALL_CLUSTER
                           : 8;
-    while (items <= alone || most.blocks > 1) {
-        int blocks = 1;
-        while (items > alone && blocks < most.blocks && (long long)blocks * SMALL_THREADS < items) blocks *= 2;
+    while (want == 1 || most.blocks > 1) {
+        const int blocks = want == 1 || want < most.blocks ? want : most.blocks;
         cudaLaunchConfig_t c = {};
         c.gridDim = dim3((unsigned)blocks);
         c.blockDim = dim3(SMALL_THREADS);
@@ -140,11 +148,17 @@ void launch_fp64_bonds(const Views &V, int side, int *cnt, int *wfo, int *scan_s
 // shelter: some field of the batch has sheltering; drag: 8 N doubles; out:
 // pinned host memory for the status word and the first expired step; done: an
 // int that is zero): as one launch of one cluster up to ONE_CLUSTER_* items
-// (positions, bonds and floes; one block up to ONE_BLOCK_*), else, or where
-// the cluster is refused, as two to four launches a step.  Returns the kernels
+// (positions, bonds and floes; one block where one_block_* says so), else, or
+// where the cluster is refused, as two to four launches a step.  Returns the kernels
 // launched.
 constexpr int ONE_CLUSTER_FP64 = 1024, ONE_CLUSTER_MIXED = 4096;
-constexpr int ONE_BLOCK_FP64 = 640, ONE_BLOCK_MIXED = 1024;
+// (FP64: no thread has a second pair or a second floe; mixed, where a pair is
+// lighter: no second floe, or hardly a pair; see cluster_blocks)
+inline bool one_block_fp64(int N, int n) { return N <= SMALL_THREADS && n <= SMALL_THREADS; }
+inline bool one_block_mixed(int N, long long items)
+{
+    return items <= (N <= SMALL_THREADS ? 4 : 2) * SMALL_THREADS;
+}
 int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
                        const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
                        const int *up_n, double *drag, int *out, int *done, cudaStream_t st);

@@ -83,7 +83,7 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
     A.lo_n = lo_n; A.up_n = up_n; A.drag = drag; A.out = out; A.done = done;
     const long long items = (long long)n + V.N;
     if (!shelter && items <= ONE_CLUSTER_FP64 &&
-        launch_cluster(most, V.pdl != 0, k_steps_fp64, items, ONE_BLOCK_FP64, st, V, A))
+        launch_cluster(most, V.pdl != 0, k_steps_fp64, cluster_blocks(items, one_block_fp64(V.N, n)), st, V, A))
         return 1;
     const GroupSums how = group_sums(V.N, shelter);
     // the drag planes of floes out of sheltering fields, then the sums

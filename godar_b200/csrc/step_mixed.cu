@@ -1499,7 +1499,7 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
     A.done = done;
     const long long all = (long long)n + NB + V.N;
     if (!shelter && all <= ONE_CLUSTER_MIXED &&
-        launch_cluster(most, V.pdl != 0, k_steps_mixed, all, ONE_BLOCK_MIXED, st, V, A, B))
+        launch_cluster(most, V.pdl != 0, k_steps_mixed, cluster_blocks(all, one_block_mixed(V.N, all)), st, V, A, B))
         return 1;
     const GroupSums how = group_sums(V.N, shelter);
     const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;

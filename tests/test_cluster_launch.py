@@ -33,7 +33,7 @@ __global__ void k(int) {}
 static void go(ClusterLimit &m, long long items)
 {
     launched = 0;
-    const bool ok = launch_cluster(m, true, k, items, 1024, (cudaStream_t)0, 1);
+    const bool ok = launch_cluster(m, true, k, cluster_blocks(items, items <= 1024), (cudaStream_t)0, 1);
     std::printf("%lld:%d:%d:%d ", items, (int)ok, launched, refused);
 }
 int main()

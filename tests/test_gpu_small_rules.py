@@ -1,0 +1,40 @@
+"""The rules that choose a small batch's form, on either side of each line:
+one block or a cluster, the diagnostic step with its chunk or apart from it, the
+floes' sums by groups of lanes or by a thread each.  Every form gives the
+separate kernels' bits."""
+import numpy as np
+import pytest
+
+from godar_b200 import generators as gen
+from godar_b200.params import BC_OPEN_BOTTOM, BC_OPEN_LEFT, BC_OPEN_RIGHT, BC_OPEN_TOP, PREC_FP64, PREC_MIXED, make_params
+
+from .test_gpu_merged import _same
+
+pytestmark = pytest.mark.gpu
+
+OPEN = BC_OPEN_LEFT | BC_OPEN_RIGHT | BC_OPEN_BOTTOM | BC_OPEN_TOP
+
+
+def _free(n, rtree=200.0, sp=400.0, **kw):
+    """Floes on a jittered grid, out of touch."""
+    rng = np.random.default_rng(n)
+    m = int(np.ceil(np.sqrt(n)))
+    at = rng.permutation(m * m)[:n]
+    x = (at % m + 0.5) * sp + rng.uniform(-9.0, 9.0, n)
+    y = (at // m + 0.5) * sp + rng.uniform(-9.0, 9.0, n)
+    p = make_params(m * sp, m * sp, **{**dict(cohesion=0, shelter=0, ridging=0, dt=1e-2, rtree=rtree, ua=9.0, va=-4.0,
+                                              boundary=OPEN), **kw})
+    return gen.Field("free", p, x, y, rng.uniform(15.0, 20.0, n), rng.uniform(0.5, 2.0, n), 10,
+                     u=rng.uniform(-1.0, 1.0, n), v=rng.uniform(-1.0, 1.0, n))
+
+
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 512, 513, 1024, 1025])
+def test_one_block_of_free_floes(n, precision, monkeypatch):
+    _same(_free(n), precision, monkeypatch)
+
+
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("n", [200, 215, 230, 256, 257, 285])
+def test_one_block_of_bonded_floes(n, precision, monkeypatch):
+    _same(gen.bonded_field(n=n, seed=1), precision, monkeypatch)

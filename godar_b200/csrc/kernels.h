@@ -149,8 +149,8 @@ void launch_fp64_bonds(const Views &V, int side, int *cnt, int *wfo, int *scan_s
 // pinned host memory for the status word and the first expired step; done: an
 // int that is zero): as one launch of one cluster up to ONE_CLUSTER_* items
 // (positions, bonds and floes; one block where one_block_* says so), else, or
-// where the cluster is refused, as two to four launches a step.  Returns the kernels
-// launched.
+// where the cluster is refused and on large diagnostic steps (diag_apart), as
+// two to four launches a step.  Returns the kernels launched.
 constexpr int ONE_CLUSTER_FP64 = 1024, ONE_CLUSTER_MIXED = 4096;
 // (FP64: no thread has a second pair or a second floe; mixed, where a pair is
 // lighter: no second floe, or hardly a pair; see cluster_blocks)
@@ -162,6 +162,12 @@ inline bool one_block_mixed(int N, long long items)
 int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
                        const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
                        const int *up_n, double *drag, int *out, int *done, cudaStream_t st);
+// Whether a diagnostic step, which visits all E owner entries, leaves the launch
+// of its chunk: a cluster has few threads, and the two launches of a step as
+// many as there are entries.  A call of one such step: 400 floes with 5,214
+// entries FP64 105 and 89 us, 2,299: 72 and 69; 2,000 floes with 700,000
+// entries mixed 369 and 98, 1,000 with 13,000: 48 and 45.
+inline bool diag_apart(int E, int blocks) { return E > 4LL * blocks * SMALL_THREADS; }
 
 // How a plain step of the merged kernels sums the pairs of a floe: one thread
 // a floe; by groups of lanes in the update's kernel, up to one wave of its

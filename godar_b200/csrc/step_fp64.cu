@@ -82,18 +82,28 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
     A.n = n; A.E = E; A.plist = plist; A.erow = erow; A.pfl = pfl; A.rec = (PairRec64 *)rec;
     A.lo_n = lo_n; A.up_n = up_n; A.drag = drag; A.out = out; A.done = done;
     const long long items = (long long)n + V.N;
-    if (!shelter && items <= ONE_CLUSTER_FP64 &&
-        launch_cluster(most, V.pdl != 0, k_steps_fp64, cluster_blocks(items, one_block_fp64(V.N, n)), st, V, A))
-        return 1;
+    int kernels = 0, first = 0;
+    if (!shelter && items <= ONE_CLUSTER_FP64) {
+        const int blocks = cluster_blocks(items, one_block_fp64(V.N, n));
+        auto W = A;
+        if (diag_last && diag_apart(E, blocks)) {
+            W.K = K - 1;
+            W.diag_last = 0;
+        }
+        if (W.K > 0 && launch_cluster(most, V.pdl != 0, k_steps_fp64, blocks, st, V, W)) {
+            kernels = 1;
+            first = W.K;
+        }
+        if (first == K) return kernels;
+    }
     const GroupSums how = group_sums(V.N, shelter);
     // the drag planes of floes out of sheltering fields, then the sums
     double *fs = drag + 8 * (size_t)V.N;
-    int kernels = 0;
     const auto launch = [&](auto kern, int grid, int block, auto... args) {
         launch_step(V.pdl != 0, kern, grid, block, st, args...);
         kernels++;
     };
-    for (int k = 0; k < K; k++) {
+    for (int k = first; k < K; k++) {
         const int c = cur ^ (k & 1);
         const bool diag = diag_last && k == K - 1;
         const long long work = (long long)(diag ? E : n) + 32 + V.N;

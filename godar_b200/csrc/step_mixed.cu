@@ -1498,18 +1498,28 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
     A.out = out;
     A.done = done;
     const long long all = (long long)n + NB + V.N;
-    if (!shelter && all <= ONE_CLUSTER_MIXED &&
-        launch_cluster(most, V.pdl != 0, k_steps_mixed, cluster_blocks(all, one_block_mixed(V.N, all)), st, V, A, B))
-        return 1;
+    int kernels = 0, first = 0;
+    if (!shelter && all <= ONE_CLUSTER_MIXED) {
+        const int blocks = cluster_blocks(all, one_block_mixed(V.N, all));
+        auto W = A;
+        if (diag_last && diag_apart(E, blocks)) {
+            W.K = K - 1;
+            W.diag_last = 0;
+        }
+        if (W.K > 0 && launch_cluster(most, V.pdl != 0, k_steps_mixed, blocks, st, V, W, B)) {
+            kernels = 1;
+            first = W.K;
+        }
+        if (first == K) return kernels;
+    }
     const GroupSums how = group_sums(V.N, shelter);
     const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
     float4 *fs = B.fdg;   // (a plain step has no diagnostic sums)
-    int kernels = 0;
     const auto launch = [&](auto kern, int grid, int block, auto... args) {
         launch_step(V.pdl != 0, kern, grid, block, st, args...);
         kernels++;
     };
-    for (int k = 0; k < K; k++) {
+    for (int k = first; k < K; k++) {
         const int c = cur ^ (k & 1);
         const int diag = diag_last && k == K - 1;
         B.bfl_rd = A.bfl + (size_t)c * NB;

@@ -38,3 +38,11 @@ def test_one_block_of_free_floes(n, precision, monkeypatch):
 @pytest.mark.parametrize("n", [200, 215, 230, 256, 257, 285])
 def test_one_block_of_bonded_floes(n, precision, monkeypatch):
     _same(gen.bonded_field(n=n, seed=1), precision, monkeypatch)
+
+
+# every floe a candidate of every other: 990 and 1,035 entries for a block's
+# four rounds, and far more than a cluster's
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("n", [45, 46, 130, 300, 600])
+def test_diagnostic_steps_of_many_candidates(n, precision, monkeypatch):
+    _same(_free(n, rtree=50000.0, sp=60.0, cohesion=1, bond_lim_rel=0.7, dt=1e-3), precision, monkeypatch)

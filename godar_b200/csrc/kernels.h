@@ -150,7 +150,8 @@ void launch_fp64_bonds(const Views &V, int side, int *cnt, int *wfo, int *scan_s
 // int that is zero): as one launch of one cluster up to ONE_CLUSTER_* items
 // (positions, bonds and floes; one block where one_block_* says so), else, or
 // where the cluster is refused and on large diagnostic steps (diag_apart), as
-// two to four launches a step.  Returns the kernels launched.
+// two to four launches a step (one where no pair can act).  Returns the kernels
+// launched.
 constexpr int ONE_CLUSTER_FP64 = 1024, ONE_CLUSTER_MIXED = 4096;
 // (FP64: no thread has a second pair or a second floe; mixed, where a pair is
 // lighter: no second floe, or hardly a pair; see cluster_blocks)
@@ -172,11 +173,14 @@ inline bool diag_apart(int E, int blocks) { return E > 4LL * blocks * SMALL_THRE
 // How a plain step of the merged kernels sums the pairs of a floe: one thread
 // a floe; by groups of lanes in the update's kernel, up to one wave of its
 // blocks; by groups of lanes in a kernel of their own (sheltering fields, whose
-// every candidate has a record).
+// every candidate has a record).  rows: entries and bonds the sums walk; where
+// there is hardly one a floe, seven of a group's lanes only wait (6,000 free
+// floes FP64 9.5 us a step by groups and 8.3 by threads, mixed 8.1 and 7.8;
+// bonded 18.8 and 21.6, 12.9 and 13.5).
 enum GroupSums { SUMS_THREAD, SUMS_GROUP, SUMS_GROUP_APART };
-inline GroupSums group_sums(int N, int shelter)
+inline GroupSums group_sums(int N, int shelter, long long rows)
 {
-    if (N <= 148 * 2 * GRP_FLOES) return SUMS_GROUP;
+    if (N <= 148 * 2 * GRP_FLOES) return shelter || 4 * rows > N ? SUMS_GROUP : SUMS_THREAD;
     return shelter ? SUMS_GROUP_APART : SUMS_THREAD;
 }
 

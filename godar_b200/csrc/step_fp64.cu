@@ -96,7 +96,7 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
         }
         if (first == K) return kernels;
     }
-    const GroupSums how = group_sums(V.N, shelter);
+    const GroupSums how = group_sums(V.N, shelter, n);
     // the drag planes of floes out of sheltering fields, then the sums
     double *fs = drag + 8 * (size_t)V.N;
     const auto launch = [&](auto kern, int grid, int block, auto... args) {
@@ -109,9 +109,11 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
         const long long work = (long long)(diag ? E : n) + 32 + V.N;
         const int gp = fp64_grid(work, 128);
         const bool dense = work > 148 * 2 * 128;
+        // (nothing to visit: the update computes its drag itself)
+        A.drag = diag || n > 0 ? drag : nullptr;
         if (diag) launch(dense ? k_step_pairs_fp64<true, 4> : k_step_pairs_fp64<true, 2>, gp, 128, V, A, c);
         else if (shelter && n > SHEL_WAVE) launch(k_step_pairs_shel_fp64, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, A, c);
-        else launch(dense ? k_step_pairs_fp64<false, 4> : k_step_pairs_fp64<false, 2>, gp, 128, V, A, c);
+        else if (n > 0) launch(dense ? k_step_pairs_fp64<false, 4> : k_step_pairs_fp64<false, 2>, gp, 128, V, A, c);
         const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
         if (diag) {
             launch(walls ? k_step_floes_fp64<true, true> : k_step_floes_fp64<true, false>, fp64_grid(V.N, 64), 64, V, A, c, k);

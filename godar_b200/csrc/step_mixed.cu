@@ -1512,7 +1512,7 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
         }
         if (first == K) return kernels;
     }
-    const GroupSums how = group_sums(V.N, shelter);
+    const GroupSums how = group_sums(V.N, shelter, (long long)E + NB);
     const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
     float4 *fs = B.fdg;   // (a plain step has no diagnostic sums)
     const auto launch = [&](auto kern, int grid, int block, auto... args) {
@@ -1525,9 +1525,12 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
         B.bfl_rd = A.bfl + (size_t)c * NB;
         B.bfl_wr = A.bfl + (size_t)(c ^ 1) * NB;
         const long long items = (long long)(diag ? E : n) + (ridging ? 0 : NB) + 64 + V.N;
+        // (nothing to visit: the update computes its drag itself)
+        const bool pairs = diag || n > 0 || NB > 0;
+        A.drag = pairs ? B.fsum : nullptr;
         if (shelter && !diag && n > SHEL_WAVE)
             launch(k_step_pairs_shel_mixed, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, A, B, c);
-        else launch(items > 148 * 5 * 128 ? k_step_pairs_mixed<8> : k_step_pairs_mixed<5>, grid_of(items, 128),
+        else if (pairs) launch(items > 148 * 5 * 128 ? k_step_pairs_mixed<8> : k_step_pairs_mixed<5>, grid_of(items, 128),
                     128, V, A, B, c, diag);
         if (ridging && NB > 0)
             launch(k_bonds_mixed, grid_of(NB, 128), 128, V, c, diag, NB, B.bsp, B.bst, B.brec,

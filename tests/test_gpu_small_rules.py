@@ -46,3 +46,17 @@ def test_one_block_of_bonded_floes(n, precision, monkeypatch):
 @pytest.mark.parametrize("n", [45, 46, 130, 300, 600])
 def test_diagnostic_steps_of_many_candidates(n, precision, monkeypatch):
     _same(_free(n, rtree=50000.0, sp=60.0, cohesion=1, bond_lim_rel=0.7, dt=1e-3), precision, monkeypatch)
+
+
+# pairs in touch for fewer and for more than a quarter of the floes
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("n,pairs", [(4200, 0), (4200, 1), (5000, 1240), (5000, 1260), (9472, 40), (9473, 40)])
+def test_sums_of_few_pairs(n, pairs, precision, monkeypatch):
+    f = _free(n, rtree=60.0, cohesion=1, bond_lim=2.0, dt=1e-3)
+    # the last floes join earlier ones, near enough for a bond
+    for k in range(pairs):
+        i, j = k, n - 1 - k
+        a = 0.7 * k
+        f.x[j] = f.x[i] + np.cos(a) * (f.r[i] + f.r[j] + 0.5)
+        f.y[j] = f.y[i] + np.sin(a) * (f.r[i] + f.r[j] + 0.5)
+    _same(f, precision, monkeypatch)

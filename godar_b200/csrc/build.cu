@@ -378,7 +378,8 @@ static_assert(sizeof(RowEntry) <= sizeof(Hist4<float>), "raw owner rows lie wher
 constexpr int ROW_THREADS = 128, ROW_CAP = 112;
 __global__ void __launch_bounds__(ROW_THREADS) k_nbr_fill(Views V, int side, const int *coff, const int *off2,
                                                           int up_by_id, int *lo_off, int *up_off, int2 *ent_lo,
-                                                          int2 *ent_up, int2 *lo_raw, RowEntry *up_raw)
+                                                          int2 *ent_up, int2 *lo_raw, RowEntry *up_raw,
+                                                          int *row_max)
 {
     constexpr int T = ROW_THREADS;
     __shared__ GroupBag<ROW_CAP> bags[T / GRP];
@@ -397,6 +398,7 @@ __global__ void __launch_bounds__(ROW_THREADS) k_nbr_fill(Views V, int side, con
         const int lo = on ? off2[s] : 0, up = on ? off2[N + s] - P : 0;
         const int m = on ? off2[s + 1] - lo + (off2[N + s + 1] - P) - up : 0;
         const bool lng = m > ROW_CAP;
+        if (m > LONG_ROW && sub == 0) atomicMax(row_max, m);
         if (on && sub == 0) {
             lo_off[s] = lo;
             up_off[s] = up;
@@ -554,7 +556,7 @@ __global__ void k_copy_ids(Views V, int from)
 }
 
 // The state fresh rows start from: no error and no expiry, an empty work
-// list and, mixed, no displacement (the contact list holds the gaps at the
+// list (nwork's first two; the third is the next rebuild's longest row) and, mixed, no displacement (the contact list holds the gaps at the
 // rebuild).
 __global__ void k_rows_ready(int *status, int *nwork, unsigned *dsp)
 {
@@ -562,7 +564,7 @@ __global__ void k_rows_ready(int *status, int *nwork, unsigned *dsp)
         status[0] = 0;
         status[1] = 0x7fffffff;
     }
-    if (threadIdx.x < 2) nwork[threadIdx.x] = 0;
+    if (threadIdx.x < 3) nwork[threadIdx.x] = 0;
     if (threadIdx.x < 4) dsp[threadIdx.x] = 0;
 }
 
@@ -595,10 +597,11 @@ void launch_nbr_count(const Views &V, int side, const int *coff, int *cnt, int *
 }
 
 void launch_nbr_fill(const Views &V, int side, const int *coff, const int *off2, int up_by_id, int *lo_off,
-                     int *up_off, int2 *ent_lo, int2 *ent_up, void *lo_raw, void *up_raw, cudaStream_t st)
+                     int *up_off, int2 *ent_lo, int2 *ent_up, void *lo_raw, void *up_raw, int *row_max,
+                     cudaStream_t st)
 {
     k_nbr_fill<<<grid_for((long long)V.N * GRP, ROW_THREADS), ROW_THREADS, 0, st>>>(
-        V, side, coff, off2, up_by_id, lo_off, up_off, ent_lo, ent_up, (int2 *)lo_raw, (RowEntry *)up_raw);
+        V, side, coff, off2, up_by_id, lo_off, up_off, ent_lo, ent_up, (int2 *)lo_raw, (RowEntry *)up_raw, row_max);
 }
 
 void launch_row_finish(const Views &V, int mixed, int side, const int *old_slot, const int *old_up_off,

@@ -444,6 +444,7 @@ struct Engine {
     bool overlap_bonds = false;
     bool shelter_any = false;      // some field of the batch has sheltering
     bool walls_any = false;        // some field of the batch has a solid wall
+    bool rows_long = false;        // mixed: some floe has more than LONG_ROW partners
     // Batches of at most SMALL_FLOES_* floes run their steps as one to three
     // launches (launch_small): below these sizes the four kernels of a step
     // are mostly gaps and one thread's latency; above them the registers of
@@ -1481,8 +1482,12 @@ struct Engine {
         TRY(ens(dist2, (size_t)(Ecap + 2) * 8));
         TRY(ens(ent_up2, (size_t)Ecap * 8)); TRY(ens(ent_lo2, (size_t)Ecap * 8));
         TRY(ens(bidx2, (size_t)Ecap * 4)); TRY(ens(hist2, (size_t)Ecap * he));
+        if (!nwork_b.p) {
+            TRY(nwork_b.ensure(16, &bytes, &mp));
+            CK(cudaMemsetAsync(nwork_b.p, 0, 16, st));
+        }
         launch_nbr_fill(V, nxt, coff_b.as<int>(), row_off2.as<int>(), fp64 ? 0 : 1, lo_off2.as<int>(),
-                        up_off2.as<int>(), ent_lo2.as<int2>(), ent_up2.as<int2>(), dist2.p, hist2.p, st);
+                        up_off2.as<int>(), ent_lo2.as<int2>(), ent_up2.as<int2>(), dist2.p, hist2.p, nwork_b.as<int>() + 2, st);
         if (fp64 && NB > 0) {
             // the bonds' working order, which the pairs' bond indices count in
             TRY(ens(wdyn_b, (size_t)NB * sizeof(BondDyn))); TRY(ens(wgeo_b, (size_t)NB * sizeof(BondGeom64)));
@@ -1508,14 +1513,16 @@ struct Engine {
             E = Pn;
             TRY(fp64_rows(nxt));
         }
-        TRY(nwork_b.ensure(16, &bytes, &mp));
         // per-floe sums: the FP64 path's ordered record sums, the mixed path's window partials
         TRY(fsum_b.ensure((size_t)N * (fp64 ? 8 * FP64_FLOE_SUMS : 32), &bytes, &mp));
         if (!fp64) {
             TRY(frex_b.ensure((size_t)N * 4, &bytes, &mp));
             TRY(fdg_b.ensure((size_t)N * 32, &bytes, &mp));
             launch_pack_snap(V, nxt, st);
+            // (read once the contact list's length is)
+            CK(cudaMemcpyAsync(h_status + 3, nwork_b.as<int>() + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
             TRY(contact_list(nxt, Pn));
+            rows_long = Pn > 0 && h_status[3] > LONG_ROW;
             TRY(mixed_bond_lists(nxt));
         }
         E = Pn;
@@ -1695,7 +1702,7 @@ struct Engine {
             if (conc) CK(cudaStreamWaitEvent(st, ev_join, 0));
             else launch_bonds_mixed(V, side, diag, NB, B, cfg_block(bs[2]), cfg_variant(bs[2]), test_wait_spins, st);
             if (ev) TRY(record(ev[3], capturing));
-            if (shelter_any && !diag) launch_group_sums_mixed(V, B, st);
+            if (shelter_any && !diag) launch_group_sums_mixed(V, rows_long ? 1 : 0, B, st);
             else launch_floe_sums(V, diag, light, B, cfg_block(bs[3]), st);
             if (ev) TRY(record(ev[4], capturing));
             // (without a contact list only diagnostic steps would advance the bound)
@@ -1721,7 +1728,7 @@ struct Engine {
             return launch_steps_fp64(V, cluster, c0, K, diag_last, gbase, (int)Lc, (int)E, shelter_any ? 1 : 0, walls_any ? 1 : 0, fplist_b.as<int>(),
                                      erow_up.as<unsigned>(), pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
                                      fupn_b.as<int>(), fsum_b.as<double>(), out, step_base_b.as<int>() + 1, st);
-        return launch_steps_mixed(V, cluster, c0, K, diag_last, gbase, (int)Ec, (int)E, NB, shelter_any ? 1 : 0, walls_any ? 1 : 0, ridging_any ? 1 : 0,
+        return launch_steps_mixed(V, cluster, c0, K, diag_last, gbase, (int)Ec, (int)E, NB, rows_long ? 1 : 0, shelter_any ? 1 : 0, walls_any ? 1 : 0, ridging_any ? 1 : 0,
                                   clist_b.as<int2>(), clist_b.as<int2>() + Ecap, erow_up.as<unsigned>(),
                                   bflag_b.as<unsigned char>(), mixed_bufs(), out, step_base_b.as<int>() + 1, st);
     }

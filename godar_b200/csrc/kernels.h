@@ -101,11 +101,13 @@ void launch_cell_list(const Views &V, int cur, int s0, int n, long long C, uint3
 void launch_cell_place(const Views &V, int cur, const uint32_t *keys, const int *coff, const int *list,
                        const int *repack, int *old_slot, cudaStream_t st);
 // The counts of every floe's partners (cnt: 2 N) and their scan (off2: 2 N + 1;
-// off2[N] pairs), then the rows (lo_raw, up_raw: 8 and 16 bytes for every pair).
+// off2[N] pairs), then the rows (lo_raw, up_raw: 8 and 16 bytes for every pair;
+// row_max: raised to the partners of any floe with more than LONG_ROW).
+constexpr int LONG_ROW = 192;
 void launch_nbr_count(const Views &V, int side, const int *coff, int *cnt, int *off2, int *scan_scratch,
                       cudaStream_t st);
 void launch_nbr_fill(const Views &V, int side, const int *coff, const int *off2, int up_by_id, int *lo_off,
-                     int *up_off, int2 *ent_lo, int2 *ent_up, void *lo_raw, void *up_raw, cudaStream_t st);
+                     int *up_off, int2 *ent_lo, int2 *ent_up, void *lo_raw, void *up_raw, int *row_max, cudaStream_t st);
 void launch_rows_ready(int *status, int *nwork, unsigned *dsp, cudaStream_t st);
 void launch_row_finish(const Views &V, int mixed, int side, const int *old_slot, const int *old_up_off,
                        const int2 *old_ent_up, const int *old_id, const void *old_hist, const int *up_off,
@@ -225,7 +227,7 @@ void launch_pairs_diag(const Views &V, int cur, int P, const unsigned *erow_up, 
 // pair kernel advances the displacement bound in every step since the rebuild.
 void launch_floe_sums(const Views &V, int diag, int light, MixedBufs B, int block, cudaStream_t st);
 void launch_pairs_shel_mixed(const Views &V, int cur, int n, int2 *eb, const int2 *stl, MixedBufs B, cudaStream_t st);
-void launch_group_sums_mixed(const Views &V, MixedBufs B, cudaStream_t st);
+void launch_group_sums_mixed(const Views &V, int long_rows, MixedBufs B, cudaStream_t st);
 void launch_bonds_mixed(const Views &V, int cur, int diag, int NB, MixedBufs B, int block, int variant,
                         unsigned test_spins, cudaStream_t st);
 void launch_floes_mixed(const Views &V, int cur, int diag, int sic, int walls, int light, int bounded, MixedBufs B,
@@ -233,8 +235,8 @@ void launch_floes_mixed(const Views &V, int cur, int diag, int sic, int walls, i
 
 // The same on the mixed path (n contact-list items eb/stl, bfl: the live-bond
 // flags of both sides).
-int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
-                        int walls, int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
+int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int long_rows,
+                        int shelter, int walls, int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
                         int *done, cudaStream_t st);
 
 // Checkpoints: pair histories out and back in.

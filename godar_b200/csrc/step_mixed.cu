@@ -1170,6 +1170,11 @@ GD_DEV void small_pairs32(const Views &V, const SmallArgs32 &A, const MixedBufs 
 // the warp calls.
 GD_DEV float shfl_grp(float v, int src) { return __shfl_sync(0xffffffffu, v, src, GRP); }
 
+// SEEK: a batch with a row of more than LONG_ROW entries, whose flags are
+// searched 64 at a time to the next that is set: of a large floe's 3,272 entries
+// hardly one has a record (4,000 floes 73 -> 23 us a step; batches without such
+// a row lose 2 % to the search's code).
+template <bool SEEK>
 GD_DEV void group_sum32(const Views &V, const MixedBufs &B, bool on, int g, FloeSum32 &F)
 {
     const int lane = threadIdx.x & 31, sub = lane & (GRP - 1);
@@ -1184,6 +1189,17 @@ GD_DEV void group_sum32(const Views &V, const MixedBufs &B, bool on, int g, Floe
         const unsigned char *fl = side ? B.lfl : B.pfl;
         const int e0 = on ? off[g] : 0, e1 = on ? off[g + 1] : 0;
         for (int b = e0; __any_sync(0xffffffffu, b < e1); b += GRP) {
+            bool seek = SEEK && e1 - b > 8 * GRP;
+            while (SEEK && __any_sync(0xffffffffu, seek)) {
+                const int w = (b >> 3) + sub;
+                const bool set = seek && flag_word(fl, w, b, e1, 0x0a0a0a0a0a0a0a0aULL) != 0;
+                const unsigned bal = __ballot_sync(0xffffffffu, set) >> (lane & ~(GRP - 1)) & ((1u << GRP) - 1u);
+                if (seek) {
+                    const int at = ((b >> 3) + (bal ? __ffs(bal) - 1 : GRP)) << 3;
+                    b = at > b ? at : b;
+                    seek = !bal && e1 - b > 8 * GRP;
+                }
+            }
             const int e = b + sub;
             unsigned f = e < e1 ? fl[e] : 0u;
             int p = e;
@@ -1395,6 +1411,7 @@ __global__ void __launch_bounds__(128, WALLS ? 3 : 6) k_step_floes_mixed(Views V
 
 // The second half of a plain step with the floes' sums by groups of lanes
 // (k_step_floes_grp_fp64).
+template <bool SEEK>
 __global__ void __launch_bounds__(SMALL_THREADS, 2) k_step_floes_grp_mixed(Views V, SmallArgs32 A, MixedBufs B,
                                                                            int cur, int sic)
 {
@@ -1409,7 +1426,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) k_step_floes_grp_mixed(Views
     for (int g0 = blockIdx.x * GRP_FLOES; !stopped && g0 < V.N; g0 += gridDim.x * GRP_FLOES) {
         const bool on = g0 + grp < V.N;
         FloeSum32 F;
-        group_sum32(V, B, on, g0 + grp, F);
+        group_sum32<SEEK>(V, B, on, g0 + grp, F);
         if (on && threadIdx.x % GRP == 0) {
             sum[0][grp] = F.fcx; sum[1][grp] = F.fcy; sum[2][grp] = F.mc;
             sum[3][grp] = F.fbx; sum[4][grp] = F.fby; sum[5][grp] = F.mb;
@@ -1432,6 +1449,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) k_step_floes_grp_mixed(Views
 
 // The sums as a kernel of their own (k_group_sums_fp64), two float4 a floe in
 // fs: 65,536 sheltering floes 112 -> 84 us a step.
+template <bool SEEK>
 __global__ void __launch_bounds__(SMALL_THREADS, 8) k_group_sums_mixed(Views V, MixedBufs B, float4 *fs)
 {
     step_kernel_entry();
@@ -1441,7 +1459,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 8) k_group_sums_mixed(Views V, 
         const int g = g0 + grp;
         const bool on = g < V.N;
         FloeSum32 F;
-        group_sum32(V, B, on, g, F);
+        group_sum32<SEEK>(V, B, on, g, F);
         if (on && threadIdx.x % GRP == 0) {
             fs[2 * (size_t)g] = make_float4(F.fcx, F.fcy, F.mc, F.fbx);
             fs[2 * (size_t)g + 1] = make_float4(F.fby, F.mb, F.sca, F.scw);
@@ -1481,13 +1499,13 @@ void launch_pairs_shel_mixed(const Views &V, int cur, int n, int2 *eb, const int
     if (n > 0) launch_step(V.pdl != 0, k_step_pairs_shel_mixed, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, B, cur);
 }
 
-void launch_group_sums_mixed(const Views &V, MixedBufs B, cudaStream_t st)
+void launch_group_sums_mixed(const Views &V, int long_rows, MixedBufs B, cudaStream_t st)
 {
-    launch_step(V.pdl != 0, k_group_sums_mixed, (V.N + GRP_FLOES - 1) / GRP_FLOES, SMALL_THREADS, st, V, B, B.fsum);
+    launch_step(V.pdl != 0, long_rows ? k_group_sums_mixed<true> : k_group_sums_mixed<false>, (V.N + GRP_FLOES - 1) / GRP_FLOES, SMALL_THREADS, st, V, B, B.fsum);
 }
 
-int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int shelter,
-                        int walls, int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
+int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int long_rows,
+                        int shelter, int walls, int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
                         int *done, cudaStream_t st)
 {
     SmallArgs32 A;
@@ -1540,9 +1558,9 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
         } else if (how == SUMS_THREAD) {
             launch(walls ? k_step_floes_mixed<false, true> : k_step_floes_mixed<false, false>, grid_of(V.N, 64), 64, V, A, B, c, k);
         } else if (how == SUMS_GROUP) {
-            launch(k_step_floes_grp_mixed, groups, SMALL_THREADS, V, A, B, c, k);
+            launch(long_rows ? k_step_floes_grp_mixed<true> : k_step_floes_grp_mixed<false>, groups, SMALL_THREADS, V, A, B, c, k);
         } else {
-            launch(k_group_sums_mixed, groups, SMALL_THREADS, V, B, fs);
+            launch(long_rows ? k_group_sums_mixed<true> : k_group_sums_mixed<false>, groups, SMALL_THREADS, V, B, fs);
             launch(walls ? k_step_update_mixed<true> : k_step_update_mixed<false>, grid_of(V.N, 64), 64, V, A, B, c, k, fs);
         }
     }

@@ -8,6 +8,7 @@ import pytest
 from godar_b200 import generators as gen
 from godar_b200.params import BC_OPEN_BOTTOM, BC_OPEN_LEFT, BC_OPEN_RIGHT, BC_OPEN_TOP, PREC_FP64, PREC_MIXED, make_params
 
+from .test_gpu_long_rows import _packed, _ring
 from .test_gpu_merged import _same
 
 pytestmark = pytest.mark.gpu
@@ -60,3 +61,22 @@ def test_sums_of_few_pairs(n, pairs, precision, monkeypatch):
         f.x[j] = f.x[i] + np.cos(a) * (f.r[i] + f.r[j] + 0.5)
         f.y[j] = f.y[i] + np.sin(a) * (f.r[i] + f.r[j] + 0.5)
     _same(f, precision, monkeypatch)
+
+
+# rows of hundreds of entries of which few, or all, add to a floe's sums
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("shelter", [0, 1])
+def test_sums_along_long_rows(shelter, precision, monkeypatch):
+    fields = [_packed(300), _ring(200, 0), _ring(200, 100), _ring(1500, 700)]
+    # one small floe in five touches the large one
+    k = fields[3]
+    big = int(np.argmax(k.r))
+    dx, dy = k.x - k.x[big], k.y - k.y[big]
+    d = np.hypot(dx, dy)
+    d[big] = 1.0
+    to = np.where(np.arange(k.n) % 5 == 0, k.r[big] + k.r - 0.01, d)
+    to[big] = 0.0
+    k.x, k.y = k.x[big] + dx / d * to, k.y[big] + dy / d * to
+    for f in fields:
+        f.params.shelter = f.params.ridging = shelter
+        _same(f, precision, monkeypatch)

@@ -172,6 +172,13 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
 // entries mixed 369 and 98, 1,000 with 13,000: 48 and 45.
 inline bool diag_apart(int E, int blocks) { return E > 4LL * blocks * SMALL_THREADS; }
 
+// Whether a diagnostic step of the merged kernels sums its floes in a kernel of
+// their own: the rows of every candidate are long, and the sums wait for them
+// with the update's registers otherwise.  Sums and update, merged and apart, of
+// 70,000 floes of many sizes: 189 and 130 us FP64, 139 and 85 mixed; of 20,000
+// no difference (a call 160 and 162, 132 and 134 us).
+inline bool diag_sums_apart(int N) { return N > 32 * 1024; }
+
 // How a plain step of the merged kernels sums the pairs of a floe: one thread
 // a floe; by groups of lanes in the update's kernel, up to one wave of its
 // blocks; by groups of lanes in a kernel of their own (sheltering fields, whose

@@ -110,12 +110,19 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
         const int gp = fp64_grid(work, 128);
         const bool dense = work > 148 * 2 * 128;
         // (nothing to visit: the update computes its drag itself)
-        A.drag = diag || n > 0 ? drag : nullptr;
+        const bool apart = diag && diag_sums_apart(V.N);
+        A.drag = !apart && (diag || n > 0) ? drag : nullptr;
         if (diag) launch(dense ? k_step_pairs_fp64<true, 4> : k_step_pairs_fp64<true, 2>, gp, 128, V, A, c);
         else if (shelter && n > SHEL_WAVE) launch(k_step_pairs_shel_fp64, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, A, c);
         else if (n > 0) launch(dense ? k_step_pairs_fp64<false, 4> : k_step_pairs_fp64<false, 2>, gp, 128, V, A, c);
         const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
-        if (diag) {
+        if (apart) {
+            // (every plane of the sums: the drag is the update's)
+            launch(k_row_sums_fp64<true, false>, fp64_grid(V.N, 128), 128, V, c, (const unsigned char *)pfl,
+                   (const PairRec64 *)A.rec, lo_n, up_n, drag);
+            launch(walls ? k_step_update_fp64<true, true> : k_step_update_fp64<true, false>, fp64_grid(V.N, 64), 64, V,
+                   A, c, k, (const double *)drag);
+        } else if (diag) {
             launch(walls ? k_step_floes_fp64<true, true> : k_step_floes_fp64<true, false>, fp64_grid(V.N, 64), 64, V, A, c, k);
         } else if (how == SUMS_THREAD) {
             launch(walls ? k_step_floes_fp64<false, true> : k_step_floes_fp64<false, false>, fp64_grid(V.N, 64), 64, V, A, c, k);
@@ -123,7 +130,7 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
             launch(k_step_floes_grp_fp64, groups, SMALL_THREADS, V, A, c, k);
         } else {
             launch(k_group_sums_fp64, groups, SMALL_THREADS, V, c, pfl, A.rec, lo_n, up_n, fs);
-            launch(walls ? k_step_update_fp64<true> : k_step_update_fp64<false>, fp64_grid(V.N, 64), 64, V, A, c, k, fs);
+            launch(walls ? k_step_update_fp64<false, true> : k_step_update_fp64<false, false>, fp64_grid(V.N, 64), 64, V, A, c, k, fs);
         }
     }
     return kernels;

@@ -876,8 +876,9 @@ GD_DEV void small_pairs64(const Views &V, const SmallArgs64 &A, int cur)
     const int nthr = gridDim.x * blockDim.x;
     const int n = DIAG ? A.E : A.n;
     const int n0 = (n + 31) & ~31;      // the floes start on a warp of their own
+    const int end = n0 + (A.drag ? V.N : 0);
     Counts64 C = {0, 0, 0, 0};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n0 + V.N; i += nthr) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < end; i += nthr) {
         if (i < n) {
             pair_entry64<DIAG>(V, cur, DIAG ? i : A.plist[i], A.erow, A.pfl, A.rec, C);
         } else if (i >= n0) {
@@ -1092,12 +1093,14 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4) k_group_sums_fp64(Views V, i
     }
 }
 
-// ... and the update from them, as the last kernel of a small batch's step.
-template <bool WALLS>
+// ... and the update from them, as the last kernel of a small batch's step; on
+// a diagnostic step from k_row_sums_fp64's.
+template <bool DIAG, bool WALLS>
 __global__ void __launch_bounds__(64) k_step_update_fp64(Views V, SmallArgs64 A, int cur, int sic, const double *fs)
 {
     step_kernel_entry();
     const size_t N = (size_t)V.N;
+    Counts64 C = {0, 0, 0, 0};
     if (!floe_update_stopped(V, A.base, sic))
         for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < V.N; g += gridDim.x * blockDim.x) {
             const InstParams &P = V.P[V.inst[g]];
@@ -1105,9 +1108,18 @@ __global__ void __launch_bounds__(64) k_step_update_fp64(Views V, SmallArgs64 A,
             S.fcx = fs[FS64_FCX * N + g]; S.fcy = fs[FS64_FCY * N + g]; S.mc = fs[FS64_MC * N + g];
             S.fbx = fs[FS64_FBX * N + g]; S.fby = fs[FS64_FBY * N + g]; S.mb = fs[FS64_MB * N + g];
             S.hsfa = fs[FS64_HSFA * N + g]; S.hsfw = fs[FS64_HSFW * N + g];
+            if (DIAG) {
+                S.tac = fs[FS64_TAC * N + g]; S.pc = fs[FS64_PC * N + g];
+                S.tab = fs[FS64_TAB * N + g]; S.pb = fs[FS64_PB * N + g];
+                S.sxx = fs[FS64_SXX * N + g]; S.syy = fs[FS64_SYY * N + g];
+                S.sxy = fs[FS64_SXY * N + g]; S.syx = fs[FS64_SYX * N + g];
+            }
             const Shape run = make_shape(P, fs[FS64_R * N + g], fs[FS64_H * N + g]);
-            floe_update64<false, WALLS>(V, cur, A.base, sic, g, P, S, run, P.shelter != 0 ? nullptr : A.drag);
+            C.plast += floe_update64<DIAG, WALLS>(V, cur, A.base, sic, g, P, S, run,
+                                                  P.shelter != 0 ? nullptr : A.drag);
         }
+    __syncwarp();
+    if (DIAG) add_counts(C, V.counters);
     if (sic == A.K - 1) publish_status_last(V, A.done, A.out);
 }
 

@@ -1129,7 +1129,8 @@ GD_DEV void small_pairs32(const Views &V, const SmallArgs32 &A, const MixedBufs 
     const int n0 = (n + 31) & ~31;
     const int n1 = n0 + (A.ridging ? 0 : (A.NB + 31) & ~31);
     unsigned long long n_cand = 0, n_cont = 0, n_plast = 0, n_bond = 0;
-    for (int i = first; i < n1 + V.N; i += nthr) {
+    const int end = n1 + (A.drag ? V.N : 0);
+    for (int i = first; i < end; i += nthr) {
         if (i < n) {
             int e = i, s, t;
             if (diag) {
@@ -1468,8 +1469,9 @@ __global__ void __launch_bounds__(SMALL_THREADS, 8) k_group_sums_mixed(Views V, 
     }
 }
 
-// ... and the update from them, as the last kernel of a small batch's step.
-template <bool WALLS>
+// ... and the update from them, as the last kernel of a small batch's step; on
+// a diagnostic step from k_floe_sums'.
+template <bool DIAG, bool WALLS>
 __global__ void __launch_bounds__(128, WALLS ? 4 : 6) k_step_update_mixed(Views V, SmallArgs32 A, MixedBufs B, int cur, int sic,
                                                            const float4 *fs)
 {
@@ -1482,8 +1484,13 @@ __global__ void __launch_bounds__(128, WALLS ? 4 : 6) k_step_update_mixed(Views 
             F.fcx = s0.x; F.fcy = s0.y; F.mc = s0.z; F.fbx = s0.w; F.fby = s1.x; F.mb = s1.y;
             F.sca = s1.z; F.scw = s1.w;
             F.rex = B.frex[g];
+            if (DIAG) {
+                const float4 d0 = B.fdg[2 * (size_t)g], d1 = B.fdg[2 * (size_t)g + 1];
+                F.tac = d0.x; F.pc = d0.y; F.tab = d0.z; F.pb = d0.w;
+                F.sxx = d1.x; F.syy = d1.y; F.sxy = d1.z; F.syx = d1.w;
+            }
             const bool shel = V.P[V.inst[g]].shelter != 0;
-            dmx = max(dmx, floe_update<false, WALLS>(V, cur, A.base, sic, g, F, shel ? nullptr : A.drag));
+            dmx = max(dmx, floe_update<DIAG, WALLS>(V, cur, A.base, sic, g, F, shel ? nullptr : A.drag));
         }
         __syncwarp();
         raise_step(dmx, B.dsp + cur);
@@ -1545,7 +1552,8 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
         const long long items = (long long)(diag ? E : n) + (ridging ? 0 : NB) + 64 + V.N;
         // (nothing to visit: the update computes its drag itself)
         const bool pairs = diag || n > 0 || NB > 0;
-        A.drag = pairs ? B.fsum : nullptr;
+        const bool apart = diag && diag_sums_apart(V.N);
+        A.drag = pairs && !apart ? B.fsum : nullptr;
         if (shelter && !diag && n > SHEL_WAVE)
             launch(k_step_pairs_shel_mixed, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, A, B, c);
         else if (pairs) launch(items > 148 * 5 * 128 ? k_step_pairs_mixed<8> : k_step_pairs_mixed<5>, grid_of(items, 128),
@@ -1553,7 +1561,11 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
         if (ridging && NB > 0)
             launch(k_bonds_mixed, grid_of(NB, 128), 128, V, c, diag, NB, B.bsp, B.bst, B.brec,
                         B.bdg, B.bfl_wr, B.wdyn);
-        if (diag) {
+        if (apart) {
+            launch(k_floe_sums<true, false>, grid_of(V.N, 128), 128, V, B);
+            launch(walls ? k_step_update_mixed<true, true> : k_step_update_mixed<true, false>, grid_of(V.N, 64), 64, V,
+                   A, B, c, k, (const float4 *)B.fsum);
+        } else if (diag) {
             launch(walls ? k_step_floes_mixed<true, true> : k_step_floes_mixed<true, false>, grid_of(V.N, 64), 64, V, A, B, c, k);
         } else if (how == SUMS_THREAD) {
             launch(walls ? k_step_floes_mixed<false, true> : k_step_floes_mixed<false, false>, grid_of(V.N, 64), 64, V, A, B, c, k);
@@ -1561,7 +1573,7 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
             launch(long_rows ? k_step_floes_grp_mixed<true> : k_step_floes_grp_mixed<false>, groups, SMALL_THREADS, V, A, B, c, k);
         } else {
             launch(long_rows ? k_group_sums_mixed<true> : k_group_sums_mixed<false>, groups, SMALL_THREADS, V, B, fs);
-            launch(walls ? k_step_update_mixed<true> : k_step_update_mixed<false>, grid_of(V.N, 64), 64, V, A, B, c, k, fs);
+            launch(walls ? k_step_update_mixed<false, true> : k_step_update_mixed<false, false>, grid_of(V.N, 64), 64, V, A, B, c, k, (const float4 *)fs);
         }
     }
     return kernels;

@@ -51,6 +51,14 @@ def test_merged_steps_of_sheltering_fields(precision, monkeypatch):
     assert got == [4 * (3 + bonds), 3 * (3 + bonds) + 2 + bonds]
 
 
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
+def test_diagnostic_steps_of_larger_merged_batches(precision, monkeypatch):
+    # the sums of a diagnostic step in a kernel of their own beyond 32,768 floes
+    for n, diag in ((32768, 2), (32769, 3)):
+        f = gen.bonded_field(n=n, seed=2, device="gpu")
+        assert _launched(f, precision, [(4, False, False), (4, True, False)], monkeypatch) == [8, 6 + diag]
+
+
 def test_separate_kernels(monkeypatch):
     calls = [(4, False, False), (4, True, False)]
     bonded = gen.bonded_field(n=3000, seed=2)

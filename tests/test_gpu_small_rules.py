@@ -80,3 +80,18 @@ def test_sums_along_long_rows(shelter, precision, monkeypatch):
     for f in fields:
         f.params.shelter = f.params.ridging = shelter
         _same(f, precision, monkeypatch)
+
+
+# diagnostic steps with the sums in the update's kernel and apart
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("n", [32768, 32769])
+@pytest.mark.parametrize("kind", ["bonded", "poly", "walls"])
+def test_diagnostic_sums(kind, n, precision, monkeypatch):
+    if kind == "poly":
+        f = gen.polydisperse_field(n=n, seed=2, phi=0.6, dt=1e-3)
+    else:
+        f = gen.bonded_field(n=n, seed=2, device="gpu")
+        f.params.ridging = 1
+        if kind == "walls":
+            f.params.boundary = 0
+    _same(f, precision, monkeypatch)

@@ -183,7 +183,7 @@ struct Views {
 
 #define GD_DEV __device__ __forceinline__
 
-// the FP64 pair work list: contacts, and candidates of sheltering fields
+// the FP64 pair work list: contacts
 struct __align__(32) FP64Item {
     int p, g, t, bi;     // pair index, owner slot, partner slot, bond index
     double dx, dy;       // the pair's minimum-image offset x_g - x_t, y_g - y_t

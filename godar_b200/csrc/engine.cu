@@ -1654,15 +1654,18 @@ struct Engine {
             L.n = nwork_b.as<int>();
             // a plain step visits the pairs that can act before the next
             // rebuild; a diagnostic step every owner entry
-            if (shelter_any && !diag) {
+            if (diag) {
+                launch_pairs_diag_fp64(V, side, (int)E, erow_up.as<unsigned>(), pfl.as<unsigned char>(), frec_b.p, st);
+                if (ev) TRY(record(ev[1], capturing));
+            } else if (shelter_any) {
                 launch_pairs_shel_fp64(V, side, (int)Lc, fplist_b.as<int>(), erow_up.as<unsigned>(),
                                        pfl.as<unsigned char>(), frec_b.p, st);
                 if (ev) TRY(record(ev[1], capturing));
             } else {
-                launch_pairs_fp64(V, side, diag, diag ? (int)E : (int)Lc, diag ? nullptr : fplist_b.as<int>(),
-                                  erow_up.as<unsigned>(), pfl.as<unsigned char>(), L, frec_b.p, cfg_block(bs[0]), st);
+                launch_pairs_fp64(V, side, (int)Lc, fplist_b.as<int>(), erow_up.as<unsigned>(),
+                                  pfl.as<unsigned char>(), L, frec_b.p, cfg_block(bs[0]), st);
                 if (ev) TRY(record(ev[1], capturing));
-                launch_pairs_list_fp64(V, side, diag, (int)E, pfl.as<unsigned char>(), L, frec_b.p, cfg_block(bs[1]), st);
+                launch_pairs_list_fp64(V, side, (int)Lc, pfl.as<unsigned char>(), L, frec_b.p, cfg_block(bs[1]), st);
             }
             // (the third phase has no kernel of its own)
             if (ev) TRY(record(ev[2], capturing));
@@ -1741,7 +1744,7 @@ struct Engine {
 
     // The separate kernels of a plain or of a diagnostic step (launch_one).
     int step_kernels(bool diag) const {
-        if (prec == GODAR_PREC_FP64) return shelter_any && !diag ? (Lc > 0) + 2 : 4;
+        if (prec == GODAR_PREC_FP64) return diag ? (E > 0) + 2 : shelter_any ? (Lc > 0) + 2 : 4;
         return (diag ? (E > 0 ? 2 : 0) : (Ec > 0)) + (NB > 0) + 2;
     }
 

@@ -122,10 +122,13 @@ void launch_row_finish(const Views &V, int mixed, int side, const int *old_slot,
 // (c)-(e) walls, forcing and the FP64 update (which also clears the work list).
 constexpr int FP64_PAIR_REC_BYTES = 160;
 constexpr int FP64_FLOE_SUMS = 18;
-void launch_pairs_fp64(const Views &V, int cur, int diag, int n, const int *plist, const unsigned *erow,
-                       unsigned char *pfl, FP64List L, void *rec, int block, cudaStream_t st);
-void launch_pairs_list_fp64(const Views &V, int cur, int diag, int E, unsigned char *pfl, FP64List L, void *rec,
-                            int block, cudaStream_t st);
+void launch_pairs_fp64(const Views &V, int cur, int n, const int *plist, const unsigned *erow, unsigned char *pfl,
+                       FP64List L, void *rec, int block, cudaStream_t st);
+void launch_pairs_list_fp64(const Views &V, int cur, int n, unsigned char *pfl, FP64List L, void *rec, int block,
+                            cudaStream_t st);
+// Diagnostic steps: the pairs of every owner entry, in one kernel.
+void launch_pairs_diag_fp64(const Views &V, int cur, int E, const unsigned *erow, unsigned char *pfl, void *rec,
+                            cudaStream_t st);
 // (light: no field of the batch has ridging, sheltering or walls)
 void launch_row_sums_fp64(const Views &V, int cur, int diag, int light, const unsigned char *pfl, const void *rec,
                           const int *lo_n, const int *up_n, double *fs, int block, cudaStream_t st);

@@ -15,23 +15,19 @@ static int fp64_grid(long long n, int block)
     return (int)std::max(1LL, std::min<long long>((n + block - 1) / block, 148LL * (4096 / block)));
 }
 
-void launch_pairs_fp64(const Views &V, int cur, int diag, int n, const int *plist, const unsigned *erow,
-                       unsigned char *pfl, FP64List L, void *rec, int block, cudaStream_t st)
+void launch_pairs_fp64(const Views &V, int cur, int n, const int *plist, const unsigned *erow, unsigned char *pfl,
+                       FP64List L, void *rec, int block, cudaStream_t st)
 {
-    const int grid = fp64_grid(n, block);
-    PairRec64 *r = (PairRec64 *)rec;
-    if (diag) launch_step(V.pdl != 0, k_pairs_fp64<true>, grid, block, st, V, cur, n, plist, erow, pfl, L, r);
-    else launch_step(V.pdl != 0, k_pairs_fp64<false>, grid, block, st, V, cur, n, plist, erow, pfl, L, r);
+    launch_step(V.pdl != 0, k_pairs_fp64, fp64_grid(n, block), block, st, V, cur, n, plist, erow, pfl, L,
+                (PairRec64 *)rec);
 }
 
-void launch_pairs_list_fp64(const Views &V, int cur, int diag, int E, unsigned char *pfl, FP64List L, void *rec,
-                            int block, cudaStream_t st)
+void launch_pairs_list_fp64(const Views &V, int cur, int n, unsigned char *pfl, FP64List L, void *rec, int block,
+                            cudaStream_t st)
 {
     // the list's length is known on the device only: at most one wave, grid-stride
-    const int grid = (int)std::max(1LL, std::min<long long>((E + block - 1) / block, 148LL * (1024 / block)));
-    PairRec64 *r = (PairRec64 *)rec;
-    if (diag) launch_step(V.pdl != 0, k_pairs_list_fp64<true>, grid, block, st, V, cur, L, pfl, r);
-    else launch_step(V.pdl != 0, k_pairs_list_fp64<false>, grid, block, st, V, cur, L, pfl, r);
+    const int grid = (int)std::max(1LL, std::min<long long>(((long long)n + block - 1) / block, 148LL * (1024 / block)));
+    launch_step(V.pdl != 0, k_pairs_list_fp64, grid, block, st, V, cur, L, pfl, (PairRec64 *)rec);
 }
 
 void launch_row_sums_fp64(const Views &V, int cur, int diag, int light, const unsigned char *pfl, const void *rec,
@@ -49,7 +45,15 @@ void launch_pairs_shel_fp64(const Views &V, int cur, int n, const int *plist, co
 {
     SmallArgs64 A{};
     A.n = n; A.plist = plist; A.erow = erow; A.pfl = pfl; A.rec = (PairRec64 *)rec;
-    if (n > 0) launch_step(V.pdl != 0, k_step_pairs_shel_fp64, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, cur);
+    if (n > 0) launch_step(V.pdl != 0, k_step_pairs_shel_fp64<false>, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, cur);
+}
+
+void launch_pairs_diag_fp64(const Views &V, int cur, int E, const unsigned *erow, unsigned char *pfl, void *rec,
+                            cudaStream_t st)
+{
+    SmallArgs64 A{};
+    A.n = E; A.erow = erow; A.pfl = pfl; A.rec = (PairRec64 *)rec;
+    if (E > 0) launch_step(V.pdl != 0, k_step_pairs_shel_fp64<true>, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, cur);
 }
 
 void launch_group_sums_fp64(const Views &V, int cur, const unsigned char *pfl, const void *rec, const int *lo_n,
@@ -112,8 +116,12 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
         // (nothing to visit: the update computes its drag itself)
         const bool apart = diag && diag_sums_apart(V.N);
         A.drag = !apart && (diag || n > 0) ? drag : nullptr;
-        if (diag) launch(dense ? k_step_pairs_fp64<true, 4> : k_step_pairs_fp64<true, 2>, gp, 128, V, A, c);
-        else if (shelter && n > SHEL_WAVE) launch(k_step_pairs_shel_fp64, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, A, c);
+        if (diag && E > SHEL_WAVE) {
+            auto W = A;
+            W.n = E;
+            launch(k_step_pairs_shel_fp64<true>, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, W, c);
+        } else if (diag) launch(dense ? k_step_pairs_fp64<true, 4> : k_step_pairs_fp64<true, 2>, gp, 128, V, A, c);
+        else if (shelter && n > SHEL_WAVE) launch(k_step_pairs_shel_fp64<false>, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, A, c);
         else if (n > 0) launch(dense ? k_step_pairs_fp64<false, 4> : k_step_pairs_fp64<false, 2>, gp, 128, V, A, c);
         const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
         if (apart) {

@@ -2,7 +2,8 @@
 // (stepper.f90:44-343) as four kernels, bit-identical to the reference's
 // sequential order.
 //
-//   k_pairs_fp64, one thread per owner entry (pair of candidates i < j by
+//   k_pairs_fp64 (diagnostic steps and sheltering fields:
+//   k_step_pairs_shel_fp64), one thread per owner entry (pair of candidates i < j by
 //   id, stored in the row of the lower-id floe i): the FP64 distance of the
 //   pair and the candidate test (dist <= r_i + rtree, stepper.f90:89-92);
 //   pairs that need no pair physics and bonded pairs out of contact are done
@@ -227,23 +228,23 @@ GD_DEV void pair_work64(const Views &V, int cur, Hist4<double> *Hs, int p, int g
     }
 }
 
-// Owner entries: the FP64 distance (kept for the row sort), the candidate
-// test, and every pair that is not in contact in a field without sheltering.
+// Owner entries on a plain step of a batch without sheltering: the FP64
+// distance (kept for the row sort), the candidate test, and every pair that is
+// not in contact.
 // A non-candidate keeps its history and bond state.  A candidate without a
 // bond is a quiet_candidate.  A bonded one goes through the pair physics with
 // the contact branch compiled out.  The others go on the work list with
 // their slots, bond index and offset.
-// A plain step visits the positions of plist only (n of them: the pairs that
-// can act before the next rebuild, see k_fp64_mark; nine in ten are bonded on
-// the benchmark's fields); a diagnostic step every owner entry (plist null,
-// n = E).
+// It visits the positions of plist only (n of them: the pairs that can act
+// before the next rebuild, see k_fp64_mark; nine in ten are bonded on the
+// benchmark's fields); a diagnostic step visits every owner entry
+// (k_step_pairs_shel_fp64<true>).
 // Latency bounds it (half its warps' registers are the bond's FP64 chain), so
 // what it waits for is kept short: the screen and the bonds were two kernels
 // with a 32-byte item a bond between them, each gathering both floes, the bond
 // state in reference order, and every pair's history read and written back.
 // 529,113 floes, 0.82 M bonds: 41 + 84 us then, 77 us now.
-template <bool DIAG>
-__global__ void __launch_bounds__(128, DIAG ? 4 : 6) k_pairs_fp64(Views V, int cur, int n, const int *plist, const unsigned *erow,
+__global__ void __launch_bounds__(128, 6) k_pairs_fp64(Views V, int cur, int n, const int *plist, const unsigned *erow,
                                                     unsigned char *pfl, FP64List L, PairRec64 *rec)
 {
     step_kernel_entry();
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(128, DIAG ? 4 : 6) k_pairs_fp64(Views V, int c
         const int i = i0 + lane;
         const bool on = i < n;
         // lanes past the end read item 0 and store nothing
-        const int e = plist ? plist[on ? i : 0] : on ? i : 0;
+        const int e = plist[on ? i : 0];
         const int g = (int)erow[e];
         const int2 en = V.ent_up[e];
         const int t = en.x, p = en.y;
@@ -271,7 +272,7 @@ __global__ void __launch_bounds__(128, DIAG ? 4 : 6) k_pairs_fp64(Views V, int c
         const double dist = sqrt(dx * dx + dy * dy);
         const double deltan = (rg + rt) - dist;
         const bool cand = on && dist <= rg + P.rtree;
-        const bool heavy = cand && (deltan > 0.0 || P.shelter != 0);
+        const bool heavy = cand && deltan > 0.0;
         if (on) V.edist[e] = dist;
         const unsigned m = __ballot_sync(0xffffffffu, heavy);
         if (m) {
@@ -289,20 +290,15 @@ __global__ void __launch_bounds__(128, DIAG ? 4 : 6) k_pairs_fp64(Views V, int c
         if (!cand) {
             // history and bond state stay as they are
             pfl[p] = (unsigned char)(old & PR_HIST);
-            if (DIAG) V.pdn[p] = __int_as_float(0x7fc00000);
         } else if (bi >= 0) {
-            pair_work64<true, DIAG>(V, cur, Hs, p, g, t, bi, dx, dy, old, pfl, rec, C);
+            pair_work64<true, false>(V, cur, Hs, p, g, t, bi, dx, dy, old, pfl, rec, C);
         } else {
-            pfl[p] = (unsigned char)quiet_candidate<DIAG>(V, Hs, p, dx, dy, dist, deltan, rg, rt, old, rec);
-            if (DIAG) C.cand++;
+            pfl[p] = (unsigned char)quiet_candidate<false>(V, Hs, p, dx, dy, dist, deltan, rg, rt, old, rec);
         }
     }
-    __syncwarp();
-    if (DIAG) add_counts(C, V.counters);
 }
 
-// The work list: contacts, and every candidate of a sheltering field.
-template <bool DIAG>
+// The work list: contacts.
 __global__ void __launch_bounds__(128, 4) k_pairs_list_fp64(Views V, int cur, FP64List L, unsigned char *pfl,
                                                          PairRec64 *rec)
 {
@@ -315,10 +311,8 @@ __global__ void __launch_bounds__(128, 4) k_pairs_list_fp64(Views V, int cur, FP
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
         // the pair, both slots, the bond index and the pair's offset come along
         const FP64Item w = L.work[k];
-        pair_work64<false, DIAG>(V, cur, Hs, w.p, w.g, w.t, w.bi, w.dx, w.dy, pfl[w.p], pfl, rec, C);
+        pair_work64<false, false>(V, cur, Hs, w.p, w.g, w.t, w.bi, w.dx, w.dy, pfl[w.p], pfl, rec, C);
     }
-    __syncwarp();
-    if (DIAG) add_counts(C, V.counters);
 }
 
 // The pair result one floe's sums need, from the pair's record.  A group the
@@ -944,9 +938,15 @@ __global__ void __launch_bounds__(128, MINB) k_step_pairs_fp64(Views V, SmallArg
 // shelter factors only, and such pairs stay on their lane; the others (one in
 // five of a packed field's, in nearly every warp) collect in shared memory and
 // go through the physics 32 at a time, so that a warp does not run it for a few
-// lanes.  65,536 floes: 198 -> 143 us a
-// step; 9,473 (little more than one wave of items) as without.
+// lanes.  65,536 floes: 198 -> 143 us a step; 9,473 (little more than one wave
+// of items) as without.
+// DIAG: the pairs of a diagnostic step, every owner entry (n of them; plist null),
+// most of which are candidates out of contact: a call of one such step of
+// 600,000 bonded floes 659 -> 580 us, of 130,000 of many sizes 372 -> 346, of
+// 70,000 259 -> 226 (three or six blocks an SM 604 and 612, 361 and 342, 231 and
+// 226).
 constexpr int SHEL_THREADS = 128, SHEL_WAVE = 148 * 4 * SHEL_THREADS;
+template <bool DIAG>
 __global__ void __launch_bounds__(SHEL_THREADS, 4) k_step_pairs_shel_fp64(Views V, SmallArgs64 A, int cur)
 {
     struct Item { int p, g, t, bi; double dx, dy; unsigned old; };
@@ -964,7 +964,7 @@ __global__ void __launch_bounds__(SHEL_THREADS, 4) k_step_pairs_shel_fp64(Views 
         bool heavy = false;
         Item it;
         if (i0 + lane < A.n) {
-            const int e = A.plist[i0 + lane];
+            const int e = DIAG ? i0 + lane : A.plist[i0 + lane];
             const int g = (int)A.erow[e];
             const int2 en = V.ent_up[e];
             const int t = en.x, p = en.y;
@@ -981,15 +981,17 @@ __global__ void __launch_bounds__(SHEL_THREADS, 4) k_step_pairs_shel_fp64(Views 
             if (!(dist <= rg + P.rtree)) {
                 // history and bond state stay as they are
                 A.pfl[p] = (unsigned char)(old & PR_HIST);
-            } else if (deltan > 0.0 || bi >= 0) {
+                if (DIAG) V.pdn[p] = __int_as_float(0x7fc00000);
+            } else if (deltan > 0.0 || bi >= 0 || (DIAG && P.shelter != 0)) {
                 heavy = true;
                 it.p = p; it.g = g; it.t = t; it.bi = bi;
                 it.dx = dx; it.dy = dy; it.old = old;
-            } else if (P.shelter != 0) {
+            } else if (!DIAG && P.shelter != 0) {
                 A.pfl[p] = (unsigned char)sheltered_candidate(V, P, cur, Hs, p, g, t, x, y, dx, dy, dist, deltan, rg,
                                                               rt, old, A.rec);
             } else {
-                A.pfl[p] = (unsigned char)quiet_candidate<false>(V, Hs, p, dx, dy, dist, deltan, rg, rt, old, A.rec);
+                A.pfl[p] = (unsigned char)quiet_candidate<DIAG>(V, Hs, p, dx, dy, dist, deltan, rg, rt, old, A.rec);
+                if (DIAG) C.cand++;
             }
         }
         const unsigned m = __ballot_sync(0xffffffffu, heavy);
@@ -1000,7 +1002,7 @@ __global__ void __launch_bounds__(SHEL_THREADS, 4) k_step_pairs_shel_fp64(Views 
             const int k = max(waiting - 32, 0);
             if (k + lane < waiting) {
                 it = L[k + lane];
-                pair_work64<false, false>(V, cur, Hs, it.p, it.g, it.t, it.bi, it.dx, it.dy, it.old, A.pfl, A.rec, C);
+                pair_work64<false, DIAG>(V, cur, Hs, it.p, it.g, it.t, it.bi, it.dx, it.dy, it.old, A.pfl, A.rec, C);
             }
             waiting = k;
             __syncwarp();
@@ -1008,8 +1010,10 @@ __global__ void __launch_bounds__(SHEL_THREADS, 4) k_step_pairs_shel_fp64(Views 
     }
     if (lane < waiting) {
         const Item it = L[lane];
-        pair_work64<false, false>(V, cur, Hs, it.p, it.g, it.t, it.bi, it.dx, it.dy, it.old, A.pfl, A.rec, C);
+        pair_work64<false, DIAG>(V, cur, Hs, it.p, it.g, it.t, it.bi, it.dx, it.dy, it.old, A.pfl, A.rec, C);
     }
+    __syncwarp();
+    if (DIAG) add_counts(C, V.counters);
     // the drag of the floes out of sheltering fields (a small batch's update
     // takes it from here)
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; A.drag && g < V.N; g += nthr)

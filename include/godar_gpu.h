@@ -353,8 +353,8 @@ int godar_batch_stats(godar_batch *b, double *kernel_ms, int64_t *launches,
 /* The same device time split by kernel (CUDA events between the kernels of
  * each timed step), up to nphase entries: GODAR_PREC_MIXED [pair screen and
  * physics, every candidate (diagnostic steps only), bonds, floe sums, floe
- * update], GODAR_PREC_FP64 [entry screen and bonded pairs (sheltering fields:
- * every pair), work list, none, row sums, floe update]; the number of
+ * update], GODAR_PREC_FP64 [entry screen and bonded pairs (sheltering fields and
+ * diagnostic steps: every pair), work list, none, row sums, floe update]; the number of
  * step kernels launched; and the number of steps timed.  No counterpart in
  * the reference (its timers are the wall-clock prints of godar.f90). */
 #define GODAR_NPHASES 5

@@ -2404,6 +2404,10 @@ struct Engine {
         // the list's first `want` pairs in one pass; how many there are comes
         // back beside them, or before them where they do not fit a staging slot
         const long long bound = which == 2 ? I->nb : E;
+        if (bound == 0) {
+            if (count) *count = 0;
+            return GODAR_OK;
+        }
         int want = (int)std::max(0LL, std::min<long long>(cap, bound));
         auto launch = [&](int m) {
             double *v = tmp_v.as<double>();

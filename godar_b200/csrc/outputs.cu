@@ -106,6 +106,24 @@ __global__ void __launch_bounds__(256) k_list_counts(Views V, int cur, int off, 
     }
 }
 
+// The length of the list only (total: zero before).
+__global__ void __launch_bounds__(256) k_list_length(Views V, int cur, int off, int n, int which, int *total)
+{
+    const int sub = threadIdx.x & (GRP - 1), step = gridDim.x * (blockDim.x / GRP);
+    int c = 0;
+    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) / GRP; k < n; k += step) {
+        int e0, e1;
+        list_row(V, cur, off, which, k, e0, e1);
+        for (int e = e0 + sub; e < e1; e += GRP) {
+            int j;
+            double v;
+            c += list_entry(V, cur, which, e, j, v);
+        }
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(total, c);
+}
+
 // Every pair at base[lower id] + its rank in its row, up to cap of them (base:
 // n + 1).
 constexpr int LIST_THREADS = 128, LIST_CAP = 64;
@@ -395,10 +413,15 @@ const int *launch_list_pairs(const Views &V, int cur, int off, int n, long long 
         return total;
     }
     const auto grid = [&](int per) { return (int)std::min<long long>(((long long)n + per - 1) / per, 148 * 16); };
+    if (cap <= 0) {
+        // (two launches where the counts and their scan are four)
+        cudaMemsetAsync(total, 0, sizeof(int), st);
+        k_list_length<<<grid(256 / GRP), 256, 0, st>>>(V, cur, off, n, which, total);
+        return total;
+    }
     k_list_counts<<<grid(256 / GRP), 256, 0, st>>>(V, cur, off, n, which, cnt);
     scan_excl(cnt, base, n, scan_scratch, st);
-    if (cap > 0)
-        k_list_fill<<<grid(LIST_THREADS / GRP), LIST_THREADS, 0, st>>>(V, cur, off, n, which, base, cap, pi, pj, val);
+    k_list_fill<<<grid(LIST_THREADS / GRP), LIST_THREADS, 0, st>>>(V, cur, off, n, which, base, cap, pi, pj, val);
     return base + n;
 }
 

@@ -1705,7 +1705,7 @@ struct Engine {
             if (conc) CK(cudaStreamWaitEvent(st, ev_join, 0));
             else launch_bonds_mixed(V, side, diag, NB, B, cfg_block(bs[2]), cfg_variant(bs[2]), test_wait_spins, st);
             if (ev) TRY(record(ev[3], capturing));
-            if (shelter_any && !diag) launch_group_sums_mixed(V, rows_long ? 1 : 0, B, st);
+            if (shelter_any && !diag) launch_group_sums_mixed(V, B, st);
             else launch_floe_sums(V, diag, light, B, cfg_block(bs[3]), st);
             if (ev) TRY(record(ev[4], capturing));
             // (without a contact list only diagnostic steps would advance the bound)

@@ -159,11 +159,13 @@ void launch_fp64_bonds(const Views &V, int side, int *cnt, int *wfo, int *scan_s
 // launched.
 constexpr int ONE_CLUSTER_FP64 = 1024, ONE_CLUSTER_MIXED = 4096;
 // (FP64: no thread has a second pair or a second floe; mixed, where a pair is
-// lighter: no second floe, or hardly a pair; see cluster_blocks)
+// lighter: four rounds of items, in which a bond counts twice once there are two
+// of floes; see cluster_blocks.  271 floes in touch without bonds 10.6 us a step,
+// a cluster 13.8)
 inline bool one_block_fp64(int N, int n) { return N <= SMALL_THREADS && n <= SMALL_THREADS; }
-inline bool one_block_mixed(int N, long long items)
+inline bool one_block_mixed(int N, long long items, int NB)
 {
-    return items <= (N <= SMALL_THREADS ? 4 : 2) * SMALL_THREADS;
+    return N <= SMALL_THREADS ? items <= 4 * SMALL_THREADS : N <= 2 * SMALL_THREADS && items + NB <= 4 * SMALL_THREADS;
 }
 int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
                        const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
@@ -179,8 +181,9 @@ inline bool diag_apart(int E, int blocks) { return E > 4LL * blocks * SMALL_THRE
 // their own: the rows of every candidate are long, and the sums wait for them
 // with the update's registers otherwise.  Sums and update, merged and apart, of
 // 70,000 floes of many sizes: 189 and 130 us FP64, 139 and 85 mixed; of 20,000
-// no difference (a call 160 and 162, 132 and 134 us).
-inline bool diag_sums_apart(int N) { return N > 32 * 1024; }
+// no difference (a call 160 and 162, 132 and 134 us), and of 112,870 with hardly
+// a candidate each mixed a call 62 and 69.
+inline bool diag_sums_apart(int N, int E) { return N > 32 * 1024 && E > 4LL * N; }
 
 // How a plain step of the merged kernels sums the pairs of a floe: one thread
 // a floe; by groups of lanes in the update's kernel, up to one wave of its
@@ -237,7 +240,7 @@ void launch_pairs_diag(const Views &V, int cur, int P, const unsigned *erow_up, 
 // pair kernel advances the displacement bound in every step since the rebuild.
 void launch_floe_sums(const Views &V, int diag, int light, MixedBufs B, int block, cudaStream_t st);
 void launch_pairs_shel_mixed(const Views &V, int cur, int n, int2 *eb, const int2 *stl, MixedBufs B, cudaStream_t st);
-void launch_group_sums_mixed(const Views &V, int long_rows, MixedBufs B, cudaStream_t st);
+void launch_group_sums_mixed(const Views &V, MixedBufs B, cudaStream_t st);
 void launch_bonds_mixed(const Views &V, int cur, int diag, int NB, MixedBufs B, int block, int variant,
                         unsigned test_spins, cudaStream_t st);
 void launch_floes_mixed(const Views &V, int cur, int diag, int sic, int walls, int light, int bounded, MixedBufs B,

@@ -114,9 +114,9 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
         const int gp = fp64_grid(work, 128);
         const bool dense = work > 148 * 2 * 128;
         // (nothing to visit: the update computes its drag itself)
-        const bool apart = diag && diag_sums_apart(V.N);
+        const bool apart = diag && diag_sums_apart(V.N, E);
         A.drag = !apart && (diag || n > 0) ? drag : nullptr;
-        if (diag && E > SHEL_WAVE) {
+        if (diag && !shelter && E > SHEL_WAVE) {
             auto W = A;
             W.n = E;
             launch(k_step_pairs_shel_fp64<true>, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, W, c);

@@ -1171,10 +1171,11 @@ GD_DEV void small_pairs32(const Views &V, const SmallArgs32 &A, const MixedBufs 
 // the warp calls.
 GD_DEV float shfl_grp(float v, int src) { return __shfl_sync(0xffffffffu, v, src, GRP); }
 
-// SEEK: a batch with a row of more than LONG_ROW entries, whose flags are
-// searched 64 at a time to the next that is set: of a large floe's 3,272 entries
-// hardly one has a record (4,000 floes 73 -> 23 us a step; batches without such
-// a row lose 2 % to the search's code).
+// SEEK: a batch without sheltering (whose every candidate has a record: 1,065
+// floes 106 us a step, 138 searched) with a row of more than LONG_ROW entries,
+// whose flags are searched 64 at a time to the next that is set: of a large
+// floe's 3,272 entries hardly one has a record (4,000 floes 73 -> 23 us a step;
+// batches without such a row lose 2 % to the search's code).
 template <bool SEEK>
 GD_DEV void group_sum32(const Views &V, const MixedBufs &B, bool on, int g, FloeSum32 &F)
 {
@@ -1450,7 +1451,6 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) k_step_floes_grp_mixed(Views
 
 // The sums as a kernel of their own (k_group_sums_fp64), two float4 a floe in
 // fs: 65,536 sheltering floes 112 -> 84 us a step.
-template <bool SEEK>
 __global__ void __launch_bounds__(SMALL_THREADS, 8) k_group_sums_mixed(Views V, MixedBufs B, float4 *fs)
 {
     step_kernel_entry();
@@ -1460,7 +1460,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 8) k_group_sums_mixed(Views V, 
         const int g = g0 + grp;
         const bool on = g < V.N;
         FloeSum32 F;
-        group_sum32<SEEK>(V, B, on, g, F);
+        group_sum32<false>(V, B, on, g, F);
         if (on && threadIdx.x % GRP == 0) {
             fs[2 * (size_t)g] = make_float4(F.fcx, F.fcy, F.mc, F.fbx);
             fs[2 * (size_t)g + 1] = make_float4(F.fby, F.mb, F.sca, F.scw);
@@ -1506,9 +1506,9 @@ void launch_pairs_shel_mixed(const Views &V, int cur, int n, int2 *eb, const int
     if (n > 0) launch_step(V.pdl != 0, k_step_pairs_shel_mixed, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, B, cur);
 }
 
-void launch_group_sums_mixed(const Views &V, int long_rows, MixedBufs B, cudaStream_t st)
+void launch_group_sums_mixed(const Views &V, MixedBufs B, cudaStream_t st)
 {
-    launch_step(V.pdl != 0, long_rows ? k_group_sums_mixed<true> : k_group_sums_mixed<false>, (V.N + GRP_FLOES - 1) / GRP_FLOES, SMALL_THREADS, st, V, B, B.fsum);
+    launch_step(V.pdl != 0, k_group_sums_mixed, (V.N + GRP_FLOES - 1) / GRP_FLOES, SMALL_THREADS, st, V, B, B.fsum);
 }
 
 int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int long_rows,
@@ -1525,7 +1525,7 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
     const long long all = (long long)n + NB + V.N;
     int kernels = 0, first = 0;
     if (!shelter && all <= ONE_CLUSTER_MIXED) {
-        const int blocks = cluster_blocks(all, one_block_mixed(V.N, all));
+        const int blocks = cluster_blocks(all, one_block_mixed(V.N, all, NB));
         auto W = A;
         if (diag_last && diag_apart(E, blocks)) {
             W.K = K - 1;
@@ -1538,6 +1538,7 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
         if (first == K) return kernels;
     }
     const GroupSums how = group_sums(V.N, shelter, (long long)E + NB);
+    const bool seek = long_rows && !shelter;
     const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
     float4 *fs = B.fdg;   // (a plain step has no diagnostic sums)
     const auto launch = [&](auto kern, int grid, int block, auto... args) {
@@ -1552,7 +1553,7 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
         const long long items = (long long)(diag ? E : n) + (ridging ? 0 : NB) + 64 + V.N;
         // (nothing to visit: the update computes its drag itself)
         const bool pairs = diag || n > 0 || NB > 0;
-        const bool apart = diag && diag_sums_apart(V.N);
+        const bool apart = diag && diag_sums_apart(V.N, E);
         A.drag = pairs && !apart ? B.fsum : nullptr;
         if (shelter && !diag && n > SHEL_WAVE)
             launch(k_step_pairs_shel_mixed, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, A, B, c);
@@ -1570,9 +1571,9 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
         } else if (how == SUMS_THREAD) {
             launch(walls ? k_step_floes_mixed<false, true> : k_step_floes_mixed<false, false>, grid_of(V.N, 64), 64, V, A, B, c, k);
         } else if (how == SUMS_GROUP) {
-            launch(long_rows ? k_step_floes_grp_mixed<true> : k_step_floes_grp_mixed<false>, groups, SMALL_THREADS, V, A, B, c, k);
+            launch(seek ? k_step_floes_grp_mixed<true> : k_step_floes_grp_mixed<false>, groups, SMALL_THREADS, V, A, B, c, k);
         } else {
-            launch(long_rows ? k_group_sums_mixed<true> : k_group_sums_mixed<false>, groups, SMALL_THREADS, V, B, fs);
+            launch(k_group_sums_mixed, groups, SMALL_THREADS, V, B, fs);
             launch(walls ? k_step_update_mixed<false, true> : k_step_update_mixed<false, false>, grid_of(V.N, 64), 64, V, A, B, c, k, (const float4 *)fs);
         }
     }

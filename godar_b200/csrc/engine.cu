@@ -1649,13 +1649,12 @@ struct Engine {
         if (NB > 0) wdirty = true;
         const int light = !ridging_any && !shelter_any && !walls_any;
         if (prec == GODAR_PREC_FP64) {
-            FP64List L;
-            L.work = work_b.as<FP64Item>();
-            L.n = nwork_b.as<int>();
+            const FP64List L = fp64_list();
             // a plain step visits the pairs that can act before the next
             // rebuild; a diagnostic step every owner entry
             if (diag) {
-                launch_pairs_diag_fp64(V, side, (int)E, erow_up.as<unsigned>(), pfl.as<unsigned char>(), frec_b.p, st);
+                launch_pairs_diag_fp64(V, side, (int)E, shelter_any ? 1 : 0, erow_up.as<unsigned>(),
+                                       pfl.as<unsigned char>(), L, frec_b.p, st);
                 if (ev) TRY(record(ev[1], capturing));
             } else if (shelter_any) {
                 launch_pairs_shel_fp64(V, side, (int)Lc, fplist_b.as<int>(), erow_up.as<unsigned>(),
@@ -1721,6 +1720,13 @@ struct Engine {
         return fused_on && every == 0 && N > 0 && N <= (prec == GODAR_PREC_FP64 ? SMALL_FLOES_FP64 : SMALL_FLOES_MIXED);
     }
 
+    FP64List fp64_list() const {
+        FP64List L;
+        L.work = work_b.as<FP64Item>();
+        L.n = nwork_b.as<int>();
+        return L;
+    }
+
     // K steps from side c0 as merged steps; out receives the status word and
     // the first expired step.  Returns the kernels launched.
     int launch_small(int K, int c0, int diag_last, int *out) {
@@ -1728,9 +1734,9 @@ struct Engine {
         V.pdl = step_pdl();
         graph_launches++;
         if (prec == GODAR_PREC_FP64)
-            return launch_steps_fp64(V, cluster, c0, K, diag_last, gbase, (int)Lc, (int)E, shelter_any ? 1 : 0, walls_any ? 1 : 0, fplist_b.as<int>(),
+            return launch_steps_fp64(V, cluster, c0, K, diag_last, gbase, (int)Lc, (int)E, NB, shelter_any ? 1 : 0, walls_any ? 1 : 0, fplist_b.as<int>(),
                                      erow_up.as<unsigned>(), pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
-                                     fupn_b.as<int>(), fsum_b.as<double>(), out, step_base_b.as<int>() + 1, st);
+                                     fupn_b.as<int>(), fsum_b.as<double>(), fp64_list(), out, step_base_b.as<int>() + 1, st);
         return launch_steps_mixed(V, cluster, c0, K, diag_last, gbase, (int)Ec, (int)E, NB, rows_long ? 1 : 0, shelter_any ? 1 : 0, walls_any ? 1 : 0, ridging_any ? 1 : 0,
                                   clist_b.as<int2>(), clist_b.as<int2>() + Ecap, erow_up.as<unsigned>(),
                                   bflag_b.as<unsigned char>(), mixed_bufs(), out, step_base_b.as<int>() + 1, st);
@@ -1744,7 +1750,7 @@ struct Engine {
 
     // The separate kernels of a plain or of a diagnostic step (launch_one).
     int step_kernels(bool diag) const {
-        if (prec == GODAR_PREC_FP64) return diag ? (E > 0) + 2 : shelter_any ? (Lc > 0) + 2 : 4;
+        if (prec == GODAR_PREC_FP64) return diag ? (E > 0 ? (shelter_any ? 1 : 2) : 0) + 2 : shelter_any ? (Lc > 0) + 2 : 4;
         return (diag ? (E > 0 ? 2 : 0) : (Ec > 0)) + (NB > 0) + 2;
     }
 

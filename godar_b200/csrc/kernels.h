@@ -126,9 +126,10 @@ void launch_pairs_fp64(const Views &V, int cur, int n, const int *plist, const u
                        FP64List L, void *rec, int block, cudaStream_t st);
 void launch_pairs_list_fp64(const Views &V, int cur, int n, unsigned char *pfl, FP64List L, void *rec, int block,
                             cudaStream_t st);
-// Diagnostic steps: the pairs of every owner entry, in one kernel.
-void launch_pairs_diag_fp64(const Views &V, int cur, int E, const unsigned *erow, unsigned char *pfl, void *rec,
-                            cudaStream_t st);
+// Diagnostic steps: the pairs of every owner entry (shelter: some field of the
+// batch has sheltering).
+void launch_pairs_diag_fp64(const Views &V, int cur, int E, int shelter, const unsigned *erow, unsigned char *pfl,
+                            FP64List L, void *rec, cudaStream_t st);
 // (light: no field of the batch has ridging, sheltering or walls)
 void launch_row_sums_fp64(const Views &V, int cur, int diag, int light, const unsigned char *pfl, const void *rec,
                           const int *lo_n, const int *up_n, double *fs, int block, cudaStream_t st);
@@ -158,18 +159,22 @@ void launch_fp64_bonds(const Views &V, int side, int *cnt, int *wfo, int *scan_s
 // two to four launches a step (one where no pair can act).  Returns the kernels
 // launched.
 constexpr int ONE_CLUSTER_FP64 = 1024, ONE_CLUSTER_MIXED = 4096;
-// (FP64: no thread has a second pair or a second floe; mixed, where a pair is
-// lighter: four rounds of items, in which a bond counts twice once there are two
-// of floes; see cluster_blocks.  271 floes in touch without bonds 10.6 us a step,
-// a cluster 13.8)
-inline bool one_block_fp64(int N, int n) { return N <= SMALL_THREADS && n <= SMALL_THREADS; }
+// (FP64: no thread has a second floe or a second bond, nor a third item; mixed,
+// where a pair is lighter: four rounds of items, in which a bond counts twice once
+// there are two of floes; see cluster_blocks.  Floes in touch without bonds, one
+// block and a cluster: 221 FP64 8.7 and 10.6 us a step, 271 mixed 10.6 and 13.8)
+inline bool one_block_fp64(int N, int n, int NB)
+{
+    return N <= SMALL_THREADS && NB <= SMALL_THREADS && n + N <= 5 * SMALL_THREADS / 2;
+}
 inline bool one_block_mixed(int N, long long items, int NB)
 {
     return N <= SMALL_THREADS ? items <= 4 * SMALL_THREADS : N <= 2 * SMALL_THREADS && items + NB <= 4 * SMALL_THREADS;
 }
-int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
+int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB,
+                       int shelter, int walls,
                        const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
-                       const int *up_n, double *drag, int *out, int *done, cudaStream_t st);
+                       const int *up_n, double *drag, FP64List L, int *out, int *done, cudaStream_t st);
 // Whether a diagnostic step, which visits all E owner entries, leaves the launch
 // of its chunk: a cluster has few threads, and the two launches of a step as
 // many as there are entries.  A call of one such step: 400 floes with 5,214
@@ -178,12 +183,18 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
 inline bool diag_apart(int E, int blocks) { return E > 4LL * blocks * SMALL_THREADS; }
 
 // Whether a diagnostic step of the merged kernels sums its floes in a kernel of
-// their own: the rows of every candidate are long, and the sums wait for them
-// with the update's registers otherwise.  Sums and update, merged and apart, of
-// 70,000 floes of many sizes: 189 and 130 us FP64, 139 and 85 mixed; of 20,000
-// no difference (a call 160 and 162, 132 and 134 us), and of 112,870 with hardly
-// a candidate each mixed a call 62 and 69.
-inline bool diag_sums_apart(int N, int E) { return N > 32 * 1024 && E > 4LL * N; }
+// their own (FP64: and leaves the pair physics to a work list): the rows of
+// every candidate are long, and the sums wait for them with the update's
+// registers otherwise.  Sums and update, merged and apart, of 70,000 floes of
+// many sizes: 189 and 130 us FP64, 139 and 85 mixed.  A call, us: mixed 20,000
+// floes of many sizes 132 and 134, 112,870 with hardly a candidate each 62 and
+// 69; FP64 30,000 with 351,000 entries 119 and 108, with 987,000 256 and 209,
+// 20,000 with 240,000 96 and 104; 60,000 bonded ones with six entries each 138
+// and 111, 41,250 without bonds 81 and 90.
+inline bool diag_sums_apart(int N, int E, int NB, bool fp64)
+{
+    return E + 4LL * NB > (fp64 ? 10LL : 16LL) * N && (N > 32 * 1024 || (fp64 && E > 320 * 1024));
+}
 
 // How a plain step of the merged kernels sums the pairs of a floe: one thread
 // a floe; by groups of lanes in the update's kernel, up to one wave of its

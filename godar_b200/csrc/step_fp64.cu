@@ -27,7 +27,7 @@ void launch_pairs_list_fp64(const Views &V, int cur, int n, unsigned char *pfl, 
 {
     // the list's length is known on the device only: at most one wave, grid-stride
     const int grid = (int)std::max(1LL, std::min<long long>(((long long)n + block - 1) / block, 148LL * (1024 / block)));
-    launch_step(V.pdl != 0, k_pairs_list_fp64, grid, block, st, V, cur, L, pfl, (PairRec64 *)rec);
+    launch_step(V.pdl != 0, k_pairs_list_fp64<false>, grid, block, st, V, cur, L, pfl, (PairRec64 *)rec);
 }
 
 void launch_row_sums_fp64(const Views &V, int cur, int diag, int light, const unsigned char *pfl, const void *rec,
@@ -45,15 +45,32 @@ void launch_pairs_shel_fp64(const Views &V, int cur, int n, const int *plist, co
 {
     SmallArgs64 A{};
     A.n = n; A.plist = plist; A.erow = erow; A.pfl = pfl; A.rec = (PairRec64 *)rec;
-    if (n > 0) launch_step(V.pdl != 0, k_step_pairs_shel_fp64<false>, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, cur);
+    if (n > 0) launch_step(V.pdl != 0, k_step_pairs_shel_fp64, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, cur);
 }
 
-void launch_pairs_diag_fp64(const Views &V, int cur, int E, const unsigned *erow, unsigned char *pfl, void *rec,
-                            cudaStream_t st)
+// The two kernels of k_pairs_diag_fp64 (the list's length is known on the device
+// only: at most one wave, grid-stride).
+template <class Launch>
+static void pairs_diag(const Views &V, int cur, int E, const unsigned *erow, unsigned char *pfl, FP64List L, void *rec,
+                       Launch launch)
 {
-    SmallArgs64 A{};
-    A.n = E; A.erow = erow; A.pfl = pfl; A.rec = (PairRec64 *)rec;
-    if (E > 0) launch_step(V.pdl != 0, k_step_pairs_shel_fp64<true>, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, st, V, A, cur);
+    launch(k_pairs_diag_fp64, fp64_grid(E, 128), 128, V, cur, E, erow, pfl, L, (PairRec64 *)rec);
+    launch(k_pairs_list_fp64<true>, std::min((E + 127) / 128, 148 * 8), 128, V, cur, L, pfl, (PairRec64 *)rec);
+}
+
+void launch_pairs_diag_fp64(const Views &V, int cur, int E, int shelter, const unsigned *erow, unsigned char *pfl,
+                            FP64List L, void *rec, cudaStream_t st)
+{
+    if (E <= 0) return;
+    if (shelter) {
+        SmallArgs64 A{};
+        A.n = A.E = E; A.erow = erow; A.pfl = pfl; A.rec = (PairRec64 *)rec;
+        launch_step(V.pdl != 0, k_step_pairs_fp64<true, 4>, fp64_grid(E, 128), 128, st, V, A, cur);
+        return;
+    }
+    pairs_diag(V, cur, E, erow, pfl, L, rec, [&](auto kern, int grid, int block, auto... args) {
+        launch_step(V.pdl != 0, kern, grid, block, st, args...);
+    });
 }
 
 void launch_group_sums_fp64(const Views &V, int cur, const unsigned char *pfl, const void *rec, const int *lo_n,
@@ -77,18 +94,19 @@ void launch_floes_fp64(const Views &V, int cur, int diag, int sic, int walls, in
     }
 }
 
-int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int shelter, int walls,
+int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB,
+                       int shelter, int walls,
                        const int *plist, const unsigned *erow, unsigned char *pfl, void *rec, const int *lo_n,
-                       const int *up_n, double *drag, int *out, int *done, cudaStream_t st)
+                       const int *up_n, double *drag, FP64List L, int *out, int *done, cudaStream_t st)
 {
     SmallArgs64 A;
     A.cur = cur; A.K = K; A.diag_last = diag_last; A.base = base;
     A.n = n; A.E = E; A.plist = plist; A.erow = erow; A.pfl = pfl; A.rec = (PairRec64 *)rec;
-    A.lo_n = lo_n; A.up_n = up_n; A.drag = drag; A.out = out; A.done = done;
+    A.lo_n = lo_n; A.up_n = up_n; A.drag = drag; A.nd = V.N; A.out = out; A.done = done;
     const long long items = (long long)n + V.N;
     int kernels = 0, first = 0;
     if (!shelter && items <= ONE_CLUSTER_FP64) {
-        const int blocks = cluster_blocks(items, one_block_fp64(V.N, n));
+        const int blocks = cluster_blocks(items, one_block_fp64(V.N, n, NB));
         auto W = A;
         if (diag_last && diag_apart(E, blocks)) {
             W.K = K - 1;
@@ -114,22 +132,21 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
         const int gp = fp64_grid(work, 128);
         const bool dense = work > 148 * 2 * 128;
         // (nothing to visit: the update computes its drag itself)
-        const bool apart = diag && diag_sums_apart(V.N, E);
+        const bool apart = diag && diag_sums_apart(V.N, E, NB, true);
         A.drag = !apart && (diag || n > 0) ? drag : nullptr;
-        if (diag && !shelter && E > SHEL_WAVE) {
-            auto W = A;
-            W.n = E;
-            launch(k_step_pairs_shel_fp64<true>, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, W, c);
-        } else if (diag) launch(dense ? k_step_pairs_fp64<true, 4> : k_step_pairs_fp64<true, 2>, gp, 128, V, A, c);
-        else if (shelter && n > SHEL_WAVE) launch(k_step_pairs_shel_fp64<false>, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, A, c);
+        A.nd = A.drag ? V.N : 0;
+        if (apart && !shelter) pairs_diag(V, c, E, erow, pfl, L, rec, launch);
+        else if (diag) launch(dense ? k_step_pairs_fp64<true, 4> : k_step_pairs_fp64<true, 2>, gp, 128, V, A, c);
+        else if (shelter && n > SHEL_WAVE) launch(k_step_pairs_shel_fp64, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, A, c);
         else if (n > 0) launch(dense ? k_step_pairs_fp64<false, 4> : k_step_pairs_fp64<false, 2>, gp, 128, V, A, c);
         const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
         if (apart) {
             // (every plane of the sums: the drag is the update's)
-            launch(k_row_sums_fp64<true, false>, fp64_grid(V.N, 128), 128, V, c, (const unsigned char *)pfl,
+            const int block = V.N > 148 * 256 ? 128 : 32;      // (on as many SMs as there are blocks for)
+            launch(k_row_sums_fp64<true, false>, fp64_grid(V.N, block), block, V, c, (const unsigned char *)pfl,
                    (const PairRec64 *)A.rec, lo_n, up_n, drag);
             launch(walls ? k_step_update_fp64<true, true> : k_step_update_fp64<true, false>, fp64_grid(V.N, 64), 64, V,
-                   A, c, k, (const double *)drag);
+                   A, c, k, (const double *)drag, L.n);
         } else if (diag) {
             launch(walls ? k_step_floes_fp64<true, true> : k_step_floes_fp64<true, false>, fp64_grid(V.N, 64), 64, V, A, c, k);
         } else if (how == SUMS_THREAD) {
@@ -138,7 +155,7 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
             launch(k_step_floes_grp_fp64, groups, SMALL_THREADS, V, A, c, k);
         } else {
             launch(k_group_sums_fp64, groups, SMALL_THREADS, V, c, pfl, A.rec, lo_n, up_n, fs);
-            launch(walls ? k_step_update_fp64<false, true> : k_step_update_fp64<false, false>, fp64_grid(V.N, 64), 64, V, A, c, k, fs);
+            launch(walls ? k_step_update_fp64<false, true> : k_step_update_fp64<false, false>, fp64_grid(V.N, 64), 64, V, A, c, k, (const double *)fs, L.n);
         }
     }
     return kernels;

@@ -2,8 +2,9 @@
 // (stepper.f90:44-343) as four kernels, bit-identical to the reference's
 // sequential order.
 //
-//   k_pairs_fp64 (diagnostic steps and sheltering fields:
-//   k_step_pairs_shel_fp64), one thread per owner entry (pair of candidates i < j by
+//   k_pairs_fp64 (diagnostic steps: k_pairs_diag_fp64; sheltering fields:
+//   k_step_pairs_shel_fp64, k_step_pairs_fp64), one thread per owner entry (pair of
+//   candidates i < j by
 //   id, stored in the row of the lower-id floe i): the FP64 distance of the
 //   pair and the candidate test (dist <= r_i + rtree, stepper.f90:89-92);
 //   pairs that need no pair physics and bonded pairs out of contact are done
@@ -238,7 +239,7 @@ GD_DEV void pair_work64(const Views &V, int cur, Hist4<double> *Hs, int p, int g
 // It visits the positions of plist only (n of them: the pairs that can act
 // before the next rebuild, see k_fp64_mark; nine in ten are bonded on the
 // benchmark's fields); a diagnostic step visits every owner entry
-// (k_step_pairs_shel_fp64<true>).
+// (k_pairs_diag_fp64, k_step_pairs_fp64<true>).
 // Latency bounds it (half its warps' registers are the bond's FP64 chain), so
 // what it waits for is kept short: the screen and the bonds were two kernels
 // with a 32-byte item a bond between them, each gathering both floes, the bond
@@ -298,7 +299,67 @@ __global__ void __launch_bounds__(128, 6) k_pairs_fp64(Views V, int cur, int n, 
     }
 }
 
-// The work list: contacts.
+// The pairs of a diagnostic step of a batch without sheltering: every owner
+// entry (n of them), most of which are candidates out of contact, with the pair
+// physics of the others left to the work list.  Few registers, so that many
+// entries' loads wait side by side: a call of one such step, this and the list
+// against one kernel of both: 130,000 floes of many sizes 299 and 372 us,
+// 300,000 526 and 666, 600,000 bonded 577 and 659.
+__global__ void __launch_bounds__(128, 12) k_pairs_diag_fp64(Views V, int cur, int n, const unsigned *erow,
+                                                             unsigned char *pfl, FP64List L, PairRec64 *rec)
+{
+    step_kernel_entry();
+    if (*(volatile int *)V.status & ST_ABORT) return;
+    Hist4<double> *Hs = (Hist4<double> *)V.hist[0];   // in place: one thread per pair
+    Counts64 C = {0, 0, 0, 0};
+    const int lane = threadIdx.x & 31;
+    const int stride = gridDim.x * blockDim.x;
+    // every lane of a warp runs the same iterations (the list append is warp-wide)
+    for (int i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += stride) {
+        const int e = i0 + lane;
+        bool heavy = false;
+        FP64Item it;
+        if (e < n) {
+            const int g = (int)erow[e];
+            const int2 en = V.ent_up[e];
+            const int t = en.x, p = en.y;
+            const InstParams &P = V.P[V.inst[g]];
+            const double rg = V.r[cur][g], rt = V.r[cur][t];
+            const int bi = V.bidx[p];
+            const unsigned old = pfl[p];
+            const bool px = P.boundary & BC_PERIODIC_X, py = P.boundary & BC_PERIODIC_Y;
+            const double dx = wrap_d(V.x[cur][g] - V.x[cur][t], P.nx, px);
+            const double dy = wrap_d(V.y[cur][g] - V.y[cur][t], P.ny, py);
+            const double dist = sqrt(dx * dx + dy * dy);
+            const double deltan = (rg + rt) - dist;
+            V.edist[e] = dist;
+            if (!(dist <= rg + P.rtree)) {
+                // history and bond state stay as they are
+                pfl[p] = (unsigned char)(old & PR_HIST);
+                V.pdn[p] = __int_as_float(0x7fc00000);
+            } else if (deltan > 0.0 || bi >= 0) {
+                heavy = true;
+                it.p = p; it.g = g; it.t = t; it.bi = bi;
+                it.dx = dx; it.dy = dy;
+            } else {
+                pfl[p] = (unsigned char)quiet_candidate<true>(V, Hs, p, dx, dy, dist, deltan, rg, rt, old, rec);
+                C.cand++;
+            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, heavy);
+        if (m) {
+            int base = 0;
+            if (lane == 0) base = atomicAdd(L.n, __popc(m));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (heavy) L.work[base + __popc(m & ((1u << lane) - 1))] = it;
+        }
+    }
+    __syncwarp();
+    add_counts(C, V.counters);
+}
+
+// The work list: contacts (on a diagnostic step bonds too).
+template <bool DIAG>
 __global__ void __launch_bounds__(128, 4) k_pairs_list_fp64(Views V, int cur, FP64List L, unsigned char *pfl,
                                                          PairRec64 *rec)
 {
@@ -311,8 +372,10 @@ __global__ void __launch_bounds__(128, 4) k_pairs_list_fp64(Views V, int cur, FP
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
         // the pair, both slots, the bond index and the pair's offset come along
         const FP64Item w = L.work[k];
-        pair_work64<false, false>(V, cur, Hs, w.p, w.g, w.t, w.bi, w.dx, w.dy, pfl[w.p], pfl, rec, C);
+        pair_work64<false, DIAG>(V, cur, Hs, w.p, w.g, w.t, w.bi, w.dx, w.dy, pfl[w.p], pfl, rec, C);
     }
+    __syncwarp();
+    if (DIAG) add_counts(C, V.counters);
 }
 
 // The pair result one floe's sums need, from the pair's record.  A group the
@@ -812,6 +875,7 @@ struct SmallArgs64 {
     PairRec64 *rec;
     const int *lo_n, *up_n;
     double *drag;                  // [8][N]
+    int nd;                        // floes whose drag the pair kernel computes: N or 0
     int *out;                      // pinned host memory: the status word and the first expired step
     int *done;                     // blocks of k_step_floes_fp64 that have finished
 };
@@ -870,9 +934,8 @@ GD_DEV void small_pairs64(const Views &V, const SmallArgs64 &A, int cur)
     const int nthr = gridDim.x * blockDim.x;
     const int n = DIAG ? A.E : A.n;
     const int n0 = (n + 31) & ~31;      // the floes start on a warp of their own
-    const int end = n0 + (A.drag ? V.N : 0);
     Counts64 C = {0, 0, 0, 0};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < end; i += nthr) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n0 + A.nd; i += nthr) {
         if (i < n) {
             pair_entry64<DIAG>(V, cur, DIAG ? i : A.plist[i], A.erow, A.pfl, A.rec, C);
         } else if (i >= n0) {
@@ -940,13 +1003,7 @@ __global__ void __launch_bounds__(128, MINB) k_step_pairs_fp64(Views V, SmallArg
 // go through the physics 32 at a time, so that a warp does not run it for a few
 // lanes.  65,536 floes: 198 -> 143 us a step; 9,473 (little more than one wave
 // of items) as without.
-// DIAG: the pairs of a diagnostic step, every owner entry (n of them; plist null),
-// most of which are candidates out of contact: a call of one such step of
-// 600,000 bonded floes 659 -> 580 us, of 130,000 of many sizes 372 -> 346, of
-// 70,000 259 -> 226 (three or six blocks an SM 604 and 612, 361 and 342, 231 and
-// 226).
 constexpr int SHEL_THREADS = 128, SHEL_WAVE = 148 * 4 * SHEL_THREADS;
-template <bool DIAG>
 __global__ void __launch_bounds__(SHEL_THREADS, 4) k_step_pairs_shel_fp64(Views V, SmallArgs64 A, int cur)
 {
     struct Item { int p, g, t, bi; double dx, dy; unsigned old; };
@@ -964,7 +1021,7 @@ __global__ void __launch_bounds__(SHEL_THREADS, 4) k_step_pairs_shel_fp64(Views 
         bool heavy = false;
         Item it;
         if (i0 + lane < A.n) {
-            const int e = DIAG ? i0 + lane : A.plist[i0 + lane];
+            const int e = A.plist[i0 + lane];
             const int g = (int)A.erow[e];
             const int2 en = V.ent_up[e];
             const int t = en.x, p = en.y;
@@ -981,17 +1038,15 @@ __global__ void __launch_bounds__(SHEL_THREADS, 4) k_step_pairs_shel_fp64(Views 
             if (!(dist <= rg + P.rtree)) {
                 // history and bond state stay as they are
                 A.pfl[p] = (unsigned char)(old & PR_HIST);
-                if (DIAG) V.pdn[p] = __int_as_float(0x7fc00000);
-            } else if (deltan > 0.0 || bi >= 0 || (DIAG && P.shelter != 0)) {
+            } else if (deltan > 0.0 || bi >= 0) {
                 heavy = true;
                 it.p = p; it.g = g; it.t = t; it.bi = bi;
                 it.dx = dx; it.dy = dy; it.old = old;
-            } else if (!DIAG && P.shelter != 0) {
+            } else if (P.shelter != 0) {
                 A.pfl[p] = (unsigned char)sheltered_candidate(V, P, cur, Hs, p, g, t, x, y, dx, dy, dist, deltan, rg,
                                                               rt, old, A.rec);
             } else {
-                A.pfl[p] = (unsigned char)quiet_candidate<DIAG>(V, Hs, p, dx, dy, dist, deltan, rg, rt, old, A.rec);
-                if (DIAG) C.cand++;
+                A.pfl[p] = (unsigned char)quiet_candidate<false>(V, Hs, p, dx, dy, dist, deltan, rg, rt, old, A.rec);
             }
         }
         const unsigned m = __ballot_sync(0xffffffffu, heavy);
@@ -1002,7 +1057,7 @@ __global__ void __launch_bounds__(SHEL_THREADS, 4) k_step_pairs_shel_fp64(Views 
             const int k = max(waiting - 32, 0);
             if (k + lane < waiting) {
                 it = L[k + lane];
-                pair_work64<false, DIAG>(V, cur, Hs, it.p, it.g, it.t, it.bi, it.dx, it.dy, it.old, A.pfl, A.rec, C);
+                pair_work64<false, false>(V, cur, Hs, it.p, it.g, it.t, it.bi, it.dx, it.dy, it.old, A.pfl, A.rec, C);
             }
             waiting = k;
             __syncwarp();
@@ -1010,13 +1065,11 @@ __global__ void __launch_bounds__(SHEL_THREADS, 4) k_step_pairs_shel_fp64(Views 
     }
     if (lane < waiting) {
         const Item it = L[lane];
-        pair_work64<false, DIAG>(V, cur, Hs, it.p, it.g, it.t, it.bi, it.dx, it.dy, it.old, A.pfl, A.rec, C);
+        pair_work64<false, false>(V, cur, Hs, it.p, it.g, it.t, it.bi, it.dx, it.dy, it.old, A.pfl, A.rec, C);
     }
-    __syncwarp();
-    if (DIAG) add_counts(C, V.counters);
     // the drag of the floes out of sheltering fields (a small batch's update
     // takes it from here)
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; A.drag && g < V.N; g += nthr)
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < A.nd; g += nthr)
         drag_ahead64(V, cur, g, A.drag);
 }
 
@@ -1100,9 +1153,12 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4) k_group_sums_fp64(Views V, i
 // ... and the update from them, as the last kernel of a small batch's step; on
 // a diagnostic step from k_row_sums_fp64's.
 template <bool DIAG, bool WALLS>
-__global__ void __launch_bounds__(64) k_step_update_fp64(Views V, SmallArgs64 A, int cur, int sic, const double *fs)
+__global__ void __launch_bounds__(64) k_step_update_fp64(Views V, SmallArgs64 A, int cur, int sic, const double *fs,
+                                                         int *nwork)
 {
     step_kernel_entry();
+    // the work list was used by the pair kernels before this one
+    if (DIAG && blockIdx.x == 0 && threadIdx.x == 0) *nwork = 0;
     const size_t N = (size_t)V.N;
     Counts64 C = {0, 0, 0, 0};
     if (!floe_update_stopped(V, A.base, sic))

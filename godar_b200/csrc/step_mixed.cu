@@ -1098,6 +1098,7 @@ struct SmallArgs32 {
     const unsigned *erow;
     unsigned char *bfl;            // live-bond flags of both sides
     float4 *drag;                  // [2N]
+    int nd;                        // floes whose drag the pair kernel computes: N or 0
     int *out;                      // pinned host memory: the status word and the first expired step
     int *done;                     // blocks of k_step_floes_mixed that have finished
 };
@@ -1129,8 +1130,7 @@ GD_DEV void small_pairs32(const Views &V, const SmallArgs32 &A, const MixedBufs 
     const int n0 = (n + 31) & ~31;
     const int n1 = n0 + (A.ridging ? 0 : (A.NB + 31) & ~31);
     unsigned long long n_cand = 0, n_cont = 0, n_plast = 0, n_bond = 0;
-    const int end = n1 + (A.drag ? V.N : 0);
-    for (int i = first; i < end; i += nthr) {
+    for (int i = first; i < n1 + A.nd; i += nthr) {
         if (i < n) {
             int e = i, s, t;
             if (diag) {
@@ -1396,8 +1396,7 @@ __global__ void __launch_bounds__(SHEL_THREADS, SHEL_BLOCKS) k_step_pairs_shel_m
     if (!A.ridging)
         for (int b = first; b < A.NB; b += nthr)
             bond_step(V, S, 0, b, B.bsp[b], B.wdyn[b], B.bst[b], B.brec, B.bdg, B.bfl_wr, B.wdyn);
-    if (A.drag)
-        for (int g = first; g < V.N; g += nthr) drag_ahead32(V, cur, g, A.drag);
+    for (int g = first; g < A.nd; g += nthr) drag_ahead32(V, cur, g, A.drag);
 }
 
 // A batch without walls runs the instance without their code, whose 80
@@ -1520,6 +1519,7 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
     A.n = n; A.E = E; A.NB = NB; A.ridging = ridging;
     A.eb = eb; A.stl = stl; A.erow = erow; A.bfl = bfl;
     A.drag = B.fsum;      // two float4 a floe: the sums stay in registers here
+    A.nd = V.N;
     A.out = out;
     A.done = done;
     const long long all = (long long)n + NB + V.N;
@@ -1553,8 +1553,9 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
         const long long items = (long long)(diag ? E : n) + (ridging ? 0 : NB) + 64 + V.N;
         // (nothing to visit: the update computes its drag itself)
         const bool pairs = diag || n > 0 || NB > 0;
-        const bool apart = diag && diag_sums_apart(V.N, E);
+        const bool apart = diag && diag_sums_apart(V.N, E, NB, false);
         A.drag = pairs && !apart ? B.fsum : nullptr;
+        A.nd = A.drag ? V.N : 0;
         if (shelter && !diag && n > SHEL_WAVE)
             launch(k_step_pairs_shel_mixed, SHEL_WAVE / SHEL_THREADS, SHEL_THREADS, V, A, B, c);
         else if (pairs) launch(items > 148 * 5 * 128 ? k_step_pairs_mixed<8> : k_step_pairs_mixed<5>, grid_of(items, 128),

@@ -1,7 +1,7 @@
 """The count of step kernels in godar_batch_phase_stats: every kernel a step
 launches, whether the batch runs merged steps (one launch a chunk, or two to
-four a step) or the separate kernels (four; FP64 three on diagnostic steps and
-of sheltering fields; mixed one more on diagnostic steps)."""
+five a step) or the separate kernels (four, FP64 three of sheltering fields;
+mixed one more on diagnostic steps)."""
 import pytest
 
 from godar_b200 import generators as gen
@@ -51,18 +51,20 @@ def test_merged_steps_of_sheltering_fields(precision, monkeypatch):
     assert got == [4 * (3 + bonds), 3 * (3 + bonds) + 2 + bonds]
 
 
-@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
-def test_diagnostic_steps_of_larger_merged_batches(precision, monkeypatch):
-    # the sums of a diagnostic step in a kernel of their own beyond 32,768 floes
-    for n, diag in ((32768, 2), (32769, 3)):
+def test_diagnostic_steps_of_larger_merged_batches(monkeypatch):
+    # beyond 32,768 floes with enough candidates a diagnostic step's sums have a
+    # kernel of their own, FP64 behind two kernels of pairs
+    calls = [(4, False, False), (4, True, False)]
+    for n, diag in ((32768, 2), (32769, 4)):
         f = gen.bonded_field(n=n, seed=2, device="gpu")
-        assert _launched(f, precision, [(4, False, False), (4, True, False)], monkeypatch) == [8, 6 + diag]
+        assert _launched(f, PREC_FP64, calls, monkeypatch) == [8, 6 + diag]
+        assert _launched(f, PREC_MIXED, calls, monkeypatch) == [8, 8]
 
 
 def test_separate_kernels(monkeypatch):
     calls = [(4, False, False), (4, True, False)]
     bonded = gen.bonded_field(n=3000, seed=2)
-    assert _launched(bonded, PREC_FP64, calls, monkeypatch, "0") == [16, 15]
+    assert _launched(bonded, PREC_FP64, calls, monkeypatch, "0") == [16, 16]
     assert _launched(bonded, PREC_MIXED, calls, monkeypatch, "0") == [16, 17]
     poly = gen.polydisperse_field(n=3000, seed=2, phi=0.6, dt=1e-3)
     assert _launched(poly, PREC_FP64, calls, monkeypatch, "0") == [12, 12]

@@ -95,3 +95,10 @@ def test_diagnostic_sums(kind, n, precision, monkeypatch):
         if kind == "walls":
             f.params.boundary = 0
     _same(f, precision, monkeypatch)
+
+
+# FP64: by the entries too, 327,680 of them (each floe a candidate of all others)
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("n", [809, 810, 811])
+def test_diagnostic_sums_of_many_entries(n, precision, monkeypatch):
+    _same(_free(n, rtree=50000.0, sp=60.0, cohesion=1, bond_lim_rel=0.7, dt=1e-3), precision, monkeypatch)

@@ -444,7 +444,7 @@ struct Engine {
     bool overlap_bonds = false;
     bool shelter_any = false;      // some field of the batch has sheltering
     bool walls_any = false;        // some field of the batch has a solid wall
-    bool rows_long = false;        // mixed: some floe has more than LONG_ROW partners
+    int row_max = 0;               // mixed: the most partners of a floe (0: at most LONG_ROW)
     // Batches of at most SMALL_FLOES_* floes run their steps as one to three
     // launches (launch_small): below these sizes the four kernels of a step
     // are mostly gaps and one thread's latency; above them the registers of
@@ -1522,7 +1522,7 @@ struct Engine {
             // (read once the contact list's length is)
             CK(cudaMemcpyAsync(h_status + 3, nwork_b.as<int>() + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
             TRY(contact_list(nxt, Pn));
-            rows_long = Pn > 0 && h_status[3] > LONG_ROW;
+            row_max = Pn > 0 ? h_status[3] : 0;
             TRY(mixed_bond_lists(nxt));
         }
         E = Pn;
@@ -1737,7 +1737,7 @@ struct Engine {
             return launch_steps_fp64(V, cluster, c0, K, diag_last, gbase, (int)Lc, (int)E, NB, shelter_any ? 1 : 0, walls_any ? 1 : 0, fplist_b.as<int>(),
                                      erow_up.as<unsigned>(), pfl.as<unsigned char>(), frec_b.p, flon_b.as<int>(),
                                      fupn_b.as<int>(), fsum_b.as<double>(), fp64_list(), out, step_base_b.as<int>() + 1, st);
-        return launch_steps_mixed(V, cluster, c0, K, diag_last, gbase, (int)Ec, (int)E, NB, rows_long ? 1 : 0, shelter_any ? 1 : 0, walls_any ? 1 : 0, ridging_any ? 1 : 0,
+        return launch_steps_mixed(V, cluster, c0, K, diag_last, gbase, (int)Ec, (int)E, NB, row_max, shelter_any ? 1 : 0, walls_any ? 1 : 0, ridging_any ? 1 : 0,
                                   clist_b.as<int2>(), clist_b.as<int2>() + Ecap, erow_up.as<unsigned>(),
                                   bflag_b.as<unsigned char>(), mixed_bufs(), out, step_base_b.as<int>() + 1, st);
     }

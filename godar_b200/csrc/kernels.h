@@ -179,21 +179,32 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
 // of its chunk: a cluster has few threads, and the two launches of a step as
 // many as there are entries.  A call of one such step: 400 floes with 5,214
 // entries FP64 105 and 89 us, 2,299: 72 and 69; 2,000 floes with 700,000
-// entries mixed 369 and 98, 1,000 with 13,000: 48 and 45.
-inline bool diag_apart(int E, int blocks) { return E > 4LL * blocks * SMALL_THREADS; }
+// entries mixed 369 and 98, 1,000 with 13,000: 48 and 45.  FP64 sums walk their
+// rows entry by entry, on one block through its L1: 85 floes, all candidates of
+// one another, 107 and 128.
+inline bool diag_apart(int N, int E, int blocks, bool fp64)
+{
+    return E > 4LL * blocks * SMALL_THREADS && !(fp64 && N <= SMALL_THREADS / 2);
+}
 
 // Whether a diagnostic step of the merged kernels sums its floes in a kernel of
-// their own (FP64: and leaves the pair physics to a work list): the rows of
-// every candidate are long, and the sums wait for them with the update's
-// registers otherwise.  Sums and update, merged and apart, of 70,000 floes of
-// many sizes: 189 and 130 us FP64, 139 and 85 mixed.  A call, us: mixed 20,000
-// floes of many sizes 132 and 134, 112,870 with hardly a candidate each 62 and
-// 69; FP64 30,000 with 351,000 entries 119 and 108, with 987,000 256 and 209,
-// 20,000 with 240,000 96 and 104; 60,000 bonded ones with six entries each 138
-// and 111, 41,250 without bonds 81 and 90.
-inline bool diag_sums_apart(int N, int E, int NB, bool fp64)
+// their own: the rows of every candidate are long, and the sums wait for them
+// with the update's registers otherwise.  FP64 (which then leaves the pair
+// physics to a work list too), a call, us, merged and apart: 60,000 bonded floes
+// with six entries each 138 and 111, 41,250 without bonds 81 and 90; 30,000 with
+// 351,000 entries 119 and 108, with 987,000 256 and 209; 20,000 with 240,000 96
+// and 104; 5,000 with 1.2 M 1,073 and 1,108.
+inline bool diag_sums_apart_fp64(int N, int E, int NB)
 {
-    return E + 4LL * NB > (fp64 ? 10LL : 16LL) * N && (N > 32 * 1024 || (fp64 && E > 320 * 1024));
+    return E + 4LL * NB > 10LL * N && (N > 32 * 1024 || (N > 8 * 1024 && E > 320 * 1024));
+}
+// Mixed, where the sums are short beside one long row (row_max: the most
+// partners of a floe, 0 if no more than LONG_ROW): sums and update of 70,000
+// floes of many sizes 139 and 85 us; a call of 51,476 alike sheltering ones 508
+// and 627, of 112,870 with hardly a candidate each 62 and 69.
+inline bool diag_sums_apart_mixed(int N, int E, int row_max)
+{
+    return N > 32 * 1024 && (long long)row_max * N > 16LL * E;
 }
 
 // How a plain step of the merged kernels sums the pairs of a floe: one thread
@@ -259,7 +270,7 @@ void launch_floes_mixed(const Views &V, int cur, int diag, int sic, int walls, i
 
 // The same on the mixed path (n contact-list items eb/stl, bfl: the live-bond
 // flags of both sides).
-int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int long_rows,
+int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int row_max,
                         int shelter, int walls, int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
                         int *done, cudaStream_t st);
 

@@ -108,7 +108,7 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
     if (!shelter && items <= ONE_CLUSTER_FP64) {
         const int blocks = cluster_blocks(items, one_block_fp64(V.N, n, NB));
         auto W = A;
-        if (diag_last && diag_apart(E, blocks)) {
+        if (diag_last && diag_apart(V.N, E, blocks, true)) {
             W.K = K - 1;
             W.diag_last = 0;
         }
@@ -132,7 +132,7 @@ int launch_steps_fp64(const Views &V, ClusterLimit &most, int cur, int K, int di
         const int gp = fp64_grid(work, 128);
         const bool dense = work > 148 * 2 * 128;
         // (nothing to visit: the update computes its drag itself)
-        const bool apart = diag && diag_sums_apart(V.N, E, NB, true);
+        const bool apart = diag && diag_sums_apart_fp64(V.N, E, NB);
         A.drag = !apart && (diag || n > 0) ? drag : nullptr;
         A.nd = A.drag ? V.N : 0;
         if (apart && !shelter) pairs_diag(V, c, E, erow, pfl, L, rec, launch);

@@ -1510,7 +1510,7 @@ void launch_group_sums_mixed(const Views &V, MixedBufs B, cudaStream_t st)
     launch_step(V.pdl != 0, k_group_sums_mixed, (V.N + GRP_FLOES - 1) / GRP_FLOES, SMALL_THREADS, st, V, B, B.fsum);
 }
 
-int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int long_rows,
+int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int diag_last, int base, int n, int E, int NB, int row_max,
                         int shelter, int walls, int ridging, int2 *eb, const int2 *stl, const unsigned *erow, unsigned char *bfl, MixedBufs B, int *out,
                         int *done, cudaStream_t st)
 {
@@ -1527,7 +1527,7 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
     if (!shelter && all <= ONE_CLUSTER_MIXED) {
         const int blocks = cluster_blocks(all, one_block_mixed(V.N, all, NB));
         auto W = A;
-        if (diag_last && diag_apart(E, blocks)) {
+        if (diag_last && diag_apart(V.N, E, blocks, false)) {
             W.K = K - 1;
             W.diag_last = 0;
         }
@@ -1538,7 +1538,7 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
         if (first == K) return kernels;
     }
     const GroupSums how = group_sums(V.N, shelter, (long long)E + NB);
-    const bool seek = long_rows && !shelter;
+    const bool seek = row_max > 0 && !shelter;
     const int groups = (V.N + GRP_FLOES - 1) / GRP_FLOES;
     float4 *fs = B.fdg;   // (a plain step has no diagnostic sums)
     const auto launch = [&](auto kern, int grid, int block, auto... args) {
@@ -1553,7 +1553,7 @@ int launch_steps_mixed(const Views &V, ClusterLimit &most, int cur, int K, int d
         const long long items = (long long)(diag ? E : n) + (ridging ? 0 : NB) + 64 + V.N;
         // (nothing to visit: the update computes its drag itself)
         const bool pairs = diag || n > 0 || NB > 0;
-        const bool apart = diag && diag_sums_apart(V.N, E, NB, false);
+        const bool apart = diag && diag_sums_apart_mixed(V.N, E, row_max);
         A.drag = pairs && !apart ? B.fsum : nullptr;
         A.nd = A.drag ? V.N : 0;
         if (shelter && !diag && n > SHEL_WAVE)

@@ -97,8 +97,27 @@ def test_diagnostic_sums(kind, n, precision, monkeypatch):
     _same(f, precision, monkeypatch)
 
 
-# FP64: by the entries too, 327,680 of them (each floe a candidate of all others)
+# FP64: by the entries too, 327,680 of them beyond 8,192 floes
 @pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
-@pytest.mark.parametrize("n", [809, 810, 811])
-def test_diagnostic_sums_of_many_entries(n, precision, monkeypatch):
-    _same(_free(n, rtree=50000.0, sp=60.0, cohesion=1, bond_lim_rel=0.7, dt=1e-3), precision, monkeypatch)
+@pytest.mark.parametrize("n,rtree", [(8192, 360.0), (8300, 300.0), (8300, 360.0)])
+def test_diagnostic_sums_of_many_entries(n, rtree, precision, monkeypatch):
+    _same(_free(n, rtree=rtree, sp=60.0, cohesion=1, bond_lim_rel=0.7, dt=1e-3), precision, monkeypatch)
+
+
+# one block, FP64: 128 floes keep a diagnostic step of all pairs, 129 do not
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("n", [128, 129])
+def test_diagnostic_steps_on_one_block(n, precision, monkeypatch):
+    _same(_free(n, rtree=50000.0, sp=60.0, dt=1e-3), precision, monkeypatch)
+
+
+# mixed: a large floe whose row is far longer than the others', and none
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("large", [0, 1])
+def test_diagnostic_sums_of_one_long_row(large, precision, monkeypatch):
+    n = 33000
+    f = _free(n, rtree=100.0, sp=60.0, cohesion=1, bond_lim_rel=0.7, dt=1e-3)
+    if large:
+        f.params.nx += 5000.0
+        f.x[17], f.y[17], f.r[17] = f.x.max() + 2040.0, 0.5 * f.y.max(), 2000.0
+    _same(f, precision, monkeypatch)

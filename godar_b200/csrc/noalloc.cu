@@ -3,9 +3,9 @@
 // Some callers cannot call cudaMalloc: a host program whose own memory
 // manager has already reserved the GPU's memory, or a time-critical loop that
 // must not pay cudaMalloc's implicit device synchronisation.  This entry point
-// runs the same neighbour search as the step (cell keys, radix sort, cell
-// ranges, exact radius predicate) but keeps all of its scratch in one
-// file-scope device array of fixed size (about 2.4 MB).
+// answers the step's radius query (the same predicate) by cell keys, a radix
+// sort and cell ranges, with all of its scratch in one file-scope device array
+// of fixed size (about 2.4 MB).
 //
 // When the array exists on a device: CUDA loads a library's device code
 // lazily by default, so the array (with the module's code) is allocated on a

@@ -250,15 +250,13 @@ GD_DEV void warp_count(unsigned long long a, unsigned long long *counters, int k
     if ((threadIdx.x & 31) == 0 && a) atomicAdd(&counters[k], a);
 }
 
-// Screening pass: one lane per owner entry, few registers.  A pair with no
-// contact history in a field without sheltering can only matter if it
-// touches, and d2 > (ri + rj)^2 (1 + 1e-9) is safely beyond contact in FP64;
-// such a lane only clears stale record flags.  Every other pair (and every
-// pair on a diagnostic step) is appended to the work list (one atomic per
-// warp for the slots; the results do not depend on the list's order).
+// The screen's FP64 test.  A pair with no contact history in a field without
+// sheltering can only matter if it touches, and d2 > (ri + rj)^2 (1 + 1e-9) is
+// safely beyond contact in FP64; such a pair only clears a stale record flag.
+// Every other pair goes through the physics.
 // The contact list of the current rows is two arrays: {entry, bound bits}
-// (eb) and {row slot, partner slot} (st) per item (eb null: every owner
-// entry, as on diagnostic steps); the bound test reads only the first.
+// (eb) and {row slot, partner slot} (st) per item; the bound test reads only the
+// first.
 //
 // Conservative advancement.  D_k bounds how far any floe of the batch has
 // moved since the rebuild: D grows each step by the largest step of any
@@ -272,7 +270,7 @@ GD_DEV void warp_count(unsigned long long a, unsigned long long *counters, int k
 // b = -inf marks pairs that are always tested (sheltering or ridging
 // fields, whose radii change).
 // The FP64 test of contact-list item k (entry c.x, bound c.y, slots st;
-// f0 the entry's flags): whether the pair goes on the work list.  A pair
+// f0 the entry's flags): whether the pair goes through the physics.  A pair
 // found apart drops a stale record flag and stores a fresh bound.
 GD_DEV bool screen_test(const Views &V, const Snap *S, int2 *eb, int k, const int2 c, const int2 st, unsigned f0,
                         float Dk, const MixedBufs &B)

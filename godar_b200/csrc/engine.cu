@@ -928,18 +928,20 @@ struct Engine {
 
     // Uploads of a commit, in stream order: ranges of up to a quarter of a
     // megabyte through the two pinned read-back slots (idle here), one filling
-    // while the other is copied, larger ones directly.  Ranges that follow one
-    // another on the device leave as one copy: thousands of small fields have
-    // eight arrays each, and every copy from pinned memory takes 1.4 us longer
-    // than a small one that the driver inlines.
+    // while the other is copied, larger ones directly.  Ranges of one buffer that
+    // follow one another leave as one copy (one copy does not cross buffers, which
+    // may lie side by side in the pool): thousands of small fields have eight
+    // arrays each, and every copy from pinned memory takes 1.4 us longer than a
+    // small one that the driver inlines.
     struct Upload {
         Engine &E;
-        char *dst = nullptr, *src = nullptr;      // the range being gathered
+        const Buf *in = nullptr;                  // the buffer of ...
+        char *dst = nullptr, *src = nullptr;      // ... the range being gathered
         size_t len = 0, at = 0;                   // ... and the slot's end
         int slot = 0;
         bool used[2] = {false, false};
 
-        int put(void *to, const void *from, size_t nbytes) {
+        int put(const Buf &buf, void *to, const void *from, size_t nbytes) {
             cudaStream_t st = E.st;
             if (nbytes > 2 * STAGE_SLOT) {
                 TRY(flush());
@@ -949,7 +951,7 @@ struct Engine {
             const char *f = (const char *)from;
             char *t = (char *)to;
             while (nbytes > 0) {
-                if (len > 0 && t != dst + len) TRY(flush());
+                if (len > 0 && (in != &buf || t != dst + len)) TRY(flush());
                 if (at == STAGE_SLOT) {
                     TRY(flush());
                     CK(cudaEventRecord(E.stage_ev[slot], st));
@@ -958,7 +960,7 @@ struct Engine {
                     if (used[slot]) CK(cudaEventSynchronize(E.stage_ev[slot]));
                     at = 0;
                 }
-                if (len == 0) { dst = t; src = E.h_stage + slot * STAGE_SLOT + at; }
+                if (len == 0) { in = &buf; dst = t; src = E.h_stage + slot * STAGE_SLOT + at; }
                 const size_t n = std::min(nbytes, STAGE_SLOT - at);
                 std::memcpy(src + len, f, n);
                 len += n; at += n; f += n; t += n; nbytes -= n;
@@ -1165,12 +1167,14 @@ struct Engine {
         TRY(alloc_scratch(n_tot));
         const int sn = 0;
         Upload U{*this};
-        auto up = [&](void *dst, const void *src, size_t nbytes) { return U.put(dst, src, nbytes); };
+        const auto up = [&](const Buf &buf, void *dst, const void *src, size_t nbytes) {
+            return U.put(buf, dst, src, nbytes);
+        };
         TRY(params_b.ensure(std::max<size_t>(hp.size(), 1) * sizeof(InstParams), &bytes, &mp));
-        TRY(up(params_b.p, hp.data(), hp.size() * sizeof(InstParams)));
+        TRY(up(params_b, params_b.p, hp.data(), hp.size() * sizeof(InstParams)));
         hparams = hp;
         TRY(field_b.ensure(std::max<size_t>(hfield.size(), 1) * 8, &bytes, &mp));
-        TRY(up(field_b.p, hfield.data(), hfield.size() * 8));
+        TRY(up(field_b, field_b.p, hfield.data(), hfield.size() * 8));
         // the layout's table, every slot's field and origin, and the resident
         // floes, device to device
         TRY(repack_b.ensure((size_t)std::max(N, 1) * 4, &bytes, &mp));
@@ -1181,7 +1185,7 @@ struct Engine {
             tab[3 * ni + k] = old_boff[k];
         }
         TRY(layout_b.ensure(tab.size() * 4, &bytes, &mp));
-        TRY(up(layout_b.p, tab.data(), tab.size() * 4));
+        TRY(up(layout_b, layout_b.p, tab.data(), tab.size() * 4));
         RelayoutTable T;
         T.ni = ni;
         T.off = layout_b.as<int>(); T.old_off = T.off + ni; T.boff = T.off + 2 * ni; T.old_boff = T.off + 3 * ni;
@@ -1193,7 +1197,7 @@ struct Engine {
         // admitted floes, host to device, an array of every field after the other
         const auto upload = [&](Piece &to, std::vector<double> Inst::*from) -> int {
             for (const Inst &I : insts)
-                if (I.pending) TRY(up(to.as<double>() + I.off, (I.*from).data(), (size_t)I.n * 8));
+                if (I.pending) TRY(up(F->mem, to.as<double>() + I.off, (I.*from).data(), (size_t)I.n * 8));
             return GODAR_OK;
         };
         TRY(upload(F->x[sn], &Inst::x)); TRY(upload(F->y[sn], &Inst::y)); TRY(upload(F->th[sn], &Inst::th));
@@ -1202,10 +1206,10 @@ struct Engine {
         for (Inst &I : insts) {
             if (!I.pending || !I.rx) continue;
             const size_t o = (size_t)I.off, nb8 = (size_t)I.n * 8;
-            TRY(up(F->dtb1[sn].as<double>() + o, I.rx->dtb1.data(), nb8));
-            TRY(up(F->dtb2[sn].as<double>() + o, I.rx->dtb2.data(), nb8));
-            TRY(up(F->thb1[sn].as<double>() + o, I.rx->thb1.data(), nb8));
-            TRY(up(F->thb2[sn].as<double>() + o, I.rx->thb2.data(), nb8));
+            TRY(up(F->mem, F->dtb1[sn].as<double>() + o, I.rx->dtb1.data(), nb8));
+            TRY(up(F->mem, F->dtb2[sn].as<double>() + o, I.rx->dtb2.data(), nb8));
+            TRY(up(F->mem, F->thb1[sn].as<double>() + o, I.rx->thb1.data(), nb8));
+            TRY(up(F->mem, F->thb2[sn].as<double>() + o, I.rx->thb2.data(), nb8));
         }
         TRY(U.flush());
         // bonds: the fresh fields' counts from the device, then every
@@ -1225,7 +1229,7 @@ struct Engine {
         TRY(ens(BS->bdyn[0], (size_t)NB * sizeof(BondDyn)));
         if (oldB && oldN > 0) {
             for (int k = 0; k < ni; k++) tab[k] = insts[k].boff;
-            TRY(up(layout_b.as<int>() + 2 * ni, tab.data(), (size_t)ni * 4));
+            TRY(up(layout_b, layout_b.as<int>() + 2 * ni, tab.data(), (size_t)ni * 4));
             TRY(U.flush());
             launch_relayout_bonds(oldB->bond_off.as<int>(), BS->bond_off.as<int>(), inst_b.as<int>(),
                                   oldB->bond_hi.as<int>(), oldB->bstat.as<BondStat>(), oldB->bdyn[0].as<BondDyn>(),
@@ -1241,7 +1245,7 @@ struct Engine {
             return GODAR_OK;
         };
         TRY(each([&](const Inst &I, const HostBonds &B) {
-            return up(BS->bond_hi.as<int>() + I.boff, B.hi.data(), (size_t)I.nb * 4);
+            return up(BS->bond_hi, BS->bond_hi.as<int>() + I.boff, B.hi.data(), (size_t)I.nb * 4);
         }));
         TRY(each([&](const Inst &I, const HostBonds &B) {
             std::vector<BondStat> st_(I.nb);
@@ -1259,7 +1263,7 @@ struct Engine {
                 bs.inv_l = (float)(1.0 / L);
                 st_[q] = bs;
             }
-            return up(BS->bstat.as<BondStat>() + I.boff, st_.data(), (size_t)I.nb * sizeof(BondStat));
+            return up(BS->bstat, BS->bstat.as<BondStat>() + I.boff, st_.data(), (size_t)I.nb * sizeof(BondStat));
         }));
         TRY(each([&](const Inst &I, const HostBonds &B) {
             std::vector<BondDyn> dyn(I.nb);
@@ -1269,14 +1273,14 @@ struct Engine {
                 bd.flag = B.flag[q];
                 dyn[q] = bd;
             }
-            return up(BS->bdyn[sn].as<BondDyn>() + I.boff, dyn.data(), (size_t)I.nb * sizeof(BondDyn));
+            return up(BS->bdyn[sn], BS->bdyn[sn].as<BondDyn>() + I.boff, dyn.data(), (size_t)I.nb * sizeof(BondDyn));
         }));
         TRY(each([&](const Inst &I, const HostBonds &B) {
             std::vector<int> off(I.n);
             for (int i = 0; i < I.n; i++) off[i] = I.boff + (B.off.empty() ? 0 : B.off[i]);
-            return up(BS->bond_off.as<int>() + I.off, off.data(), (size_t)I.n * 4);
+            return up(BS->bond_off, BS->bond_off.as<int>() + I.off, off.data(), (size_t)I.n * 4);
         }));
-        TRY(up(BS->bond_off.as<int>() + N, &NB, sizeof(int)));
+        TRY(up(BS->bond_off, BS->bond_off.as<int>() + N, &NB, sizeof(int)));
         TRY(U.flush());
         CK(cudaStreamSynchronize(st));
         for (auto &I : insts) {

@@ -60,3 +60,33 @@ def test_fields_admitted_together(precision):
             assert b.field(hid, name).tobytes() == one.field(i, name).tobytes(), (sizes[k], name)
         one.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("fields", [1, 2, 3, 4, 8, 15, 16, 24, 32, 48, 64])
+def test_parameters_and_forcing_grids_of_many_fields(fields, precision):
+    # one copy must not cross from one buffer into the next, which for some
+    # numbers of fields begins where the first ends
+    rng = np.random.default_rng(fields)
+    made = []
+    for k in range(fields):
+        p, s, _ = _field(6 + k % 3, k, False)
+        p.field_nx, p.field_ny = 4, 4
+        made.append((p, s, rng.uniform(-1.0, 1.0, 64)))
+
+    def add(b, f):
+        p, s, grid = f
+        return b.add(p, s["x"], s["y"], s["r"], s["h"], s["theta"], s["omega"], s["u"], s["v"], field=grid)
+
+    for _ in range(2):
+        b = Batch(precision)
+        ids = [add(b, f) for f in made]
+        b.step(3)
+        for k in {0, fields // 2, fields - 1}:
+            one = Batch(precision)
+            i = add(one, made[k])
+            one.step(3)
+            for name in STATE:
+                assert b.field(ids[k], name).tobytes() == one.field(i, name).tobytes(), (k, name)
+            one.close()
+        b.close()

@@ -1523,8 +1523,6 @@ struct Engine {
             TRY(frex_b.ensure((size_t)N * 4, &bytes, &mp));
             TRY(fdg_b.ensure((size_t)N * 32, &bytes, &mp));
             launch_pack_snap(V, nxt, st);
-            // (read once the contact list's length is)
-            CK(cudaMemcpyAsync(h_status + 3, nwork_b.as<int>() + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
             TRY(contact_list(nxt, Pn));
             row_max = Pn > 0 ? h_status[3] : 0;
             TRY(mixed_bond_lists(nxt));
@@ -1547,9 +1545,9 @@ struct Engine {
         if (P <= 0) return GODAR_OK;
         int *mark = dist2.as<int>(), *pos = mark + P;
         launch_contact_list(views(), side, P, erow_up.as<unsigned>(), pfl.as<unsigned char>(), mark, pos,
-                            cscan_b.as<int>(), clist_b.as<int2>(), clist_b.as<int2>() + Ecap, st);
-        int &ec = h_status[2];
-        CK(cudaMemcpyAsync(&ec, pos + P, sizeof(int), cudaMemcpyDeviceToHost, st));
+                            cscan_b.as<int>(), clist_b.as<int2>(), clist_b.as<int2>() + Ecap,
+                            nwork_b.as<int>() + 2, h_status + 2, st);
+        const int &ec = h_status[2];
         CK(cudaStreamSynchronize(st));
         Ec = ec;
         return GODAR_OK;

@@ -254,7 +254,8 @@ void launch_bond_work_scatter(const int *perm, int nb, const BondDyn *wdyn, Bond
 void launch_pairs_screen(const Views &V, int cur, int diag, int P, int2 *eb, const int2 *stl,
                          MixedBufs B, int block, int variant, cudaStream_t st);
 void launch_contact_list(const Views &V, int side, int P, const unsigned *erow, const unsigned char *pfl, int *mark,
-                         int *pos, int *scan_scratch, int2 *eb, int2 *stl, cudaStream_t st);
+                         int *pos, int *scan_scratch, int2 *eb, int2 *stl, const int *row_max, int *hs,
+                         cudaStream_t st);
 // Diagnostic steps: the pair physics of every owner entry.
 void launch_pairs_diag(const Views &V, int cur, int P, const unsigned *erow_up, MixedBufs B, int block,
                        cudaStream_t st);

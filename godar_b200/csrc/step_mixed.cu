@@ -1730,10 +1730,16 @@ __global__ void k_contact_mark(Views V, int side, int P, const unsigned *erow, c
 // (the bound of k_pairs_screen with D = 0).  A pair that carries a contact
 // history gets a bound of at most -1, so that the screen always tests it
 // (the screen reads a pair's flags only for the items it tests).
-// side: the rows' side, whose positions are the floes' rebuild origins.
+// side: the rows' side, whose positions are the floes' rebuild origins.  hs
+// (pinned host memory): the list's length and the longest row.
 __global__ void k_contact_fill(Views V, int side, int P, const unsigned *erow, const unsigned char *pfl,
-                               const int *mark, const int *pos, int2 *eb, int2 *stl)
+                               const int *mark, const int *pos, int2 *eb, int2 *stl, const int *row_max,
+                               int *hs)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        hs[0] = pos[P];
+        hs[1] = *row_max;
+    }
     const Snap *S = V.snap[side];
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < P; e += gridDim.x * blockDim.x) {
         if (!mark[e]) continue;
@@ -1755,12 +1761,13 @@ __global__ void k_contact_fill(Views V, int side, int P, const unsigned *erow, c
 }
 
 void launch_contact_list(const Views &V, int side, int P, const unsigned *erow, const unsigned char *pfl, int *mark,
-                         int *pos, int *scan_scratch, int2 *eb, int2 *stl, cudaStream_t st)
+                         int *pos, int *scan_scratch, int2 *eb, int2 *stl, const int *row_max, int *hs,
+                         cudaStream_t st)
 {
     if (P <= 0) return;
     k_contact_mark<<<grid_of(P, 256), 256, 0, st>>>(V, side, P, erow, pfl, mark);
     scan_excl(mark, pos, P, scan_scratch, st);
-    k_contact_fill<<<grid_of(P, 256), 256, 0, st>>>(V, side, P, erow, pfl, mark, pos, eb, stl);
+    k_contact_fill<<<grid_of(P, 256), 256, 0, st>>>(V, side, P, erow, pfl, mark, pos, eb, stl, row_max, hs);
 }
 
 void launch_bond_lists(const Views &V, int side, int nb, int *slot_of, int4 *bsp, int *cnt, int *blo, int *list,
